@@ -65,3 +65,29 @@ def test_select_then_attend(built_lib, oracle):
                                      block_table=case["block_table"], page_block_size=64)
     check_out(out.view(torch.int16).cpu().numpy().view(np.uint16), r_out, **TOL_FP8)
     check_lse(lse.cpu().numpy(), r_lse)
+
+
+@pytest.mark.parametrize("rows,kv_len,topk,stride", [
+    (2, 4095, 7, 4095),          # one CTA per row, rows that are not 16-byte aligned
+    (300, 8192, 2048, 8192),     # many rows: the small CTAs, a full register file
+    (3, 8193, 2048, 8196),       # the first length above it
+    (1, 131072, 2048, 131072),   # eight CTAs per row
+    (300, 20001, 500, 20004),    # many long rows: the large CTAs
+    (2, 300001, 2048, 300004),   # more than eight CTAs hold in registers: the slices are read again
+])
+def test_select_over_the_slices(built_lib, rows, kv_len, topk, stride):
+    """Every way a row is cut over CTAs and registers, with values that fall into one bin of the first pass (more than
+    the candidate list holds), ties over slice borders, and lengths that end inside a slice."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(kv_len)
+    buf = torch.randn(rows, stride, generator=g, device="cuda")
+    scores = buf[:, :kv_len]
+    scores[0] = 1.0 + torch.randint(0, 1000, (kv_len,), generator=g, device="cuda") * 2.0 ** -20   # one 12-bit bin, heavy ties
+    if rows > 1:
+        scores[1] = torch.round(scores[1])
+    valid = torch.randint(topk, kv_len + 1, (rows,), generator=g, device="cuda").to(torch.int32)
+    valid[0] = kv_len
+    got = api.topk_select(scores, topk, valid).cpu().numpy()
+    check = sorted({0, 1 % rows, rows // 2, rows - 1})
+    want = numpy_select(scores[check].cpu().numpy(), topk, valid[check].cpu().numpy())
+    assert np.array_equal(got[check], want)
