@@ -17,7 +17,7 @@ cudaError_t launch_attn(bool fp8, bool ext, int num_lists, const CUtensorMap& tq
                         const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const int32_t* reduce_indptr,
                            const int32_t* reduce_slots, const ReduceDst* reduce_dst, int num_reduce_rows, const OutTargets& tgt,
-                           int64_t stride_o_row, int64_t stride_o_head, int H, cudaStream_t stream);
+                           int64_t stride_o_row, int64_t stride_o_head, int H, int tile_rows, cudaStream_t stream);
 cudaError_t launch_peer_sync(const PeerSync& s, cudaStream_t stream);
 cudaError_t launch_peer_push(int n_peers, int my_rank, const void* src, void* const* dst, int64_t bytes, cudaStream_t stream);
 cudaError_t launch_topk_select(const float* scores, int64_t stride_row, const int32_t* valid_len, int total_q, int kv_len, int topk,
@@ -289,6 +289,13 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }
 
+// Rows of the 128-row tile that can carry a head: H, or the stacked query rows' heads together (a stacking plan has
+// s_q * H <= 128).
+int live_tile_rows(const WorkspaceHeader& h) {
+    const int r = h.has_stacked ? h.s_q * h.H : h.H;
+    return r < kHeadsPerBlock ? r : kHeadsPerBlock;
+}
+
 int launch_merge(const dsa_v32_attn_args* a, cudaStream_t stream, const WorkspaceHeader* known = nullptr,
                  const dsa_v32_peer_outputs* peers = nullptr) {
     WorkspaceHeader h;
@@ -316,7 +323,7 @@ int launch_merge(const dsa_v32_attn_args* a, cudaStream_t stream, const Workspac
                                    reinterpret_cast<const int32_t*>(ws + h.off_reduce_indptr),
                                    reinterpret_cast<const int32_t*>(ws + h.off_reduce_slots),
                                    reinterpret_cast<const ReduceDst*>(ws + h.off_reduce_dst), h.num_reduce_rows, tgt,
-                                   a->stride_o_row, a->stride_o_head, a->H, stream);
+                                   a->stride_o_row, a->stride_o_head, a->H, live_tile_rows(h), stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }
 

@@ -1324,19 +1324,35 @@ done:
 }
 
 // ------------------------------------------------------------------ split merge
-// One warp per (reduce row, head).  Same arithmetic as the reference's two-pass merge
-// (opus_attn/dsa_v32/common/mla_reduce.hpp:92-156): m = max lse_i, w_i = exp2((lse_i - m) log2e)
-// (0 for an empty split), out = sum w_i O_i / sum w_i, lse = m + ln(sum w_i); all empty -> 0, +inf.
-__global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
+// Same arithmetic as the reference's two-pass merge (opus_attn/dsa_v32/common/mla_reduce.hpp:92-156): m = max lse_i,
+// w_i = exp2((lse_i - m) log2e) (0 for an empty split), out = sum w_i O_i / sum w_i, lse = m + ln(sum w_i); all
+// empty -> 0, +inf.
+// The partials were written by the kernel before and come from L2 (16 splits x 128 heads: 4 MB), so the time is a
+// chain of load latencies, not bytes: the plan's tables are read before the wait for the attention kernel, lane i then
+// fetches the lse of split i while the first partial rows (eight float4 per lane) are already on their way.
+// kV = float4 per lane and split: a warp covers 128 kV columns of one tile row, a block four warps.  kV = 1 (a block per
+// row) while all blocks are resident at once, else kV = 4 (a warp per row), which needs a quarter of the blocks.
+// Measured: decode of one sequence (16 splits) 25.3 -> 19.8 us, batch 16 37.1 -> 35.4 us, two sequences of 16 heads on a bf16
+// cache 21.5 -> 15.9 us, against one warp per row that walked the splits one by one (slot, then lse, then four float4).
+// With kV = 1 throughout, a prefill chunk of 64 split rows x 64 heads took 8.9 us for its merge instead of 5.2.
+constexpr int kMergeFlight = 8;                       // float4 in flight per lane
+constexpr int kMergeResidentRows = 148 * 8;           // blocks of 128 threads resident at once (64 registers per thread)
+template <int kV>
+__global__ void __launch_bounds__(128) combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
                                                       const int32_t* __restrict__ reduce_indptr,
                                                       const int32_t* __restrict__ reduce_slots,
                                                       const ReduceDst* __restrict__ reduce_dst, const OutTargets tgt,
                                                       int64_t stride_o_row, int64_t stride_o_head, int H) {
+    constexpr int kF = kMergeFlight / kV;    // splits in flight
     const int rr = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int hrow = blockIdx.y * 8 + warp;  // head inside the 128-head block
-    grid_dependency_wait();   // launched ahead of the attention kernel's end (programmatic stream serialization)
+    const int hrow = kV == 1 ? blockIdx.y : blockIdx.y * 4 + warp;   // row of the 128-row tile
+    const int col = (kV == 1 ? warp * 128 : 0) + lane * 4;
+    // the tables belong to the plan: no kernel writes them
     const ReduceDst dst = reduce_dst[rr];
+    const int s0 = reduce_indptr[rr], ns = reduce_indptr[rr + 1] - s0;
+    int slot = lane < ns ? __ldg(reduce_slots + s0 + lane) : 0;
+    grid_dependency_wait();   // launched ahead of the attention kernel's end (programmatic stream serialization)
     int head = dst.head_block * kHeadsPerBlock + hrow, q_row = dst.q_row;
     if (dst.head_block < 0) {   // stacked unit: -head_block query rows of H heads each
         const int sub = hrow / H;
@@ -1344,43 +1360,65 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
         head = hrow - sub * H;
         q_row += sub;
     }
-    if (head >= H) return;
-    const int s0 = reduce_indptr[rr], ns = reduce_indptr[rr + 1] - s0;
-    float m = -FLT_MAX;
-    for (int i = lane; i < ns; i += 32) m = fmaxf(m, lse_accum[(size_t)reduce_slots[s0 + i] * kHeadsPerBlock + hrow]);
+    if (head >= H || hrow >= kHeadsPerBlock) return;
+    float lse_i = lane < ns ? lse_accum[(size_t)slot * kHeadsPerBlock + hrow] : -FLT_MAX;
+    const float* src = o_accum + (size_t)hrow * kDV + col;
+    float4 x[kF][kV];
+    auto load = [&](int j, int n) {   // splits [j, j + kF) of the chunk's n; j + k <= 31, so the source lane is always in range
+#pragma unroll
+        for (int k = 0; k < kF; ++k) {
+            const int sl = __shfl_sync(0xffffffffu, slot, j + k);
+#pragma unroll
+            for (int v = 0; v < kV; ++v) {
+                x[k][v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (j + k < n) x[k][v] = *reinterpret_cast<const float4*>(src + (size_t)sl * kHeadsPerBlock * kDV + v * 128);
+            }
+        }
+    };
+    load(0, min(32, ns));
+    float m = lse_i;
+    for (int i = lane + 32; i < ns; i += 32) m = fmaxf(m, lse_accum[(size_t)reduce_slots[s0 + i] * kHeadsPerBlock + hrow]);
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    float acc[16];
+    float4 acc[kV];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = 0.0f;
+    for (int v = 0; v < kV; ++v) acc[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float denom = 0.0f;
-    for (int i = 0; i < ns; ++i) {
-        const int slot = reduce_slots[s0 + i];
-        const float li = lse_accum[(size_t)slot * kHeadsPerBlock + hrow];
-        const float wgt = (li > -FLT_MAX) ? exp2f((li - m) * 1.4426950408889634f) : 0.0f;
-        denom += wgt;
-        const float4* src = reinterpret_cast<const float4*>(o_accum + ((size_t)slot * kHeadsPerBlock + hrow) * kDV);
+    for (int c0 = 0; c0 < ns; c0 += 32) {
+        if (c0) {
+            slot = c0 + lane < ns ? __ldg(reduce_slots + s0 + c0 + lane) : 0;
+            lse_i = c0 + lane < ns ? lse_accum[(size_t)slot * kHeadsPerBlock + hrow] : -FLT_MAX;
+        }
+        const float wgt = (lse_i > -FLT_MAX) ? exp2f((lse_i - m) * 1.4426950408889634f) : 0.0f;
+        const int n = min(32, ns - c0);
+        for (int j = 0; j < n; j += kF) {
+            if (c0 + j) load(j, n);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const float4 x = src[v * 32 + lane];
-            acc[4 * v + 0] += wgt * x.x;
-            acc[4 * v + 1] += wgt * x.y;
-            acc[4 * v + 2] += wgt * x.z;
-            acc[4 * v + 3] += wgt * x.w;
+            for (int k = 0; k < kF; ++k) {   // in split order, whatever the number in flight; past the end the weight is 0
+                const float wk = __shfl_sync(0xffffffffu, wgt, j + k);
+                denom += wk;
+#pragma unroll
+                for (int v = 0; v < kV; ++v) {
+                    acc[v].x += wk * x[k][v].x;
+                    acc[v].y += wk * x[k][v].y;
+                    acc[v].z += wk * x[k][v].z;
+                    acc[v].w += wk * x[k][v].w;
+                }
+            }
         }
     }
     const float inv = denom > 0.0f ? 1.0f / denom : 0.0f;
     const float lse_val = denom > 0.0f ? m + log2f(denom) * 0.69314718055994531f : INFINITY;
     for (int d = 0; d < tgt.n_peers; ++d) {   // one destination, or every peer's gathered buffer
-        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(tgt.out[d]) + (size_t)q_row * stride_o_row + (size_t)head * stride_o_head;
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(tgt.out[d]) + (size_t)q_row * stride_o_row + (size_t)head * stride_o_head + col;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
+        for (int v = 0; v < kV; ++v) {
             uint2 u;
-            u.x = pack_bf16x2(acc[4 * v + 0] * inv, acc[4 * v + 1] * inv);
-            u.y = pack_bf16x2(acc[4 * v + 2] * inv, acc[4 * v + 3] * inv);
-            *reinterpret_cast<uint2*>(o + (v * 32 + lane) * 4) = u;
+            u.x = pack_bf16x2(acc[v].x * inv, acc[v].y * inv);
+            u.y = pack_bf16x2(acc[v].z * inv, acc[v].w * inv);
+            *reinterpret_cast<uint2*>(o + v * 128) = u;
         }
-        if (lane == 0 && tgt.lse[d] != nullptr) tgt.lse[d][(size_t)q_row * tgt.lse_stride_row + head] = lse_val;
+        if (col == 0 && tgt.lse[d] != nullptr) tgt.lse[d][(size_t)q_row * tgt.lse_stride_row + head] = lse_val;
     }
 }
 
@@ -1537,19 +1575,20 @@ cudaError_t launch_attn(bool fp8, bool ext, int num_lists, const CUtensorMap& tq
 
 cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const int32_t* reduce_indptr,
                            const int32_t* reduce_slots, const ReduceDst* reduce_dst, int num_reduce_rows, const OutTargets& tgt,
-                           int64_t stride_o_row, int64_t stride_o_head, int H, cudaStream_t stream) {
+                           int64_t stride_o_row, int64_t stride_o_head, int H, int tile_rows, cudaStream_t stream) {
     if (num_reduce_rows <= 0) return cudaSuccess;
-    dim3 grid(num_reduce_rows, kHeadsPerBlock / 8);
+    const bool wide = (int64_t)num_reduce_rows * tile_rows > kMergeResidentRows;
+    dim3 grid(num_reduce_rows, wide ? (tile_rows + 3) / 4 : tile_rows);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.blockDim = dim3(128, 1, 1);
     cfg.stream = stream;
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, combine_kernel, o_accum, lse_accum, reduce_indptr, reduce_slots, reduce_dst, tgt, stride_o_row,
+    return cudaLaunchKernelEx(&cfg, wide ? combine_kernel<4> : combine_kernel<1>, o_accum, lse_accum, reduce_indptr, reduce_slots, reduce_dst, tgt, stride_o_row,
                               stride_o_head, H);
 }
 

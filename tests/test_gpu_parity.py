@@ -52,6 +52,14 @@ def test_decode_bf16_config1(oracle):
     assert plan.info.num_partials > 0   # the list is split across CTA pairs and merged
 
 
+@pytest.mark.parametrize("B,H,topk", [(1, 128, 6000), (1, 40, 4500), (2, 200, 900), (20, 128, 512), (5, 72, 1200)])
+def test_merge_splits(oracle, B, H, topk):
+    """Merge kernel: more than 32 splits of a row, few and many reduce rows (both widths), head counts off the block size."""
+    case = synth.make_decode_case(B, H, 64 * (topk // 64 + 2), topk, seed=topk)
+    _, _, plan = compare(case, oracle, TOL_BF16)
+    assert plan.info.num_partials > 0
+
+
 def test_decode_bf16_padding_anywhere_and_poison(oracle):
     from gpu_util import poison_unselected
     case = synth.make_decode_case(3, 128, 1024, 300, pad_frac=0.3, scatter_pad=True, seed=5)
