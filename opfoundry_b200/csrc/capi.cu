@@ -15,6 +15,7 @@ namespace dsa {
 int max_resident_pairs(bool fp8, int* out);
 cudaError_t launch_attn(bool fp8, bool ext, int num_lists, const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ttail,
                         const AttnParams& p, cudaStream_t stream);
+cudaError_t launch_small_heads(bool fp8, int tile_rows, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const int32_t* reduce_indptr,
                            const int32_t* reduce_slots, const ReduceDst* reduce_dst, int num_reduce_rows, const OutTargets& tgt,
                            int64_t stride_o_row, int64_t stride_o_head, int H, int tile_rows, cudaStream_t stream);
@@ -233,6 +234,13 @@ TmapCache& tmap_cache() {
     return c;
 }
 
+// Rows of the 128-row tile that can carry a head: H, or the stacked query rows' heads together (a stacking plan has
+// s_q * H <= 128).
+int live_tile_rows(const WorkspaceHeader& h) {
+    const int r = h.has_stacked ? h.s_q * h.H : h.H;
+    return r < kHeadsPerBlock ? r : kHeadsPerBlock;
+}
+
 int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t stream, const WorkspaceHeader* known = nullptr,
                      const dsa_v32_peer_outputs* peers = nullptr, const dsa_v32_v4_ext* ext = nullptr) {
     WorkspaceHeader h;
@@ -264,6 +272,17 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     std::memset(&tkv, 0, sizeof(tkv));
     std::memset(&ttail, 0, sizeof(ttail));
     const bool fp8 = want_dtype == DSA_V32_KV_FP8;
+    // Up to 32 tile rows per item: the kernel that puts the slots on the tensor-core tile's rows.
+    // It is the faster one at every size measured (batch 2 to 128, 16 and 32 rows, both caches: 1.0 to 1.6 times); beyond 32 rows
+    // Q, the P copies and three tile stages no longer fit shared memory.
+    if (live_tile_rows(h) <= kSmallHeads) {
+        const uint64_t qdims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
+        const uint64_t qstr[2] = {uint64_t(a->stride_q_head) * 2, uint64_t(a->stride_q_row) * 2};
+        const uint32_t qbox[3] = {64, uint32_t(a->H), 1};
+        if (tmap_cache().get(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->q, qdims, qstr, qbox, CU_TENSOR_MAP_SWIZZLE_128B)) return DSA_V32_ERR_DRIVER;
+        cudaError_t e = launch_small_heads(fp8, live_tile_rows(h), h.num_lists, tq, p, stream);
+        return e == cudaSuccess ? DSA_V32_OK : (int)e;
+    }
     if (fp8) {
         {   // Q: the 64 rope columns of a head block, 128-byte swizzle (the latent columns go to TMEM by plain loads)
             const uint64_t dims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
@@ -287,13 +306,6 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     const bool use_ext = h.has_stacked != 0 || p.attn_sink != nullptr || p.kv2 != nullptr || p.n_peers > 0;
     cudaError_t e = launch_attn(fp8, use_ext, h.num_lists, tq, tkv, ttail, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
-}
-
-// Rows of the 128-row tile that can carry a head: H, or the stacked query rows' heads together (a stacking plan has
-// s_q * H <= 128).
-int live_tile_rows(const WorkspaceHeader& h) {
-    const int r = h.has_stacked ? h.s_q * h.H : h.H;
-    return r < kHeadsPerBlock ? r : kHeadsPerBlock;
 }
 
 int launch_merge(const dsa_v32_attn_args* a, cudaStream_t stream, const WorkspaceHeader* known = nullptr,

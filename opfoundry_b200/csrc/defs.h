@@ -11,6 +11,7 @@ constexpr int kDRope = DSA_V32_D_ROPE;  // 64
 constexpr int kHeadsPerBlock = 128;     // MMA M: one head per TMEM lane
 constexpr int kDvHalf = 256;            // output columns accumulated by one CTA of a pair
 constexpr int kTileRows = 32;           // top-k slots per pipeline step
+constexpr int kSmallHeads = 32;         // most tile rows an item may have for the few-heads kernel
 constexpr int kFp8RowBytes = DSA_V32_FP8_ROW_BYTES;
 
 constexpr uint32_t kWorkspaceMagic = 0x44534133u;  // "DSA3"

@@ -116,6 +116,13 @@ __device__ __forceinline__ void ldg_nc_256(const void* p, uint32_t (&r)[8]) {
                  : "l"(p));
 }
 
+// 16-byte read-only global load that does not allocate in L1 (a gathered row is read once per SM).
+__device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // 32-byte global store (sm_100).
 __device__ __forceinline__ void stg_256(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f, uint32_t g, uint32_t h) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h)
@@ -235,6 +242,11 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* m, 
         :
         : "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
         : "memory");
+}
+
+// Asks for `bytes` bytes (a multiple of 16, 16-byte aligned) to be brought into L2.
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // 4-byte asynchronous copy global -> shared (src_bytes = 0 writes zeros without reading), and an
@@ -371,6 +383,20 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t saddr, uint32_
     return d;
 }
 
+// MN-major operand whose rows hold N = 16 or 32 bf16 (one K index per row): 32- or 64-byte swizzle (mode 6 or 4), groups of
+// eight rows follow one another.  There is a single MN block, so the leading offset is not used.
+template <int N>
+__device__ __forceinline__ uint64_t make_smem_desc_mn_narrow(uint32_t saddr, uint32_t lbo_bytes) {
+    static_assert(N == 16 || N == 32, "32- or 64-byte rows");
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
+    d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
+    d |= static_cast<uint64_t>((8 * 2 * N) >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(N == 16 ? 6 : 4) << 61;
+    return d;
+}
+
 // Instruction descriptor for kind::f16 with bf16 A and B, fp32 accumulate.
 //   bits 4-5 D format (1 = f32), 7-9 A format (1 = bf16), 10-12 B format (1 = bf16),
 //   bit 15 A major (0 = K), bit 16 B major (0 = K, 1 = MN), bits 17-22 N >> 3, bits 24-28 M >> 4.
@@ -378,6 +404,7 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool b_mn_m
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) |
            (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
 }
+constexpr uint32_t kIdescATransposed = 1u << 15;   // A is MN-major
 
 // D[tmem] (+)= A[smem] * B[smem]; issued by one thread.  accumulate == 0 overwrites D.
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,

@@ -1,0 +1,49 @@
+// Device helpers that both attention kernels use: index translation and the exact e4m3 -> bf16 conversion.
+#pragma once
+#include "defs.h"
+#include "ptx.cuh"
+
+namespace dsa {
+
+// ------------------------------------------------------------------ index translation
+// Top-k slot value -> physical cache row, or -1 when the slot is padding / unusable.  Split in two so
+// the loader warps can issue the block-table load of one tile and finish the arithmetic tiles later:
+//   block_of(idx)        issues the block-table load (0 when there is nothing to load)
+//   row_of(idx, phys)    the physical row from the loaded block number
+__device__ __forceinline__ int block_of(int idx, int seq, const AttnParams& p) {
+    if (idx < 0 || p.block_table == nullptr) return 0;
+    const int blk = p.page_shift >= 0 ? (idx >> p.page_shift) : idx / p.page_block_size;
+    if (blk >= p.block_table_stride) return -1;
+    return __ldg(p.block_table + (size_t)seq * p.block_table_stride + blk);
+}
+__device__ __forceinline__ int row_of(int idx, int phys, int seq, const AttnParams& p) {
+    if (idx < 0) return -1;
+    long long row;
+    if (p.block_table != nullptr) {
+        if (phys < 0) return -1;
+        const int in_page = p.page_shift >= 0 ? (idx & (p.page_block_size - 1)) : idx % p.page_block_size;
+        row = (long long)phys * p.page_block_size + in_page;
+    } else {
+        row = (long long)seq * p.kv_batch_stride_rows + idx;
+    }
+    if (row < 0 || row >= p.num_kv_rows) return -1;
+    return (int)row;
+}
+__device__ __forceinline__ int translate_row(int idx, int seq, const AttnParams& p) {
+    return row_of(idx, block_of(idx, seq, p), seq, p);
+}
+
+// ------------------------------------------------------------------ e4m3 -> bf16, exact, two at a time
+// Input: the two e4m3 bytes in the high byte of each 16-bit half.  Moving the 7 magnitude bits down
+// by 4 puts the 4 exponent bits and 3 mantissa bits where bf16 keeps them; read as bf16 that number
+// is the e4m3 value times 2^-120 (normal and subnormal codes alike), so one exact multiply by 2^120
+// finishes the conversion without going through the conversion unit.  (0x7F, the e4m3 NaN, becomes
+// 480 instead of NaN; a cache row that is never selected is never converted.)
+__device__ __forceinline__ uint32_t e4m3x2_to_bf16x2(uint32_t hi_bytes) {
+    const uint32_t y = (hi_bytes & 0x80008000u) | ((hi_bytes >> 4) & 0x07F007F0u);
+    uint32_t z;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(z) : "r"(y), "r"(0x7B807B80u));
+    return z;
+}
+
+}  // namespace dsa
