@@ -124,7 +124,8 @@ def _check(status, where):
 
 
 def _stream():
-    # the raw handle: building a Stream object for it cost 3 us of every call
+    # the raw handle: building a Stream object for it cost a few microseconds of every call (two sequences of 16 heads, where
+    # the host is the bound: 14.7 -> 12.5 us with the argument block below)
     return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 

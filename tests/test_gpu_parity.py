@@ -225,6 +225,24 @@ def test_pack_fp8_rows_bit_exact(oracle):
     assert np.array_equal(got.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("n,mag", [(1, 1.0), (2049, 1.0), (7, 1e-20), (9, 1e-26), (5, 1e-38), (9, 1e20), (5, 1e28), (6, 1e36)])
+def test_pack_fp8_rows_divisions(oracle, n, mag):
+    """The quotients of the packer round like a division: many rows, signed zeros and values far below the row's
+    largest one, rows on both sides of the range in which the quotient is formed from the reciprocal.  (Rows whose largest
+    value is below 448 * 2^-150 = 3e-43 have a scale of 0 and infinite quotients, which the packer saturates and the codec does not.)"""
+    rng = np.random.default_rng(n)
+    latent = (rng.standard_normal((n, 512)) * np.exp2(rng.integers(-30, 1, (n, 512)) * (rng.random((n, 512)) < 0.3)) * mag).astype(np.float32)
+    latent[:, ::37] = np.float32(-0.0)
+    latent[-1, 128:256] = np.float32(-0.0)
+    rope = synth.normal_bf16(n, "kv2", (n, 64))
+    want = oracle.pack_fp8_rows(latent, rope)
+    dst = torch.from_numpy(rng.permutation(n)).cuda()
+    got = torch.zeros(n, 656, dtype=torch.uint8, device="cuda")
+    api.pack_fp8_rows(torch.from_numpy(latent).cuda(), torch.from_numpy(rope.view(np.int16)).cuda().view(torch.bfloat16), out=got, dst_rows=dst)
+    assert np.array_equal(got[dst].cpu().numpy(), want)
+
+
+
 def test_repeated_launches_are_deterministic(oracle):
     from gpu_util import run_gpu
     case = synth.make_decode_case(8, 128, 2048, 512, fp8=True, paged=True, seed=50)
