@@ -476,8 +476,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             const int n_tiles = (wi.k_end - wi.k_begin + kTileRows - 1) / kTileRows;
             const uint32_t it_end = it_base + n_tiles;
             // Q of item n goes into TMEM once the score MMAs of item n - 1 have all read theirs: for the
-            // list's first item here, for every later item during the epilogue of the item before it (so
-            // the next item's scores start while this item's output is still being written).
+            // list's first item here; for every later item during the epilogue of the item before it (fp8 cache; the next
+            // item's scores start while this item's output is still being written), or by the loader warps (bf16 cache).
             auto q_store = [&](const dsa_v32_work_info& wq, int n) -> bool {
                 q_fetch(wq);
                 if (!tile_wait<kFp8>(smem_u32(&ctl->q_empty), (n & 1) ^ 1, abort_flag)) return false;
@@ -828,7 +828,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 // finished early cannot know of another team's barrier.)
                 // the next work item is read before the barrier: its Q is fetched right after the row sums below, and
                 // the addresses of those loads should not wait for this one
-                const dsa_v32_work_info wnext = p.works[w + 1 < w_end ? w + 1 : w];
+                const dsa_v32_work_info wnext = p.works[kFp8 && w + 1 < w_end ? w + 1 : w];
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&ctl->e_bar));
                 if (!tile_wait<kFp8>(smem_u32(&ctl->e_bar), item_n & 1, abort_flag)) goto done;
@@ -854,7 +854,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         if (kRowSplit) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->l_bar), peer));
                     }
                 }
-                if (w + 1 < w_end)
+                if (kFp8 && w + 1 < w_end)   // (bf16 cache: the loaders have stored it already)
                     if (!q_store(wnext, item_n + 1)) goto done;
                 if (!warp_wait_cluster(smem_u32(&ctl->l_bar), item_n & 1, abort_flag)) goto done;
                 float l = 0.0f;
@@ -1065,7 +1065,43 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             uint8_t* mask_bytes = reinterpret_cast<uint8_t*>(ctl->tile_mask);
             const uint8_t* kv_bytes = reinterpret_cast<const uint8_t*>(p.kv);
             uint32_t it_base = 0;
-            for (int w = w_begin; w < w_end; ++w) {
+            // Q of every item but the list's first goes into TMEM from here: the score MMAs of the item before have read theirs
+            // a whole softmax chain (5 300 cycles) before that item's last P V product, so the loaders can store the next Q, and
+            // the next item's first scores be there, while the softmax warps still work on the last tiles and the output.
+            // From the epilogue, as the fp8 kernel has it, the fetch and the store were on the way to the next scores.  Items of
+            // 640 slots with sink and second pool (1024 queries): 307 -> 292 us; items of 2048 slots are as fast either way
+            // (2265 us, under the power cap).  Storing after the group's first tile instead of before it, with the test for it in the
+            // tile loop, cost 5 % there.
+            // Thread = head row of the TMEM lane quadrant; a group of loader warps stores half of the slice's columns.
+            auto store_q = [&](const dsa_v32_work_info& wq, int n) -> bool {
+                const int quad = warp & 3;
+                const RowMap rm = map_row<kExt>(wq, quad * 32 + lane, p.H);
+                const char* base = reinterpret_cast<const char*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)rm.q_row * p.stride_q_row +
+                                                                 (size_t)rm.head * p.stride_q_head);
+                const uint32_t qcol = tmem + (static_cast<uint32_t>(quad * 32) << 16) + kColQ;
+                if (!tile_wait<kFp8>(smem_u32(&ctl->q_empty), (n & 1) ^ 1, abort_flag)) return false;
+                tc_fence_after();
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {   // 32 bf16 = 16 TMEM columns a round
+                    uint32_t a[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, b[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+                    if (rm.live) {
+                        ldg_nc_256(base + col0 * 2 + grp * 256 + j * 64, a);
+                        ldg_nc_256(base + col0 * 2 + grp * 256 + j * 64 + 32, b);
+                    }
+                    tmem_st_n<8>(qcol + grp * 64 + j * 16, a);
+                    tmem_st_n<8>(qcol + grp * 64 + j * 16 + 8, b);
+                }
+                uint32_t a[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+                if (rm.live) ldg_nc_256(base + (kDV + rope0) * 2 + grp * 32, a);
+                tmem_st_n<8>(qcol + 128 + grp * 8, a);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(smem_u32(&ctl->q_full), kSoftmaxWarps / kLoaderWarps);   // for two of the sixteen softmax warps
+                return true;
+            };
+            int item_n = 0;
+            for (int w = w_begin; w < w_end; ++w, ++item_n) {
                 const dsa_v32_work_info wi = p.works[w];
                 const int seq = wi.q_row / p.s_q;
                 const int n_tiles = (wi.k_end - wi.k_begin + kTileRows - 1) / kTileRows;
@@ -1082,6 +1118,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 int idx_a = load_slot(kb0), idx_b = load_slot(kb0 + 2 * kTileRows);
                 int idx_c = load_slot(kb0 + 4 * kTileRows), idx_d = load_slot(kb0 + 6 * kTileRows);
                 int phys_a = block_of(idx_a, seq, p), phys_b = block_of(idx_b, seq, p);
+                if (item_n > 0)
+                    if (!store_q(wi, item_n)) goto done;
                 for (int u = u0; u < n_tiles; u += 2) {
                     const uint32_t it = it_base + u;
                     const int k0 = wi.k_begin + u * kTileRows;
