@@ -57,10 +57,14 @@ constexpr int kXBytes = 2 * 128 * 16 * 4;          // 16 384: the peer's sums of
 constexpr int kLoadWarp0 = 8;
 constexpr int kLoadWarps = kSlots / 4;             // 12: four rows of every tile each, eight lanes per row
 constexpr int kWarps = kLoadWarp0 + kLoadWarps;    // 20: five warpgroups
-// Registers per thread after the role split (setmaxnreg), of the launch's 640 x 96 = 61 440: 128 x 128 + 512 x 88 for 16 heads,
-// 128 x 152 + 512 x 80 for 32.
-template <int kN> constexpr int kRegsSoftmax = kN == 16 ? 128 : 152;
-template <int kN> constexpr int kRegsOther = kN == 16 ? 88 : 80;
+// Registers per thread after the role split (setmaxnreg): softmax warpgroup + issuers' + three of loaders <= 480, five times the
+// launch's 96.  16 heads, fp8: the loaders hold the next row and the one being converted (64 sequences 53 -> 51 us against loading
+// it after the conversion); 32 heads, fp8: the scores need the room (128 sequences of 2 x 16 heads 206 us that way, 186 without);
+// bf16: the rows never pass through registers.
+template <bool kFp8, int kN> constexpr bool kTwoRows = kFp8 && kN == 16;
+template <bool kFp8, int kN> constexpr int kRegsLoaders = !kFp8 ? 72 : (kN == 16 ? 104 : 80);
+template <bool kFp8, int kN> constexpr int kRegsSoftmax = kTwoRows<kFp8, kN> ? 112 : 152;
+constexpr int kRegsIssuers = 56;
 constexpr int kCtlBytes = 5120;
 
 // kN: tile rows (heads) an item may have = N of both MMAs, 16 or 32
@@ -210,7 +214,8 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
 
     if (warp < 4) {
         // ============================================================ softmax + epilogue
-        setmaxnreg_inc<kRegsSoftmax<kN>>();
+        setmaxnreg_inc<kRegsSoftmax<kFp8, kN>>();
+        static_assert(kRegsSoftmax<kFp8, kN> + kRegsIssuers + 3 * kRegsLoaders<kFp8, kN> <= 5 * 96, "more registers than the launch has");
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(warp * 32) << 16);
         const bool live_lane = lane < 16 && warp < kSlots / 16;   // this thread has a slot
         const int slot = 16 * warp + (lane & 15);
@@ -555,8 +560,8 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                 }
             }
         }
-    } else {
-        setmaxnreg_dec<kRegsOther<kN>>();
+    } else if (warp < kLoadWarp0) {
+        setmaxnreg_dec<kRegsIssuers>();
         if (warp == 4) {
             // ======================================================== Q and score issuer
             const uint32_t el = elect_one() ? 1u : 0u;
@@ -632,7 +637,11 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     if (t + 1 == pt.n_tiles) tc_commit_el(smem_u32(&ctl->o_full), el);
                 }
             }
-        } else if (warp >= kLoadWarp0) {
+        }
+    } else {
+        if constexpr (kTwoRows<kFp8, kN>) setmaxnreg_inc<kRegsLoaders<kFp8, kN>>();
+        else setmaxnreg_dec<kRegsLoaders<kFp8, kN>>();
+        {
             // ======================================================== row loaders: four rows of every tile per warp, eight lanes per row
             const int r = 4 * (warp - kLoadWarp0) + (lane >> 3);   // tile row
             const int oc = lane & 7;                               // 16-byte chunks oc, oc + 8, ... of the row
@@ -688,46 +697,49 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     phys3 = phys4;
                 };
                 if (kFp8) {
-                    uint4 raw[4], rope;
-                    float sc;   // lanes oc < 4: scale oc of the row
-                    bool ok;
-                    auto load_row = [&](int row) {
-                        ok = row >= 0;
+                    struct Row {
+                        uint4 raw[4], rope;
+                        float sc;   // lanes oc < 4: scale oc of the row
+                        bool ok;
+                    };
+                    auto load_row = [&](int row) -> Row {
+                        Row x;
+                        x.ok = row >= 0;
                         const uint8_t* src = address(row);
-                        sc = 0.0f;
-                        if (ok) {
+                        x.sc = 0.0f;
+                        if (x.ok) {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) raw[k] = ldg_stream_16(src + (oc + 8 * k) * 16);
-                            rope = ldg_stream_16(src + kDV + 16 + oc * 16);
-                            if (oc < 4) sc = __ldg(reinterpret_cast<const float*>(src + kDV) + oc);
+                            for (int k = 0; k < 4; ++k) x.raw[k] = ldg_stream_16(src + (oc + 8 * k) * 16);
+                            x.rope = ldg_stream_16(src + kDV + 16 + oc * 16);
+                            if (oc < 4) x.sc = __ldg(reinterpret_cast<const float*>(src + kDV) + oc);
                         } else {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) raw[k] = make_uint4(0u, 0u, 0u, 0u);
-                            rope = make_uint4(0u, 0u, 0u, 0u);
+                            for (int k = 0; k < 4; ++k) x.raw[k] = make_uint4(0u, 0u, 0u, 0u);
+                            x.rope = make_uint4(0u, 0u, 0u, 0u);
                         }
+                        return x;
                     };
-                    load_row(row0);
+                    Row next = load_row(row0);
                     for (int t = 0; t < pt.n_tiles; ++t, ring.next()) {
+                        const Row cur = next;
+                        advance(t);
+                        if (kTwoRows<kFp8, kN>) next = load_row(row0);   // a whole tile ahead
                         // e4m3 -> bf16 before the wait for a stage: a stage is the scarce resource
                         uint32_t o[32];
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            const uint32_t wv[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
+                            const uint32_t wv[4] = {cur.raw[k].x, cur.raw[k].y, cur.raw[k].z, cur.raw[k].w};
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
                                 o[8 * k + 2 * q + 0] = e4m3x2_to_bf16x2(__byte_perm(wv[q], 0u, 0x1404u));
                                 o[8 * k + 2 * q + 1] = e4m3x2_to_bf16x2(__byte_perm(wv[q], 0u, 0x3424u));
                             }
                         }
-                        const uint4 rope_t = rope;
-                        const float sc_t = sc;
-                        const bool ok_t = ok;
-                        advance(t);
-                        load_row(row0);   // the next tile's row is on its way during the wait
+                        if (!kTwoRows<kFp8, kN>) next = load_row(row0);
                         if (!wait_on(&ctl->kv_empty[ring.s], ring.ph ^ 1u, abort_flag)) goto done;
                         uint8_t* tile = sKV + ring.s * kTileBytes + r * 128;
-                        if (oc < 4) reinterpret_cast<float*>(&ctl->row_scale[ring.s][r])[oc] = sc_t;
-                        if (oc == 0) ctl->ok[ring.s][r] = ok_t;
+                        if (oc < 4) reinterpret_cast<float*>(&ctl->row_scale[ring.s][r])[oc] = cur.sc;
+                        if (oc == 0) ctl->ok[ring.s][r] = cur.ok;
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             const int j = oc + 8 * k;   // raw chunk -> 64-column block j / 4, its 16-byte chunks 2 c and 2 c + 1
@@ -740,7 +752,7 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                             *reinterpret_cast<uint4*>(dst_row + (((2 * c + h0) ^ (r & 7)) * 16)) = h0 ? hi : lo;
                             *reinterpret_cast<uint4*>(dst_row + (((2 * c + (h0 ^ 1)) ^ (r & 7)) * 16)) = h0 ? lo : hi;
                         }
-                        *reinterpret_cast<uint4*>(tile + 8 * kKvBlock + ((oc ^ (r & 7)) * 16)) = rope_t;
+                        *reinterpret_cast<uint4*>(tile + 8 * kKvBlock + ((oc ^ (r & 7)) * 16)) = cur.rope;
                         fence_proxy_async_smem();
                         warp_arrive(&ctl->kv_full[ring.s], lane);
                     }
