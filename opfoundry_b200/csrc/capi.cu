@@ -161,6 +161,7 @@ void fill_params(const dsa_v32_attn_args* a, const WorkspaceHeader& h, AttnParam
     p->block_table_stride = a->block_table_stride;
     set_page(p, a->page_block_size);
     p->scale_log2 = a->sm_scale * 1.4426950408889634f;
+    p->wide = 0;
     p->n_peers = 0;
     p->lse_stride_row = a->H;
     for (int i = 0; i < DSA_V32_MAX_PEERS; ++i) {
@@ -303,7 +304,12 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         if (tmap_cache().get(&ttail, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, a->kv, dims, str, box_b, CU_TENSOR_MAP_SWIZZLE_NONE))
             return DSA_V32_ERR_DRIVER;
     }
-    const bool use_ext = h.has_stacked != 0 || p.attn_sink != nullptr || p.kv2 != nullptr || p.n_peers > 0;
+    // 32-byte loads of q and stores of out want rows on 32-byte boundaries; what the checks above admit is 16
+    uintptr_t low = reinterpret_cast<uintptr_t>(a->q) | reinterpret_cast<uintptr_t>(a->out) |
+                    uintptr_t(2 * (a->stride_q_head | a->stride_q_row | a->stride_o_head | a->stride_o_row));
+    for (int i = 0; i < p.n_peers; ++i) low |= reinterpret_cast<uintptr_t>(p.out_peers[i]);
+    p.wide = (low & 31u) == 0;
+    const bool use_ext = !p.wide || h.has_stacked != 0 || p.attn_sink != nullptr || p.kv2 != nullptr || p.n_peers > 0;
     cudaError_t e = launch_attn(fp8, use_ext, h.num_lists, tq, tkv, ttail, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }

@@ -132,6 +132,26 @@ __device__ __forceinline__ void stg_256(void* p, uint32_t a, uint32_t b, uint32_
                  : "memory");
 }
 
+// The same for addresses that may be aligned to 16 bytes only; kMaybe = false: the caller knows that they are not.
+template <bool kMaybe> __device__ __forceinline__ void ldg_nc_32(const void* p, uint32_t (&r)[8], bool wide) {
+    if (!kMaybe || wide) {
+        ldg_nc_256(p, r);
+    } else {
+        const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+        r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+        r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+    }
+}
+template <bool kMaybe>
+__device__ __forceinline__ void stg_32(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f, uint32_t g, uint32_t h, bool wide) {
+    if (!kMaybe || wide) {
+        stg_256(p, a, b, c, d, e, f, g, h);
+    } else {
+        reinterpret_cast<uint4*>(p)[0] = make_uint4(a, b, c, d);
+        reinterpret_cast<uint4*>(p)[1] = make_uint4(e, f, g, h);
+    }
+}
+
 // ------------------------------------------------------------------ thread-block cluster
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;

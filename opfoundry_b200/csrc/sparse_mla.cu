@@ -281,7 +281,8 @@ __device__ __forceinline__ bool tile_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // ------------------------------------------------------------------ the kernel
-// kExt: the instantiation that also handles stacked query rows, the attention sink and the second KV pool;
+// kExt: the instantiation that also handles stacked query rows, the attention sink, the second KV pool and rows of q and out
+// that start on 16-byte boundaries (views with such offsets or strides);
 // the plain one keeps those branches out of the loaders and the epilogue.
 template <bool kFp8, bool kExt>
 __global__ void __launch_bounds__(Cfg<kFp8>::kThreads, 1)
@@ -448,7 +449,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint32_t v[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-                if (live) ldg_nc_256(reinterpret_cast<const char*>(src) + 32 * j, v);
+                if (live) ldg_nc_32<kExt>(reinterpret_cast<const char*>(src) + 32 * j, v, p.wide);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) qreg[8 * j + k] = v[k];
             }
@@ -889,8 +890,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll 1
                             for (int d = 0; d < n_dst; ++d) {
                                 __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.n_peers > 0 ? p.out_peers[d] : p.out);
-                                stg_256(base + o_off + oc, u[0].x, u[0].y, u[0].z, u[0].w, u[1].x, u[1].y, u[1].z, u[1].w);
-                                stg_256(base + o_off + oc + 16, u[2].x, u[2].y, u[2].z, u[2].w, u[3].x, u[3].y, u[3].z, u[3].w);
+                                stg_32<kExt>(base + o_off + oc, u[0].x, u[0].y, u[0].z, u[0].w, u[1].x, u[1].y, u[1].z, u[1].w, p.wide);
+                                stg_32<kExt>(base + o_off + oc + 16, u[2].x, u[2].y, u[2].z, u[2].w, u[3].x, u[3].y, u[3].z, u[3].w, p.wide);
                             }
                         }
                     }
@@ -916,8 +917,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                             uint32_t u[16];
 #pragma unroll
                             for (int v = 0; v < 16; ++v) u[v] = pack_bf16x2(__uint_as_float(o[2 * v]) * inv, __uint_as_float(o[2 * v + 1]) * inv);
-                            stg_256(o_dst + oc, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7]);
-                            stg_256(o_dst + oc + 16, u[8], u[9], u[10], u[11], u[12], u[13], u[14], u[15]);
+                            stg_32<kExt>(o_dst + oc, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], p.wide);
+                            stg_32<kExt>(o_dst + oc + 16, u[8], u[9], u[10], u[11], u[12], u[13], u[14], u[15], p.wide);
                         }
                     }
                     if (live && (kRowSplit ? own : half == 0) && cg == 0 && p.lse != nullptr) p.lse[(size_t)rm.q_row * p.H + head] = lse_nat;
@@ -1085,14 +1086,14 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 for (int j = 0; j < 4; ++j) {   // 32 bf16 = 16 TMEM columns a round
                     uint32_t a[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, b[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
                     if (rm.live) {
-                        ldg_nc_256(base + col0 * 2 + grp * 256 + j * 64, a);
-                        ldg_nc_256(base + col0 * 2 + grp * 256 + j * 64 + 32, b);
+                        ldg_nc_32<kExt>(base + col0 * 2 + grp * 256 + j * 64, a, p.wide);
+                        ldg_nc_32<kExt>(base + col0 * 2 + grp * 256 + j * 64 + 32, b, p.wide);
                     }
                     tmem_st_n<8>(qcol + grp * 64 + j * 16, a);
                     tmem_st_n<8>(qcol + grp * 64 + j * 16 + 8, b);
                 }
                 uint32_t a[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-                if (rm.live) ldg_nc_256(base + (kDV + rope0) * 2 + grp * 32, a);
+                if (rm.live) ldg_nc_32<kExt>(base + (kDV + rope0) * 2 + grp * 32, a, p.wide);
                 tmem_st_n<8>(qcol + 128 + grp * 8, a);
                 tmem_wait_st();
                 tc_fence_before();
@@ -1585,7 +1586,7 @@ static cudaError_t launch_attn_t(int num_lists, const CUtensorMap& tq, const CUt
     return cudaLaunchKernelEx(&cfg, sparse_mla_kernel<kFp8, kExt>, tq, tkv, ttail, p);
 }
 
-// ext: the plan holds stacked items, or a sink / second pool is given
+// ext: the plan holds stacked items, a sink, second pool or peers are given, or rows of q / out are aligned to 16 bytes only
 cudaError_t launch_attn(bool fp8, bool ext, int num_lists, const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ttail,
                         const AttnParams& p, cudaStream_t stream) {
     if (fp8) return ext ? launch_attn_t<true, true>(num_lists, tq, tkv, ttail, p, stream) : launch_attn_t<true, false>(num_lists, tq, tkv, ttail, p, stream);

@@ -243,6 +243,26 @@ def test_pack_fp8_rows_divisions(oracle, n, mag):
 
 
 
+@pytest.mark.parametrize("fp8,H,topk", [(False, 128, 300), (True, 128, 300), (False, 16, 300), (True, 16, 300), (False, 128, 1500)])
+def test_rows_on_16_byte_boundaries(oracle, fp8, H, topk):
+    """q and out as views whose rows start on 16- but not on 32-byte boundaries (offset and strides of 8 elements)."""
+    from gpu_util import run_oracle, to_dev
+    case = synth.make_decode_case(90, H, 2048, topk, fp8=fp8, paged=fp8, seed=topk + H) if topk < 1000 else synth.make_decode_case(2, H, 2048, topk, seed=1)
+    d = to_dev(case)
+    n = d["q"].shape[0]
+    q = torch.zeros(n * H * 584 + 8, dtype=torch.bfloat16, device="cuda")[8:].view(n, H, 584)[:, :, :576]
+    q.copy_(d["q"])
+    out = torch.full((n * H * 520 + 8,), float("nan"), dtype=torch.bfloat16, device="cuda")[8:].view(n, H, 520)[:, :, :512]
+    lse = torch.empty(n, H, device="cuda")
+    plan = api.mla_decode_plan_create(n, H, topk)
+    api.mla_decode_launch_pipeline(q, d["kv"], d["indices"], plan, SCALE, block_table=d["block_table"], page_block_size=case["page_block_size"],
+                                   kv_batch_stride_rows=case["kv_batch_stride_rows"], out=out, lse=lse)
+    rows = list(range(0, n, 9))
+    r_out, r_lse = run_oracle(oracle, case, SCALE, subset=rows)
+    check_out(out.contiguous().view(torch.int16).cpu().numpy().view(np.uint16)[rows], r_out[rows], **(TOL_FP8 if fp8 else TOL_BF16))
+    check_lse(lse.cpu().numpy()[rows], r_lse[rows])
+
+
 def test_repeated_launches_are_deterministic(oracle):
     from gpu_util import run_gpu
     case = synth.make_decode_case(8, 128, 2048, 512, fp8=True, paged=True, seed=50)
