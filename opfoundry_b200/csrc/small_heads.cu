@@ -16,9 +16,9 @@
 // Warp roles (20 warps):
 //   warps 0-3   softmax: thread = slot (the M = 64 accumulator puts its rows on lanes 0-15 of every TMEM lane
 //              quadrant), holding the scores of its slot, 16 heads at a time.  A head's reference maximum is only moved
-//              when a score exceeds it by more than the lazy margin of 8 - one vote of the four warps per tile, whose result
-//              is awaited under the exponentials; the row sums stay per slot in fp32 registers and cross the lanes once per
-//              item.  P goes to shared memory (fp8 cache: one copy per 128-column scale group, pre-multiplied by that
+//              when a score exceeds it by more than the lazy margin of 8 - one vote of the four warps per tile (taking the
+//              exponentials while it is under way gained nothing); the row sums stay per slot in fp32 registers and cross
+//              the lanes once per item.  P goes to shared memory (fp8 cache: one copy per 128-column scale group, pre-multiplied by that
 //              group's row scale).  Epilogue: merge, normalise, store.
 //   warp 4      score issuer; it also fetches the item's Q (TMA).     warp 5  P V issuer.     warps 6, 7 idle.
 //   warps 8-19  row loaders, four rows of every tile each.  bf16 cache: 16-byte cp.async copies straight into the
@@ -31,7 +31,7 @@
 // 48 slots; the tensor pipe is busy for 2 000 of them (a score MMA of M = 64, N = 16 takes 33 cycles, a P V MMA 62).
 // Measured against the kernel of sparse_mla.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 226 -> 186 us, 64
 // sequences of 16 heads 79 -> 53, 128 of 32 heads 151 -> 130; bf16, 64 sequences of 16 heads 52 -> 39, prefill of 2048 tokens with
-// 16 heads 661 -> 414, two sequences of 16 heads 15.9 -> 14.7 (the last with the merge).  out against 64 bits: 2.08e-3 (2.10e-3
+// 16 heads 661 -> 409, two sequences of 16 heads 15.9 -> 14.7 (the last with the merge).  out against 64 bits: 2.08e-3 (2.10e-3
 // there), lse 2e-7 (7e-7: no 16-bit exchange of partial scores).
 //
 // Every mbarrier wait is bounded, as in sparse_mla.cu, and the warps of the softmax group meet on mbarriers only, so a
@@ -222,18 +222,12 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
         uint32_t team_n = 0, xn = 0, it = 0, rb = 0;   // rb: which of ctl->ref holds the current references
         Ring ring;
         const uint64_t c2 = pack2(p.scale_log2, p.scale_log2);
-        // 16 heads: the exponentials are taken while the vote is under way (and again if it moves a reference); with 32 heads that
-        // needs 32 more registers, and the spills cost more than the wait (223 against 190 us on 128 sequences of 2 x 16 heads)
-        constexpr bool kEarly = kN == 16;
         // the four softmax warps meet: what they wrote to shared memory before is visible after
-        auto meet_wait = [&]() -> bool {
+        auto meet = [&]() -> bool {
+            warp_arrive(&ctl->team, lane);
             const bool ok = wait_on(&ctl->team, team_n & 1u, abort_flag);
             ++team_n;
             return ok;
-        };
-        auto meet = [&]() -> bool {
-            warp_arrive(&ctl->team, lane);
-            return meet_wait();
         };
         int item_n = 0;
         for (int w = w_begin; w < w_end; ++w, ++item_n) {
@@ -297,36 +291,11 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                         }
                     }
                 }
-                // ---- P = 2^(score - reference), at most 2^8; a masked slot gives 0
-                uint64_t early[kEarly ? kN / 2 : 1];
-                uint64_t* pr = kEarly ? early : v2;
-                auto exponentials = [&]() {
-#pragma unroll
-                    for (int hh = 0; hh < C::kHalves; ++hh) {
-                        if (hh && n_halves < 2) break;
-                        const float4* rf = reinterpret_cast<const float4*>(&ctl->ref[rb][16 * hh]);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float4 r4 = rf[j];
-                            const float rr[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-                            for (int k = 0; k < 2; ++k) {
-                                const int i = 8 * hh + 2 * j + k;
-                                const float r0 = rr[2 * k] == -INFINITY ? 0.0f : rr[2 * k], r1 = rr[2 * k + 1] == -INFINITY ? 0.0f : rr[2 * k + 1];
-                                float y0, y1;
-                                unpack2(fma2(v2[i], c2, pack2(-r0, -r1)), y0, y1);
-                                pr[i] = pack2(ok_slot ? ex2_approx(y0) : 0.0f, ok_slot ? ex2_approx(y1) : 0.0f);
-                            }
-                        }
-                    }
-                };
                 bool move = t == 0;   // the first tile sets the references
                 if (t > 0) {
                     over = __any_sync(0xffffffffu, over && ok_slot);
                     if (lane == 0) ctl->vote[sb][warp] = over;
-                    warp_arrive(&ctl->team, lane);
-                    if (kEarly) exponentials();   // with the references as they are: right unless the vote moves one
-                    if (!meet_wait()) goto done;
+                    if (!meet()) goto done;
                     const uint4 vt = *reinterpret_cast<const uint4*>(ctl->vote[sb]);
                     move = (vt.x | vt.y | vt.z | vt.w) != 0u;
                 }
@@ -380,14 +349,27 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                         tmem_wait_st();
                     }
                 }
-                if (move || !kEarly) exponentials();
+                // ---- P = 2^(score - reference), at most 2^8; a masked slot gives 0
 #pragma unroll
-                for (int j = 0; j < kN / 2; ++j) {
-                    if (j >= 8 && n_halves < 2) break;
-                    float p0, p1;
-                    unpack2(pr[j], p0, p1);
-                    l[2 * j] += p0;
-                    l[2 * j + 1] += p1;
+                for (int hh = 0; hh < C::kHalves; ++hh) {
+                    if (hh && n_halves < 2) break;
+                    const float4* rf = reinterpret_cast<const float4*>(&ctl->ref[rb][16 * hh]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 r4 = rf[j];
+                        const float rr[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int i = 8 * hh + 2 * j + k;
+                            const float r0 = rr[2 * k] == -INFINITY ? 0.0f : rr[2 * k], r1 = rr[2 * k + 1] == -INFINITY ? 0.0f : rr[2 * k + 1];
+                            float y0, y1;
+                            unpack2(fma2(v2[i], c2, pack2(-r0, -r1)), y0, y1);
+                            const float p0 = ok_slot ? ex2_approx(y0) : 0.0f, p1 = ok_slot ? ex2_approx(y1) : 0.0f;
+                            l[2 * i] += p0;
+                            l[2 * i + 1] += p1;
+                            v2[i] = pack2(p0, p1);
+                        }
+                    }
                 }
                 if (it > 0)   // the product that read the P buffer last is complete
                     if (!wait_on(&ctl->pv_done, (it - 1) & 1u, abort_flag)) goto done;
@@ -405,7 +387,7 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                             uint32_t u[8];
                             const uint64_t sg = pack2(scv[g], scv[g]);
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) u[j] = pack_bf16x2_from2(kFp8 ? mul2(pr[8 * hh + j], sg) : pr[8 * hh + j]);
+                            for (int j = 0; j < 8; ++j) u[j] = pack_bf16x2_from2(kFp8 ? mul2(v2[8 * hh + j], sg) : v2[8 * hh + j]);
                             *reinterpret_cast<uint4*>(sP + g * C::kPCopy + (lin ^ x)) = make_uint4(u[0], u[1], u[2], u[3]);
                             *reinterpret_cast<uint4*>(sP + g * C::kPCopy + ((lin + 16u) ^ x)) = make_uint4(u[4], u[5], u[6], u[7]);
                         }
@@ -668,10 +650,12 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     return row >= -1 ? kv_bytes + (size_t)(row < 0 ? 0 : row) * row_bytes
                                      : reinterpret_cast<const uint8_t*>(p.kv2) + (size_t)(-2 - row) * row_bytes;
                 };
-                // Three tiles ahead of its use a row is asked into L2; its block number is loaded a step before that and its slot
-                // two steps before, so no load is consumed in the step that issues it.
+                // A row's block number is loaded a step before its address is needed and its slot two steps before, so no load is
+                // consumed in the step that issues it.  fp8 cache: three tiles ahead of its use the row is asked into L2 (without it
+                // 205 instead of 189 us on 128 sequences of 2 x 16 heads); the bf16 copies of two tiles are in flight anyway, and
+                // asking made them slower (prefill of 2048 tokens with 16 heads 406 -> 414 us).
                 auto ask = [&](int row) {
-                    if (oc == 0 && row != -1) bulk_prefetch_l2(address(row), row_bytes);
+                    if (kFp8 && oc == 0 && row != -1) bulk_prefetch_l2(address(row), row_bytes);
                 };
                 int row0, row1, row2, idx3 = load_slot(3), idx4 = load_slot(4), phys3;
                 {
