@@ -37,7 +37,7 @@
 //              maximum exceeds it by more than the lazy margin (the reference's threshold of 8:
 //              ..16mx4_64nx1_template.hpp:700-725); P = 2^(s - reference) -> bf16 -> tcgen05.st.
 //              Epilogue: O / l -> bf16 (to out, or to every peer GPU's gathered buffer when the all-gather
-//              is fused), or the fp32 partial + lse of a split item; during its waits the next item's Q
+//              is fused), or the fp32 partial + lse of a split item; fp8 cache: during its waits the next item's Q
 //              slice is stored into TMEM (A operand of the score MMAs).
 //   warp 16    score MMA issuer: S_c = Q_c K_c^T (tcgen05.mma M=128, N=32, K=16, A = the Q slice in TMEM,
 //              accumulator in TMEM; fp8 cache: the 64 rope columns of Q stay in shared memory)
@@ -45,6 +45,7 @@
 //              MN-major).  Two issuers so that neither stream waits behind the other's barriers.
 //   bf16 cache: warp 18 second score issuer (alternate tiles), warp 19 asks the next item's Q into L2 near the end of
 //              an item; warps 20-27 loaders, two groups of four on alternate tiles, 8 rows of the tile per warp:
+//              the next item's Q slice into TMEM as soon as the score MMAs have read the old one, then
 //              top-k slots -> block table -> the row's bytes of this CTA's slice as 16-byte cp.async copies
 //              straight into the 128-byte swizzled MMA tile (a TMA tile::gather4 moves one 128-byte block
 //              of four rows per request, 40 requests per tile, and the issue rate of those requests was
