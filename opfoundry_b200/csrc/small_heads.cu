@@ -1,5 +1,5 @@
 // Sparse MLA attention for few heads: work items of at most 32 tile rows (16 or 32 heads of a head-sharded
-// deployment, or the stacked rows of an MTP pair).
+// deployment, or the stacked rows of an MTP pair) that hold enough slots on average (few_heads_form in plan.h).
 //
 // The kernel in sparse_mla.cu puts the heads on the 128 rows of the tensor-core tile, so an item of 16 heads pays
 // for 128: a tile of 32 slots takes the same 1 800-2 600 cycles whatever H is, while the rows it gathers would take

@@ -17,6 +17,11 @@ def load_golden(name):
     return dict(np.load(os.path.join(GOLDEN, name)))
 
 
+def few_heads_form(blob):
+    """Which kernel a plan's items run on: 16 or 32 tile rows of the few-heads kernel, 0 = the 128-row kernel (the header's last field)."""
+    return int(np.frombuffer(blob, np.int32, 1, 112)[0])
+
+
 def csr_to_lists(kv_indptr, kv_indices, B, s_q, topk=None):
     """The reference selects rows per batch through a CSR page table and trims token t of an s_q
     group causally (host.cc:482,526).  Returns the equivalent per-query lists with -1 padding."""

@@ -1,12 +1,13 @@
-"""Items of at most 32 tile rows run on a kernel of their own (slots on the rows of the tensor-core tile, the pair splits
-the slots): edges of its 48-slot tiles and of its 16- and 32-row forms, moving references, sink and second pool."""
+"""Items of at most 32 tile rows, most of which run on a kernel of their own (slots on the rows of the tensor-core tile, the pair
+splits the slots; items that are short on average stay on the 128-row kernel): edges of its 48-slot tiles and of its 16- and
+32-row forms, moving references, sink and second pool."""
 import math
 
 import numpy as np
 import pytest
 
-from helpers import TOL_BF16, TOL_FP8, check_lse, check_out
-from opfoundry_b200 import synth
+from helpers import TOL_BF16, TOL_FP8, check_lse, check_out, few_heads_form
+from opfoundry_b200 import api, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +67,35 @@ def test_sink_and_second_pool(built_lib, oracle, H):
     r_out, r_lse = oracle.sparse_mla_v4(case["q"], case["kv"], idx, SCALE, attn_sink=sink, kv2=kv2, pool_split=split, s_q=120)
     check_out(out.view(torch.int16).cpu().numpy().view(np.uint16), r_out, **TOL_BF16)
     check_lse(lse.cpu().numpy(), r_lse)
+
+
+EDGES = [1, 2, 3, 31, 47, 48, 49, 94, 95, 96, 97, 98, 143, 144, 145, 192, 193, 0]   # a CTA takes half of the slots, 48 a tile
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H", [1, 16, 17, 32])
+def test_tile_edges_among_long_items(built_lib, oracle, H, fp8):
+    """Items at the edges of the 48-slot tiles, in one list with items long enough for the few-heads kernel."""
+    from gpu_util import run_gpu, run_oracle
+    lens = np.array([x for n in EDGES for x in (n, 1100)] + [1100] * (0 if H <= 16 else 42), np.int32)
+    case = synth.make_decode_case(len(lens), H, 1216, 1100, fp8=fp8, paged=fp8, seed=H)
+    for r, n in enumerate(lens):
+        case["indices"][r, n:] = -1
+    kw = dict(num_sms=14, valid_len_hint=lens)
+    assert few_heads_form(api.plan_host(len(lens), H, 1100, **kw)) == (16 if H <= 16 else 32)
+    g_out, g_lse, _ = run_gpu(case, SCALE, **kw)
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    check_out(g_out, r_out, **(TOL_FP8 if fp8 else TOL_BF16))
+    check_lse(g_lse, r_lse)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,topk", [(16, 96), (16, 128), (32, 128), (32, 500)])
+def test_short_items_stay_on_the_128_row_kernel(built_lib, H, topk, fp8):
+    """There a head's result does not depend on the other heads, so it has the bits that it has among 64 heads."""
+    from gpu_util import run_gpu
+    case = synth.make_decode_case(40, 64, 1024, topk, fp8=fp8, paged=fp8, seed=topk)
+    few = dict(case, q=np.ascontiguousarray(case["q"][:, :H]))
+    w_out, w_lse, _ = run_gpu(case, SCALE)
+    g_out, g_lse, _ = run_gpu(few, SCALE)
+    assert np.array_equal(g_out, w_out[:, :H]) and np.array_equal(g_lse, w_lse[:, :H])
