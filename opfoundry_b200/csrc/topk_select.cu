@@ -16,6 +16,7 @@
 // for the list, written), and the chain of block- and cluster-wide steps when there are few.  Measured against one CTA of
 // 512 threads per row that reads the row in each of five passes and scans every 512 positions: 64 rows of 32768 84.0 ->
 // 14.4 us, 2048 rows of up to 8192 247.6 -> 53.3 us (0.6 and 1.4 TB/s of scores and lists).
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "defs.h"
@@ -35,7 +36,7 @@ __device__ __forceinline__ uint32_t order_key(float x) {
     return x != x ? 1u : k;
 }
 
-struct SelShared {
+struct alignas(16) SelShared {
     int hist[kSelBins];     // first pass
     int hist2[2][1024];     // the two others
     int coarse[3][64];
@@ -45,6 +46,7 @@ struct SelShared {
     int total[2];           // this CTA's sums of the two
     int found[3];           // bin, how many more to take in it, how many it holds
 };
+static_assert(alignof(SelShared) == 16 && offsetof(SelShared, hist) % 16 == 0 && offsetof(SelShared, hist2) % 16 == 0, "cleared 16 bytes at a time");
 
 __device__ __forceinline__ void count_in(int* bin) {
     asm volatile("red.shared::cta.add.u32 [%0], 1;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(bin))) : "memory");
