@@ -89,6 +89,7 @@ template <int kThreads, int kPer, bool kCluster, bool kReload>
 __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3) : 1) topk_select_kernel(const float* __restrict__ scores, int64_t stride_row,
                                                                 const int32_t* __restrict__ valid_len, int kv_len, int topk,
                                                                 int n_cta, int vec_ok, int32_t* __restrict__ indices_out) {
+    static_assert(kCluster || !kReload, "a row longer than the registers of one CTA is cut over a cluster first");
     static_assert(kPer % 4 == 0 && kThreads * kPer / 128 <= 1024, "counts table");
     constexpr int kChunk = kThreads * kPer;          // positions per round of the register file
     constexpr int kWarps = kThreads / 32;
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             eq_base += p->total[1];
         }
     };
-    if (kCluster && kReload) {          // the slices' sums take a reading of their own
+    if (kReload) {                      // the slices' sums take a reading of their own
         int g = 0, e = 0;
         for (int c = 0; c < n_chunks; ++c) {
             load_chunk(c);
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
 template <int kThreads, int kPer, bool kReload>
 static cudaError_t launch_sel(const float* scores, int64_t stride_row, const int32_t* valid_len, int total_q, int kv_len, int topk,
                               int n_cta, int vec_ok, int32_t* indices_out, cudaStream_t stream) {
-    if (n_cta == 1) {
+    if constexpr (!kReload) if (n_cta == 1) {   // (slices that are read again are those of eight CTAs)
         topk_select_kernel<kThreads, kPer, false, kReload><<<total_q, kThreads, 0, stream>>>(scores, stride_row, valid_len, kv_len, topk, 1, vec_ok, indices_out);
         return cudaGetLastError();
     }
