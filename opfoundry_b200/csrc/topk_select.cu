@@ -56,8 +56,8 @@ __device__ __forceinline__ const SelShared* sel_peer(const SelShared* s, uint32_
     asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(s)), "r"(rank));
     return reinterpret_cast<const SelShared*>(out);
 }
-template <bool kCluster> __device__ __forceinline__ void sel_sync() {
-    if (kCluster) {
+template <bool kShared> __device__ __forceinline__ void sel_sync() {
+    if (kShared) {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
@@ -84,40 +84,31 @@ __device__ __forceinline__ void sel_find_bin(int v0, int v1, int need, int& bin,
     holds = __shfl_sync(0xffffffffu, hi ? v1 : v0, src);
 }
 
+// The k largest of the first n positions of a row (0 < k < n), by one CTA or (kShared) by all n_cta of a cluster, a slice each.
 // kThreads x kPer positions per CTA are kept in registers; kReload: slices of any length, read again in every pass.
-template <int kThreads, int kPer, bool kCluster, bool kReload>
-__global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3) : 1) topk_select_kernel(const float* __restrict__ scores, int64_t stride_row,
-                                                                const int32_t* __restrict__ valid_len, int kv_len, int topk,
-                                                                int n_cta, int vec_ok, int32_t* __restrict__ indices_out) {
-    static_assert(kCluster || !kReload, "a row longer than the registers of one CTA is cut over a cluster first");
+template <int kThreads, int kPer, bool kShared, bool kReload>
+__device__ __forceinline__ void select_row(SelShared& sh, const float* __restrict__ row, int32_t* __restrict__ out, int n, int k, int rank, int n_cta, int vec_ok) {
+    static_assert(kShared || !kReload, "a row longer than the registers of one CTA is cut over a cluster first");
     static_assert(kPer % 4 == 0 && kThreads * kPer / 128 <= 1024, "counts table");
     constexpr int kChunk = kThreads * kPer;          // positions per round of the register file
     constexpr int kWarps = kThreads / 32;
     constexpr int kRounds = kPer / 4;                // four consecutive positions per thread and round
-    __shared__ SelShared sh;
+    constexpr int kRound = 4 * kThreads;             // positions of a round
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rank = kCluster ? (int)(blockIdx.x % n_cta) : 0;
-    const int q = kCluster ? (int)(blockIdx.x / n_cta) : (int)blockIdx.x;
-    const float* row = scores + (size_t)q * stride_row;
-    int32_t* out = indices_out + (size_t)q * topk;
-    int n = valid_len ? valid_len[q] : kv_len;
-    n = n < 0 ? 0 : (n > kv_len ? kv_len : n);
-    const int k = topk < n ? topk : n;
-    if (k == n) {   // everything valid is selected (all CTAs of the cluster take this exit)
-        for (int i = rank * kThreads + tid; i < topk; i += n_cta * kThreads) out[i] = i < n ? i : -1;
-        return;
-    }
     const int per_cta = ((n + n_cta - 1) / n_cta + 3) & ~3;
     const int begin = min(rank * per_cta, n), end = min(begin + per_cta, n);
     const int n_chunks = kReload ? (per_cta + kChunk - 1) / kChunk : 1;
+    // Rounds that hold a position: the work follows the row's own length, not the width that the form is made for.
+    constexpr bool kGuard = !kReload;
+    const int live = kGuard ? min(kRounds, (max(0, end - begin) + kRound - 1) / kRound) : kRounds;
 
     uint32_t key[kPer];
     auto load_chunk = [&](int c) {
         const int base = begin + c * kChunk + 4 * tid;
-        if (vec_ok && base + (kRounds - 1) * 4 * kThreads + 4 <= end) {   // all of the thread's positions are there
+        if (vec_ok && base + (kRounds - 1) * kRound + 4 <= end) {   // all of the thread's positions are there
 #pragma unroll
             for (int r = 0; r < kRounds; ++r) {
-                const float4 v = __ldg(reinterpret_cast<const float4*>(row + base + r * 4 * kThreads));
+                const float4 v = __ldg(reinterpret_cast<const float4*>(row + base + r * kRound));
                 key[4 * r + 0] = order_key(v.x);
                 key[4 * r + 1] = order_key(v.y);
                 key[4 * r + 2] = order_key(v.z);
@@ -126,14 +117,14 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
         } else {
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
-                const int p = base + (j >> 2) * 4 * kThreads + (j & 3);
+                const int p = base + (j >> 2) * kRound + (j & 3);
                 key[j] = p < end ? order_key(__ldg(row + p)) : 0u;
             }
         }
     };
     if (!kReload) load_chunk(0);
-    for (int i = 4 * tid; i < kSelBins; i += 4 * kThreads) *reinterpret_cast<int4*>(sh.hist + i) = make_int4(0, 0, 0, 0);
-    for (int i = 4 * tid; i < 2048; i += 4 * kThreads) *reinterpret_cast<int4*>(&sh.hist2[0][0] + i) = make_int4(0, 0, 0, 0);
+    for (int i = 4 * tid; i < kSelBins; i += kRound) *reinterpret_cast<int4*>(sh.hist + i) = make_int4(0, 0, 0, 0);
+    for (int i = 4 * tid; i < 2048; i += kRound) *reinterpret_cast<int4*>(&sh.hist2[0][0] + i) = make_int4(0, 0, 0, 0);
     if (tid == 0) sh.list_n = 0;
     __syncthreads();
 
@@ -152,7 +143,10 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             for (int c = 0; c < n_chunks; ++c) {
                 if (kReload) load_chunk(c);
 #pragma unroll
-                for (int j = 0; j < kPer; ++j) count_in(&hist[key[j] >> 20]);
+                for (int r = 0; r < kRounds; ++r)
+                    if (r < live)
+#pragma unroll
+                        for (int j = 4 * r; j < 4 * r + 4; ++j) count_in(&hist[key[j] >> 20]);
             }
         } else if (sh.list_n <= kSelList) {
             for (int i = tid; i < sh.list_n; i += kThreads) {
@@ -169,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             }
         }
         __syncthreads();
-        if (pass == 0 && tid == 0) hist[0] -= n_chunks * kChunk - (end - begin);   // "no position" keys do not count
+        if (pass == 0 && tid == 0) hist[0] -= (kGuard ? live * kRound : n_chunks * kChunk) - (end - begin);   // "no position" keys do not count
         if (pass == 0) __syncthreads();
         for (int b = warp; b < 64; b += kWarps) {
             int s = 0;
@@ -177,11 +171,11 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             s = __reduce_add_sync(0xffffffffu, s);
             if (lane == 0) sh.coarse[pass][b] = s;
         }
-        sel_sync<kCluster>();
+        sel_sync<kShared>();
         if (warp == 0) {
             int v0 = 0, v1 = 0, cb, fb, left, holds;
             for (int r = 0; r < n_cta; ++r) {
-                const SelShared* p = kCluster ? sel_peer(&sh, r) : &sh;
+                const SelShared* p = kShared ? sel_peer(&sh, r) : &sh;
                 v0 += p->coarse[pass][2 * lane];
                 v1 += p->coarse[pass][2 * lane + 1];
             }
@@ -189,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             v0 = v1 = 0;
             if (2 * lane < per_coarse)
                 for (int r = 0; r < n_cta; ++r) {
-                    const SelShared* p = kCluster ? sel_peer(&sh, r) : &sh;
+                    const SelShared* p = kShared ? sel_peer(&sh, r) : &sh;
                     const int* h = (pass == 0 ? p->hist : p->hist2[pass == 0 ? 0 : pass - 1]) + cb * per_coarse;
                     v0 += h[2 * lane];
                     v1 += h[2 * lane + 1];
@@ -210,11 +204,14 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             for (int c = 0; c < n_chunks; ++c) {
                 if (kReload) load_chunk(c);
 #pragma unroll
-                for (int j = 0; j < kPer; ++j)
-                    if ((key[j] ^ prefix) < (1u << 20) && key[j] != 0u) {
-                        const int at = atomicAdd(&sh.list_n, 1);
-                        if (at < kSelList) sh.list[at] = key[j];
-                    }
+                for (int r = 0; r < kRounds; ++r)
+                    if (r < live)
+#pragma unroll
+                        for (int j = 4 * r; j < 4 * r + 4; ++j)
+                            if ((key[j] ^ prefix) < (1u << 20) && key[j] != 0u) {
+                                const int at = atomicAdd(&sh.list_n, 1);
+                                if (at < kSelList) sh.list[at] = key[j];
+                            }
             }
             __syncthreads();
         }
@@ -225,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
     const uint32_t floor_key = tie ? prefix + 1u : prefix;
     int gt_base = 0, eq_base = 0;       // positions of the row before this CTA's slice (and before the chunk)
     auto add_slices_before = [&]() {    // a CTA's first output slot depends on the CTAs before it
-        sel_sync<kCluster>();
+        sel_sync<kShared>();
         for (int r = 0; r < rank; ++r) {
             const SelShared* p = sel_peer(&sh, r);
             gt_base += p->total[0];
@@ -258,6 +255,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
         uint32_t before_g[(kRounds + 3) / 4], before_e[(kRounds + 3) / 4];   // of the lanes before this one
 #pragma unroll
         for (int w = 0; w < (kRounds + 3) / 4; ++w) {
+            if (4 * w >= live) break;
             uint32_t g = 0, e = 0;
 #pragma unroll
             for (int j = 0; j < 16 && 16 * w + j < kPer; ++j) {
@@ -289,7 +287,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             int v[kEach], g = 0, e = 0;
 #pragma unroll
             for (int i = 0; i < kEach; ++i) {
-                v[i] = lane * kEach + i < kN ? sh.counts[lane * kEach + i] : 0;
+                v[i] = lane * kEach + i < live * kWarps ? sh.counts[lane * kEach + i] : 0;
                 g += v[i] & 0xFFFF;
                 e += v[i] >> 16;
             }
@@ -315,23 +313,24 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
                 sums[1] = ei;
             }
         }
-        if (kCluster && !kReload) add_slices_before();
+        if (kShared && !kReload) add_slices_before();
         else __syncthreads();
         const int base = begin + c * kChunk + 4 * tid;
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
+            if (r >= live) break;
             const uint32_t before = (uint32_t)sh.counts[r * kWarps + warp];
             int g = gt_base + (int)(before & 0xFFFFu) + (int)((before_g[r >> 2] >> (8 * (r & 3))) & 255u);
             if (!tie) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (key[4 * r + j] >= floor_key) out[g++] = base + r * 4 * kThreads + j;
+                    if (key[4 * r + j] >= floor_key) out[g++] = base + r * kRound + j;
             } else {
                 int e = eq_base + (int)(before >> 16) + (int)((before_e[r >> 2] >> (8 * (r & 3))) & 255u);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const bool eq = key[4 * r + j] == prefix, gt = key[4 * r + j] > prefix;
-                    if (gt || (eq && e < need)) out[g + min(e, need)] = base + r * 4 * kThreads + j;
+                    if (gt || (eq && e < need)) out[g + min(e, need)] = base + r * kRound + j;
                     g += gt;
                     e += eq;
                 }
@@ -343,29 +342,62 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3)
             __syncthreads();
         }
     }
-    for (int i = k + rank * kThreads + tid; i < topk; i += n_cta * kThreads) out[i] = -1;
-    if (kCluster) sel_sync<kCluster>();   // no CTA leaves while another may still read its tables
+    if (kShared) sel_sync<kShared>();   // no CTA leaves while another may still read its tables
 }
 
-template <int kThreads, int kPer, bool kReload>
+// Not inlined: the registers of the cluster's own path are not shared with it.
+template <int kThreads, int kPer>
+__device__ __noinline__ void select_row_alone(SelShared* sh, const float* row, int32_t* out, int n, int k, int vec_ok) {
+    select_row<kThreads, kPer, false, false>(*sh, row, out, n, k, 0, 1, vec_ok);
+}
+
+// One CTA or one cluster per row.  The lengths are on the device and the form is chosen by the buffer's width, so a row that fits the
+// registers of one CTA is left to the first of its cluster, and one whose valid positions are all selected needs no selection.
+// Rows of 2100-3000 in a buffer of 131072: 160 rows 23 us (74 when the whole cluster worked on the width; one CTA of 512 threads that
+// scanned the row five times 31), 300 rows 40 (146; 33).  CTAs and clusters that stay and deal the rows out among themselves
+// took 20 us for the latter, but 5 to 12 % more for full rows and up to 65 % for mixed ones, whose order they fix beforehand.
+template <int kThreads, int kPer, bool kCluster, bool kReload>
+__global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3) : 1) topk_select_kernel(const float* __restrict__ scores, int64_t stride_row,
+                                                                const int32_t* __restrict__ valid_len, int kv_len, int topk,
+                                                                int n_cta, int vec_ok, int32_t* __restrict__ indices_out) {
+    __shared__ SelShared sh;
+    const int rank = kCluster ? (int)(blockIdx.x % n_cta) : 0;
+    const int q = kCluster ? (int)(blockIdx.x / n_cta) : (int)blockIdx.x;
+    const float* row = scores + (size_t)q * stride_row;
+    int32_t* out = indices_out + (size_t)q * topk;
+    int n = valid_len ? valid_len[q] : kv_len;
+    n = n < 0 ? 0 : (n > kv_len ? kv_len : n);
+    if (n <= topk) {   // everything valid is selected
+        for (int i = rank * kThreads + threadIdx.x; i < topk; i += n_cta * kThreads) out[i] = i < n ? i : -1;
+        return;
+    }
+    if (!kCluster || n <= kThreads * kPer) {
+        if (rank == 0) {
+            if constexpr (kCluster) select_row_alone<kThreads, kPer>(&sh, row, out, n, topk, vec_ok);
+            else select_row<kThreads, kPer, false, false>(sh, row, out, n, topk, 0, 1, vec_ok);
+        }
+        return;
+    }
+    if constexpr (kCluster) select_row<kThreads, kPer, true, kReload>(sh, row, out, n, topk, rank, n_cta, vec_ok);
+}
+
+template <int kThreads, int kPer, bool kCluster, bool kReload>
 static cudaError_t launch_sel(const float* scores, int64_t stride_row, const int32_t* valid_len, int total_q, int kv_len, int topk,
                               int n_cta, int vec_ok, int32_t* indices_out, cudaStream_t stream) {
-    if constexpr (!kReload) if (n_cta == 1) {   // (slices that are read again are those of eight CTAs)
-        topk_select_kernel<kThreads, kPer, false, kReload><<<total_q, kThreads, 0, stream>>>(scores, stride_row, valid_len, kv_len, topk, 1, vec_ok, indices_out);
-        return cudaGetLastError();
-    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3((unsigned)total_q * n_cta, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.stream = stream;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = n_cta;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, topk_select_kernel<kThreads, kPer, true, kReload>, scores, stride_row, valid_len, kv_len, topk, n_cta, vec_ok, indices_out);
+    if (kCluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = n_cta;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, topk_select_kernel<kThreads, kPer, kCluster, kReload>, scores, stride_row, valid_len, kv_len, topk, n_cta, vec_ok, indices_out);
 }
 
 cudaError_t launch_topk_select(const float* scores, int64_t stride_row, const int32_t* valid_len, int total_q, int kv_len, int topk,
@@ -380,9 +412,10 @@ cudaError_t launch_topk_select(const float* scores, int64_t stride_row, const in
     const int per_cta = ((kv_len + n_cta - 1) / n_cta + 3) & ~3;
     // Slices of up to 8192 positions: 16 keys per thread, three CTAs on an SM (2048 rows of 8192: 49.6 us; 32 keys in 256
     // threads 51.6, 8 in 1024 threads 61.7).
-    if (per_cta <= 8192) return launch_sel<512, 16, false>(scores, stride_row, valid_len, total_q, kv_len, topk, n_cta, vec_ok, indices_out, stream);
-    if (per_cta <= 32768) return launch_sel<1024, 32, false>(scores, stride_row, valid_len, total_q, kv_len, topk, n_cta, vec_ok, indices_out, stream);
-    return launch_sel<1024, 32, true>(scores, stride_row, valid_len, total_q, kv_len, topk, n_cta, vec_ok, indices_out, stream);
+    auto launch = [&](auto form) { return form(scores, stride_row, valid_len, total_q, kv_len, topk, n_cta, vec_ok, indices_out, stream); };
+    if (per_cta <= 8192) return launch(n_cta > 1 ? launch_sel<512, 16, true, false> : launch_sel<512, 16, false, false>);
+    if (per_cta <= 32768) return launch(n_cta > 1 ? launch_sel<1024, 32, true, false> : launch_sel<1024, 32, false, false>);
+    return launch(launch_sel<1024, 32, true, true>);   // only a cluster of eight gets here
 }
 
 }  // namespace dsa

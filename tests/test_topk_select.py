@@ -91,3 +91,49 @@ def test_select_over_the_slices(built_lib, rows, kv_len, topk, stride):
     check = sorted({0, 1 % rows, rows // 2, rows - 1})
     want = numpy_select(scores[check].cpu().numpy(), topk, valid[check].cpu().numpy())
     assert np.array_equal(got[check], want)
+
+
+def test_time_follows_the_rows_own_length(built_lib):
+    """Short rows in a buffer made for long ones (a serving batch) take a small multiple of their time in a narrow buffer (a
+    CTA that makes, counts and tests keys for the whole width took 14 times as long), and give the same lists."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(11)
+    wide = torch.randn(300, 131072, generator=g, device="cuda")
+    narrow = wide[:, :3000].contiguous()
+    valid = torch.randint(2100, 3001, (300,), generator=g, device="cuda").to(torch.int32)
+
+    def best(scores):
+        out = api.topk_select(scores, 2048, valid)
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(20):
+                api.topk_select(scores, 2048, valid, out=out)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times), out
+
+    t_wide, o_wide = best(wide)
+    t_narrow, o_narrow = best(narrow)
+    assert torch.equal(o_wide, o_narrow)
+    assert t_wide < 6 * t_narrow, (t_wide, t_narrow)
+
+
+@pytest.mark.parametrize("rows,kv_len", [(64, 32768), (300, 20004), (40, 131072), (2, 300004)])
+def test_lengths_at_the_edges_of_rounds_and_slices(built_lib, rows, kv_len):
+    """Rows of one buffer that end around a round of a CTA's registers (2048 or 4096 positions), around what one CTA holds
+    (8192 or 32768) and around a slice."""
+    edges = [n + d for n in (2048, 4096, 6144, 8192, 12288, 16384, 32768, 32768 + 4096, 65536, 131072, kv_len) for d in (-3, -1, 0, 1, 2)]
+    edges = [n for n in edges if 0 < n <= kv_len]
+    topk = 300
+    g = torch.Generator(device="cuda")
+    g.manual_seed(kv_len)
+    for i0 in range(0, len(edges), rows):
+        lens = (edges[i0:i0 + rows] * rows)[:rows]
+        scores = torch.round(torch.randn(rows, kv_len, generator=g, device="cuda") * 64) / 64
+        valid = torch.tensor(lens, dtype=torch.int32, device="cuda")
+        got = api.topk_select(scores, topk, valid).cpu().numpy()
+        n = min(rows, len(edges) - i0)
+        assert np.array_equal(got[:n], numpy_select(scores[:n].cpu().numpy(), topk, np.array(lens[:n])))
