@@ -354,8 +354,9 @@ __device__ __noinline__ void select_row_alone(SelShared* sh, const float* row, i
 // One CTA or one cluster per row.  The lengths are on the device and the form is chosen by the buffer's width, so a row that fits the
 // registers of one CTA is left to the first of its cluster, and one whose valid positions are all selected needs no selection.
 // Rows of 2100-3000 in a buffer of 131072: 160 rows 23 us (74 when the whole cluster worked on the width; one CTA of 512 threads that
-// scanned the row five times 31), 300 rows 40 (146; 33).  CTAs and clusters that stay and deal the rows out among themselves
-// took 20 us for the latter, but 5 to 12 % more for full rows and up to 65 % for mixed ones, whose order they fix beforehand.
+// scanned the row five times 31), 300 rows 40 (146; 33).  Small CTAs for the short rows in a launch before, and then clusters that
+// stay and deal the long ones out among themselves, took 12.5 us for the 300, but 5 to 12 % more for full rows and up to 65 % for mixed
+// ones, whose order they fix beforehand.
 template <int kThreads, int kPer, bool kCluster, bool kReload>
 __global__ void __launch_bounds__(kThreads, kThreads == 512 ? (kCluster ? 2 : 3) : 1) topk_select_kernel(const float* __restrict__ scores, int64_t stride_row,
                                                                 const int32_t* __restrict__ valid_len, int kv_len, int topk,
