@@ -1,6 +1,8 @@
 // Internal definitions shared by the host launcher, the planner and the kernels.
 #pragma once
+#include <atomic>
 #include <cstdint>
+#include <cuda_runtime.h>
 #include "../../include/dsa_v32.h"
 
 namespace dsa {
@@ -13,6 +15,22 @@ constexpr int kDvHalf = 256;            // output columns accumulated by one CTA
 constexpr int kTileRows = 32;           // top-k slots per pipeline step
 constexpr int kSmallHeads = 32;         // most tile rows an item may have for the few-heads kernel
 constexpr int kFp8RowBytes = DSA_V32_FP8_ROW_BYTES;
+
+// SMs of the current device, for the rules that ask whether a launch fills it.
+inline cudaError_t sm_count(int* out) {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int n = dev >= 0 && dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
+    }
+    *out = n;
+    return cudaSuccess;
+}
 
 constexpr uint32_t kWorkspaceMagic = 0x44534133u;  // "DSA3"
 

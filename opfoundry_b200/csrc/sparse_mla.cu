@@ -1336,9 +1336,9 @@ done:
 // cache 21.5 -> 15.9 us, against one warp per row that walked the splits one by one (slot, then lse, then four float4).
 // With kV = 1 throughout, a prefill chunk of 64 split rows x 64 heads took 8.9 us for its merge instead of 5.2.
 constexpr int kMergeFlight = 8;                       // float4 in flight per lane
-constexpr int kMergeResidentRows = 148 * 8;           // blocks of 128 threads resident at once (64 registers per thread)
+constexpr int kMergeBlocks = 8;                       // blocks per SM of the form with kV = 1 (64 registers per thread)
 template <int kV>
-__global__ void __launch_bounds__(128) combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
+__global__ void __launch_bounds__(128, kV == 1 ? kMergeBlocks : kMergeBlocks - 1) combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
                                                       const int32_t* __restrict__ reduce_indptr,
                                                       const int32_t* __restrict__ reduce_slots,
                                                       const ReduceDst* __restrict__ reduce_dst, const OutTargets tgt,
@@ -1598,7 +1598,10 @@ cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const i
                            const int32_t* reduce_slots, const ReduceDst* reduce_dst, int num_reduce_rows, const OutTargets& tgt,
                            int64_t stride_o_row, int64_t stride_o_head, int H, int tile_rows, cudaStream_t stream) {
     if (num_reduce_rows <= 0) return cudaSuccess;
-    const bool wide = (int64_t)num_reduce_rows * tile_rows > kMergeResidentRows;
+    int sms = 0;
+    cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    const bool wide = (int64_t)num_reduce_rows * tile_rows > int64_t(sms) * kMergeBlocks;
     dim3 grid(num_reduce_rows, wide ? (tile_rows + 3) / 4 : tile_rows);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];

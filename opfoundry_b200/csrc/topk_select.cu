@@ -405,11 +405,14 @@ cudaError_t launch_topk_select(const float* scores, int64_t stride_row, const in
                                int32_t* indices_out, cudaStream_t stream) {
     if (total_q <= 0) return cudaSuccess;
     const int vec_ok = (stride_row % 4 == 0 && (reinterpret_cast<uintptr_t>(scores) & 15u) == 0) ? 1 : 0;
+    int sms = 0;
+    cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
     // CTAs per row: up to two waves' worth of an SM each (64 rows of 32768 positions: four CTAs of 512 threads 14.8 us, one of
     // 1024 threads 15.0, eight 27, the exchange of a cluster growing with its size), and enough that a slice fits the
     // registers.
     int n_cta = 1;
-    while (n_cta < 8 && (((int64_t)total_q * n_cta * 2 <= 296 && kv_len / (2 * n_cta) >= 4096) || kv_len > n_cta * 32768)) n_cta *= 2;
+    while (n_cta < 8 && (((int64_t)total_q * n_cta * 2 <= 2 * sms && kv_len / (2 * n_cta) >= 4096) || kv_len > n_cta * 32768)) n_cta *= 2;
     const int per_cta = ((kv_len + n_cta - 1) / n_cta + 3) & ~3;
     // Slices of up to 8192 positions: 16 keys per thread, three CTAs on an SM (2048 rows of 8192: 49.6 us; 32 keys in 256
     // threads 51.6, 8 in 1024 threads 61.7).
