@@ -6,8 +6,11 @@
 // the tables the merge kernel walks.  The unit of cost here is one pipeline step of
 // kTileRows top-k slots plus a fixed per-piece overhead (query load + epilogue), mirroring the
 // reference's "kv blocks + fixed_overhead" cost (get_mla_metadata.hpp:27-37).  A work list
-// belongs to one CTA pair (the two CTAs of a pair each accumulate one 256-column half of the
-// output), so there are num_sms / 2 lists instead of the reference's 256 compute units.
+// belongs to one CTA pair, so there are num_sms / 2 lists instead of the reference's 256 compute units.
+// The two CTAs of a pair split an item by columns in the 128-row kernel and by slots in the few-heads kernel; the
+// plan is the same for both, its unit and its overhead being those of the 128-row kernel.  (Of the few-heads kernel's own: an
+// overhead of 12 steps was neutral, a merge cost of 60 made 128 sequences of 2 x 16 heads 195 us instead of 186, least pieces of
+// two or three steps 19.1-20.3 us for one sequence against 19.6.)
 //
 // The plan depends only on shapes (and the optional per-query valid-length hint), never on the
 // index values, so it is computed on the host and uploaded once per shape.

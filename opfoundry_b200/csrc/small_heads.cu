@@ -26,10 +26,11 @@
 //              ahead), converted e4m3 -> bf16 exactly and stored.  No staging of raw rows: the room it would take is the
 //              third tile stage.
 //
-// What bounds it (cycle stamps, fp8, 16 heads): a tile holds its stage for 8 500 cycles (load and convert 900, the other warps'
+// What bounds it (cycle stamps of an instrumented copy, fp8, 16 heads): a tile holds its stage for 8 500 cycles (load and convert 900, the other warps'
 // rows 700, scores 2 000, softmax 2 100, P V 750 and the hand-offs between them), three stages: 2 850-3 300 cycles per
-// 48 slots; the tensor pipe is busy for 2 000 of them (a score MMA of M = 64, N = 16 takes 33 cycles, a P V MMA 62).
-// Measured against the kernel of sparse_mla.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 226 -> 186 us, 64
+// 48 slots; its MMAs take 2 000 of them to issue (36 for the scores of M = 64, N = 16 at 33 cycles, 12 for P V at 62), though
+// the counter has the tensor pipe active for 8 %.
+// Measured against the kernel of sparse_mla.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 219 -> 177 us, 64
 // sequences of 16 heads 79 -> 51, 128 of 32 heads 151 -> 127; bf16, 64 sequences of 16 heads 52 -> 39, prefill of 2048 tokens with
 // 16 heads 661 -> 409, two sequences of 16 heads 15.9 -> 14.7 (the last with the merge).  out against 64 bits: 2.08e-3 (2.10e-3
 // there), lse 2e-7 (7e-7: no 16-bit exchange of partial scores).
