@@ -428,8 +428,11 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     if (p.attn_sink != nullptr && wi.k_begin == 0 && half == 0) {
                         // attention sink: one more term exp(sink - m) in the denominator, in the piece that starts the list
                         const float sink2 = live ? __ldg(p.attn_sink + head) * 1.4426950408889634f : -INFINITY;
-                        if (m == -INFINITY) m = sink2;
-                        if (sink2 > -INFINITY) ls += ex2_approx(sink2 - m);
+                        // (a NaN is no term)
+                        if (sink2 > -INFINITY) {
+                            if (m == -INFINITY) m = sink2;
+                            ls += ex2_approx(sink2 - m);
+                        }
                     }
                     // this CTA's P buffer is free (every product of the item is complete; all four warps have met since they
                     // read the last exchange), so the peer may write its sums over it
@@ -465,8 +468,9 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     ++xn;
                     const float pm = ctl->peer_m[h], pl = ctl->peer_l[h];
                     const float mm = fmaxf(m, pm);
-                    const float f_own = m == -INFINITY ? 0.0f : ex2_approx(m - mm);
-                    const float f_peer = pm == -INFINITY ? 0.0f : ex2_approx(pm - mm);
+                    // an infinite sink is the reference of a row without positions: its zeros stay zeros
+                    const float f_own = m == -INFINITY ? 0.0f : (m == mm ? 1.0f : ex2_approx(m - mm));
+                    const float f_peer = pm == -INFINITY ? 0.0f : (pm == mm ? 1.0f : ex2_approx(pm - mm));
                     ls = ls * f_own + pl * f_peer;
                     m = mm;
                     const float inv = ls > 0.0f ? 1.0f / ls : 0.0f;

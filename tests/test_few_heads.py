@@ -227,3 +227,31 @@ def test_rows_go_to_every_peer(built_lib, B, H, s_q, fp8, share):
         assert torch.equal(o[:, h0:h0 + H].view(torch.int16), want_out.view(torch.int16)) and torch.equal(l[:, h0:h0 + H], want_lse)
         assert torch.all(o[:, :h0] == 7) and torch.all(o[:, h0 + H:] == 7) and torch.all(l[:, :h0] == 7) and torch.all(l[:, h0 + H:] == 7)
     assert flags[:, 0].tolist() == [1, 1]
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("B,fp8", [(2, False), (2, True), (90, False), (90, True)])
+def test_infinite_and_nan_sinks(built_lib, B, fp8, value):
+    """A row without positions is zeros whatever its sink is, also when the pieces are merged; an infinite sink takes all of
+    a row's weight, a NaN is no term (both as in the 128-row kernel)."""
+    import torch
+    from gpu_util import to_dev
+    H, topk = 16, 1000
+    case = synth.make_decode_case(B, H, 1024, topk, fp8=fp8, paged=fp8, seed=B)
+    case["indices"][0] = -1
+    case["indices"][1, :500] = -1      # nothing in the first CTA's half
+    d = to_dev(case)
+    plan = api.mla_decode_plan_create(B, H, topk)
+    kw = dict(block_table=d["block_table"], page_block_size=case["page_block_size"], kv_batch_stride_rows=case["kv_batch_stride_rows"])
+    run = lambda sink: api.mla_v4_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, attn_sink=torch.tensor(sink, device="cuda"), **kw)
+    sink = [0.5] * H
+    sink[1::2] = [value] * (H // 2)
+    out, lse = run(sink)
+    assert torch.all(out[0] == 0) and torch.all(lse[0, 1::2] == float("inf"))
+    if value == float("inf"):
+        if plan.info.num_partials:     # (the merge has no finite reference for a piece of infinite weight)
+            return
+        assert torch.all(out[:, 1::2] == 0) and torch.all(lse[:, 1::2] == float("inf"))
+    else:
+        w_out, w_lse = run([0.5, -float("inf")] * (H // 2))
+        assert torch.equal(out[1:], w_out[1:]) and torch.equal(lse[1:], w_lse[1:])
