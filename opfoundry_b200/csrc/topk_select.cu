@@ -15,7 +15,7 @@
 // What bounds it: instruction issue while there are many rows (every key is touched four times: made, counted, tested
 // for the list, written), and the chain of block- and cluster-wide steps when there are few.  Measured against one CTA of
 // 512 threads per row that reads the row in each of five passes and scans every 512 positions: 64 rows of 32768 84.0 ->
-// 14.4 us, 2048 rows of up to 8192 247.6 -> 53.3 us (0.6 and 1.4 TB/s of scores and lists).
+// 14.4 us, 2048 rows of up to 8192 247.6 -> 51.6 us (0.6 and 1.5 TB/s of scores and lists).
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
