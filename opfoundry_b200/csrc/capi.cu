@@ -16,6 +16,7 @@ int max_resident_pairs(bool fp8, int* out);
 cudaError_t launch_attn(bool fp8, bool ext, int num_lists, const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ttail,
                         const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_small_heads(bool fp8, int tile_rows, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
+cudaError_t launch_paired_heads(bool ext, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const int32_t* reduce_indptr,
                            const int32_t* reduce_slots, const ReduceDst* reduce_dst, int num_reduce_rows, const OutTargets& tgt,
                            int64_t stride_o_row, int64_t stride_o_head, int H, int tile_rows, cudaStream_t stream);
@@ -162,6 +163,7 @@ void fill_params(const dsa_v32_attn_args* a, const WorkspaceHeader& h, AttnParam
     set_page(p, a->page_block_size);
     p->scale_log2 = a->sm_scale * 1.4426950408889634f;
     p->wide = 0;
+    p->q_box = 0;
     p->n_peers = 0;
     p->lse_stride_row = a->H;
     for (int i = 0; i < DSA_V32_MAX_PEERS; ++i) {
@@ -308,6 +310,16 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     for (int i = 0; i < p.n_peers; ++i) low |= reinterpret_cast<uintptr_t>(p.out_peers[i]);
     p.wide = (low & 31u) == 0;
     const bool use_ext = !p.wide || h.has_stacked != 0 || p.attn_sink != nullptr || p.kv2 != nullptr || p.n_peers > 0;
+    if (!fp8) {
+        // stacked query rows follow one another every H (a multiple of 8) tile rows, so their boxes are eight heads high
+        p.q_box = h.has_stacked ? 8 : 64;
+        const uint64_t dims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
+        const uint64_t str[2] = {uint64_t(a->stride_q_head) * 2, uint64_t(a->stride_q_row) * 2};
+        const uint32_t box[3] = {64, uint32_t(p.q_box), 1};
+        if (tmap_cache().get(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->q, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return DSA_V32_ERR_DRIVER;
+        cudaError_t e = launch_paired_heads(use_ext, h.num_lists, tq, p, stream);
+        return e == cudaSuccess ? DSA_V32_OK : (int)e;
+    }
     cudaError_t e = launch_attn(fp8, use_ext, h.num_lists, tq, tkv, ttail, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }

@@ -74,6 +74,7 @@ struct AttnParams {
     int32_t H, topk, s_q, block_table_stride, page_block_size;
     int32_t page_shift;  // log2(page_block_size) when that is a power of two, else -1
     float scale_log2;  // sm_scale * log2(e)
+    int32_t q_box;     // heads in a box of the tensor map of Q (paired_heads.cu)
     int32_t wide;      // rows of q and out start on 32-byte boundaries (else they are accessed 16 bytes at a time)
     // fused all-gather: when n_peers > 0 finished rows go to every peer's gathered buffer instead of out / lse
     int32_t n_peers;

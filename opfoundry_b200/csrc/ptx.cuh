@@ -29,6 +29,9 @@ __device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {   // no arrival
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -190,6 +193,12 @@ __device__ __forceinline__ void st_async_u32(uint32_t caddr, uint32_t v, uint32_
 // arrive on an mbarrier of another CTA of the cluster; releases this thread's earlier writes
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t caddr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(caddr) : "memory");
+}
+// The same at CTA scope: what it orders must already be visible where it is needed - TMEM accesses before a
+// tcgen05.fence::before_thread_sync, shared memory made visible to the async proxy by fence.proxy.async - and a release at
+// cluster scope, which waits for every earlier write of the thread, is then not paid for.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t caddr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(caddr) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -527,6 +536,79 @@ __device__ __forceinline__ void tc_commit_el(uint32_t bar, uint32_t elected) {
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
         :
         : "r"(bar), "r"(elected)
+        : "memory");
+}
+
+// ------------------------------------------------------------------ the pair forms (cta_group::2)
+// One instruction over the tensor cores of both CTAs of a cluster, issued by the even one: each CTA's shared memory holds
+// its half of A's rows and its half of B's N rows at the same offsets, and each CTA's TMEM gets its half of D's rows.
+// With M = 128 a CTA has 64 rows: TMEM lanes 0-63 hold columns [0, N / 2) of them and lanes 64-127 columns [N / 2, N), so
+// all lanes work and the rate is the full one; an A operand in TMEM has its 64 rows in both halves of the lanes.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {   // one warp of either CTA
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// All pair MMAs this thread has issued arrive, when complete, on the barrier at this offset in both CTAs.
+__device__ __forceinline__ void tc_commit_pair_el(uint32_t bar, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "mov.b16 m, 3;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
+        :
+        : "r"(bar), "r"(elected)
+        : "memory");
+}
+__device__ __forceinline__ void umma_pair_ss_el(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
+        : "memory");
+}
+// four K = 16 steps of one 64-column block, as umma_ts_x4_el and umma_ss_x4_el
+__device__ __forceinline__ void umma_pair_ts_x4_el(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                                   uint32_t first_accumulates, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred q, pt, pf;\n\t.reg .b32 a, l;\n\t.reg .b64 bd;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "setp.ne.b32 pf, %5, 0;\n\t"
+        "setp.eq.b32 pt, %6, %6;\n\t"
+        "mov.b64 bd, {%2, %3};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], bd, %4, pf;\n\t"
+        "add.u32 a, %1, 8;\n\tadd.u32 l, %2, 2;\n\tmov.b64 bd, {l, %3};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a], bd, %4, pt;\n\t"
+        "add.u32 a, %1, 16;\n\tadd.u32 l, %2, 4;\n\tmov.b64 bd, {l, %3};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a], bd, %4, pt;\n\t"
+        "add.u32 a, %1, 24;\n\tadd.u32 l, %2, 6;\n\tmov.b64 bd, {l, %3};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a], bd, %4, pt;\n\t}"
+        :
+        : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates), "r"(elected)
+        : "memory");
+}
+__device__ __forceinline__ void umma_pair_ss_x4_el(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                                   uint32_t idesc, uint32_t first_accumulates, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred q, pt, pf;\n\t.reg .b32 la, lb;\n\t.reg .b64 ad, bd;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "setp.ne.b32 pf, %6, 0;\n\t"
+        "setp.eq.b32 pt, %7, %7;\n\t"
+        "mov.b64 ad, {%1, %2};\n\tmov.b64 bd, {%3, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], ad, bd, %5, pf;\n\t"
+        "add.u32 la, %1, 2;\n\tadd.u32 lb, %3, 2;\n\tmov.b64 ad, {la, %2};\n\tmov.b64 bd, {lb, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], ad, bd, %5, pt;\n\t"
+        "add.u32 la, %1, 4;\n\tadd.u32 lb, %3, 4;\n\tmov.b64 ad, {la, %2};\n\tmov.b64 bd, {lb, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], ad, bd, %5, pt;\n\t"
+        "add.u32 la, %1, 6;\n\tadd.u32 lb, %3, 6;\n\tmov.b64 ad, {la, %2};\n\tmov.b64 bd, {lb, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], ad, bd, %5, pt;\n\t}"
+        :
+        : "r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates), "r"(elected)
         : "memory");
 }
 

@@ -1,0 +1,57 @@
+"""The 128-row kernel (one pair MMA over the two CTAs of a cluster, 64 tile rows and 32 of a tile's 64 slots each): edges of its
+tiles and row halves, lists of many short items (the ring of stages that Q and the tiles share), moving references, stacked rows."""
+import math
+
+import numpy as np
+import pytest
+
+from helpers import TOL_BF16, TOL_FP8, check_lse, check_out, few_heads_form
+from opfoundry_b200 import api, synth
+from test_few_heads import _moving_references
+
+pytestmark = pytest.mark.gpu
+
+SCALE = 1.0 / math.sqrt(192.0)
+
+
+def _compare(oracle, case, **kw):
+    from gpu_util import run_gpu, run_oracle
+    T, H = case["q"].shape[:2]
+    assert few_heads_form(api.plan_host(T, H, case["topk"], case["s_q"], **kw)) == 0
+    g_out, g_lse, plan = run_gpu(case, SCALE, **kw)
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    check_out(g_out, r_out, **(TOL_FP8 if case["fp8"] else TOL_BF16))
+    check_lse(g_lse, r_lse)
+    return plan
+
+
+EDGES = [1, 2, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 191, 193, 255, 256, 257, 321, 0]
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,num_sms", [(33, 2), (64, 4), (72, 6), (128, 2), (128, 148), (200, 4)])
+def test_tile_edges_in_lists_of_short_items(built_lib, oracle, H, num_sms, fp8):
+    lens = np.array(EDGES + EDGES[::-1], np.int32)
+    case = synth.make_decode_case(len(lens), H, 512, 321, fp8=fp8, paged=fp8, seed=H + num_sms)
+    for r, n in enumerate(lens):
+        case["indices"][r, n:] = -1
+    _compare(oracle, case, num_sms=num_sms, valid_len_hint=lens)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,s_q", [(64, 1), (128, 1), (64, 2)])
+def test_references_move_in_long_items(built_lib, oracle, H, s_q, fp8):
+    B, topk = 6, 1216
+    case = _moving_references(B, H, topk, s_q=s_q, fp8=fp8, share=s_q > 1, seed=H + s_q)
+    _compare(oracle, case, num_sms=4, mtp_shared=[b % 2 == 0 for b in range(B)] if s_q > 1 else None)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,s_q", [(24, 4), (40, 3), (64, 2), (56, 2)])
+def test_stacked_rows_over_both_ctas(built_lib, oracle, H, s_q, fp8):
+    """Stacked query rows that end inside, at and beyond the 64 tile rows of a CTA, among items of a single row."""
+    case = synth.make_decode_case(7, H, 1024, 200, s_q=s_q, fp8=fp8, paged=fp8, share_mtp="coin", seed=H + s_q)
+    case["mtp_shared"][:2] = [True, False]
+    case["indices"][:s_q] = case["indices"][0]
+    plan = _compare(oracle, case, num_sms=6, mtp_shared=case["mtp_shared"])
+    assert any(w.stacked_rows > 1 for w in plan.read_works()[0])
