@@ -12,8 +12,9 @@
 #include "tmap.h"
 
 namespace dsa {
-int max_resident_pairs(bool fp8, int* out);
-cudaError_t launch_attn(bool fp8, bool ext, int num_lists, const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ttail,
+int max_resident_pairs(int* out);
+int max_resident_pairs_paired(int* out);
+cudaError_t launch_attn(bool ext, int num_lists, const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ttail,
                         const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_small_heads(bool fp8, int tile_rows, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_paired_heads(bool ext, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
@@ -88,9 +89,9 @@ Registry& registry() {
 // keeps resident at once, which can be below the SM count when a GPC holds an odd number of SMs.
 int device_sm_count(int* out) {
     int a = 0, b = 0;
-    int rc = max_resident_pairs(true, &a);
+    int rc = max_resident_pairs(&a);
     if (rc) return rc;
-    rc = max_resident_pairs(false, &b);
+    rc = max_resident_pairs_paired(&b);
     if (rc) return rc;
     const int pairs = a < b ? a : b;
     if (pairs < 1) return DSA_V32_ERR_DRIVER;
@@ -269,7 +270,6 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         p.pool_split = ext->kv2 ? ext->pool_split : nullptr;
         p.num_kv2_rows = ext->num_kv2_rows;
     }
-    // bf16 cache: the 128-row kernel reads Q and the cache rows with plain loads and takes no tensor map
     CUtensorMap tq, tkv, ttail;
     std::memset(&tq, 0, sizeof(tq));
     std::memset(&tkv, 0, sizeof(tkv));
@@ -320,7 +320,7 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         cudaError_t e = launch_paired_heads(use_ext, h.num_lists, tq, p, stream);
         return e == cudaSuccess ? DSA_V32_OK : (int)e;
     }
-    cudaError_t e = launch_attn(fp8, use_ext, h.num_lists, tq, tkv, ttail, p, stream);
+    cudaError_t e = launch_attn(use_ext, h.num_lists, tq, tkv, ttail, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }
 

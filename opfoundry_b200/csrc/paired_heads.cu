@@ -687,41 +687,63 @@ done:
     }
 }
 
+// The opt-in for more than 48 KB of dynamic shared memory is a per-device attribute of the kernel.
 template <bool kExt>
-static cudaError_t launch(int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream) {
+static cudaError_t configure() {
     static std::mutex mu;
     static bool done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    {   // the opt-in for more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
-        std::lock_guard<std::mutex> guard(mu);
-        if (dev < 0 || dev >= 64 || !done[dev]) {
-            e = cudaFuncSetAttribute(paired_heads_kernel<kExt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-            if (e != cudaSuccess) return e;
-            if (dev >= 0 && dev < 64) done[dev] = true;
-        }
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
-    cfg.gridDim = dim3(2 * num_lists, 1, 1);
-    cfg.blockDim = dim3(32 * kWarps, 1, 1);
-    cfg.dynamicSmemBytes = kSmemBytes;
-    cfg.stream = stream;
+    std::lock_guard<std::mutex> guard(mu);
+    if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+    e = cudaFuncSetAttribute(paired_heads_kernel<kExt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) done[dev] = true;
+    return cudaSuccess;
+}
+
+static void fill_launch(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int num_lists, cudaStream_t stream) {
+    cfg->gridDim = dim3(2 * num_lists, 1, 1);
+    cfg->blockDim = dim3(32 * kWarps, 1, 1);
+    cfg->dynamicSmemBytes = kSmemBytes;
+    cfg->stream = stream;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg->attrs = attr;
+    cfg->numAttrs = 2;
+}
+
+template <bool kExt>
+static cudaError_t launch(int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream) {
+    cudaError_t e = configure<kExt>();
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    fill_launch(&cfg, attr, num_lists, stream);
     return cudaLaunchKernelEx(&cfg, paired_heads_kernel<kExt>, tq, p);
 }
 
 }  // namespace paired
 
-// tq: boxes of 64 columns x p.q_box heads of one query row
+int max_resident_pairs_paired(int* out) {
+    cudaError_t e = paired::configure<false>();
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    paired::fill_launch(&cfg, attr, 1, nullptr);
+    e = cudaOccupancyMaxActiveClusters(&n, paired::paired_heads_kernel<false>, &cfg);
+    if (e != cudaSuccess) return (int)e;
+    *out = n;
+    return 0;
+}
+
+// ext: a sink, second pool or peers are given, or rows of out are aligned to 16 bytes only; tq: boxes of 64 columns x p.q_box heads of one query row
 cudaError_t launch_paired_heads(bool ext, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream) {
     return ext ? paired::launch<true>(num_lists, tq, p, stream) : paired::launch<false>(num_lists, tq, p, stream);
 }
