@@ -276,12 +276,13 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     std::memset(&ttail, 0, sizeof(ttail));
     const bool fp8 = want_dtype == DSA_V32_KV_FP8;
     // Few heads: the kernel that puts the slots on the tensor-core tile's rows, where the plan says so (few_heads_form).
-    if (h.few_heads) {
+    const int few_heads = fp8 ? h.few_heads : h.few_heads_bf16;
+    if (few_heads) {
         const uint64_t qdims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
         const uint64_t qstr[2] = {uint64_t(a->stride_q_head) * 2, uint64_t(a->stride_q_row) * 2};
         const uint32_t qbox[3] = {64, uint32_t(a->H), 1};
         if (tmap_cache().get(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->q, qdims, qstr, qbox, CU_TENSOR_MAP_SWIZZLE_128B)) return DSA_V32_ERR_DRIVER;
-        cudaError_t e = launch_small_heads(fp8, h.few_heads, h.num_lists, tq, p, stream);
+        cudaError_t e = launch_small_heads(fp8, few_heads, h.num_lists, tq, p, stream);
         return e == cudaSuccess ? DSA_V32_OK : (int)e;
     }
     if (fp8) {

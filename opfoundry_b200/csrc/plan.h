@@ -63,22 +63,26 @@ inline void enumerate_units(const dsa_v32_shape& sh, std::vector<PlanUnit>& unit
 // The kernel a plan's items run on: 16 or 32 = the few-heads kernel's form for that many tile rows, 0 = the 128-row kernel.
 // Beyond 32 rows Q, the P copies and three tile stages of the few-heads kernel do not fit shared memory.
 // Up to 32 rows it takes less time per slot but more per change of item (its softmax group is also its epilogue), so the line is
-// drawn by the slots that an item has on average.  Measured time over that of the 128-row kernel, 1 to 12 items per list, fp8 | bf16:
-//   16 rows, whole items of  64: 1.04-1.12 | 1.02-1.14   128: 1.01-1.05 | 1.03-1.11   192: 0.81-0.90 | 0.90-0.94   2048: 0.59-0.63 | 0.71-0.75
-//   32 rows, whole items of 128: 1.42-1.69 | 1.34-1.61   448: 1.02-1.07 | 1.06-1.12   800: 0.95-0.99 | 1.00-1.02   2048: 0.87      | 0.85-0.87
+// drawn by the slots that an item has on average.  Measured time over that of the 128-row kernel, fp8, 1 to 12 items per list:
+//   16 rows, whole items of  64: 1.04-1.12   128: 1.01-1.05   192: 0.81-0.90   2048: 0.59-0.63
+//   32 rows, whole items of 128: 1.42-1.69   448: 1.02-1.07   800: 0.95-0.99   2048: 0.87
 // A piece of a split item has a cheaper end there (fp32 rows of the live heads only): pieces of 128 slots and more
-//   16 rows: 0.57-0.82 | 0.61-0.81   32 rows: 0.82-1.05 | 0.78-0.98
+//   16 rows: 0.57-0.82   32 rows: 0.82-1.05
+// bf16, against its own 128-row kernel (paired_heads.cu), 4 to 16 items per list:
+//   16 rows, whole items of 192: 1.05-1.15   320: 1.20-1.24   448: 1.05   640: 0.97-1.04   1024: 0.97   2048: 0.87   pieces: 0.71-0.85
+//   32 rows, whole items of 640: 0.90-0.94   800: 1.17   1500: 1.04-1.07   2048: 1.05   pieces: 0.87-1.02 (no line is clear: the fp8 one)
 constexpr int kFewRows16Slots = 160;       // least slots of a whole item of at most 16 rows, on average
-constexpr int kFewRows32Slots = 768;       // the same for 17 to 32 rows
+constexpr int kFewRows16SlotsBf16 = 512;   // the same for a bf16 cache
+constexpr int kFewRows32Slots = 768;       // the same for 17 to 32 rows, either cache
 constexpr int kFewRows32PieceSlots = 128;  // the same for a piece of a split item of 17 to 32 rows
-inline int few_heads_form(const dsa_v32_shape& sh, const std::vector<dsa_v32_work_info>& works) {
+inline int few_heads_form(const dsa_v32_shape& sh, const std::vector<dsa_v32_work_info>& works, bool fp8) {
     int rows = 0;
     int64_t slots = 0, wanted = 0;
     for (const auto& w : works) {
         const int r = sh.H * std::max(1, w.stacked_rows);
         rows = std::max(rows, r);
         slots += w.k_end - w.k_begin;
-        if (w.partial_slot < 0) wanted += r <= 16 ? kFewRows16Slots : kFewRows32Slots;
+        if (w.partial_slot < 0) wanted += r > 16 ? kFewRows32Slots : (fp8 ? kFewRows16Slots : kFewRows16SlotsBf16);
         else if (r > 16) wanted += kFewRows32PieceSlots;
     }
     if (rows > kSmallHeads || slots < wanted) return 0;
@@ -102,7 +106,8 @@ inline void finish_plan(const dsa_v32_shape& sh, int L, int n_hb, int next_slot,
     h.has_stacked = 0;
     for (const auto& w : P.works)
         if (w.stacked_rows > 1) h.has_stacked = 1;
-    h.few_heads = few_heads_form(sh, P.works);
+    h.few_heads = few_heads_form(sh, P.works, true);
+    h.few_heads_bf16 = few_heads_form(sh, P.works, false);
     int64_t off = 256;
     h.off_list_indptr = off;
     off = align256(off + int64_t(L + 1) * 4);
