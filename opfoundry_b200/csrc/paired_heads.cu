@@ -45,7 +45,8 @@
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises its own and its peer's abort flag, records DSA_V32_ERR_DEVICE_WAIT in
 // the workspace status word and both drain to the normal exit.  A parity wait is only issued on a barrier whose previous phase
-// the waiting warp knows to be complete.
+// the waiting warp knows to be complete, and that cannot complete its next one before that warp has looked (tests/test_paired_protocol.py:
+// a model of the barriers in which any one role may be held back for as long as the others can run).
 #include <cuda_bf16.h>
 #include <cfloat>
 #include <cstddef>
@@ -99,7 +100,7 @@ struct Ctl {
     int32_t late_row[kStages][kOwn];     // rows of the tile that the other CTA gathers
     uint8_t tile_mask[kStages][2][8];    // which slots of CTA 0 / CTA 1 hold a row, four slots a byte
     uint64_t kv_full[kStages], kv_empty[kStages];      // own rows landed | P V of the tile complete (a stage with Q: it has been copied)
-    uint64_t tile_ready[kStages];                      // CTA 0: both CTAs' rows have landed
+    uint64_t tile_ready[2][kStages];                   // CTA 0: both CTAs' rows have landed, by the score issuer (tile number mod 2) that takes the tile
     uint64_t dead[kStages], late_full[kStages];        // scores complete: the other X region may be overwritten | late rows landed
     uint64_t peer_late[kStages];                       // CTA 0: late rows of CTA 1 landed
     uint64_t s_full[2], s_empty[2], p_full[2], pv_done[2];
@@ -190,7 +191,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
     if (tid < kStages) {
         mbar_init(smem_u32(&ctl->kv_full[tid]), kLoadWarps * 33);   // the lanes (their copies) and one plain arrival per warp (mask, rows)
         mbar_init(smem_u32(&ctl->kv_empty[tid]), 1);
-        mbar_init(smem_u32(&ctl->tile_ready[tid]), 2);
+        mbar_init(smem_u32(&ctl->tile_ready[0][tid]), 2);
+        mbar_init(smem_u32(&ctl->tile_ready[1][tid]), 2);
         mbar_init(smem_u32(&ctl->peer_late[tid]), 1);
         mbar_init(smem_u32(&ctl->dead[tid]), 1);
         mbar_init(smem_u32(&ctl->late_full[tid]), 4 * 32);
@@ -509,11 +511,13 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
                 const int n_tiles = tiles_of(p.works[w]);
                 ring.skip(kQStages);
                 if (!wait_on(&ctl->q_full, item_n & 1, abort_flag)) goto done;
-                for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
+                for (int t = 0; t < n_tiles; ++t, ++it) {
                     const uint32_t sb = it & 1u;
-                    // every tile's barrier, in order, so that neither issuer ever waits on a phase whose predecessor it has not seen complete
-                    if (!wait_on(&ctl->tile_ready[ring.s], ring.ph(), abort_flag)) goto done;
-                    if (sb != par) continue;   // the other issuer's
+                    if (sb != par) {   // the other issuer's.  (It has its own barriers: on common ones this warp would have to look at every
+                        ring.skip(1);  // phase, and nothing keeps a stage from its next tile until a warp that is not needed for this one has looked.)
+                        continue;
+                    }
+                    if (!wait_on(&ctl->tile_ready[par][ring.s], ring.ph(), abort_flag)) goto done;
                     if (it >= 2)
                         if (!wait_on(&ctl->s_empty[sb], ((it >> 1) & 1u) ^ 1u, abort_flag)) goto done;
                     tc_fence_after();
@@ -528,6 +532,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
                     }
                     tc_commit_pair_el(smem_u32(&ctl->s_full[sb]), el);
                     tc_commit_pair_el(smem_u32(&ctl->dead[ring.s]), el);
+                    ring.next();
                 }
                 tc_commit_pair_el(smem_u32(&ctl->q_empty), el);
             }
@@ -538,14 +543,16 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
             const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(sKV), kKvBlock, 1024);   // MN-major: 64-column blocks kKvBlock apart
             const uint64_t p_desc0 = make_smem_desc_sw128(smem_u32(sP), 16, 1024);
             uint32_t it = 0;
+            uint32_t ready_bits = 0;   // parities of tile_ready
             Ring ring;
             int item_n = 0;
             for (int w = w_begin; w < w_end; ++w, ++item_n) {
                 const int n_tiles = tiles_of(p.works[w]);
                 ring.skip(kQStages);
                 for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
-                    const uint32_t sb = it & 1u;
-                    if (!wait_on(&ctl->tile_ready[ring.s], ring.ph(), abort_flag)) goto done;
+                    const uint32_t sb = it & 1u, rb = sb * kStages + ring.s;
+                    if (!wait_on(&ctl->tile_ready[0][0] + rb, (ready_bits >> rb) & 1u, abort_flag)) goto done;
+                    ready_bits ^= 1u << rb;
                     if (!wait_on(&ctl->late_full[ring.s], ring.ph(), abort_flag)) goto done;
                     fence_proxy_async_smem();   // written by cp.async (generic proxy)
                     if (!wait_on(&ctl->peer_late[ring.s], ring.ph(), abort_flag)) goto done;
@@ -570,15 +577,17 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
         } else if (warp == kReadyWarp || (rank == 1 && warp == kPvWarp)) {
             // ======================================================== this CTA's rows' (late rows') arrival, passed on to the issuers
             uint64_t* const from = warp == kReadyWarp ? ctl->kv_full : ctl->late_full;
-            uint64_t* const to = warp == kReadyWarp ? ctl->tile_ready : ctl->peer_late;
+            uint64_t* const to0 = warp == kReadyWarp ? ctl->tile_ready[0] : ctl->peer_late;   // for even and odd tiles
+            uint64_t* const to1 = warp == kReadyWarp ? ctl->tile_ready[1] : ctl->peer_late;
+            uint32_t it = 0;
             Ring ring;
             for (int w = w_begin; w < w_end; ++w) {
                 const int n_tiles = tiles_of(p.works[w]);
                 ring.skip(kQStages);
-                for (int t = 0; t < n_tiles; ++t, ring.next()) {
+                for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
                     if (!wait_on(&from[ring.s], ring.ph(), abort_flag)) goto done;
                     fence_proxy_async_smem();   // written by cp.async (generic proxy)
-                    warp_arrive_lead(&to[ring.s], lane);
+                    warp_arrive_lead((it & 1u ? to1 : to0) + ring.s, lane);
                 }
             }
         }
