@@ -105,6 +105,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return mbar_wait_budget(bar, parity, abort_flag, DSA_WAIT_BUDGET_NS);
 }
 
+// After a wait has given up, copies and MMAs issued before it may still be on their way into shared memory and TMEM.  Nothing waits
+// for them any more, so the CTA gives them time to land before it gives that memory back: they end by themselves within microseconds.
+#ifndef DSA_SETTLE_NS
+#define DSA_SETTLE_NS 200000ull
+#endif
+__device__ __forceinline__ void settle_in_flight() {
+    const uint64_t t0 = global_ns();
+    for (uint32_t it = 0; it < DSA_WAIT_LIMIT && global_ns() - t0 < DSA_SETTLE_NS; ++it) {
+    }
+}
+
 // Warp-uniform forms for warps that run converged code (shuffles, tcgen05.ld/st) after a wait:
 // either every lane saw the phase complete or the whole warp gives up together.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {

@@ -770,6 +770,10 @@ done:
     __syncthreads();
     if (tid == 0 && ctl->abort_flag) atomicExch(p.status, DSA_V32_ERR_DEVICE_WAIT);
     cluster_sync_all();   // nothing is on its way to either CTA any more: every send has been waited for by its receiver
+    if (ctl->abort_flag) {   // unless a wait gave up; then the flag is up in both, and neither issues anything after the barrier
+        settle_in_flight();
+        cluster_sync_all();
+    }
     if (warp == 4) {
         tc_fence_after();
         tmem_dealloc(tmem, C::kTmemCols);

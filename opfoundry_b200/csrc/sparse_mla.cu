@@ -946,6 +946,10 @@ done:
     __syncthreads();
     if (tid == 0 && ctl->abort_flag) atomicExch(p.status, DSA_V32_ERR_DEVICE_WAIT);
     cluster_sync_all();
+    if (ctl->abort_flag) {   // a wait gave up; then the flag is up in both CTAs, and neither issues anything after the barrier
+        settle_in_flight();
+        cluster_sync_all();
+    }
     if (warp == kMmaWarp) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
@@ -1145,6 +1149,7 @@ __global__ void __launch_bounds__(32) wait_expiry_selftest_kernel(int32_t* statu
     __syncwarp();
     const bool ok = __all_sync(0xffffffffu, mbar_wait_budget(smem_u32(&bar), 0, &abort_flag, budget_ns));
     __syncwarp();
+    if (abort_flag) settle_in_flight();
     if (threadIdx.x == 0) {
         if (abort_flag) atomicExch(status, DSA_V32_ERR_DEVICE_WAIT);
         result[0] = ok ? 0 : 1;
