@@ -315,7 +315,9 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         // stacked query rows follow one another every H (a multiple of 8) tile rows, so their boxes are eight heads high
         p.q_box = h.has_stacked ? 8 : 64;
         const uint64_t dims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
-        const uint64_t str[2] = {uint64_t(a->stride_q_head) * 2, uint64_t(a->stride_q_row) * 2};
+        // the stride of a single head or row may be anything, and a map takes strides below 2^40 bytes only
+        const int64_t head = a->H > 1 ? a->stride_q_head : kDQK;
+        const uint64_t str[2] = {uint64_t(head) * 2, uint64_t(a->total_q > 1 ? a->stride_q_row : head * a->H) * 2};
         const uint32_t box[3] = {64, uint32_t(p.q_box), 1};
         if (tmap_cache().get(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->q, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return DSA_V32_ERR_DRIVER;
         cudaError_t e = launch_paired_heads(use_ext, h.num_lists, tq, p, stream);

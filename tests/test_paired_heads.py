@@ -55,3 +55,17 @@ def test_stacked_rows_over_both_ctas(built_lib, oracle, H, s_q, fp8):
     case["indices"][:s_q] = case["indices"][0]
     plan = _compare(oracle, case, num_sms=6, mtp_shared=case["mtp_shared"])
     assert any(w.stacked_rows > 1 for w in plan.read_works()[0])
+
+
+@pytest.mark.parametrize("T,H,topk,strides", [(1, 128, 512, (1 << 41, 576, 1)), (1, 64, 100, (1 << 50, 576, 1)), (40, 1, 64, (576, 1 << 41, 1)), (1, 1, 31, (1 << 45, 1 << 41, 1))])
+def test_any_stride_of_a_single_row_or_head(built_lib, T, H, topk, strides):
+    """A stride that nothing follows is not used, so it may be larger than a tensor map takes."""
+    import torch
+    case = synth.make_decode_case(T, H, 1024, topk, seed=H)
+    bf = lambda a: torch.from_numpy(a.view(np.int16)).cuda().view(torch.bfloat16)
+    q, kv, idx = bf(case["q"]), bf(case["kv"]), torch.from_numpy(case["indices"]).cuda()
+    plan = api.mla_decode_plan_create(T, H, topk)
+    kw = dict(kv_batch_stride_rows=1024)
+    want, want_lse = api.mla_decode_launch_pipeline(q, kv, idx, plan, SCALE, **kw)
+    out, lse = api.mla_decode_launch_pipeline(q.as_strided((T, H, 576), strides), kv, idx, plan, SCALE, **kw)
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16)) and torch.equal(lse, want_lse)
