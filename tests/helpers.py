@@ -17,9 +17,10 @@ def load_golden(name):
     return dict(np.load(os.path.join(GOLDEN, name)))
 
 
-def few_heads_form(blob):
-    """Which kernel a plan's items run on: 16 or 32 tile rows of the few-heads kernel, 0 = the 128-row kernel (the header's last field)."""
-    return int(np.frombuffer(blob, np.int32, 1, 112)[0])
+def few_heads_form(blob, fp8=True):
+    """Which kernel a plan's items run on with either cache type: 16 or 32 tile rows of the few-heads kernel, 0 = a 128-row kernel
+    (the last two words of the header)."""
+    return int(np.frombuffer(blob, np.int32, 2, 112)[0 if fp8 else 1])
 
 
 def csr_to_lists(kv_indptr, kv_indices, B, s_q, topk=None):

@@ -15,7 +15,7 @@ SCALE = 1.0 / math.sqrt(192.0)
 
 
 @pytest.mark.parametrize("fp8", [False, True])
-@pytest.mark.parametrize("B,H,topk", [(2, 1, 1), (2, 16, 2), (3, 16, 95), (2, 16, 96), (2, 17, 97), (2, 32, 193), (1, 7, 1000), (40, 16, 300)])
+@pytest.mark.parametrize("B,H,topk", [(2, 1, 1), (2, 16, 2), (3, 16, 95), (2, 16, 96), (2, 17, 97), (2, 32, 193), (1, 7, 1000), (40, 16, 300), (40, 16, 700)])
 def test_tile_edges(built_lib, oracle, fp8, B, H, topk):
     from gpu_util import run_gpu, run_oracle
     case = synth.make_decode_case(B, H, 1024, topk, fp8=fp8, paged=fp8, pad_frac=0.1 if topk > 90 else 0.0, scatter_pad=True, seed=H + topk)
@@ -82,7 +82,7 @@ def test_tile_edges_among_long_items(built_lib, oracle, H, fp8):
     for r, n in enumerate(lens):
         case["indices"][r, n:] = -1
     kw = dict(num_sms=14, valid_len_hint=lens)
-    assert few_heads_form(api.plan_host(len(lens), H, 1100, **kw)) == (16 if H <= 16 else 32)
+    assert few_heads_form(api.plan_host(len(lens), H, 1100, **kw), fp8) == (16 if H <= 16 else 32)
     g_out, g_lse, _ = run_gpu(case, SCALE, **kw)
     r_out, r_lse = run_oracle(oracle, case, SCALE)
     check_out(g_out, r_out, **(TOL_FP8 if fp8 else TOL_BF16))
@@ -154,7 +154,7 @@ def test_many_long_items_per_list(built_lib, oracle, H, s_q, share, fp8):
     assert min(_moves(case, topk // 2, fp8)) >= 4
     shared = [share and b % 2 == 0 for b in range(B)]
     kw = dict(num_sms=4, mtp_shared=shared if share else None)
-    assert few_heads_form(api.plan_host(B * s_q, H, topk, s_q, **kw)) == (16 if H * s_q == 16 else 32)
+    assert few_heads_form(api.plan_host(B * s_q, H, topk, s_q, **kw), fp8) == (16 if H * s_q == 16 else 32)
     g_out, g_lse, plan = run_gpu(case, SCALE, **kw)
     works, indptr = plan.read_works()
     lists = [works[a:b] for a, b in zip(indptr, indptr[1:])]
@@ -173,7 +173,7 @@ def test_stacked_rows_of_a_bf16_cache(built_lib, oracle, H, s_q):
     case["mtp_shared"][:2] = [True, False]
     case["indices"][:s_q] = case["indices"][0]
     kw = dict(mtp_shared=case["mtp_shared"])
-    assert few_heads_form(api.plan_host(5 * s_q, H, 900, s_q, **kw)) == (16 if H * s_q == 16 else 32)
+    assert few_heads_form(api.plan_host(5 * s_q, H, 900, s_q, **kw), fp8=False) == (16 if H * s_q == 16 else 32)
     g_out, g_lse, _ = run_gpu(case, SCALE, **kw)
     r_out, r_lse = run_oracle(oracle, case, SCALE)
     check_out(g_out, r_out, **TOL_BF16)
@@ -198,7 +198,8 @@ def test_sink_with_an_fp8_cache(built_lib, oracle, H, B):
     check_lse(lse.cpu().numpy(), r_lse)
 
 
-@pytest.mark.parametrize("B,H,s_q,fp8,share", [(2, 16, 1, True, False), (90, 16, 1, False, False), (3, 24, 1, True, False), (40, 16, 2, True, True), (4, 64, 1, True, False)])
+@pytest.mark.parametrize("B,H,s_q,fp8,share", [(2, 16, 1, True, False), (90, 16, 1, False, False), (3, 24, 1, True, False), (40, 16, 2, True, True), (4, 64, 1, True, False),
+                                                (4, 64, 1, False, False), (74, 128, 1, False, False), (40, 64, 2, False, True), (5, 48, 2, False, True)])
 def test_rows_go_to_every_peer(built_lib, B, H, s_q, fp8, share):
     """The gathered buffers of two destinations on this GPU (the other rank's arrival is set beforehand, so nothing is waited
     for): both hold this rank's heads, bit for bit what the call without peers gives, and nothing else is written."""
@@ -230,13 +231,13 @@ def test_rows_go_to_every_peer(built_lib, B, H, s_q, fp8, share):
 
 
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
-@pytest.mark.parametrize("B,fp8", [(2, False), (2, True), (90, False), (90, True)])
-def test_infinite_and_nan_sinks(built_lib, B, fp8, value):
+@pytest.mark.parametrize("B,fp8,H", [(2, False, 16), (2, True, 16), (90, False, 16), (90, True, 16), (2, False, 72), (74, False, 128)])
+def test_infinite_and_nan_sinks(built_lib, B, fp8, H, value):
     """A row without positions is zeros whatever its sink is, also when the pieces are merged; an infinite sink takes all of
     a row's weight, a NaN is no term (both as in the 128-row kernel)."""
     import torch
     from gpu_util import to_dev
-    H, topk = 16, 1000
+    topk = 1000
     case = synth.make_decode_case(B, H, 1024, topk, fp8=fp8, paged=fp8, seed=B)
     case["indices"][0] = -1
     case["indices"][1, :500] = -1      # nothing in the first CTA's half

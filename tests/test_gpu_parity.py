@@ -243,7 +243,7 @@ def test_pack_fp8_rows_divisions(oracle, n, mag):
 
 
 
-@pytest.mark.parametrize("fp8,H,topk", [(False, 128, 300), (True, 128, 300), (False, 16, 300), (True, 16, 300), (False, 128, 1500)])
+@pytest.mark.parametrize("fp8,H,topk", [(False, 128, 300), (True, 128, 300), (False, 16, 300), (True, 16, 300), (False, 16, 700), (False, 128, 1500)])
 def test_rows_on_16_byte_boundaries(oracle, fp8, H, topk):
     """q and out as views whose rows start on 16- but not on 32-byte boundaries (offset and strides of 8 elements)."""
     from gpu_util import run_oracle, to_dev

@@ -17,7 +17,7 @@ SCALE = 1.0 / math.sqrt(192.0)
 def _compare(oracle, case, **kw):
     from gpu_util import run_gpu, run_oracle
     T, H = case["q"].shape[:2]
-    assert few_heads_form(api.plan_host(T, H, case["topk"], case["s_q"], **kw)) == 0
+    assert few_heads_form(api.plan_host(T, H, case["topk"], case["s_q"], **kw), case["fp8"]) == 0
     g_out, g_lse, plan = run_gpu(case, SCALE, **kw)
     r_out, r_lse = run_oracle(oracle, case, SCALE)
     check_out(g_out, r_out, **(TOL_FP8 if case["fp8"] else TOL_BF16))
@@ -69,3 +69,58 @@ def test_any_stride_of_a_single_row_or_head(built_lib, T, H, topk, strides):
     want, want_lse = api.mla_decode_launch_pipeline(q, kv, idx, plan, SCALE, **kw)
     out, lse = api.mla_decode_launch_pipeline(q.as_strided((T, H, 576), strides), kv, idx, plan, SCALE, **kw)
     assert torch.equal(out.view(torch.int16), want.view(torch.int16)) and torch.equal(lse, want_lse)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("B,H", [(3, 128), (80, 72)])
+def test_repeated_launches_give_the_same_bits(built_lib, B, H, fp8):
+    """Split items with their merge, and whole items several to a list: which warp sums what is fixed by the plan."""
+    from gpu_util import run_gpu
+    case = synth.make_decode_case(B, H, 1024, 700, fp8=fp8, paged=fp8, pad_frac=0.1, seed=B)
+    first = run_gpu(case, SCALE, num_sms=40)
+    assert (first[2].info.num_partials > 0) == (B == 3)
+    for _ in range(5):
+        out, lse, _ = run_gpu(case, SCALE, num_sms=40)
+        assert np.array_equal(out, first[0]) and np.array_equal(lse, first[1])
+
+
+@pytest.mark.parametrize("what", ["sink", "pool", "both"])
+@pytest.mark.parametrize("B,H,s_q,num_sms", [(3, 128, 1, 0), (5, 40, 1, 24), (6, 24, 4, 60), (7, 64, 2, 6)])
+def test_sink_and_second_pool_of_split_and_stacked_items(built_lib, oracle, B, H, s_q, num_sms, what):
+    """Pieces (the sink counts once, in the piece that starts the list; the second pool begins inside a piece or between two) and
+    stacked rows, which share a list and the slot where the second pool begins."""
+    import torch
+    topk, T = 900, B * s_q
+    case = synth.make_decode_case(B, H, 1024, topk, s_q=s_q, pad_frac=0.1, scatter_pad=True, share_mtp="coin" if s_q > 1 else None, seed=H + B)
+    rng = np.random.default_rng(H)
+    idx, rows2 = case["indices"], 96
+    split = np.repeat(rng.choice([0, 1, 63, 128, 500, 640, topk - 1, topk], B), s_q).astype(np.int32)
+    split[:s_q] = 321
+    sink = (rng.normal(size=H) * 3.0).astype(np.float32)
+    kv2 = synth.normal_bf16(H, "kv2", (rows2, 576))
+    if what == "sink":
+        kv2 = split = None
+    else:
+        for b in range(B):     # rows of the second pool, one list for a sequence's rows where they share it
+            for r in range(b * s_q, (b + 1) * s_q):
+                if s_q > 1 and r > b * s_q and case["mtp_shared"][b]:
+                    idx[r] = idx[b * s_q]
+                else:
+                    idx[r, split[r]:] = rng.integers(-1, rows2, topk - split[r])
+    idx[T - 1] = -1            # no position
+    shared = case["mtp_shared"].astype(bool).copy() if s_q > 1 else None
+    if s_q > 1:
+        shared[B - 1] = False
+    if what == "pool":
+        sink = None
+    kw = dict(num_sms=num_sms, mtp_shared=shared)
+    plan = api.mla_decode_plan_create(T, H, topk, s_q, **kw)
+    works = plan.read_works()[0]
+    assert plan.info.num_partials > 0 and (s_q == 1 or any(w.stacked_rows > 1 for w in works))
+    bf = lambda a: torch.from_numpy(a.view(np.int16)).cuda().view(torch.bfloat16)
+    dev = lambda a: None if a is None else torch.from_numpy(a).cuda()
+    out, lse = api.mla_v4_launch_pipeline(bf(case["q"]), bf(case["kv"]), dev(idx), plan, SCALE, attn_sink=dev(sink), kv2=None if kv2 is None else bf(kv2),
+                                          pool_split=dev(split), kv_batch_stride_rows=1024)
+    r_out, r_lse = oracle.sparse_mla_v4(case["q"], case["kv"], idx, SCALE, attn_sink=sink, kv2=kv2, pool_split=split, s_q=s_q, kv_batch_stride_rows=1024)
+    check_out(out.view(torch.int16).cpu().numpy().view(np.uint16), r_out, **TOL_BF16)
+    check_lse(lse.cpu().numpy(), r_lse)
