@@ -944,12 +944,11 @@ done:
     if (ctl->abort_flag) st_cluster_u32(peer_abort, 1u);   // let the peer stop waiting for us
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && ctl->abort_flag) atomicExch(p.status, DSA_V32_ERR_DEVICE_WAIT);
-    cluster_sync_all();
-    if (ctl->abort_flag) {   // a wait gave up; then the flag is up in both CTAs, and neither issues anything after the barrier
+    if (ctl->abort_flag) {   // a wait gave up; nothing more is issued here, and the peer stays at the barrier below meanwhile
+        if (tid == 0) atomicExch(p.status, DSA_V32_ERR_DEVICE_WAIT);
         settle_in_flight();
-        cluster_sync_all();
     }
+    cluster_sync_all();
     if (warp == kMmaWarp) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
