@@ -58,7 +58,7 @@ struct ReduceDst {
 // Kernel parameters (passed by value next to the tensor maps).
 struct AttnParams {
     const void* kv;    // the cache (read directly for the row scales of an fp8 cache)
-    const void* q;     // bf16 [total_q][H][576] with the element strides below (read directly for a bf16 cache)
+    const void* q;     // bf16 [total_q][H][576] with the element strides below (read directly for an fp8 cache, else through a tensor map)
     int64_t stride_q_row, stride_q_head;
     const int32_t* indices;
     const int32_t* block_table;

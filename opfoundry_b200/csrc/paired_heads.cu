@@ -40,8 +40,8 @@
 // stores of O), a sixth of an item of 32 tiles.  One score issuer instead of two: 2 050 cycles a tile.  Arrivals at the issuing CTA with a
 // release at cluster scope: 2 970.  Q by 32-byte loads into TMEM instead of TMA and the ring: 14 000 cycles a change of item.
 // Against a pair that splits the 576 columns and sums partial scores over distributed shared memory (kept for the fp8 cache), in
-// long runs (the power cap): prefill of 4096 tokens x 128 heads 2260 -> 1658 us, 1268 tokens x 64 heads after 1733 642 -> 482, 1024
-// tokens with sink and second pool, 640 slots, 293 -> 216.
+// long runs (the power cap): prefill of 4096 tokens x 128 heads 2260 -> 1656 us, 1268 tokens x 64 heads after 1733 642 -> 483, 1024
+// tokens with sink and second pool, 640 slots, 293 -> 215.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises its own and its peer's abort flag, records DSA_V32_ERR_DEVICE_WAIT in
 // the workspace status word and both drain to the normal exit.  A parity wait is only issued on a barrier whose previous phase
@@ -126,26 +126,6 @@ struct Ring {
         skip(1);
     }
 };
-
-// tile row -> (query row, head)
-struct RowMap {
-    int q_row, head;
-    bool live;
-};
-__device__ __forceinline__ RowMap map_row(const dsa_v32_work_info& w, int row, int H) {
-    RowMap m;
-    if (w.stacked_rows > 1) {
-        const int sub = row / H;
-        m.q_row = w.q_row + sub;
-        m.head = row - sub * H;
-        m.live = sub < w.stacked_rows;
-    } else {
-        m.q_row = w.q_row;
-        m.head = w.head_block * kHeadsPerBlock + row;
-        m.live = m.head < H;
-    }
-    return m;
-}
 
 __device__ __forceinline__ bool wait_on(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     const uint32_t b = smem_u32(bar);

@@ -68,9 +68,13 @@ inline void enumerate_units(const dsa_v32_shape& sh, std::vector<PlanUnit>& unit
 //   32 rows, whole items of 128: 1.42-1.69   448: 1.02-1.07   800: 0.95-0.99   2048: 0.87
 // A piece of a split item has a cheaper end there (fp32 rows of the live heads only): pieces of 128 slots and more
 //   16 rows: 0.57-0.82   32 rows: 0.82-1.05
-// bf16, against its own 128-row kernel (paired_heads.cu), 4 to 16 items per list:
-//   16 rows, whole items of 192: 1.05-1.15   320: 1.20-1.24   448: 1.05   640: 0.97-1.04   1024: 0.97   2048: 0.87   pieces: 0.71-0.85
-//   32 rows, whole items of 640: 0.90-0.94   800: 1.17   1500: 1.04-1.07   2048: 1.05   pieces: 0.87-1.02 (no line is clear: the fp8 one)
+// bf16, over its own 128-row kernel (paired_heads.cu), both from one build, 1 to 16 items per list, short runs | after 0.8 s of the same
+// launches, when the 128-row kernel, not the few-heads one, has run into the power cap (1965 -> 1300-1900 MHz):
+//   16 rows, whole items of 128: 1.16-1.26 | 1.20-1.27   320: 1.07-1.23 | 1.00-1.12   400: 1.02-1.09 | 0.95-1.02   512: 0.97-1.07 | 0.82-1.02
+//                           640: 0.99-1.03 | 0.87-0.99   1024: 0.91-0.98 | 0.78-0.94   pieces: 0.93-0.98 | 0.93-0.98
+//   32 rows, whole items of 300: 1.38-1.69 | 1.39-1.52   640: 1.30 | 1.10-1.31   1024: 1.15-1.27 | 0.98-1.20   1500: 0.99-1.14 | 0.90-0.99
+//                          2048: 0.99-1.12 | 0.91-0.93   pieces: 1.17-1.24 | 1.18-1.21
+// The line for 17 to 32 rows is that of the fp8 cache; by these figures a bf16 cache wants its own, later one, and none for pieces.
 constexpr int kFewRows16Slots = 160;       // least slots of a whole item of at most 16 rows, on average
 constexpr int kFewRows16SlotsBf16 = 512;   // the same for a bf16 cache
 constexpr int kFewRows32Slots = 768;       // the same for 17 to 32 rows, either cache

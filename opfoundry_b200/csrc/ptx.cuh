@@ -23,9 +23,6 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -178,20 +175,11 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_cluster_f32x4(uint32_t caddr, float a, float b, float c, float d) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(caddr), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
-}
 __device__ __forceinline__ void st_cluster_u32(uint32_t caddr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(caddr), "r"(v) : "memory");
 }
 // Asynchronous 16-byte store into another CTA's shared memory; its arrival is counted (in bytes)
 // on an mbarrier of that CTA, so the receiver needs no fence from the sender.
-__device__ __forceinline__ void st_async_f32x4(uint32_t caddr, float a, float b, float c, float d, uint32_t cbar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(caddr),
-                 "f"(a), "f"(b), "f"(c), "f"(d), "r"(cbar)
-                 : "memory");
-}
 __device__ __forceinline__ void st_async_b32x4(uint32_t caddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t cbar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(caddr),
                  "r"(a), "r"(b), "r"(c), "r"(d), "r"(cbar)
@@ -330,11 +318,6 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// All previously issued tcgen05.mma of this thread arrive (once) on the mbarrier when complete.
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 // 32 lanes x 32-bit, N consecutive columns: thread t of the warp gets lane (base lane + t).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
@@ -391,19 +374,12 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&r)[4]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
-                 :
-                 : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
-                 : "memory");
-}
-// N consecutive columns, N in {8, 16, 32} for loads and {4, 8, 16, 32} for stores
+// N consecutive columns, N in {8, 16, 32}
 template <int N> __device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[N]);
 template <> __device__ __forceinline__ void tmem_ld_n<8>(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8(taddr, r); }
 template <> __device__ __forceinline__ void tmem_ld_n<16>(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 template <> __device__ __forceinline__ void tmem_ld_n<32>(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 template <int N> __device__ __forceinline__ void tmem_st_n(uint32_t taddr, const uint32_t (&r)[N]);
-template <> __device__ __forceinline__ void tmem_st_n<4>(uint32_t taddr, const uint32_t (&r)[4]) { tmem_st4(taddr, r); }
 template <> __device__ __forceinline__ void tmem_st_n<8>(uint32_t taddr, const uint32_t (&r)[8]) { tmem_st8(taddr, r); }
 template <> __device__ __forceinline__ void tmem_st_n<16>(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
 template <> __device__ __forceinline__ void tmem_st_n<32>(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st32(taddr, r); }
@@ -449,29 +425,7 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool b_mn_m
 }
 constexpr uint32_t kIdescATransposed = 1u << 15;   // A is MN-major
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.  accumulate == 0 overwrites D.
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        :
-        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
+// D[tmem] (+)= A * B, A in shared memory (ss) or TMEM (ts), B in shared memory; accumulate == 0 overwrites D.
 // Forms for an issuing warp that stays converged: every lane executes the call, the lane whose
 // `elected` is non-zero issues.  Descriptors then stay warp-uniform values.
 __device__ __forceinline__ void umma_ss_el(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -540,6 +494,7 @@ __device__ __forceinline__ void umma_ss_x4_el(uint32_t d_tmem, uint32_t a_lo, ui
         : "r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates), "r"(elected)
         : "memory");
 }
+// All tcgen05.mma the elected lane has issued arrive (once) on the mbarrier when complete.
 __device__ __forceinline__ void tc_commit_el(uint32_t bar, uint32_t elected) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
@@ -671,15 +626,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2_from2(uint64_t v) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
-}
-// four e4m3 bytes -> four f16 (exact: every e4m3 value is an f16 value; the NaN code stays NaN)
-__device__ __forceinline__ void e4m3x4_to_f16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-    asm("{\n\t.reg .b16 l, h;\n\t"
-        "mov.b32 {l, h}, %2;\n\t"
-        "cvt.rn.f16x2.e4m3x2 %0, l;\n\t"
-        "cvt.rn.f16x2.e4m3x2 %1, h;\n\t}"
-        : "=r"(lo), "=r"(hi)
-        : "r"(w));
 }
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;

@@ -1,9 +1,31 @@
-// Device helpers that both attention kernels use: index translation and the exact e4m3 -> bf16 conversion.
+// Device helpers of the attention kernels: tile rows, index translation and the exact e4m3 -> bf16 conversion.
 #pragma once
 #include "defs.h"
 #include "ptx.cuh"
 
 namespace dsa {
+
+// ------------------------------------------------------------------ tile row -> (query row, head)
+// Tile row r of a work item is head head_block * 128 + r of query row q_row, or, for an item that stacks
+// the query rows of one sequence that share an index list, head r % H of query row q_row + r / H.
+struct RowMap {
+    int q_row, head;
+    bool live;
+};
+__device__ __forceinline__ RowMap map_row(const dsa_v32_work_info& w, int row, int H) {
+    RowMap m;
+    if (w.stacked_rows > 1) {
+        const int sub = row / H;
+        m.q_row = w.q_row + sub;
+        m.head = row - sub * H;
+        m.live = sub < w.stacked_rows;
+    } else {
+        m.q_row = w.q_row;
+        m.head = w.head_block * kHeadsPerBlock + row;
+        m.live = m.head < H;
+    }
+    return m;
+}
 
 // ------------------------------------------------------------------ index translation
 // Top-k slot value -> physical cache row, or -1 when the slot is padding / unusable.  Split in two so

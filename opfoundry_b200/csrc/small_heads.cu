@@ -31,9 +31,9 @@
 // 48 slots; its MMAs take 2 000 of them to issue (36 for the scores of M = 64, N = 16 at 33 cycles, 12 for P V at 62), though
 // the counter has the tensor pipe active for 8 %.
 // Measured against the kernel of sparse_mla.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 219 -> 177 us, 64
-// sequences of 16 heads 79 -> 51, 128 of 32 heads 151 -> 127; bf16, 64 sequences of 16 heads 52 -> 39, prefill of 2048 tokens with
-// 16 heads 661 -> 409, two sequences of 16 heads 15.9 -> 14.7 (the last with the merge).  out against 64 bits: 2.08e-3 (2.10e-3
-// there), lse 2e-7 (7e-7: no 16-bit exchange of partial scores).
+// sequences of 16 heads 79 -> 51, 128 of 32 heads 151 -> 127.  Against paired_heads.cu: bf16, 296 rows of 16 heads x 1024 slots 86.6 -> 78.9,
+// eight sequences of 16 heads x 2048 in pieces 15.1 -> 14.2 with the merge; more shapes beside the rule (few_heads_form in plan.h).
+// out against 64 bits: 2.08e-3 (2.10e-3 in sparse_mla.cu), lse 2e-7 (7e-7: no 16-bit exchange of partial scores).
 //
 // Every mbarrier wait is bounded, as in sparse_mla.cu, and the warps of the softmax group meet on mbarriers only, so a
 // warp that gave up never leaves the others in a hardware barrier.

@@ -46,7 +46,7 @@ def test_decode_bf16_heads(oracle, H):
 
 
 def test_decode_bf16_config1(oracle):
-    """B=2, H=16, kv_len 4096 contiguous per sequence, top-k 2048."""
+    """The small configuration: B=2, H=16, kv_len 4096 contiguous per sequence, top-k 2048."""
     case = synth.make_decode_case(2, 16, 4096, 2048, seed=2026)
     _, _, plan = compare(case, oracle, TOL_BF16)
     assert plan.info.num_partials > 0   # the list is split across CTA pairs and merged
