@@ -501,7 +501,7 @@ def cfg4_leg(env, mode, steps, warmup):
     flops_total = flops_of(pairs_total, c["H"])
     # per GPU: tp keeps every GPU's gathered bytes and divides the flops; batch divides both
     pairs_gpu = float(total_q * c["topk"])
-    roof = roofline_block(flops_of(pairs_gpu, Hl), pairs_gpu * 656.0, ms_attn, pk, "sparse_mla_kernel")
+    roof = roofline_block(flops_of(pairs_gpu, Hl), pairs_gpu * 656.0, ms_attn, pk, "paired_fp8_kernel")
     block = dict(workload="cfg4_%s_decode_fp8_mtp_b%d_sq2_h128_topk2048_kv65536_paged64" % (mode, c["B"]), n_gpus=world,
                  heads_per_gpu=Hl, sequences_per_gpu=nseq, shared_list_fraction=W["share_frac"],
                  ms_per_step=ms_step, ms_per_step_without_gather=ms_attn, ms_per_step_nccl_gather=ms_full,
@@ -657,7 +657,7 @@ def headline_leg(env, args):
                 config=workload_config(),
                 roofline=dict(bound="tensor", achieved=attn_tf, peak=pk["bf16_tflops"], unit="TFLOP/s",
                               frac=attn_tf / pk["bf16_tflops"], traffic=measured_traffic(B),
-                              peak_source=pk["source"], kernel="sparse_mla_kernel", kernel_us=attn_ms * 1e3,
+                              peak_source=pk["source"], kernel="paired_fp8_kernel", kernel_us=attn_ms * 1e3,
                               kernel_us_between_events=attn_events_ms * 1e3,
                               flops_per_launch=step_flops, gathered_bytes_per_launch=gathered,
                               gathered_gbs=gathered / (attn_ms * 1e-3) / 1e9, hbm_peak_gbs=pk["hbm_gbs"],

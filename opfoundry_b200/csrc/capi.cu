@@ -12,10 +12,9 @@
 #include "tmap.h"
 
 namespace dsa {
-int max_resident_pairs(int* out);
+int max_resident_pairs_fp8(int* out);
 int max_resident_pairs_paired(int* out);
-cudaError_t launch_attn(bool ext, int num_lists, const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ttail,
-                        const AttnParams& p, cudaStream_t stream);
+cudaError_t launch_paired_fp8(bool ext, int num_lists, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_small_heads(bool fp8, int tile_rows, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_paired_heads(bool ext, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const int32_t* reduce_indptr,
@@ -89,7 +88,7 @@ Registry& registry() {
 // keeps resident at once, which can be below the SM count when a GPC holds an odd number of SMs.
 int device_sm_count(int* out) {
     int a = 0, b = 0;
-    int rc = max_resident_pairs(&a);
+    int rc = max_resident_pairs_fp8(&a);
     if (rc) return rc;
     rc = max_resident_pairs_paired(&b);
     if (rc) return rc;
@@ -119,7 +118,7 @@ int check_args(const dsa_v32_attn_args* a, int want_dtype, WorkspaceHeader* hdr,
     if (a->stride_q_head < kDQK || a->stride_q_row < int64_t(a->H - 1) * a->stride_q_head + kDQK) return DSA_V32_ERR_SHAPE;
     if (a->stride_o_head < kDV || a->stride_o_row < int64_t(a->H - 1) * a->stride_o_head + kDV) return DSA_V32_ERR_SHAPE;
     if (!(a->sm_scale > 0.0f) || !std::isfinite(a->sm_scale)) return DSA_V32_ERR_SHAPE;
-    // TMA: 16-byte aligned bases and strides; the epilogue stores 16-byte vectors
+    // 16-byte aligned bases and strides: tensor maps of Q and the kernels' 16-byte accesses
     if (!aligned16(a->q) || !aligned16(a->kv) || !aligned16(a->out)) return DSA_V32_ERR_ALIGN;
     if ((a->stride_q_head % 8) || (a->stride_q_row % 8) || (a->stride_o_head % 8) || (a->stride_o_row % 8)) return DSA_V32_ERR_ALIGN;
     if (reinterpret_cast<uintptr_t>(a->workspace) & 255u) return DSA_V32_ERR_ALIGN;
@@ -270,10 +269,8 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         p.pool_split = ext->kv2 ? ext->pool_split : nullptr;
         p.num_kv2_rows = ext->num_kv2_rows;
     }
-    CUtensorMap tq, tkv, ttail;
+    CUtensorMap tq;
     std::memset(&tq, 0, sizeof(tq));
-    std::memset(&tkv, 0, sizeof(tkv));
-    std::memset(&ttail, 0, sizeof(ttail));
     const bool fp8 = want_dtype == DSA_V32_KV_FP8;
     // Few heads: the kernel that puts the slots on the tensor-core tile's rows, where the plan says so (few_heads_form).
     const int few_heads = fp8 ? h.few_heads : h.few_heads_bf16;
@@ -285,29 +282,8 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         cudaError_t e = launch_small_heads(fp8, few_heads, h.num_lists, tq, p, stream);
         return e == cudaSuccess ? DSA_V32_OK : (int)e;
     }
-    if (fp8) {
-        {   // Q: the 64 rope columns of a head block, 128-byte swizzle (the latent columns go to TMEM by plain loads)
-            const uint64_t dims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
-            const uint64_t str[2] = {uint64_t(a->stride_q_head) * 2, uint64_t(a->stride_q_row) * 2};
-            const uint32_t box[3] = {64, uint32_t(a->H < kHeadsPerBlock ? a->H : kHeadsPerBlock), 1};
-            if (tmap_cache().get(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->q, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B))
-                return DSA_V32_ERR_DRIVER;
-        }
-        // the 656-byte rows seen as 164 32-bit elements (a box may then be wider than 256 bytes):
-        // CTA 0 gathers elements [0, 64) = its 256 latent bytes, CTA 1 elements [64, 164) = its 256 latent
-        // bytes + the 16 scale bytes + the 128 rope bytes
-        const uint64_t dims[2] = {uint64_t(kFp8RowBytes / 4), uint64_t(a->num_kv_rows)};
-        const uint64_t str[1] = {uint64_t(kFp8RowBytes)};
-        const uint32_t box_a[2] = {64, 1};
-        const uint32_t box_b[2] = {100, 1};
-        if (tmap_cache().get(&tkv, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, a->kv, dims, str, box_a, CU_TENSOR_MAP_SWIZZLE_NONE))
-            return DSA_V32_ERR_DRIVER;
-        if (tmap_cache().get(&ttail, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, a->kv, dims, str, box_b, CU_TENSOR_MAP_SWIZZLE_NONE))
-            return DSA_V32_ERR_DRIVER;
-    }
-    // 32-byte loads of q and stores of out want rows on 32-byte boundaries; what the checks above admit is 16
-    uintptr_t low = reinterpret_cast<uintptr_t>(a->q) | reinterpret_cast<uintptr_t>(a->out) |
-                    uintptr_t(2 * (a->stride_q_head | a->stride_q_row | a->stride_o_head | a->stride_o_row));
+    // 32-byte stores of out want rows on 32-byte boundaries; what the checks above admit is 16
+    uintptr_t low = reinterpret_cast<uintptr_t>(a->out) | uintptr_t(2 * (a->stride_o_head | a->stride_o_row));
     for (int i = 0; i < p.n_peers; ++i) low |= reinterpret_cast<uintptr_t>(p.out_peers[i]);
     p.wide = (low & 31u) == 0;
     const bool use_ext = !p.wide || h.has_stacked != 0 || p.attn_sink != nullptr || p.kv2 != nullptr || p.n_peers > 0;
@@ -323,7 +299,7 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         cudaError_t e = launch_paired_heads(use_ext, h.num_lists, tq, p, stream);
         return e == cudaSuccess ? DSA_V32_OK : (int)e;
     }
-    cudaError_t e = launch_attn(use_ext, h.num_lists, tq, tkv, ttail, p, stream);
+    cudaError_t e = launch_paired_fp8(use_ext, h.num_lists, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }
 

@@ -57,7 +57,7 @@ struct ReduceDst {
 
 // Kernel parameters (passed by value next to the tensor maps).
 struct AttnParams {
-    const void* kv;    // the cache (read directly for the row scales of an fp8 cache)
+    const void* kv;    // the cache
     const void* q;     // bf16 [total_q][H][576] with the element strides below (read directly for an fp8 cache, else through a tensor map)
     int64_t stride_q_row, stride_q_head;
     const int32_t* indices;
@@ -76,7 +76,7 @@ struct AttnParams {
     int32_t page_shift;  // log2(page_block_size) when that is a power of two, else -1
     float scale_log2;  // sm_scale * log2(e)
     int32_t q_box;     // heads in a box of the tensor map of Q (paired_heads.cu)
-    int32_t wide;      // rows of q and out start on 32-byte boundaries (else they are accessed 16 bytes at a time)
+    int32_t wide;      // rows of out start on 32-byte boundaries (else they are stored 16 bytes at a time)
     // fused all-gather: when n_peers > 0 finished rows go to every peer's gathered buffer instead of out / lse
     int32_t n_peers;
     int64_t lse_stride_row;   // elements between query rows of lse (H without peers)

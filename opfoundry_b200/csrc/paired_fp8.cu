@@ -1,0 +1,858 @@
+// Sparse MLA attention on an fp8 cache for more than 32 tile rows (heads): pair MMAs over the two CTAs of a cluster, the cache's
+// bytes as they are for the scores, dequantised to f16 for the second product.
+//
+// A work item = one query row (or the stacked rows of an MTP group) x up to 128 heads x a slice of its top-k list, as planned in
+// plan.h: an online-softmax attention over the gathered latent rows, K = all 576 columns of a row, V = its first 512 columns
+// (opus_attn/dsa_v32/gfx950/mla_decode_mxfp8_16mx8_32nx1_template.hpp:1362-1490).
+//
+// CTA c of the pair owns tile rows (heads) [64 c, 64 c + 64) and, of every tile of 64 slots, gathers slots [32 c, 32 c + 32).
+//       S_g [128 x 64]  = Q_g K_g^T  cta_group::2, M = 128, N = 64, kind::f8f6f4, one accumulator per 128-column scale group g: B = the
+//                                    gathered e4m3 bytes, A = Q as the sum of two e4m3 numbers (below); the rope with bf16 operands
+//       O [128 x 512] += P V         cta_group::2, M = 128, N = 256, twice, kind::f16 on f16: A = each CTA's 64 rows of P, B = each
+//                                    CTA's 256 columns of all 64 gathered rows, scale x byte rounded once to f16
+// so a CTA holds the whole softmax of its heads: scores, maxima, P and output rows never cross to the other SM.
+//
+// Numbers.  Scores: an element of Q has 8 significant bits, so after a power-of-two factor per row (largest magnitude into
+// [128, 256)) it is hi + lo with both in e4m3, exact down to 2^-10 of the row's largest magnitude and to 2^-18 of that magnitude below;
+// products and sums are those of the bytes themselves, and the scales (fp32) multiply the finished group sums.
+// P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15; V = byte x scale 2^-e
+// with one e for the tile's 64 rows, so that the largest |V| stays below 2^16.  e starts at the exponent of the largest scale of an
+// item's first tile and moves up when a scale exceeds it by 2^7; O is then brought to the new e like it is to a new reference maximum.
+// What falls below f16's smallest step is 2^-33 of the largest V.
+//
+// S in TMEM: lanes 0-63 = the CTA's 64 rows x slots of CTA 0, lanes 64-127 = the same rows x slots of CTA 1.
+// O in TMEM: lanes 0-63 = the rows x columns of CTA 0, lanes 64-127 = the rows x columns of CTA 1.
+//
+// Warp roles (32 warps = eight warpgroups):
+//   warps 0-15   softmax: two teams of eight warps on alternate tiles; thread = (row, quarter of the tile's slots).  A row's four
+//                threads post their maxima; its reference maximum moves, tile after tile, when a tile's maximum exceeds it by more than the
+//                lazy margin of 8 (the reference's threshold: ..16mx4_64nx1_template.hpp:700-725).  P goes to shared memory.  At the change
+//                of an item all sixteen fetch the next one's Q (global -> hi and lo -> shared memory) and read out O
+//   warps 16, 17 CTA 0: score issuers on alternate tiles
+//   warp 18      CTA 0: P V issuer
+//   warp 19      tells the issuers that the CTA's rows of a tile have landed, and follows e
+//   warps 20-23  row loaders: 16-byte cp.async copies into the swizzled tile, eight rows of every tile each, and the own output columns of
+//                eight of the other CTA's rows
+//   warps 24-31  converters: e4m3 -> f16, eight of a tile's rows each
+//
+// What bounds it (cycle stamps of an instrumented copy, 64 sequences x 128 heads x 2048 slots): a tile of 64 slots every 2 780 cycles.  Its MMAs
+// take 1 430 (measured alone; the scores' 25 an instruction are the rate of shared memory, 3 KB of operands each), all its traffic in shared
+// memory 2 100; what is in flight - three raw tiles, one and a half converted ones - over the 10 500 cycles from a load to the end of P V gives the rest:
+// landing 1 900, scores 1 500, softmax 3 100, a converter's turn 2 200.  Every role pays for the number of its instructions, 6 700 a tile and SM:
+// seven or eight warps of a scheduler on five loops miss the instruction cache (4.7 of 19.6 cycles an instruction in a form of 85 KB; a warp number known
+// to be uniform, short waits and rolled loops brought 81 us to 61).  Tried: four teams of four warps with 32 slots a thread (fewer instructions, but
+// a tile takes 5 000 cycles from scores to P: 2 880 a tile), two teams of four (2 750, and 1.5 us more for one sequence), a converter on
+// both units of a tile (3 240).
+// Against the kernel before it (the 576 columns split over the pair, partial scores summed through distributed shared memory in 16 bits, four tile
+// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots: one sequence 19.6 -> 16.8 us, 8192 positions each: 16 33.8 -> 29.0, 37 58.7 -> 43.8,
+// 64 84.4 -> 59.7, 128 161 -> 117; 32768 positions each: 16 35.5 -> 31.0, 64 82.8 -> 65.9.
+// Against 64 bits, six shapes of 40 to 128 heads: out 1.68e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to 2.30e-3),
+// lse at most 1.9e-6 (7e-5).
+//
+// Every mbarrier wait is bounded; on expiry the CTA raises its own and its peer's abort flag, records DSA_V32_ERR_DEVICE_WAIT in
+// the workspace status word and both drain to the normal exit.  A parity wait is only issued on a barrier whose previous phase
+// the waiting warp knows to be complete, and that cannot complete its next one before that warp has looked.
+#include <cuda_bf16.h>
+#include <cfloat>
+#include <cstddef>
+#include <mutex>
+#include "defs.h"
+#include "ptx.cuh"
+#include "rows.cuh"
+
+namespace dsa {
+namespace paired_fp8 {
+
+constexpr int kRows = 64;                          // tile rows (heads) of a CTA
+constexpr int kOwn = 32;                           // slots of a tile that one CTA gathers
+constexpr int kSlots = 2 * kOwn;
+constexpr int kGroups = 4;                         // 128-column scale groups
+constexpr int kBlock = kOwn * 128;                 // 4 096: 128 bytes of 32 rows
+constexpr int kOwnBytes = (kGroups + 1) * kBlock;  // own rows: the four groups, the rope
+constexpr int kRawBytes = kOwnBytes + 2 * kBlock;  // and the own output columns of the other CTA's rows
+constexpr int kStages = 3;                         // raw tiles
+constexpr int kVUnit = 4 * kBlock;                 // 32 slots x 256 columns of f16
+constexpr int kVUnits = 3;                         // a tile takes two
+constexpr int kQBlock = kRows * 128;               // 8 192
+constexpr int kPBytes = kRows * kSlots * 2;        // 8 192
+constexpr int kSoftmaxWarps = 16, kTeamWarps = 8, kScoreWarp = 16, kPvWarp = 18, kReadyWarp = 19, kLoadWarp0 = 20, kLoadWarps = 4;
+constexpr int kConvWarp0 = 24, kConvWarps = 8, kWarps = 32;
+// Registers per thread after the role split: 4 x softmax + issuers + loaders + 2 x converters <= 8 x the launch's 64
+constexpr int kRegsSoftmax = 80, kRegsIssuers = 40, kRegsLoaders = 48, kRegsConv = 48;
+static_assert(4 * kRegsSoftmax + kRegsIssuers + kRegsLoaders + 2 * kRegsConv <= 8 * 64, "more registers than the launch has");
+constexpr float kPShift = 7.0f;                    // P = 2^(score - reference + 7) <= 2^15
+
+constexpr int kOffQ = 0;                           // hi of the four groups, lo of the four groups, rope
+constexpr int kOffRaw = 9 * kQBlock;
+constexpr int kOffV = kOffRaw + kStages * kRawBytes;
+constexpr int kOffP = kOffV + kVUnits * kVUnit;
+constexpr int kOffCtl = kOffP + 2 * kPBytes;
+constexpr int kCtlBytes = 7168;
+constexpr int kSmemBytes = kOffCtl + kCtlBytes;
+static_assert(kSmemBytes <= 232448, "227 KB per CTA");
+// TMEM columns: O 256 | S: groups 0-2 of even tiles, of odd tiles, group 3, rope, 32 columns each
+constexpr uint32_t kColO = 0, kColS = 256, kColS3 = kColS + 6 * 32, kColRope = kColS3 + 32, kTmemCols = 512;
+
+struct Ctl {
+    float scale[kStages][kGroups][kSlots];   // row scales of a tile (0 where the slot holds no row)
+    float post[2][4][kRows];                 // by team and quarter of a tile's slots: the rows' maxima (log2 domain); at the end of an item its row sums
+    float m_ref[2][kRows];                   // by tile number mod 2: the rows' reference maxima after the tile
+    uint8_t q_exp[kRows];                    // biased exponent of 2^a, Q = 2^a (hi + lo); 255: a row with an infinity or a NaN
+    uint32_t tile_mask[kStages][2];          // which slots of CTA 0 / CTA 1 hold a row
+    float v_mul[kStages], v_unit[kStages], v_fix[kStages];   // 2^-e of the tile, 2^e, and 2^(e of the tile before - e)
+    float v_fin;                             // 2^e of the item's last tile
+    uint64_t kv_full[kStages], raw_empty[kStages];     // rows landed | scores complete, rows converted, scales read
+    uint64_t prep[kStages];                            // ... and e known
+    uint64_t tile_ready[2][kStages];                   // CTA 0: both CTAs' rows have landed, by the score issuer (tile number mod 2) that takes the tile
+    uint64_t v_full[kVUnits], v_empty[kVUnits];        // CTA 0: both CTAs have converted the unit | its products are complete
+    uint64_t s_full[2], s_empty[2], s3_empty, p_full[2], pv_done[2];   // s3: group 3 and the rope
+    uint64_t posted[2][2], moved[2][2];      // by team and half of the rows: a tile's maxima are posted | its reference maxima are written and those before it read
+    uint64_t q_here;                         // this CTA's Q and q_exp are written; what the item before left in post, m_ref and v_fin has been read
+    uint64_t q_full, q_empty, o_full, o_free, e_bar;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+static_assert(sizeof(Ctl) <= kCtlBytes && offsetof(Ctl, scale) % 16 == 0, "control block");
+
+// Position in a ring of kN: index and the parity of its current use
+template <int kN>
+struct Ring {
+    uint32_t s = 0, ph = 0;
+    __device__ __forceinline__ void next() {
+        if (++s == kN) {
+            s = 0;
+            ph ^= 1u;
+        }
+    }
+};
+
+__device__ __forceinline__ bool wait_on(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return warp_wait_short(smem_u32(bar), parity, abort_flag);
+}
+__device__ __forceinline__ bool wait_on2(uint64_t* a, uint32_t parity_a, uint64_t* b, uint32_t parity_b, volatile int* abort_flag) {
+    return warp_wait_short2(smem_u32(a), parity_a, smem_u32(b), parity_b, abort_flag);
+}
+__device__ __forceinline__ bool wait_on3(uint64_t* a, uint32_t parity_a, uint64_t* b, uint32_t parity_b, uint64_t* c, uint32_t parity_c, volatile int* abort_flag) {
+    return warp_wait_short3(smem_u32(a), parity_a, smem_u32(b), parity_b, smem_u32(c), parity_c, abort_flag);
+}
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(bar));
+}
+// on the barrier of the same name in the issuing CTA
+__device__ __forceinline__ void warp_arrive_lead(uint64_t* bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(bar), 0));
+}
+
+__device__ __forceinline__ int tiles_of(const dsa_v32_work_info& w) { return (w.k_end - w.k_begin + kSlots - 1) / kSlots; }
+
+// ------------------------------------------------------------------ Q as a sum of two e4m3 numbers
+// Eight bf16 elements times the power of two `mul` -> eight bytes each of hi = e4m3(x) and lo = e4m3(x - hi)
+__device__ __forceinline__ void split_e4m3(const uint4& x, float mul, uint2& hi, uint2& lo) {
+    const uint32_t in[4] = {x.x, x.y, x.z, x.w};
+    uint32_t h[4], l[4];
+    const uint64_t m2 = pack2(mul, mul), neg1 = pack2(-1.0f, -1.0f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint64_t u = mul2(pack2u(in[i] << 16, in[i] & 0xFFFF0000u), m2);
+        float u0, u1;
+        unpack2(u, u0, u1);
+        h[i] = pack_e4m3x2(u0, u1);
+        float h0, h1;
+        unpack_f16x2(e4m3x2_to_f16x2(h[i]), h0, h1);
+        float d0, d1;
+        unpack2(fma2(pack2(h0, h1), neg1, u), d0, d1);
+        l[i] = pack_e4m3x2(d0, d1);
+    }
+    hi = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+    lo = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+}
+
+template <bool kExt>
+__global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnParams p) {
+    extern __shared__ __align__(1024) uint8_t smem_paired_fp8[];   // the same offset in both CTAs of a pair
+    uint8_t* smem = smem_paired_fp8;
+    uint8_t* sQ = smem + kOffQ;
+    uint8_t* sRaw = smem + kOffRaw;
+    uint8_t* sV = smem + kOffV;
+    uint8_t* sP = smem + kOffP;
+    Ctl* ctl = reinterpret_cast<Ctl*>(smem + kOffCtl);
+    volatile int* abort_flag = &ctl->abort_flag;
+    // the warp's number by a shuffle: what depends on it is then known to be the same in all lanes, and loop counters, barrier addresses and
+    // descriptors stay in uniform registers (a score MMA takes 10 instructions instead of 20)
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int list = blockIdx.x >> 1;
+    const int rank = (int)cluster_ctarank(), peer = rank ^ 1;
+    const int w_begin = __ldg(p.list_indptr + list), w_end = __ldg(p.list_indptr + list + 1);
+
+    if (tid < kStages) {
+        mbar_init(smem_u32(&ctl->kv_full[tid]), kLoadWarps * 33);   // the lanes (their copies) and one plain arrival per warp (mask)
+        mbar_init(smem_u32(&ctl->raw_empty[tid]), 1 + kConvWarps + kTeamWarps);   // the scores, the converters, the softmax team
+        mbar_init(smem_u32(&ctl->prep[tid]), 1);
+        mbar_init(smem_u32(&ctl->tile_ready[0][tid]), 2);
+        mbar_init(smem_u32(&ctl->tile_ready[1][tid]), 2);
+        mbar_init(smem_u32(&ctl->v_full[tid]), kConvWarps);   // half of either CTA's converters
+        mbar_init(smem_u32(&ctl->v_empty[tid]), 1);
+        fence_mbar_init();
+    } else if (tid >= 32 && tid < 34) {
+        const int i = tid - 32;
+        mbar_init(smem_u32(&ctl->s_full[i]), 1);
+        mbar_init(smem_u32(&ctl->s_empty[i]), 2 * kTeamWarps);    // one team of either CTA
+        mbar_init(smem_u32(&ctl->p_full[i]), 2 * kTeamWarps);
+        mbar_init(smem_u32(&ctl->pv_done[i]), 1);
+        for (int rq = 0; rq < 2; ++rq) {
+            mbar_init(smem_u32(&ctl->posted[i][rq]), kTeamWarps / 2);
+            mbar_init(smem_u32(&ctl->moved[i][rq]), kTeamWarps / 2);
+        }
+        fence_mbar_init();
+    } else if (tid == 96) {
+        mbar_init(smem_u32(&ctl->s3_empty), 2 * kTeamWarps);
+        mbar_init(smem_u32(&ctl->q_full), 2 * kSoftmaxWarps);   // of either CTA
+        mbar_init(smem_u32(&ctl->q_here), kSoftmaxWarps);
+        mbar_init(smem_u32(&ctl->q_empty), 2);                  // two score issuers
+        mbar_init(smem_u32(&ctl->o_full), 1);
+        mbar_init(smem_u32(&ctl->o_free), 2 * kSoftmaxWarps);
+        mbar_init(smem_u32(&ctl->e_bar), kSoftmaxWarps);
+        ctl->abort_flag = 0;
+        fence_mbar_init();
+    }
+    static_assert(kVUnits == kStages, "one thread per stage and unit");
+    if (warp == kScoreWarp) {
+        tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // the peer's barriers exist before anything is sent to it
+    tc_fence_after();
+    const uint32_t tmem = ctl->tmem_base;
+    grid_dependency_wait();   // everything above may overlap the tail of the kernel before this one
+    const uint32_t peer_abort = map_to_cta(smem_u32(&ctl->abort_flag), peer);
+
+    if (warp < kSoftmaxWarps) {
+        // ============================================================ Q, softmax, epilogue
+        setmaxnreg_inc<kRegsSoftmax>();
+        const int team = warp >> 3, cs = (warp >> 2) & 1, quad = warp & 3;
+        const int h = quad >> 1, rq = quad & 1;        // half of the tile's slots (and of the output columns), half of the CTA's rows
+        const int r = 32 * rq + lane;                  // row of the CTA's 64
+        const uint32_t lane_base = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+        const uint32_t p_lo = smem_u32(sP) + team * kPBytes + r * 128 + (((4 * h + 2 * cs) ^ (r & 7)) << 4);   // 16 slots: this chunk and its neighbour
+        // Q of an item: four rows per warp; lane = columns [8 lane, 8 lane + 8) and the same of the upper 256, of the rope eight lanes a row
+        auto store_q = [&](const dsa_v32_work_info& wi) {
+            const int row0 = 4 * warp;
+            uint4 x[4][2], xr = make_uint4(0u, 0u, 0u, 0u);
+            auto row_ptr = [&](int row, bool& live) {
+                const RowMap rm = map_row(wi, kRows * rank + row, p.H);
+                live = rm.live;
+                return reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)(live ? rm.q_row : wi.q_row) * p.stride_q_row + (size_t)(live ? rm.head : 0) * p.stride_q_head;
+            };
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                bool live;
+                const __nv_bfloat16* src = row_ptr(row0 + i, live) + 8 * lane;
+                x[i][0] = x[i][1] = make_uint4(0u, 0u, 0u, 0u);
+                if (live) {
+                    x[i][0] = __ldg(reinterpret_cast<const uint4*>(src));
+                    x[i][1] = __ldg(reinterpret_cast<const uint4*>(src + 256));
+                }
+            }
+            {
+                bool live;
+                const __nv_bfloat16* src = row_ptr(row0 + (lane >> 3), live) + kDV + 8 * (lane & 7);
+                if (live) xr = __ldg(reinterpret_cast<const uint4*>(src));
+            }
+            float rope_mul = 1.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = row0 + i;
+                uint32_t m = 0u;
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    m = max_u16x2(max_u16x2(max_u16x2(x[i][k].x & 0x7FFF7FFFu, x[i][k].y & 0x7FFF7FFFu),
+                                            max_u16x2(x[i][k].z & 0x7FFF7FFFu, x[i][k].w & 0x7FFF7FFFu)), m);
+                m = __reduce_max_sync(0xffffffffu, max(m >> 16, m & 0xFFFFu));
+                // the largest magnitude into [128, 256)
+                const uint32_t e = max(m >> 7, 64u);
+                const float mul = __uint_as_float((261u - min(e, 254u)) << 23);
+                if ((lane >> 3) == i) rope_mul = mul;
+                if (lane == 0) ctl->q_exp[row] = static_cast<uint8_t>(e == 255u ? 255u : e - 7u);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    uint2 hi, lo;
+                    split_e4m3(x[i][k], mul, hi, lo);
+                    uint8_t* dst = sQ + (2 * k + (lane >> 4)) * kQBlock + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + 8 * (lane & 1);
+                    *reinterpret_cast<uint2*>(dst) = hi;
+                    *reinterpret_cast<uint2*>(dst + kGroups * kQBlock) = lo;
+                }
+            }
+            {
+                const int row = row0 + (lane >> 3);
+                *reinterpret_cast<uint4*>(sQ + 2 * kGroups * kQBlock + row * 128 + (((lane & 7) ^ (row & 7)) << 4)) =
+                    make_uint4(scale_bf16x2(xr.x, rope_mul), scale_bf16x2(xr.y, rope_mul), scale_bf16x2(xr.z, rope_mul), scale_bf16x2(xr.w, rope_mul));
+            }
+            fence_proxy_async_smem();
+            warp_arrive_lead(&ctl->q_full, lane);
+            warp_arrive(&ctl->q_here, lane);
+        };
+        uint32_t it_base = 0;
+        int item_n = 0;
+        Ring<kStages> ring;   // of this team's tiles: every other one
+        if (team) ring.next();
+        float ls = 0.0f, m_out = 0.0f, v_unit = 1.0f;   // of the last item: its row sum, last reference and 2^e
+#pragma unroll 1
+        for (int w = w_begin; w <= w_end; ++w, ++item_n) {
+            // ---- Q of this item, so that its scores can start; then the output of the one before
+            if (w < w_end) {
+                if (item_n > 0)
+                    if (!wait_on(&ctl->q_empty, (item_n - 1) & 1, abort_flag)) goto done;
+                store_q(p.works[w]);
+            }
+            if (item_n > 0) {
+                const dsa_v32_work_info wi = p.works[w - 1];
+                const RowMap rm = map_row(wi, kRows * rank + r, p.H);
+                if (kExt && p.attn_sink != nullptr) {
+                    // attention sink (opus_attn/dsa_v4/common/mla_v4_host.cc:469-472): one more term exp(sink - m) in the
+                    // denominator, counted once per query row and head: in the piece that starts the list
+                    const float sink2 = rm.live ? __ldg(p.attn_sink + rm.head) * 1.4426950408889634f : -INFINITY;
+                    if (m_out == -INFINITY) m_out = sink2;                      // no valid score in this piece: the sink is the reference
+                    if (wi.k_begin == 0 && sink2 > -INFINITY) ls += ex2_approx(sink2 - m_out + kPShift);
+                }
+                const float inv = ls > 0.0f ? v_unit / ls : 0.0f;
+                const float lse_nat = ls > 0.0f ? (m_out - kPShift + __log2f(ls)) * 0.69314718055994531f : INFINITY;
+                if (!wait_on(&ctl->o_full, (item_n - 1) & 1, abort_flag)) goto done;
+                tc_fence_after();
+                // this thread's 64 columns of the row
+                const int col0 = 64 * (warp >> 2);   // of the 256 in its lane
+                if (wi.partial_slot < 0) {
+                    const size_t off = (size_t)rm.q_row * p.stride_o_row + (size_t)rm.head * p.stride_o_head + 256 * h;
+                    const int n_dst = kExt && p.n_peers > 0 ? p.n_peers : 1;
+#pragma unroll 1
+                    for (int oc = col0; oc < col0 + 64; oc += 32) {
+                        uint32_t o[32];
+                        tmem_ld32(lane_base + kColO + oc, o);
+                        tmem_wait_ld();
+                        if (oc != col0) {   // the next item's products may overwrite O
+                            tc_fence_before();
+                            warp_arrive_lead(&ctl->o_free, lane);
+                        }
+                        if (rm.live) {
+                            // thread = row, so a store touches 32 lines whatever its width: 32-byte stores
+                            uint32_t u[16];
+#pragma unroll
+                            for (int v = 0; v < 16; ++v) u[v] = pack_bf16x2(__uint_as_float(o[2 * v]) * inv, __uint_as_float(o[2 * v + 1]) * inv);
+#pragma unroll 1
+                            for (int d = 0; d < n_dst; ++d) {
+                                __nv_bfloat16* o_dst = reinterpret_cast<__nv_bfloat16*>(kExt && p.n_peers > 0 ? p.out_peers[d] : p.out) + off + oc;
+                                stg_32<kExt>(o_dst, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], p.wide);
+                                stg_32<kExt>(o_dst + 16, u[8], u[9], u[10], u[11], u[12], u[13], u[14], u[15], p.wide);
+                            }
+                        }
+                    }
+                    if (rm.live && warp < 2) {   // the rows' first quarter of the left half
+                        const size_t l_off = (size_t)rm.q_row * p.lse_stride_row + rm.head;
+                        if (kExt && p.n_peers > 0) {
+                            for (int d = 0; d < p.n_peers; ++d)
+                                if (p.lse_peers[d] != nullptr) p.lse_peers[d][l_off] = lse_nat;
+                        } else if (p.lse != nullptr) {
+                            p.lse[l_off] = lse_nat;
+                        }
+                    }
+                } else {
+                    float* o_dst = p.o_accum + ((size_t)wi.partial_slot * kHeadsPerBlock + kRows * rank + r) * kDV + 256 * h;
+#pragma unroll 1
+                    for (int oc = col0; oc < col0 + 64; oc += 32) {
+                        uint32_t o[32];
+                        tmem_ld32(lane_base + kColO + oc, o);
+                        tmem_wait_ld();
+                        if (oc != col0) {
+                            tc_fence_before();
+                            warp_arrive_lead(&ctl->o_free, lane);
+                        }
+                        if (rm.live) {
+#pragma unroll
+                            for (int v = 0; v < 4; ++v)
+                                stg_256(o_dst + oc + 8 * v, __float_as_uint(__uint_as_float(o[8 * v + 0]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 1]) * inv),
+                                        __float_as_uint(__uint_as_float(o[8 * v + 2]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 3]) * inv),
+                                        __float_as_uint(__uint_as_float(o[8 * v + 4]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 5]) * inv),
+                                        __float_as_uint(__uint_as_float(o[8 * v + 6]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 7]) * inv));
+                        }
+                    }
+                    if (warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + kRows * rank + r] = ls > 0.0f ? lse_nat : -FLT_MAX;
+                }
+            }
+            if (w == w_end) break;
+            const uint32_t it_end = it_base + tiles_of(p.works[w]);
+            float m_ref = -INFINITY;   // reference maximum after this team's last tile
+            float l = 0.0f;            // this thread's share of the row sum, against m_ref
+            if (!wait_on(&ctl->q_here, item_n & 1, abort_flag)) goto done;
+            const uint32_t q_exp = ctl->q_exp[r];
+            const float c_log2 = p.scale_log2 * __uint_as_float(q_exp == 255u ? 0x7FC00000u : q_exp << 23);   // of scores in units of 2^a
+#pragma unroll 1
+            for (uint32_t it = it_base + ((it_base ^ team) & 1u); it < it_end; it += 2, ring.next(), ring.next()) {
+                const uint32_t ph2 = (it >> 1) & 1u;            // phase of the per-team barriers
+                const bool first = it == it_base;
+                // the tile's mask, scales and e, and its scores (the stage's phase before is complete: its tile was three earlier, and this team has
+                // seen the references move past that tile); the team has read its last tile's maxima
+                if (!wait_on3(&ctl->prep[ring.s], ring.ph, &ctl->s_full[team], ph2, &ctl->moved[team][rq], ph2 ^ 1u, abort_flag)) goto done;
+                tc_fence_after();
+                // ---- scores in units of 2^a: sum_g scale_g S_g + S_rope, in pairs of slots.  Group 3 and the rope, which have one
+                // accumulator for all tiles, first
+                uint64_t sv[8];
+                uint32_t mask;
+                float v_fix;
+                {
+                    const uint32_t ca = lane_base + kColS + 96 * team + 16 * cs;
+                    const float* sc = &ctl->scale[ring.s][0][kOwn * h + 16 * cs];
+                    uint32_t x[2][16], sr[16];
+                    tmem_ld16(lane_base + kColS3 + 16 * cs, x[1]);
+                    tmem_ld16(lane_base + kColRope + 16 * cs, sr);
+                    mask = ctl->tile_mask[ring.s][h] >> (16 * cs);
+                    v_fix = ctl->v_fix[ring.s];
+                    v_unit = ctl->v_unit[ring.s];
+                    tmem_wait_ld();
+                    tmem_loaded(x[1]);
+                    tmem_loaded(sr);
+                    tc_fence_before();
+                    warp_arrive_lead(&ctl->s3_empty, lane);
+#pragma unroll
+                    for (int g = kGroups - 1; g >= 0; --g) {   // the next group's scores are on their way while this one's are scaled
+                        if (g > 0) tmem_ld16(ca + 32 * (g - 1), x[(g - 1) & 1]);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const float4 f = *reinterpret_cast<const float4*>(sc + g * kSlots + 4 * c);
+                            const uint32_t* y = x[g & 1] + 4 * c;
+                            sv[2 * c] = fma2(pack2(f.x, f.y), pack2u(y[0], y[1]), g == kGroups - 1 ? pack2u(sr[4 * c], sr[4 * c + 1]) : sv[2 * c]);
+                            sv[2 * c + 1] = fma2(pack2(f.z, f.w), pack2u(y[2], y[3]), g == kGroups - 1 ? pack2u(sr[4 * c + 2], sr[4 * c + 3]) : sv[2 * c + 1]);
+                        }
+                        if (g > 0) {
+                            tmem_wait_ld();
+                            tmem_loaded(x[(g - 1) & 1]);
+                        }
+                        if (g == 1) {
+                            tc_fence_before();
+                            warp_arrive_lead(&ctl->s_empty[team], lane);
+                        }
+                    }
+                    warp_arrive(&ctl->raw_empty[ring.s], lane);
+                }
+                if ((mask & 0xFFFFu) != 0xFFFFu) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float s0, s1;
+                        unpack2(sv[j], s0, s1);
+                        sv[j] = pack2(((mask >> (2 * j)) & 1u) ? s0 : -INFINITY, ((mask >> (2 * j + 1)) & 1u) ? s1 : -INFINITY);
+                    }
+                }
+                // ---- maximum of this quarter, posted
+                {
+                    float t[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float s0, s1;
+                        unpack2(sv[j], s0, s1);
+                        t[j] = fmaxf(s0, s1);
+                    }
+                    ctl->post[team][2 * h + cs][r] = fmaxf(max3(max3(t[0], t[1], t[2]), t[3], t[4]), max3(t[5], t[6], t[7])) * c_log2;
+                    warp_arrive(&ctl->posted[team][rq], lane);
+                }
+                // ---- P = 2^(score - reference + 7): at most 2^15; a masked slot gives 0.  Taken against the last reference known while
+                // the other maxima are on their way, and again in the rare case that it has moved
+                const float m_was = m_ref;
+                float m_old = -INFINITY;
+                uint32_t pk[8];
+                float lsum = 0.0f;
+                bool settled = false;
+#pragma unroll 1
+                while (true) {
+                    if (settled || !first) {
+                        const float n = kPShift - (m_ref == -INFINITY ? 0.0f : m_ref);
+                        const uint64_t c2 = pack2(c_log2, c_log2), nm2 = pack2(n, n);
+                        uint64_t ls2 = pack2(0.0f, 0.0f);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            float e0, e1;
+                            unpack2(fma2(sv[j], c2, nm2), e0, e1);
+                            e0 = ex2_approx(e0);
+                            e1 = ex2_approx(e1);
+                            ls2 = add2(ls2, pack2(e0, e1));
+                            pk[j] = pack_f16x2(e0, e1);
+                        }
+                        float l0, l1;
+                        unpack2(ls2, l0, l1);
+                        lsum = l0 + l1;
+                    }
+                    if (settled) break;
+                    // the row's reference after the tile before this one, and after this one: it moves when the tile's maximum exceeds it by
+                    // more than the lazy margin
+                    // (before tile 0 the second barrier's phase -1 passes)
+                    if (!wait_on2(&ctl->posted[team][rq], ph2, &ctl->moved[team ^ 1][rq], ((it - 1) >> 1) & 1u, abort_flag)) goto done;
+                    const float mt = fmaxf(fmaxf(ctl->post[team][0][r], ctl->post[team][1][r]), fmaxf(ctl->post[team][2][r], ctl->post[team][3][r]));
+                    if (!first) m_old = ctl->m_ref[team ^ 1][r];
+                    m_ref = mt > m_old + 8.0f ? mt : m_old;
+                    if (h == 0 && cs == 0) ctl->m_ref[team][r] = m_ref;
+                    warp_arrive(&ctl->moved[team][rq], lane);
+                    if (!first && !__any_sync(0xffffffffu, m_ref != m_was)) break;
+                    settled = true;
+                }
+                if (l != 0.0f && m_was != m_ref) l *= ex2_approx(m_was - m_ref);
+                l += lsum;
+                // ---- into the P buffer, once the product that read it last is complete
+                if (it >= 2)
+                    if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) goto done;
+                sts_16(p_lo, pk[0], pk[1], pk[2], pk[3]);
+                sts_16(p_lo ^ 16u, pk[4], pk[5], pk[6], pk[7]);
+                fence_proxy_async_smem();
+                if (!first && __any_sync(0xffffffffu, m_ref != m_old || v_fix != 1.0f)) {
+                    // the reference or e moved: O so far (complete once the previous tile's product is) is brought to the new ones
+                    const float f = (m_old == m_ref ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2_approx(m_old - m_ref))) * v_fix;
+                    if (!wait_on(&ctl->pv_done[team ^ 1], ((it - 1) >> 1) & 1u, abort_flag)) goto done;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int oc = 128 * cs; oc < 128 * cs + 128; oc += 16) {
+                        uint32_t o[16];
+                        tmem_ld16(lane_base + kColO + oc, o);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                        tmem_st16(lane_base + kColO + oc, o);
+                    }
+                    tmem_wait_st();
+                }
+                tc_fence_before();
+                warp_arrive_lead(&ctl->p_full[team], lane);
+            }
+            // ---- the item's sums, last reference and last e
+            const uint32_t last = it_end - 1, last_team = last & 1u;
+            it_base = it_end;
+            if (!wait_on(&ctl->moved[last_team][rq], (last >> 1) & 1u, abort_flag)) goto done;   // the posted maxima have been read, too
+            const float m_fin = ctl->m_ref[last_team][r];
+            if (l != 0.0f && m_ref != m_fin) l *= ex2_approx(m_ref - m_fin);
+            ctl->post[team][2 * h + cs][r] = l;
+            if (team == static_cast<int>(last_team) && (warp & (kTeamWarps - 1)) == 0 && lane == 0) ctl->v_fin = v_unit;
+            warp_arrive(&ctl->e_bar, lane);
+            if (!wait_on(&ctl->e_bar, item_n & 1, abort_flag)) goto done;
+            m_out = m_fin;
+            ls = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ls += ctl->post[i >> 2][i & 3][r];
+            v_unit = ctl->v_fin;
+        }
+    } else if (warp < kLoadWarp0) {
+        setmaxnreg_dec<kRegsIssuers>();
+        if (warp < kPvWarp && rank == 0) {
+            // ======================================================== score issuers, alternate tiles
+            const uint32_t par = warp - kScoreWarp;
+            const uint32_t el = elect_one() ? 1u : 0u;
+            constexpr uint32_t idesc8 = make_idesc_e4m3(128, kSlots), idesc = make_idesc_bf16(128, kSlots, false);
+            const uint64_t q_desc = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
+            const uint64_t k_desc0 = make_smem_desc_sw128(smem_u32(sRaw), 16, 1024);
+            const uint32_t q_lo = static_cast<uint32_t>(q_desc), q_hi = static_cast<uint32_t>(q_desc >> 32);
+            uint32_t it = 0;
+            uint32_t ready_bits = 0;   // parities of this issuer's tile_ready
+            Ring<kStages> ring;
+            int item_n = 0;
+            for (int w = w_begin; w < w_end; ++w, ++item_n) {
+                const int n_tiles = tiles_of(p.works[w]);
+                if (!wait_on(&ctl->q_full, item_n & 1, abort_flag)) goto done;
+                for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
+                    if ((it & 1u) != par) continue;
+                    if (!wait_on(&ctl->tile_ready[par][ring.s], (ready_bits >> ring.s) & 1u, abort_flag)) goto done;
+                    ready_bits ^= 1u << ring.s;
+                    if (it >= 2)
+                        if (!wait_on(&ctl->s_empty[par], ((it >> 1) & 1u) ^ 1u, abort_flag)) goto done;
+                    tc_fence_after();
+                    const uint64_t k_desc = k_desc0 + static_cast<uint64_t>((ring.s * kRawBytes) >> 4);
+                    const uint32_t k_lo = static_cast<uint32_t>(k_desc), k_hi = static_cast<uint32_t>(k_desc >> 32);
+                    const uint32_t d0 = tmem + kColS + 96 * par;
+#pragma unroll 1
+                    for (int g = 0; g < kGroups; ++g) {
+                        if (g == kGroups - 1) {   // group 3 and the rope have one accumulator each: the tile before has been read
+                            if (it >= 1)
+                                if (!wait_on(&ctl->s3_empty, (it - 1) & 1u, abort_flag)) goto done;
+                            tc_fence_after();
+                        }
+                        const uint32_t d = g < kGroups - 1 ? d0 + 32 * g : tmem + kColS3;
+#pragma unroll
+                        for (int v = 0; v < 2; ++v)
+                            umma_pair_f8_ss_x4_el(d, q_lo + (((v * kGroups + g) * kQBlock) >> 4), q_hi, k_lo + ((g * kBlock) >> 4), k_hi, idesc8, v, el);
+                    }
+                    umma_pair_ss_x4_el(tmem + kColRope, q_lo + ((2 * kGroups * kQBlock) >> 4), q_hi, k_lo + ((kGroups * kBlock) >> 4), k_hi, idesc, 0u, el);
+                    tc_commit_pair_el(smem_u32(&ctl->s_full[par]), el);
+                    tc_commit_pair_el(smem_u32(&ctl->raw_empty[ring.s]), el);
+                }
+                tc_commit_pair_el(smem_u32(&ctl->q_empty), el);
+            }
+        } else if (warp == kPvWarp && rank == 0) {
+            // ======================================================== P V issuer
+            const uint32_t el = elect_one() ? 1u : 0u;
+            constexpr uint32_t idesc = make_idesc_f16(128, 256, true);
+            const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(sV), kBlock, 1024);   // MN-major: 64-column blocks kBlock apart
+            const uint64_t p_desc0 = make_smem_desc_sw128(smem_u32(sP), 16, 1024);
+            uint32_t it = 0;
+            Ring<kVUnits> unit;
+            int item_n = 0;
+            for (int w = w_begin; w < w_end; ++w, ++item_n) {
+                const int n_tiles = tiles_of(p.works[w]);
+                for (int t = 0; t < n_tiles; ++t, ++it) {
+                    const uint32_t sb = it & 1u;
+                    const uint64_t p_desc = p_desc0 + static_cast<uint64_t>((sb * kPBytes) >> 4);
+                    if (t == 0 && item_n > 0)   // the previous item's O has been read out
+                        if (!wait_on(&ctl->o_free, (item_n - 1) & 1, abort_flag)) goto done;
+                    if (!wait_on(&ctl->p_full[sb], (it >> 1) & 1u, abort_flag)) goto done;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u, unit.next()) {   // slots of CTA 0, of CTA 1
+                        if (!wait_on(&ctl->v_full[unit.s], unit.ph, abort_flag)) goto done;
+                        tc_fence_after();
+                        const uint64_t v_desc = v_desc0 + static_cast<uint64_t>((unit.s * kVUnit) >> 4);
+#pragma unroll
+                        for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+                            for (int j = 0; j < 2; ++j)
+                                umma_pair_ss_el(tmem + kColO + 128 * j, p_desc + static_cast<uint64_t>((2 * u + ks) * 2),
+                                                v_desc + static_cast<uint64_t>((2 * j * kBlock + ks * 2048) >> 4), idesc, (t > 0 || u > 0 || ks > 0) ? 1u : 0u, el);
+                        tc_commit_pair_el(smem_u32(&ctl->v_empty[unit.s]), el);
+                    }
+                    tc_commit_pair_el(smem_u32(&ctl->pv_done[sb]), el);
+                    if (t + 1 == n_tiles) tc_commit_pair_el(smem_u32(&ctl->o_full), el);
+                }
+            }
+        } else if (warp == kReadyWarp) {
+            // ======================================================== this CTA's rows' arrival, passed on to the issuers; e
+            uint32_t it = 0;
+            Ring<kStages> ring;
+            for (int w = w_begin; w < w_end; ++w) {
+                const int n_tiles = tiles_of(p.works[w]);
+                int e = 0;
+                for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
+                    if (!wait_on(&ctl->kv_full[ring.s], ring.ph, abort_flag)) goto done;
+                    fence_proxy_async_smem();   // written by cp.async (generic proxy)
+                    warp_arrive_lead(&ctl->tile_ready[it & 1u][ring.s], lane);
+                    // largest finite scale of the tile's rows (of both CTAs' slots and all groups, so both CTAs follow the same e)
+                    uint32_t m = 0u;
+#pragma unroll
+                    for (int g = 0; g < kGroups; ++g) {
+                        const float2 s = *reinterpret_cast<const float2*>(&ctl->scale[ring.s][g][2 * lane]);
+                        const uint32_t a = __float_as_uint(s.x) & 0x7FFFFFFFu, b = __float_as_uint(s.y) & 0x7FFFFFFFu;
+                        m = max(m, max(a < 0x7F800000u ? a : 0u, b < 0x7F800000u ? b : 0u));
+                    }
+                    m = __reduce_max_sync(0xffffffffu, m);
+                    const int em = max(static_cast<int>(m >> 23) - 127, -120);
+                    const int e_old = e;
+                    if (t == 0 || em >= e + 7) e = min(em, 126);
+                    if (lane == 0) {
+                        ctl->v_mul[ring.s] = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+                        ctl->v_unit[ring.s] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+                        const int d = t == 0 ? 0 : e_old - e;
+                        ctl->v_fix[ring.s] = d < -126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 + d) << 23);
+                    }
+                    warp_arrive(&ctl->prep[ring.s], lane);
+                }
+            }
+        }
+    } else if (warp < kConvWarp0) {
+        // ============================================================ row loaders: eight rows of every tile per warp, four lanes per row
+        setmaxnreg_dec<kRegsLoaders>();
+        const int lw = warp - kLoadWarp0;
+        const int r = 8 * lw + (lane >> 2), c4 = lane & 3;   // of the copies
+        const uint8_t* kv_bytes = reinterpret_cast<const uint8_t*>(p.kv);
+        // lanes 0-7 follow the slots of the warp's own rows in even tiles, 8-15 the same slots of the other CTA, 16-31 those of odd tiles:
+        // a slot is translated once, two tiles at a time
+        const int slot = kSlots * (lane >> 4) + kOwn * ((lane >> 3 & 1) ? peer : rank) + 8 * lw + (lane & 7);
+        const uint32_t d0 = smem_u32(sRaw) + r * 128 + ((c4 ^ (r & 7)) << 4), d1 = d0 ^ 64u;   // chunks 8 j + c4 and 8 j + 4 + c4
+        const uint32_t scale_own = smem_u32(&ctl->scale[0][c4][kOwn * rank + r]), scale_late = smem_u32(&ctl->scale[0][c4][kOwn * peer + r]);
+        Ring<kStages> ring;   // of raw_empty: one use behind
+        ring.ph = 1u;
+        for (int w = w_begin; w < w_end; ++w) {
+            const dsa_v32_work_info wi = p.works[w];
+            const int n_tiles = tiles_of(wi);
+            const int seq = wi.q_row / p.s_q;
+            const int32_t* idx_row = p.indices + (size_t)wi.q_row * p.topk;
+            auto load_slot = [&](int u) -> int {
+                const int k = wi.k_begin + u * kSlots + slot;
+                return (k < wi.k_end) ? __ldg(idx_row + k) : -1;
+            };
+            // rows are known two tiles ahead (and asked into L2), block numbers loaded four, slots six
+            auto ask = [&](int row) {
+                if ((lane & 8) == 0 && row >= 0) bulk_prefetch_l2(kv_bytes + (size_t)row * kFp8RowBytes, kFp8RowBytes);
+            };
+            int idx_a = load_slot(0), idx_b = load_slot(2), idx_c = load_slot(4);
+            int phys_a = block_of(idx_a, seq, p), phys_b = block_of(idx_b, seq, p);
+            int row_n = row_of(idx_a, phys_a, seq, p);
+#pragma unroll 1
+            for (int u = 0; u < n_tiles; u += 2) {
+                const int row = row_n;
+                row_n = row_of(idx_b, phys_b, seq, p);
+                ask(row_n);
+                idx_b = idx_c;
+                phys_b = block_of(idx_b, seq, p);
+                idx_c = load_slot(u + 6);
+                const uint32_t used = __ballot_sync(0xffffffffu, row != -1);
+#pragma unroll 1
+                for (int t = 0; t < 2 && u + t < n_tiles; ++t, ring.next()) {
+                    const int own = __shfl_sync(0xffffffffu, row, 16 * t + (lane >> 2)), late = __shfl_sync(0xffffffffu, row, 16 * t + 8 + (lane >> 2));
+                    if (!wait_on(&ctl->raw_empty[ring.s], ring.ph, abort_flag)) goto done;
+                    if (lane < 2) reinterpret_cast<uint8_t*>(&ctl->tile_mask[ring.s][lane ? peer : rank])[lw] = static_cast<uint8_t>(used >> (16 * t + 8 * lane));
+                    // padding and out-of-range rows: nothing is read, the row is zeros
+                    const uint32_t st = ring.s * kRawBytes, sc = ring.s * (kGroups * kSlots * 4);
+                    {
+                        const uint8_t* src = kv_bytes + (size_t)(own < 0 ? 0 : own) * kFp8RowBytes;
+                        const uint32_t n = own != -1 ? 16u : 0u;
+                        cp_async_4(scale_own + sc, src + kDV + 4 * c4, n >> 2);
+                        src += 16 * c4;
+#pragma unroll
+                        for (int j = 0; j < 5; ++j) {   // four blocks of latent columns; the rope, after 16 bytes of scales
+                            cp_async_16(d0 + st + j * kBlock, src + 128 * j + (j == 4 ? 16 : 0), n);
+                            cp_async_16(d1 + st + j * kBlock, src + 128 * j + (j == 4 ? 16 : 0) + 64, n);
+                        }
+                    }
+                    {
+                        const uint8_t* src = kv_bytes + (size_t)(late < 0 ? 0 : late) * kFp8RowBytes;
+                        const uint32_t n = late != -1 ? 16u : 0u;
+                        cp_async_4(scale_late + sc, src + kDV + 4 * c4, n >> 2);
+                        src += rank * kDvHalf + 16 * c4;
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            cp_async_16(d0 + st + kOwnBytes + j * kBlock, src + 128 * j, n);
+                            cp_async_16(d1 + st + kOwnBytes + j * kBlock, src + 128 * j + 64, n);
+                        }
+                    }
+                    cp_async_mbar_arrive_noinc(smem_u32(&ctl->kv_full[ring.s]));
+                    warp_arrive(&ctl->kv_full[ring.s], lane);
+                }
+            }
+        }
+    } else {
+        // ============================================================ converters: this CTA's 256 output columns of all 64 rows, to f16
+        setmaxnreg_dec<kRegsConv>();
+        // Warps 0-3 take the slots of CTA 0 (unit 0 of a tile), warps 4-7 those of CTA 1, eight rows each.  Sixteen columns a lane and step: one
+        // 16-byte chunk of a raw row, two of a row of V.  A quarter of a warp takes half of the block's columns of one row and the other half of its
+        // neighbour's, so that its loads and its stores touch every bank once.
+        const int cw = warp - kConvWarp0, u = cw >> 2;
+        const int r4 = 2 * (lane >> 4) + ((lane >> 2) & 1), half = ((lane >> 3) ^ (lane >> 2)) & 1, k = lane & 3;
+        const int r = 8 * (cw & 3) + r4;   // of the first two steps; the others take the row four further
+        const uint32_t raw0 = smem_u32(sRaw) + (u == rank ? 2 * rank * kBlock : kOwnBytes) + r * 128 + (((4 * half + k) ^ (r & 7)) << 4);
+        const uint32_t v0 = smem_u32(sV) + half * kBlock + r * 128 + (((2 * k) ^ (r & 7)) << 4);
+        // lane i < 16 (and i + 16): the scale of block i / 8, row i % 8
+        const float* const scale0 = &ctl->scale[0][2 * rank + ((lane >> 3) & 1)][kOwn * u + 8 * (cw & 3) + (lane & 7)];
+        Ring<kStages> ring;
+        Ring<kVUnits> unit;   // of v_empty: one use behind
+        unit.ph = 1u;
+        if (u) unit.next();
+        for (int w = w_begin; w < w_end; ++w) {
+            const int n_tiles = tiles_of(p.works[w]);
+#pragma unroll 1
+            for (int t = 0; t < n_tiles; ++t, ring.next(), unit.next(), unit.next()) {
+                if (!wait_on2(&ctl->prep[ring.s], ring.ph, &ctl->v_empty[unit.s], unit.ph, abort_flag)) goto done;
+                const uint32_t scales = split_f16(scale0[ring.s * (kGroups * kSlots)] * ctl->v_mul[ring.s]);   // as a sum of two f16
+                uint32_t src = raw0 + ring.s * kRawBytes, dst = v0 + unit.s * kVUnit;
+                uint4 x[2] = {lds_16(src), lds_16(src + kBlock)};
+#pragma unroll 1
+                for (int i = 0; i < 2; ++i) {   // row r, row r + 4: a short loop, see warp_wait_short
+                    const uint4 in[2] = {x[0], x[1]};
+                    src = (src ^ 64u) + 512u;   // four rows on, and bit 2 of the swizzle flips
+                    if (i == 0) {
+                        x[0] = lds_16(src);
+                        x[1] = lds_16(src + kBlock);
+                    } else {
+                        warp_arrive(&ctl->raw_empty[ring.s], lane);
+                    }
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const uint32_t s = __shfl_sync(0xffffffffu, scales, 8 * b + 4 * i + r4);
+                        const uint32_t hi = __byte_perm(s, 0, 0x1010), lo = __byte_perm(s, 0, 0x3232);
+                        const uint32_t v[4] = {in[b].x, in[b].y, in[b].z, in[b].w};
+                        uint32_t y[8];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            y[2 * j] = scale_f16x2(e4m3x2_to_f16x2(v[j]), hi, lo);
+                            y[2 * j + 1] = scale_f16x2(e4m3x2_to_f16x2(v[j] >> 16), hi, lo);
+                        }
+                        sts_16(dst + 2 * b * kBlock, y[0], y[1], y[2], y[3]);
+                        sts_16((dst ^ 16u) + 2 * b * kBlock, y[4], y[5], y[6], y[7]);
+                    }
+                    dst = (dst ^ 64u) + 512u;
+                }
+                fence_proxy_async_smem();
+                warp_arrive_lead(&ctl->v_full[unit.s], lane);
+            }
+        }
+    }
+
+done:
+    if (ctl->abort_flag) st_cluster_u32(peer_abort, 1u);   // let the peer stop waiting for us
+    tc_fence_before();
+    __syncthreads();
+    if (ctl->abort_flag) {   // a wait gave up; nothing more is issued here, and the peer stays at the barrier below meanwhile
+        if (tid == 0) atomicExch(p.status, DSA_V32_ERR_DEVICE_WAIT);
+        settle_in_flight();
+    }
+    cluster_sync_all();   // nothing is on its way to either CTA any more
+    if (warp == kScoreWarp) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem, kTmemCols);
+    }
+}
+
+// The opt-in for more than 48 KB of dynamic shared memory is a per-device attribute of the kernel.
+template <bool kExt>
+static cudaError_t configure() {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> guard(mu);
+    if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+    e = cudaFuncSetAttribute(paired_fp8_kernel<kExt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) done[dev] = true;
+    return cudaSuccess;
+}
+
+static void fill_launch(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int num_lists, cudaStream_t stream) {
+    cfg->gridDim = dim3(2 * num_lists, 1, 1);
+    cfg->blockDim = dim3(32 * kWarps, 1, 1);
+    cfg->dynamicSmemBytes = kSmemBytes;
+    cfg->stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 2;
+}
+
+template <bool kExt>
+static cudaError_t launch(int num_lists, const AttnParams& p, cudaStream_t stream) {
+    cudaError_t e = configure<kExt>();
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    fill_launch(&cfg, attr, num_lists, stream);
+    return cudaLaunchKernelEx(&cfg, paired_fp8_kernel<kExt>, p);
+}
+
+}  // namespace paired_fp8
+
+int max_resident_pairs_fp8(int* out) {
+    cudaError_t e = paired_fp8::configure<false>();
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    paired_fp8::fill_launch(&cfg, attr, 1, nullptr);
+    e = cudaOccupancyMaxActiveClusters(&n, paired_fp8::paired_fp8_kernel<false>, &cfg);
+    if (e != cudaSuccess) return (int)e;
+    *out = n;
+    return 0;
+}
+
+// ext: a sink or peers are given, or rows of out are aligned to 16 bytes only
+cudaError_t launch_paired_fp8(bool ext, int num_lists, const AttnParams& p, cudaStream_t stream) {
+    return ext ? paired_fp8::launch<true>(num_lists, p, stream) : paired_fp8::launch<false>(num_lists, p, stream);
+}
+
+}  // namespace dsa

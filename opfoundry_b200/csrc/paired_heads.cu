@@ -1,4 +1,4 @@
-// Sparse MLA attention for more than 32 tile rows (heads): one tcgen05 pair MMA over the two CTAs of a cluster.
+// Sparse MLA attention on a bf16 cache for more than 32 tile rows (heads): one tcgen05 pair MMA over the two CTAs of a cluster.
 //
 // A work item = one query row (or the stacked rows of an MTP group) x up to 128 heads x a slice of its top-k list, as planned in
 // plan.h: an online-softmax attention over the gathered latent rows, K = all 576 columns of a row, V = its first 512 columns
@@ -39,7 +39,7 @@
 // its MMAs; a change of item costs 7 800 more (the score MMAs of the next item wait 2 700 for its Q, its first product 4 900 for the
 // stores of O), a sixth of an item of 32 tiles.  One score issuer instead of two: 2 050 cycles a tile.  Arrivals at the issuing CTA with a
 // release at cluster scope: 2 970.  Q by 32-byte loads into TMEM instead of TMA and the ring: 14 000 cycles a change of item.
-// Against a pair that splits the 576 columns and sums partial scores over distributed shared memory (kept for the fp8 cache), in
+// Against a pair that splits the 576 columns and sums partial scores over distributed shared memory, in
 // long runs (the power cap): prefill of 4096 tokens x 128 heads 2260 -> 1656 us, 1268 tokens x 64 heads after 1733 642 -> 483, 1024
 // tokens with sink and second pool, 640 slots, 293 -> 215.
 //

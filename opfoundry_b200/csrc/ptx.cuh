@@ -1,6 +1,6 @@
 // Thin inline-PTX wrappers for the sm_100a features the sparse-MLA kernels use:
-// mbarrier (with bounded waits), TMA tile loads and tile::gather4 row gathers into this CTA's
-// shared memory, tcgen05 MMA / TMEM alloc / ld / st / commit, and the shared-memory and
+// mbarrier (with bounded waits), TMA tile loads into this CTA's shared memory,
+// tcgen05 MMA / TMEM alloc / ld / st / commit, and the shared-memory and
 // instruction descriptors tcgen05.mma consumes.
 #pragma once
 #include <cstdint>
@@ -84,12 +84,16 @@ __device__ __forceinline__ uint64_t global_ns() {
 #ifndef DSA_WAIT_HINT_NS
 #define DSA_WAIT_HINT_NS 20000u        // one parked try_wait
 #endif
+#ifndef DSA_WAIT_PARKS
+#define DSA_WAIT_PARKS 500000u         // the bound of warp_wait_short: a parked try_wait gives up after 4 us (measured, whatever the hint), so two seconds
+#endif
 #ifndef DSA_WAIT_BUDGET_NS
 #define DSA_WAIT_BUDGET_NS 2000000000ull
 #endif
 __device__ __forceinline__ bool mbar_wait_budget(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t budget_ns) {
     if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = global_ns();
+#pragma unroll 1
     for (uint32_t it = 0; it < DSA_WAIT_LIMIT; ++it) {
         if (mbar_try_wait_hint(bar, parity, DSA_WAIT_HINT_NS)) return true;
         if (*abort_flag) return false;
@@ -109,6 +113,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 #endif
 __device__ __forceinline__ void settle_in_flight() {
     const uint64_t t0 = global_ns();
+#pragma unroll 1
     for (uint32_t it = 0; it < DSA_WAIT_LIMIT && global_ns() - t0 < DSA_SETTLE_NS; ++it) {
     }
 }
@@ -119,16 +124,86 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// The same in few instructions, for code whose size counts (seven warps of a scheduler on five different loops miss the instruction
+// cache): the bound is a number of parked waits instead of a time.
+__device__ __forceinline__ bool mbar_try_wait_all(uint32_t bar, uint32_t parity) {   // parked as above; what the whole warp has seen
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(DSA_WAIT_HINT_NS)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool warp_wait_short(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+    for (uint32_t n = 0; !mbar_try_wait_all(bar, parity); ++n) {
+        if (*abort_flag) return false;
+        if (n > DSA_WAIT_PARKS) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
+}
+
+// Three barriers at once: none can leave its phase before this warp has gone on.
+__device__ __forceinline__ bool warp_wait_short3(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b, uint32_t bar_c, uint32_t parity_c,
+                                                 volatile int* abort_flag) {
+    uint32_t ok;
+#pragma unroll 1
+    for (uint32_t n = 0;; ++n) {
+        asm volatile(
+            "{\n\t.reg .pred p, q, r;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %7;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4, %7;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 r, [%5], %6, %7;\n\t"
+            "and.pred p, p, q;\n\t"
+            "and.pred p, p, r;\n\t"
+            "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+            "selp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(ok)
+            : "r"(bar_a), "r"(parity_a), "r"(bar_b), "r"(parity_b), "r"(bar_c), "r"(parity_c), "r"(DSA_WAIT_HINT_NS)
+            : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+        if (n > DSA_WAIT_PARKS) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
+
+// Two barriers at once: neither can leave its phase before this warp has gone on.
+__device__ __forceinline__ bool warp_wait_short2(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b, volatile int* abort_flag) {
+    uint32_t ok;
+#pragma unroll 1
+    for (uint32_t n = 0;; ++n) {
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %5;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4, %5;\n\t"
+            "and.pred p, p, q;\n\t"
+            "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+            "selp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(ok)
+            : "r"(bar_a), "r"(parity_a), "r"(bar_b), "r"(parity_b), "r"(DSA_WAIT_HINT_NS)
+            : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+        if (n > DSA_WAIT_PARKS) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
+
 // Programmatic dependent launch: blocks until the kernels this one depends on have completed and their
 // writes are visible (a no-op when the kernel was launched without the attribute).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// 32-byte read-only global load (sm_100: one request per lane where two 16-byte loads would make two).
-__device__ __forceinline__ void ldg_nc_256(const void* p, uint32_t (&r)[8]) {
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "l"(p));
-}
 
 // 16-byte read-only global load that does not allocate in L1 (a gathered row is read once per SM).
 __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
@@ -144,15 +219,6 @@ __device__ __forceinline__ void stg_256(void* p, uint32_t a, uint32_t b, uint32_
 }
 
 // The same for addresses that may be aligned to 16 bytes only; kMaybe = false: the caller knows that they are not.
-template <bool kMaybe> __device__ __forceinline__ void ldg_nc_32(const void* p, uint32_t (&r)[8], bool wide) {
-    if (!kMaybe || wide) {
-        ldg_nc_256(p, r);
-    } else {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
-        r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
-        r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
-    }
-}
 template <bool kMaybe>
 __device__ __forceinline__ void stg_32(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f, uint32_t g, uint32_t h, bool wide) {
     if (!kMaybe || wide) {
@@ -225,6 +291,7 @@ __device__ __forceinline__ bool mbar_try_wait_cluster_hint(uint32_t bar, uint32_
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     const uint64_t t0 = global_ns();
+#pragma unroll 1
     for (uint32_t it = 0; it < DSA_WAIT_LIMIT; ++it) {
         if (mbar_try_wait_cluster_hint(bar, parity, DSA_WAIT_HINT_NS)) return true;
         if (*abort_flag) return false;
@@ -262,19 +329,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, 
         : "memory");
 }
 
-// Four rows of a 2-D tensor, each with its own row coordinate, one shared column coordinate.
-// The tensor map's box is (width, 1).  `col * element size` must be a multiple of 16 bytes.
-// A row coordinate outside the tensor fills its row of the destination with zeros.
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* m, uint32_t bar, int col, int r0, int r1,
-                                            int r2, int r3) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-        :
-        : "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-        : "memory");
-}
-
 // Asks for `bytes` bytes (a multiple of 16, 16-byte aligned) to be brought into L2.
 __device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
@@ -288,6 +342,14 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src, uint32
 }
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ uint4 lds_16(uint32_t src) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_16(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
@@ -384,6 +446,12 @@ template <> __device__ __forceinline__ void tmem_st_n<8>(uint32_t taddr, const u
 template <> __device__ __forceinline__ void tmem_st_n<16>(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
 template <> __device__ __forceinline__ void tmem_st_n<32>(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st32(taddr, r); }
 
+// Ties values that tcgen05.ld delivers to the wait before this, where other work stands between the load and the wait.
+__device__ __forceinline__ void tmem_loaded(uint32_t (&r)[16]) {
+    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
+                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
+}
+
 // ------------------------------------------------------------------ tcgen05.mma
 // Shared-memory matrix descriptor, 128-byte swizzle: start address, leading / stride byte
 // offsets (all >> 4), descriptor version 1 (bits 46-47), swizzle mode 2 = 128B (bits 61-63).
@@ -423,6 +491,9 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool b_mn_m
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) |
            (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
 }
+// The same for f16 A and B, and for kind::f8f6f4 with e4m3 A and B (both K-major).
+__host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, bool b_mn_major) { return make_idesc_bf16(M, N, b_mn_major) & ~((1u << 7) | (1u << 10)); }
+__host__ __device__ constexpr uint32_t make_idesc_e4m3(int M, int N) { return make_idesc_f16(M, N, false); }
 constexpr uint32_t kIdescATransposed = 1u << 15;   // A is MN-major
 
 // D[tmem] (+)= A * B, A in shared memory (ss) or TMEM (ts), B in shared memory; accumulate == 0 overwrites D.
@@ -439,42 +510,12 @@ __device__ __forceinline__ void umma_ss_el(uint32_t d_tmem, uint64_t a_desc, uin
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
-__device__ __forceinline__ void umma_ts_el(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate, uint32_t elected) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        :
-        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
-        : "memory");
-}
 // Four MMAs of one 64-column block (K = 16 each) in one piece of assembly: the election predicate is
 // set up once and the operands of the steps differ by immediates (A: +8 TMEM columns or +32 bytes,
 // B: +32 bytes = +2 in descriptor units), so a step costs the issuing warp three instructions instead
 // of eight.  `first_accumulates` = 0 lets the first step overwrite D.  b_lo / b_hi (a_lo / a_hi): the two
 // halves of the shared-memory descriptor; adding to the low half cannot carry out of its 14-bit address
 // field because shared memory ends below 2^18 bytes.
-__device__ __forceinline__ void umma_ts_x4_el(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                                              uint32_t first_accumulates, uint32_t elected) {
-    asm volatile(
-        "{\n\t.reg .pred q, pt, pf;\n\t.reg .b32 a, l;\n\t.reg .b64 bd;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "setp.ne.b32 pf, %5, 0;\n\t"
-        "setp.eq.b32 pt, %6, %6;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, pf;\n\t"
-        "add.u32 a, %1, 8;\n\tadd.u32 l, %2, 2;\n\tmov.b64 bd, {l, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %4, pt;\n\t"
-        "add.u32 a, %1, 16;\n\tadd.u32 l, %2, 4;\n\tmov.b64 bd, {l, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %4, pt;\n\t"
-        "add.u32 a, %1, 24;\n\tadd.u32 l, %2, 6;\n\tmov.b64 bd, {l, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %4, pt;\n\t}"
-        :
-        : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates), "r"(elected)
-        : "memory");
-}
 __device__ __forceinline__ void umma_ss_x4_el(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                               uint32_t idesc, uint32_t first_accumulates, uint32_t elected) {
     asm volatile(
@@ -577,6 +618,26 @@ __device__ __forceinline__ void umma_pair_ss_x4_el(uint32_t d_tmem, uint32_t a_l
         : "r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates), "r"(elected)
         : "memory");
 }
+// four K = 32 steps of one block of 128 e4m3 columns
+__device__ __forceinline__ void umma_pair_f8_ss_x4_el(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                                   uint32_t idesc, uint32_t first_accumulates, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred q, pt, pf;\n\t.reg .b32 la, lb;\n\t.reg .b64 ad, bd;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "setp.ne.b32 pf, %6, 0;\n\t"
+        "setp.eq.b32 pt, %7, %7;\n\t"
+        "mov.b64 ad, {%1, %2};\n\tmov.b64 bd, {%3, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], ad, bd, %5, pf;\n\t"
+        "add.u32 la, %1, 2;\n\tadd.u32 lb, %3, 2;\n\tmov.b64 ad, {la, %2};\n\tmov.b64 bd, {lb, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], ad, bd, %5, pt;\n\t"
+        "add.u32 la, %1, 4;\n\tadd.u32 lb, %3, 4;\n\tmov.b64 ad, {la, %2};\n\tmov.b64 bd, {lb, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], ad, bd, %5, pt;\n\t"
+        "add.u32 la, %1, 6;\n\tadd.u32 lb, %3, 6;\n\tmov.b64 ad, {la, %2};\n\tmov.b64 bd, {lb, %4};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], ad, bd, %5, pt;\n\t}"
+        :
+        : "r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates), "r"(elected)
+        : "memory");
+}
 
 // ------------------------------------------------------------------ small helpers
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
@@ -625,6 +686,45 @@ __device__ __forceinline__ uint32_t pack_bf16x2_from2(uint64_t v) {
     unpack2(v, lo, hi);
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// e4m3 (saturating, to nearest even) and f16, two at a time: element 0 in the low half
+__device__ __forceinline__ uint32_t pack_e4m3x2(float lo, float hi) {
+    uint32_t r;
+    asm("{\n\t.reg .b16 t;\n\tcvt.rn.satfinite.e4m3x2.f32 t, %1, %2;\n\tmov.b32 %0, {t, 0};\n\t}" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t v) {   // the two low bytes; exact
+    uint32_t r;
+    asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, a;\n\t}" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ void unpack_f16x2(uint32_t v, float& lo, float& hi) {
+    asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.f32.f16 %0, a;\n\tcvt.f32.f16 %1, b;\n\t}" : "=f"(lo), "=f"(hi) : "r"(v));
+}
+// s = hi + lo in f16, hi in the low half: 22 significant bits
+__device__ __forceinline__ uint32_t split_f16(float s) {
+    const uint32_t hi = pack_f16x2(s, s);
+    float a, b;
+    unpack_f16x2(hi, a, b);
+    return pack_f16x2(a, s - a);
+}
+// v (hi + lo): the product with lo is small, so the sum is rounded once for all that matters
+__device__ __forceinline__ uint32_t scale_f16x2(uint32_t v, uint32_t hi, uint32_t lo) {
+    uint32_t r;
+    asm("{\n\t.reg .b32 t;\n\tmul.rn.f16x2 t, %1, %3;\n\tfma.rn.f16x2 %0, %1, %2, t;\n\t}" : "=r"(r) : "r"(v), "r"(hi), "r"(lo));
+    return r;
+}
+// two bf16 times a power of two
+__device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float mul) { return pack_bf16x2(__uint_as_float(v << 16) * mul, __uint_as_float(v & 0xFFFF0000u) * mul); }
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
 __device__ __forceinline__ float ex2_approx(float x) {

@@ -1,7 +1,7 @@
 // Sparse MLA attention for few heads: work items of at most 32 tile rows (16 or 32 heads of a head-sharded
 // deployment, or the stacked rows of an MTP pair) that hold enough slots on average (few_heads_form in plan.h).
 //
-// The kernel in sparse_mla.cu puts the heads on the 128 rows of the tensor-core tile, so an item of 16 heads pays
+// The 128-row kernels put the heads on the 128 rows of the tensor-core tile, so an item of 16 heads pays
 // for 128: a tile of 32 slots takes the same 1 800-2 600 cycles whatever H is, while the rows it gathers would take
 // 900 cycles of the SM pair's share of HBM.  Here the product is turned round:
 //       S^T [slots x heads]          = K [slots x 576] Q^T         (A = the gathered tile, B = Q in shared memory)
@@ -30,12 +30,12 @@
 // rows 700, scores 2 000, softmax 2 100, P V 750 and the hand-offs between them), three stages: 2 850-3 300 cycles per
 // 48 slots; its MMAs take 2 000 of them to issue (36 for the scores of M = 64, N = 16 at 33 cycles, 12 for P V at 62), though
 // the counter has the tensor pipe active for 8 %.
-// Measured against the kernel of sparse_mla.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 219 -> 177 us, 64
+// Measured against the 128-row kernel before paired_fp8.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 219 -> 177 us, 64
 // sequences of 16 heads 79 -> 51, 128 of 32 heads 151 -> 127.  Against paired_heads.cu: bf16, 296 rows of 16 heads x 1024 slots 86.6 -> 78.9,
 // eight sequences of 16 heads x 2048 in pieces 15.1 -> 14.2 with the merge; more shapes beside the rule (few_heads_form in plan.h).
-// out against 64 bits: 2.08e-3 (2.10e-3 in sparse_mla.cu), lse 2e-7 (7e-7: no 16-bit exchange of partial scores).
+// out against 64 bits: 2.08e-3 (1.68e-3 in paired_fp8.cu), lse 2e-7 (2e-6).
 //
-// Every mbarrier wait is bounded, as in sparse_mla.cu, and the warps of the softmax group meet on mbarriers only, so a
+// Every mbarrier wait is bounded, as in the 128-row kernels, and the warps of the softmax group meet on mbarriers only, so a
 // warp that gave up never leaves the others in a hardware barrier.
 #include <cuda_bf16.h>
 #include <cfloat>

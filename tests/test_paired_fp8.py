@@ -1,0 +1,97 @@
+"""The 128-row kernel of an fp8 cache: Q as a sum of two e4m3 numbers per row factor, V scaled to f16 with one exponent for a tile that
+moves with the largest scale.  Tile edges, split and stacked items are in test_paired_heads."""
+import math
+
+import numpy as np
+import pytest
+
+from helpers import TOL_FP8, check_lse, check_out
+from opfoundry_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+SCALE = 1.0 / math.sqrt(192.0)
+
+
+def _bf16(x):
+    return (np.ascontiguousarray(x, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+
+
+def _f32(bits):
+    return (bits.astype(np.uint32) << 16).view(np.float32)
+
+
+def _case(seed, H=72, topk=321, B=3):
+    return synth.make_decode_case(B, H, 512, topk, fp8=True, paged=True, seed=seed)
+
+
+def _scales(case):
+    return case["kv"][:, 512:528].view(np.float32)
+
+
+def _check(oracle, case, rel=4e-3):
+    """Against the oracle relative to each query row's largest output: P, V and the output are rounded to 11, 11 and 8 significant bits, the last of
+    these to half of 2^-7 of a value."""
+    from gpu_util import run_gpu, run_oracle
+    g_out, g_lse, _ = run_gpu(case, SCALE, num_sms=4)
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    g, r = _f32(g_out), _f32(r_out)
+    assert np.isfinite(g).all()
+    assert (np.abs(g - r) <= rel * np.abs(r).max(axis=-1, keepdims=True) + 2.0 ** -8 * np.abs(r)).all()
+    check_lse(g_lse, r_lse)
+
+
+@pytest.mark.parametrize("factor", [2.0 ** -60, 2.0 ** -20, 2.0 ** 12, 2.0 ** 40])
+def test_caches_far_from_one(built_lib, oracle, factor):
+    """All scales times a power of two, Q times its inverse: the scores stay, the output is that many times larger or smaller."""
+    case = _case(5)
+    kv = case["kv"].copy()
+    kv[:, 512:528].view(np.float32)[:] *= np.float32(factor)
+    q = _f32(case["q"]).copy()
+    q[..., :512] *= np.float32(1.0 / factor)
+    _check(oracle, dict(case, kv=kv, q=_bf16(q)))
+
+
+def test_the_exponent_of_v_moves_within_an_item(built_lib, oracle):
+    """Slots in order of growing scale: 2^30 from the first tile's rows to the last one's, in steps of which some exceed the 2^7 that pass without a move;
+    the latent part of Q is zero, so every row counts."""
+    case = _case(6, topk=512, B=2)
+    kv, q, idx = case["kv"].copy(), _f32(case["q"]).copy(), case["indices"]
+    q[..., :512] = 0.0
+    for b in range(idx.shape[0]):
+        pos = idx[b]
+        blocks = case["block_table"][b]
+        page = case["page_block_size"]
+        rows = blocks[pos // page] * page + pos % page
+        steps = np.array([0, 3, 6, 8, 17, 17, 29, 30], np.float32)[np.arange(512) // 64]
+        kv[rows, 512:528] = (kv[rows, 512:528].copy().view(np.float32) * np.exp2(steps - 15)[:, None]).astype(np.float32).view(np.uint8)
+    _check(oracle, dict(case, kv=kv, q=_bf16(q)))
+
+
+def test_rows_of_zeros_and_of_very_different_size(built_lib, oracle):
+    """Query rows of zeros, with one element far above the others, and with all elements tiny; cache rows whose scales are zero."""
+    case = _case(7)
+    q, kv = _f32(case["q"]).copy(), case["kv"].copy()
+    q[:, 0] = 0.0
+    q[:, 1, :512] = 0.0
+    q[:, 2, 5] = 60.0
+    q[:, 3, :512] *= 2.0 ** -90
+    q[:, 4] *= 2.0 ** -140
+    kv[::7, 512:528] = 0
+    _check(oracle, dict(case, kv=kv, q=_bf16(q)))
+
+
+def test_nan_codes_and_scales_reach_only_their_own_queries(built_lib):
+    """The e4m3 NaN code or a NaN scale in a row makes the queries that select it NaN and no others."""
+    from gpu_util import run_gpu
+    case = _case(8, topk=100)
+    kv, idx = case["kv"].copy(), case["indices"]
+    clean, _, _ = run_gpu(case, SCALE)
+    pos, page = int(idx[1, 70]), case["page_block_size"]
+    row = int(case["block_table"][1][pos // page]) * page + pos % page
+    for poison in (lambda r: r.__setitem__(130, 0x7F), lambda r: r[512:516].view(np.float32).__setitem__(0, np.nan)):
+        bad = kv.copy()
+        poison(bad[row])
+        out, _, _ = run_gpu(dict(case, kv=bad), SCALE)
+        assert np.isnan(_f32(out)[1]).any(axis=-1).all()
+        np.testing.assert_array_equal(out[[0, 2]], clean[[0, 2]])
