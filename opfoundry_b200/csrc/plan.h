@@ -63,11 +63,11 @@ inline void enumerate_units(const dsa_v32_shape& sh, std::vector<PlanUnit>& unit
 // The kernel a plan's items run on: 16 or 32 = the few-heads kernel's form for that many tile rows, 0 = the 128-row kernel.
 // Beyond 32 rows Q, the P copies and three tile stages of the few-heads kernel do not fit shared memory.
 // Up to 32 rows it takes less time per slot but more per change of item (its softmax group is also its epilogue), so the line is
-// drawn by the slots that an item has on average.  Measured time over that of the 128-row kernel, fp8, 1 to 12 items per list:
-//   16 rows, whole items of  64: 1.04-1.12   128: 1.01-1.05   192: 0.81-0.90   2048: 0.59-0.63
-//   32 rows, whole items of 128: 1.42-1.69   448: 1.02-1.07   800: 0.95-0.99   2048: 0.87
-// A piece of a split item has a cheaper end there (fp32 rows of the live heads only): pieces of 128 slots and more
-//   16 rows: 0.57-0.82   32 rows: 0.82-1.05
+// drawn by the slots that an item has on average.  Measured time over that of the 128-row kernel, fp8, 1 to 3 items per list:
+//   16 rows, whole items of  64: 1.06   128: 1.04-1.07   256: 0.96-0.97   512: 0.87-0.92   1024: 0.81-0.88   2048: 0.84-0.88   pieces: 0.89-0.99
+//   32 rows, whole items of  64: 1.53   128: 1.51-1.58   512: 1.23-1.29   2048: 1.19-1.23   pieces: 1.13-1.21
+// so a launch with an fp8 cache takes the few-heads kernel for at most 16 rows only; the plan's word still says 32 for such items, and so do plans
+// that were saved before.
 // bf16, over its own 128-row kernel (paired_heads.cu), both from one build, 1 to 16 items per list, short runs | after 0.8 s of the same
 // launches, when the 128-row kernel, not the few-heads one, has run into the power cap (1965 -> 1300-1900 MHz):
 //   16 rows, whole items of 128: 1.16-1.26 | 1.20-1.27   320: 1.07-1.23 | 1.00-1.12   400: 1.02-1.09 | 0.95-1.02   512: 0.97-1.07 | 0.82-1.02

@@ -1,4 +1,4 @@
-// Sparse MLA attention for few heads: work items of at most 32 tile rows (16 or 32 heads of a head-sharded
+// Sparse MLA attention for few heads: work items of at most 32 tile rows (fp8 cache: 16; 16 or 32 heads of a head-sharded
 // deployment, or the stacked rows of an MTP pair) that hold enough slots on average (few_heads_form in plan.h).
 //
 // The 128-row kernels put the heads on the 128 rows of the tensor-core tile, so an item of 16 heads pays
@@ -30,8 +30,8 @@
 // rows 700, scores 2 000, softmax 2 100, P V 750 and the hand-offs between them), three stages: 2 850-3 300 cycles per
 // 48 slots; its MMAs take 2 000 of them to issue (36 for the scores of M = 64, N = 16 at 33 cycles, 12 for P V at 62), though
 // the counter has the tensor pipe active for 8 %.
-// Measured against the 128-row kernel before paired_fp8.cu: fp8, 128 sequences of 2 x 16 heads (half of them stacked) 219 -> 177 us, 64
-// sequences of 16 heads 79 -> 51, 128 of 32 heads 151 -> 127.  Against paired_heads.cu: bf16, 296 rows of 16 heads x 1024 slots 86.6 -> 78.9,
+// Measured against paired_fp8.cu: 74 rows of 16 heads x 2048 slots 57.8 -> 50.9 us, 200 x 1024 90.3 -> 73.1.  (For 17 to 32 rows of an fp8 cache it
+// had a form, too: 71 us for 74 x 2048 where paired_fp8.cu takes 60.)  Against paired_heads.cu: bf16, 296 rows of 16 heads x 1024 slots 86.6 -> 78.9,
 // eight sequences of 16 heads x 2048 in pieces 15.1 -> 14.2 with the merge; more shapes beside the rule (few_heads_form in plan.h).
 // out against 64 bits: 2.08e-3 (1.68e-3 in paired_fp8.cu), lse 2e-7 (2e-6).
 //
@@ -59,12 +59,10 @@ constexpr int kLoadWarp0 = 8;
 constexpr int kLoadWarps = kSlots / 4;             // 12: four rows of every tile each, eight lanes per row
 constexpr int kWarps = kLoadWarp0 + kLoadWarps;    // 20: five warpgroups
 // Registers per thread after the role split (setmaxnreg): softmax warpgroup + issuers' + three of loaders <= 480, five times the
-// launch's 96.  16 heads, fp8: the loaders hold the next row and the one being converted (64 sequences 53 -> 51 us against loading
-// it after the conversion); 32 heads, fp8: the scores need the room (128 sequences of 2 x 16 heads 206 us that way, 186 without);
-// bf16: the rows never pass through registers.
-template <bool kFp8, int kN> constexpr bool kTwoRows = kFp8 && kN == 16;
-template <bool kFp8, int kN> constexpr int kRegsLoaders = !kFp8 ? 72 : (kN == 16 ? 104 : 80);
-template <bool kFp8, int kN> constexpr int kRegsSoftmax = kTwoRows<kFp8, kN> ? 112 : 152;
+// launch's 96.  fp8: the loaders hold the next row and the one being converted (64 sequences 53 -> 51 us against loading
+// it after the conversion); bf16: the rows never pass through registers.
+template <bool kFp8> constexpr int kRegsLoaders = kFp8 ? 104 : 72;
+template <bool kFp8> constexpr int kRegsSoftmax = kFp8 ? 112 : 152;
 constexpr int kRegsIssuers = 56;
 constexpr int kCtlBytes = 5120;
 
@@ -166,7 +164,9 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
     uint8_t* sP = smem + C::kOffP;
     Ctl* ctl = reinterpret_cast<Ctl*>(smem + C::kOffCtl);
     volatile int* abort_flag = &ctl->abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // fp8: the warp's number by a shuffle, so known to be the same in all lanes: fewer instructions (200 rows of 16 heads x 1024 slots 74.7 -> 72.0 us;
+    // bf16, two rows x 2048: 12.26 -> 12.37)
+    const int tid = threadIdx.x, warp = kFp8 ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
     const int list = blockIdx.x >> 1;
     const int half = (int)cluster_ctarank(), peer = half ^ 1;
     const int w_begin = __ldg(p.list_indptr + list), w_end = __ldg(p.list_indptr + list + 1);
@@ -215,8 +215,8 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
 
     if (warp < 4) {
         // ============================================================ softmax + epilogue
-        setmaxnreg_inc<kRegsSoftmax<kFp8, kN>>();
-        static_assert(kRegsSoftmax<kFp8, kN> + kRegsIssuers + 3 * kRegsLoaders<kFp8, kN> <= 5 * 96, "more registers than the launch has");
+        setmaxnreg_inc<kRegsSoftmax<kFp8>>();
+        static_assert(kRegsSoftmax<kFp8> + kRegsIssuers + 3 * kRegsLoaders<kFp8> <= 5 * 96, "more registers than the launch has");
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(warp * 32) << 16);
         const bool live_lane = lane < 16 && warp < kSlots / 16;   // this thread has a slot
         const int slot = 16 * warp + (lane & 15);
@@ -626,8 +626,8 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
             }
         }
     } else {
-        if constexpr (kTwoRows<kFp8, kN>) setmaxnreg_inc<kRegsLoaders<kFp8, kN>>();
-        else setmaxnreg_dec<kRegsLoaders<kFp8, kN>>();
+        if constexpr (kFp8) setmaxnreg_inc<kRegsLoaders<kFp8>>();
+        else setmaxnreg_dec<kRegsLoaders<kFp8>>();
         {
             // ======================================================== row loaders: four rows of every tile per warp, eight lanes per row
             const int r = 4 * (warp - kLoadWarp0) + (lane >> 3);   // tile row
@@ -712,7 +712,7 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     for (int t = 0; t < pt.n_tiles; ++t, ring.next()) {
                         const Row cur = next;
                         advance(t);
-                        if (kTwoRows<kFp8, kN>) next = load_row(row0);   // a whole tile ahead
+                        next = load_row(row0);   // a whole tile ahead
                         // e4m3 -> bf16 before the wait for a stage: a stage is the scarce resource
                         uint32_t o[32];
 #pragma unroll
@@ -724,7 +724,6 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                                 o[8 * k + 2 * q + 1] = e4m3x2_to_bf16x2(__byte_perm(wv[q], 0u, 0x3424u));
                             }
                         }
-                        if (!kTwoRows<kFp8, kN>) next = load_row(row0);
                         if (!wait_on(&ctl->kv_empty[ring.s], ring.ph ^ 1u, abort_flag)) goto done;
                         uint8_t* tile = sKV + ring.s * kTileBytes + r * 128;
                         if (oc < 4) reinterpret_cast<float*>(&ctl->row_scale[ring.s][r])[oc] = cur.sc;
@@ -814,10 +813,10 @@ static cudaError_t launch(int num_lists, const CUtensorMap& tq, const AttnParams
 
 }  // namespace small
 
-// tile_rows: the most rows an item of the plan has
+// tile_rows: the most rows an item of the plan has, at most 16 with an fp8 cache
 cudaError_t launch_small_heads(bool fp8, int tile_rows, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream) {
-    if (tile_rows <= 16) return fp8 ? small::launch<true, 16>(num_lists, tq, p, stream) : small::launch<false, 16>(num_lists, tq, p, stream);
-    return fp8 ? small::launch<true, 32>(num_lists, tq, p, stream) : small::launch<false, 32>(num_lists, tq, p, stream);
+    if (fp8) return tile_rows <= 16 ? small::launch<true, 16>(num_lists, tq, p, stream) : cudaErrorInvalidValue;
+    return tile_rows <= 16 ? small::launch<false, 16>(num_lists, tq, p, stream) : small::launch<false, 32>(num_lists, tq, p, stream);
 }
 
 }  // namespace dsa
