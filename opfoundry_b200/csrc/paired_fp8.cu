@@ -31,9 +31,8 @@
 //   warps 16, 17 CTA 0: score issuers on alternate tiles
 //   warp 18      CTA 0: P V issuer
 //   warp 19      tells the issuers that the CTA's rows of a tile have landed, and follows e
-//   warps 20-23  row loaders: 16-byte cp.async copies into the swizzled tile, eight rows of every tile each, and the own output columns of
-//                eight of the other CTA's rows
-//   warps 24-31  converters: e4m3 -> f16, eight of a tile's rows each
+//   warps 20-23  row loaders: 16-byte cp.async copies into the swizzled tile, eight rows of every tile each
+//   warps 24-31  converters: e4m3 -> f16, eight of a tile's rows each; four of them fetch the own output columns of the other CTA's rows
 //
 // What bounds it (cycle stamps of an instrumented copy, 64 sequences x 128 heads x 2048 slots): a tile of 64 slots every 2 780 cycles.  Its MMAs
 // take 1 430 (measured alone; the scores' 25 an instruction are the rate of shared memory, 3 KB of operands each), all its traffic in shared
@@ -68,18 +67,17 @@ constexpr int kOwn = 32;                           // slots of a tile that one C
 constexpr int kSlots = 2 * kOwn;
 constexpr int kGroups = 4;                         // 128-column scale groups
 constexpr int kBlock = kOwn * 128;                 // 4 096: 128 bytes of 32 rows
-constexpr int kOwnBytes = (kGroups + 1) * kBlock;  // own rows: the four groups, the rope
-constexpr int kRawBytes = kOwnBytes + 2 * kBlock;  // and the own output columns of the other CTA's rows
-constexpr int kStages = 3;                         // raw tiles
+constexpr int kRawBytes = (kGroups + 1) * kBlock;  // own rows: the four groups, the rope
+constexpr int kStages = 4;                         // raw tiles
 constexpr int kVUnit = 4 * kBlock;                 // 32 slots x 256 columns of f16
 constexpr int kVUnits = 3;                         // a tile takes two
 constexpr int kQBlock = kRows * 128;               // 8 192
 constexpr int kPBytes = kRows * kSlots * 2;        // 8 192
 constexpr int kSoftmaxWarps = 16, kTeamWarps = 8, kScoreWarp = 16, kPvWarp = 18, kReadyWarp = 19, kLoadWarp0 = 20, kLoadWarps = 4;
 constexpr int kConvWarp0 = 24, kConvWarps = 8, kWarps = 32;
-// Registers per thread after the role split: 4 x softmax + issuers + loaders + 2 x converters <= 8 x the launch's 64
-constexpr int kRegsSoftmax = 80, kRegsIssuers = 40, kRegsLoaders = 48, kRegsConv = 48;
-static_assert(4 * kRegsSoftmax + kRegsIssuers + kRegsLoaders + 2 * kRegsConv <= 8 * 64, "more registers than the launch has");
+// Registers per thread after the role split: 4 x softmax + issuers + loaders + converters of own and of the other CTA's rows <= 8 x the launch's 64
+constexpr int kRegsSoftmax = 80, kRegsIssuers = 40, kRegsLoaders = 40, kRegsConv = 48, kRegsLate = 56;
+static_assert(4 * kRegsSoftmax + kRegsIssuers + kRegsLoaders + kRegsConv + kRegsLate <= 8 * 64, "more registers than the launch has");
 constexpr float kPShift = 7.0f;                    // P = 2^(score - reference + 7) <= 2^15
 
 constexpr int kOffQ = 0;                           // hi of the four groups, lo of the four groups, rope
@@ -87,7 +85,7 @@ constexpr int kOffRaw = 9 * kQBlock;
 constexpr int kOffV = kOffRaw + kStages * kRawBytes;
 constexpr int kOffP = kOffV + kVUnits * kVUnit;
 constexpr int kOffCtl = kOffP + 2 * kPBytes;
-constexpr int kCtlBytes = 7168;
+constexpr int kCtlBytes = 9216;
 constexpr int kSmemBytes = kOffCtl + kCtlBytes;
 static_assert(kSmemBytes <= 232448, "227 KB per CTA");
 // TMEM columns: O 256 | S: groups 0-2 of even tiles, of odd tiles, group 3, rope, 32 columns each
@@ -98,9 +96,11 @@ struct Ctl {
     float post[2][4][kRows];                 // by team and quarter of a tile's slots: the rows' maxima (log2 domain); at the end of an item its row sums
     float m_ref[2][kRows];                   // by tile number mod 2: the rows' reference maxima after the tile
     uint8_t q_exp[kRows];                    // biased exponent of 2^a, Q = 2^a (hi + lo); 255: a row with an infinity or a NaN
+    int32_t late_row[kStages][kOwn];         // rows of the tile that the other CTA gathers
     uint32_t tile_mask[kStages][2];          // which slots of CTA 0 / CTA 1 hold a row
     float v_mul[kStages], v_unit[kStages], v_fix[kStages];   // 2^-e of the tile, 2^e, and 2^(e of the tile before - e)
     float v_fin;                             // 2^e of the item's last tile
+    uint64_t late_known[kStages];                      // late_row is written
     uint64_t kv_full[kStages], raw_empty[kStages];     // rows landed | scores complete, rows converted, scales read
     uint64_t prep[kStages];                            // ... and e known
     uint64_t tile_ready[2][kStages];                   // CTA 0: both CTAs' rows have landed, by the score issuer (tile number mod 2) that takes the tile
@@ -192,8 +192,11 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         mbar_init(smem_u32(&ctl->prep[tid]), 1);
         mbar_init(smem_u32(&ctl->tile_ready[0][tid]), 2);
         mbar_init(smem_u32(&ctl->tile_ready[1][tid]), 2);
-        mbar_init(smem_u32(&ctl->v_full[tid]), kConvWarps);   // half of either CTA's converters
-        mbar_init(smem_u32(&ctl->v_empty[tid]), 1);
+        mbar_init(smem_u32(&ctl->late_known[tid]), kLoadWarps);
+        if (tid < kVUnits) {
+            mbar_init(smem_u32(&ctl->v_full[tid]), kConvWarps);   // half of either CTA's converters
+            mbar_init(smem_u32(&ctl->v_empty[tid]), 1);
+        }
         fence_mbar_init();
     } else if (tid >= 32 && tid < 34) {
         const int i = tid - 32;
@@ -217,7 +220,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         ctl->abort_flag = 0;
         fence_mbar_init();
     }
-    static_assert(kVUnits == kStages, "one thread per stage and unit");
+    static_assert(kVUnits <= kStages, "one thread per stage and unit");
     if (warp == kScoreWarp) {
         tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols);
         tmem_relinquish_pair();
@@ -692,6 +695,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 for (int t = 0; t < 2 && u + t < n_tiles; ++t, ring.next()) {
                     const int own = __shfl_sync(0xffffffffu, row, 16 * t + (lane >> 2)), late = __shfl_sync(0xffffffffu, row, 16 * t + 8 + (lane >> 2));
                     if (!wait_on(&ctl->raw_empty[ring.s], ring.ph, abort_flag)) goto done;
+                    if (c4 == 0) ctl->late_row[ring.s][r] = late;
+                    warp_arrive(&ctl->late_known[ring.s], lane);
                     if (lane < 2) reinterpret_cast<uint8_t*>(&ctl->tile_mask[ring.s][lane ? peer : rank])[lw] = static_cast<uint8_t>(used >> (16 * t + 8 * lane));
                     // padding and out-of-range rows: nothing is read, the row is zeros
                     const uint32_t st = ring.s * kRawBytes, sc = ring.s * (kGroups * kSlots * 4);
@@ -706,17 +711,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             cp_async_16(d1 + st + j * kBlock, src + 128 * j + (j == 4 ? 16 : 0) + 64, n);
                         }
                     }
-                    {
-                        const uint8_t* src = kv_bytes + (size_t)(late < 0 ? 0 : late) * kFp8RowBytes;
-                        const uint32_t n = late != -1 ? 16u : 0u;
-                        cp_async_4(scale_late + sc, src + kDV + 4 * c4, n >> 2);
-                        src += rank * kDvHalf + 16 * c4;
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            cp_async_16(d0 + st + kOwnBytes + j * kBlock, src + 128 * j, n);
-                            cp_async_16(d1 + st + kOwnBytes + j * kBlock, src + 128 * j + 64, n);
-                        }
-                    }
+                    cp_async_4(scale_late + sc, kv_bytes + (size_t)(late < 0 ? 0 : late) * kFp8RowBytes + kDV + 4 * c4, late != -1 ? 4u : 0u);
                     cp_async_mbar_arrive_noinc(smem_u32(&ctl->kv_full[ring.s]));
                     warp_arrive(&ctl->kv_full[ring.s], lane);
                 }
@@ -724,57 +719,104 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         }
     } else {
         // ============================================================ converters: this CTA's 256 output columns of all 64 rows, to f16
-        setmaxnreg_dec<kRegsConv>();
-        // Warps 0-3 take the slots of CTA 0 (unit 0 of a tile), warps 4-7 those of CTA 1, eight rows each.  Sixteen columns a lane and step: one
-        // 16-byte chunk of a raw row, two of a row of V.  A quarter of a warp takes half of the block's columns of one row and the other half of its
-        // neighbour's, so that its loads and its stores touch every bank once.
+        // Warps 0-3 take the slots of CTA 0 (unit 0 of a tile), warps 4-7 those of CTA 1, eight rows each.  Own rows lie in shared memory, the
+        // other CTA's come from L2 through registers, a tile ahead.  Sixteen columns a lane and step: one 16-byte chunk of a row of the cache, two of a
+        // row of V.  A quarter of a warp takes half of a block's columns of one row and the other half of its neighbour's, so that its loads and
+        // its stores touch every bank once.
         const int cw = warp - kConvWarp0, u = cw >> 2;
         const int r4 = 2 * (lane >> 4) + ((lane >> 2) & 1), half = ((lane >> 3) ^ (lane >> 2)) & 1, k = lane & 3;
         const int r = 8 * (cw & 3) + r4;   // of the first two steps; the others take the row four further
-        const uint32_t raw0 = smem_u32(sRaw) + (u == rank ? 2 * rank * kBlock : kOwnBytes) + r * 128 + (((4 * half + k) ^ (r & 7)) << 4);
         const uint32_t v0 = smem_u32(sV) + half * kBlock + r * 128 + (((2 * k) ^ (r & 7)) << 4);
         // lane i < 16 (and i + 16): the scale of block i / 8, row i % 8
         const float* const scale0 = &ctl->scale[0][2 * rank + ((lane >> 3) & 1)][kOwn * u + 8 * (cw & 3) + (lane & 7)];
+        // one chunk of either block of a row, scaled, to V
+        auto convert = [&](const uint4 (&x)[2], uint32_t scales, int i, uint32_t dst) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const uint32_t s = __shfl_sync(0xffffffffu, scales, 8 * b + 4 * i + r4);
+                const uint32_t hi = __byte_perm(s, 0, 0x1010), lo = __byte_perm(s, 0, 0x3232);
+                const uint32_t v[4] = {x[b].x, x[b].y, x[b].z, x[b].w};
+                uint32_t y[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    y[2 * j] = scale_f16x2(e4m3x2_to_f16x2(v[j]), hi, lo);
+                    y[2 * j + 1] = scale_f16x2(e4m3x2_to_f16x2(v[j] >> 16), hi, lo);
+                }
+                sts_16(dst + 2 * b * kBlock, y[0], y[1], y[2], y[3]);
+                sts_16((dst ^ 16u) + 2 * b * kBlock, y[4], y[5], y[6], y[7]);
+            }
+        };
         Ring<kStages> ring;
         Ring<kVUnits> unit;   // of v_empty: one use behind
         unit.ph = 1u;
         if (u) unit.next();
-        for (int w = w_begin; w < w_end; ++w) {
-            const int n_tiles = tiles_of(p.works[w]);
+        if (u == rank) {
+            setmaxnreg_dec<kRegsConv>();
+            const uint32_t raw0 = smem_u32(sRaw) + 2 * rank * kBlock + r * 128 + (((4 * half + k) ^ (r & 7)) << 4);
+            for (int w = w_begin; w < w_end; ++w) {
+                const int n_tiles = tiles_of(p.works[w]);
 #pragma unroll 1
-            for (int t = 0; t < n_tiles; ++t, ring.next(), unit.next(), unit.next()) {
-                if (!wait_on2(&ctl->prep[ring.s], ring.ph, &ctl->v_empty[unit.s], unit.ph, abort_flag)) goto done;
-                const uint32_t scales = split_f16(scale0[ring.s * (kGroups * kSlots)] * ctl->v_mul[ring.s]);   // as a sum of two f16
-                uint32_t src = raw0 + ring.s * kRawBytes, dst = v0 + unit.s * kVUnit;
-                uint4 x[2] = {lds_16(src), lds_16(src + kBlock)};
+                for (int t = 0; t < n_tiles; ++t, ring.next(), unit.next(), unit.next()) {
+                    if (!wait_on2(&ctl->prep[ring.s], ring.ph, &ctl->v_empty[unit.s], unit.ph, abort_flag)) goto done;
+                    const uint32_t scales = split_f16(scale0[ring.s * (kGroups * kSlots)] * ctl->v_mul[ring.s]);   // as a sum of two f16
+                    uint32_t src = raw0 + ring.s * kRawBytes, dst = v0 + unit.s * kVUnit;
+                    uint4 x[2] = {lds_16(src), lds_16(src + kBlock)};
 #pragma unroll 1
-                for (int i = 0; i < 2; ++i) {   // row r, row r + 4: a short loop, see warp_wait_short
-                    const uint4 in[2] = {x[0], x[1]};
-                    src = (src ^ 64u) + 512u;   // four rows on, and bit 2 of the swizzle flips
-                    if (i == 0) {
-                        x[0] = lds_16(src);
-                        x[1] = lds_16(src + kBlock);
-                    } else {
-                        warp_arrive(&ctl->raw_empty[ring.s], lane);
-                    }
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        const uint32_t s = __shfl_sync(0xffffffffu, scales, 8 * b + 4 * i + r4);
-                        const uint32_t hi = __byte_perm(s, 0, 0x1010), lo = __byte_perm(s, 0, 0x3232);
-                        const uint32_t v[4] = {in[b].x, in[b].y, in[b].z, in[b].w};
-                        uint32_t y[8];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            y[2 * j] = scale_f16x2(e4m3x2_to_f16x2(v[j]), hi, lo);
-                            y[2 * j + 1] = scale_f16x2(e4m3x2_to_f16x2(v[j] >> 16), hi, lo);
+                    for (int i = 0; i < 2; ++i) {   // row r, row r + 4: a short loop, see warp_wait_short
+                        const uint4 cur[2] = {x[0], x[1]};
+                        src = (src ^ 64u) + 512u;   // four rows on, and bit 2 of the swizzle flips
+                        if (i == 0) {
+                            x[0] = lds_16(src);
+                            x[1] = lds_16(src + kBlock);
+                        } else {
+                            warp_arrive(&ctl->raw_empty[ring.s], lane);
                         }
-                        sts_16(dst + 2 * b * kBlock, y[0], y[1], y[2], y[3]);
-                        sts_16((dst ^ 16u) + 2 * b * kBlock, y[4], y[5], y[6], y[7]);
+                        convert(cur, scales, i, dst);
+                        dst = (dst ^ 64u) + 512u;
                     }
-                    dst = (dst ^ 64u) + 512u;
+                    fence_proxy_async_smem();
+                    warp_arrive_lead(&ctl->v_full[unit.s], lane);
                 }
-                fence_proxy_async_smem();
-                warp_arrive_lead(&ctl->v_full[unit.s], lane);
+            }
+        } else {
+            setmaxnreg_dec<kRegsLate>();
+            const uint8_t* const kv0 = reinterpret_cast<const uint8_t*>(p.kv) + rank * kDvHalf + (4 * half + k) * 16;
+            auto load = [&](uint4 (&x)[2], int row) {
+                x[0] = x[1] = make_uint4(0u, 0u, 0u, 0u);
+                if (row >= 0) {
+                    const uint8_t* src = kv0 + (size_t)row * kFp8RowBytes;
+                    x[0] = ldg_stream_16(src);
+                    x[1] = ldg_stream_16(src + 128);
+                }
+            };
+            Ring<kStages> known;   // of the tile whose rows are fetched
+            for (int w = w_begin; w < w_end; ++w) {
+                const int n_tiles = tiles_of(p.works[w]);
+                uint4 x[2][2];
+                if (!wait_on(&ctl->late_known[known.s], known.ph, abort_flag)) goto done;
+                load(x[0], ctl->late_row[known.s][r]);
+                load(x[1], ctl->late_row[known.s][r + 4]);
+                known.next();
+#pragma unroll 1
+                for (int t = 0; t < n_tiles; ++t, ring.next(), unit.next(), unit.next()) {
+                    int next0 = -1, next1 = -1;
+                    if (t + 1 < n_tiles) {
+                        if (!wait_on(&ctl->late_known[known.s], known.ph, abort_flag)) goto done;
+                        next0 = ctl->late_row[known.s][r];
+                        next1 = ctl->late_row[known.s][r + 4];
+                        known.next();
+                    }
+                    if (!wait_on2(&ctl->prep[ring.s], ring.ph, &ctl->v_empty[unit.s], unit.ph, abort_flag)) goto done;
+                    const uint32_t scales = split_f16(scale0[ring.s * (kGroups * kSlots)] * ctl->v_mul[ring.s]);
+                    const uint32_t dst = v0 + unit.s * kVUnit;
+                    convert(x[0], scales, 0, dst);
+                    load(x[0], next0);
+                    warp_arrive(&ctl->raw_empty[ring.s], lane);
+                    convert(x[1], scales, 1, (dst ^ 64u) + 512u);
+                    load(x[1], next1);
+                    fence_proxy_async_smem();
+                    warp_arrive_lead(&ctl->v_full[unit.s], lane);
+                }
             }
         }
     }

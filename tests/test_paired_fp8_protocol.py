@@ -34,6 +34,8 @@ class PairFp8(Pair):
         bars = lambda n, count: [[Bar(count) for _ in range(n)] for _ in range(2)]
         one = lambda count: [Bar(count) for _ in range(2)]
         self.kv_full, self.raw_empty, self.prep = bars(STAGES, LOADERS * 33), bars(STAGES, 1 + CONVERTERS + TEAM), bars(STAGES, 1)
+        self.late_known = bars(STAGES, LOADERS)
+        self.late = [[[None] * LOADERS for _ in range(STAGES)] for _ in range(2)]  # rows of the other CTA
         self.tile_ready = bars(STAGES, 2)   # CTA 0's, by the issuer that takes the tile
         self.v_full, self.v_empty = [Bar(CONVERTERS) for _ in range(V_UNITS)], bars(V_UNITS, 1)
         self.s_full, self.s_empty, self.p_full, self.pv_done = bars(2, 1), [Bar(2 * TEAM) for _ in range(2)], [Bar(2 * TEAM) for _ in range(2)], bars(2, 1)
@@ -219,6 +221,9 @@ class PairFp8(Pair):
             for _ in range(tiles):
                 s = ring.s
                 yield self.raw_empty[c][s], ring.ph
+                self.late[c][s][w] = it
+                self.late_known[c][s].arrive()
+                yield None
                 self.mask[c][s][w] = it
 
                 def copy(it=it, s=s):
@@ -234,12 +239,17 @@ class PairFp8(Pair):
                 ring.next()
 
     def converter(self, c, w):
-        it, u, ring, unit = 0, w // (CONVERTERS // 2), Ring(STAGES), Ring(V_UNITS, 1)
+        it, u, ring, unit, known = 0, w // (CONVERTERS // 2), Ring(STAGES), Ring(V_UNITS, 1), Ring(STAGES)
         if u:
             unit.next()
         for tiles in self.items:
-            for _ in range(tiles):
+            for t in range(tiles):
                 s = ring.s
+                for ahead in ((0, 1) if t == 0 else (1,)) if u != c else ():   # the other CTA's rows are fetched a tile ahead
+                    if t + ahead < tiles:
+                        yield self.late_known[c][known.s], known.ph
+                        assert self.late[c][known.s] == [it + ahead] * LOADERS, "rows of another tile"
+                        known.next()
                 yield self.prep[c][s], ring.ph
                 yield self.v_empty[c][unit.s], unit.ph
                 for _ in range(2):
