@@ -14,7 +14,7 @@
 namespace dsa {
 int max_resident_pairs_fp8(int* out);
 int max_resident_pairs_paired(int* out);
-cudaError_t launch_paired_fp8(bool ext, int num_lists, const AttnParams& p, cudaStream_t stream);
+cudaError_t launch_paired_fp8(bool ext, int tile_rows, int num_lists, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_small_heads(bool fp8, int tile_rows, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_paired_heads(bool ext, int num_lists, const CUtensorMap& tq, const AttnParams& p, cudaStream_t stream);
 cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const int32_t* reduce_indptr,
@@ -300,7 +300,7 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         cudaError_t e = launch_paired_heads(use_ext, h.num_lists, tq, p, stream);
         return e == cudaSuccess ? DSA_V32_OK : (int)e;
     }
-    cudaError_t e = launch_paired_fp8(use_ext, h.num_lists, p, stream);
+    cudaError_t e = launch_paired_fp8(use_ext, live_tile_rows(h), h.num_lists, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }
 

@@ -5,7 +5,7 @@
 // plan.h: an online-softmax attention over the gathered latent rows, K = all 576 columns of a row, V = its first 512 columns
 // (opus_attn/dsa_v32/gfx950/mla_decode_mxfp8_16mx8_32nx1_template.hpp:1362-1490).
 //
-// CTA c of the pair owns tile rows (heads) [64 c, 64 c + 64) and, of every tile of 64 slots, gathers slots [32 c, 32 c + 32).
+// CTA c of the pair owns tile rows (heads) [64 c, 64 c + 64), or [32 c, 32 c + 32) where no item has more than 64, and, of every tile of 64 slots, gathers slots [32 c, 32 c + 32).
 //       S_g [128 x 64]  = Q_g K_g^T  cta_group::2, M = 128, N = 64, kind::f8f6f4, one accumulator per 128-column scale group g: B = the
 //                                    gathered e4m3 bytes, A = Q as the sum of two e4m3 numbers (below); the rope with bf16 operands
 //       O [128 x 512] += P V         cta_group::2, M = 128, N = 256, twice, kind::f16 on f16: A = each CTA's 64 rows of P, B = each
@@ -145,6 +145,7 @@ __device__ __forceinline__ void warp_arrive_lead(uint64_t* bar, int lane) {
     if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(bar), 0));
 }
 
+__device__ __forceinline__ int rows_of(const dsa_v32_work_info& w, int H) { return w.stacked_rows > 1 ? w.stacked_rows * H : H - w.head_block * kHeadsPerBlock; }
 __device__ __forceinline__ int tiles_of(const dsa_v32_work_info& w) { return (w.k_end - w.k_begin + kSlots - 1) / kSlots; }
 
 // ------------------------------------------------------------------ Q as a sum of two e4m3 numbers
@@ -169,7 +170,11 @@ __device__ __forceinline__ void split_e4m3(const uint4& x, float mul, uint2& hi,
     lo = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
 }
 
-template <bool kExt>
+// kShare: tile rows that a CTA owns, 64, or 32 for plans without items of more than 64: softmax warps without a live row only take part in the
+// barriers (128 sequences of 2 x 16 heads 144 -> 134 us), and with 32 that is half of either CTA's (64 sequences of 64 heads 55.5 -> 52.5 us; decided
+// at run time it costs 0.4 us a launch).
+// kExt: a sink, peers, stacked rows, or rows of out on 16-byte boundaries
+template <bool kExt, int kShare>
 __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnParams p) {
     extern __shared__ __align__(1024) uint8_t smem_paired_fp8[];   // the same offset in both CTAs of a pair
     uint8_t* smem = smem_paired_fp8;
@@ -246,8 +251,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             const int row0 = 4 * warp;
             uint4 x[4][2], xr = make_uint4(0u, 0u, 0u, 0u);
             auto row_ptr = [&](int row, bool& live) {
-                const RowMap rm = map_row(wi, kRows * rank + row, p.H);
-                live = rm.live;
+                const RowMap rm = map_row(wi, kShare * rank + row, p.H);
+                live = rm.live && row < kShare;
                 return reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)(live ? rm.q_row : wi.q_row) * p.stride_q_row + (size_t)(live ? rm.head : 0) * p.stride_q_head;
             };
 #pragma unroll
@@ -313,7 +318,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             }
             if (item_n > 0) {
                 const dsa_v32_work_info wi = p.works[w - 1];
-                const RowMap rm = map_row(wi, kRows * rank + r, p.H);
+                const int row = kShare * rank + r;   // of the item's tile
+                const RowMap rm = map_row(wi, row, p.H);
                 if (kExt && p.attn_sink != nullptr) {
                     // attention sink (opus_attn/dsa_v4/common/mla_v4_host.cc:469-472): one more term exp(sink - m) in the
                     // denominator, counted once per query row and head: in the piece that starts the list
@@ -327,7 +333,10 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 tc_fence_after();
                 // this thread's 64 columns of the row
                 const int col0 = 64 * (warp >> 2);   // of the 256 in its lane
-                if (wi.partial_slot < 0) {
+                if (32 * rq >= kShare) {   // none of the warp's rows is live
+                    tc_fence_before();
+                    warp_arrive_lead(&ctl->o_free, lane);
+                } else if (wi.partial_slot < 0) {
                     const size_t off = (size_t)rm.q_row * p.stride_o_row + (size_t)rm.head * p.stride_o_head + 256 * h;
                     const int n_dst = kExt && p.n_peers > 0 ? p.n_peers : 1;
 #pragma unroll 1
@@ -362,7 +371,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                         }
                     }
                 } else {
-                    float* o_dst = p.o_accum + ((size_t)wi.partial_slot * kHeadsPerBlock + kRows * rank + r) * kDV + 256 * h;
+                    float* o_dst = p.o_accum + ((size_t)wi.partial_slot * kHeadsPerBlock + row) * kDV + 256 * h;
 #pragma unroll 1
                     for (int oc = col0; oc < col0 + 64; oc += 32) {
                         uint32_t o[32];
@@ -381,18 +390,35 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                                         __float_as_uint(__uint_as_float(o[8 * v + 6]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 7]) * inv));
                         }
                     }
-                    if (warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + kRows * rank + r] = ls > 0.0f ? lse_nat : -FLT_MAX;
+                    if (rm.live && warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + row] = ls > 0.0f ? lse_nat : -FLT_MAX;
                 }
             }
             if (w == w_end) break;
             const uint32_t it_end = it_base + tiles_of(p.works[w]);
             float m_ref = -INFINITY;   // reference maximum after this team's last tile
             float l = 0.0f;            // this thread's share of the row sum, against m_ref
+            const bool idle = 32 * rq >= kShare || kShare * rank + 32 * rq >= rows_of(p.works[w], p.H);   // none of the warp's rows is live
             if (!wait_on(&ctl->q_here, item_n & 1, abort_flag)) goto done;
             const uint32_t q_exp = ctl->q_exp[r];
             const float c_log2 = p.scale_log2 * __uint_as_float(q_exp == 255u ? 0x7FC00000u : q_exp << 23);   // of scores in units of 2^a
+            uint32_t it = it_base + ((it_base ^ team) & 1u);
+            if (idle) {   // the warp's part in the barriers; what P holds for such rows is used for such rows of O only
 #pragma unroll 1
-            for (uint32_t it = it_base + ((it_base ^ team) & 1u); it < it_end; it += 2, ring.next(), ring.next()) {
+                for (; it < it_end; it += 2, ring.next(), ring.next()) {
+                    const uint32_t ph2 = (it >> 1) & 1u;
+                    if (!wait_on(&ctl->s_full[team], ph2, abort_flag)) goto done;
+                    warp_arrive_lead(&ctl->s3_empty, lane);
+                    warp_arrive_lead(&ctl->s_empty[team], lane);
+                    warp_arrive(&ctl->raw_empty[ring.s], lane);
+                    if (it >= 2)   // every warp of the team has come to the end of its last tile
+                        if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) goto done;
+                    warp_arrive(&ctl->posted[team][rq], lane);
+                    warp_arrive(&ctl->moved[team][rq], lane);
+                    warp_arrive_lead(&ctl->p_full[team], lane);
+                }
+            }
+#pragma unroll 1
+            for (; it < it_end; it += 2, ring.next(), ring.next()) {
                 const uint32_t ph2 = (it >> 1) & 1u;            // phase of the per-team barriers
                 const bool first = it == it_base;
                 // the tile's mask, scales and e, and its scores (the stage's phase before is complete: its tile was three earlier, and this team has
@@ -837,7 +863,7 @@ done:
 }
 
 // The opt-in for more than 48 KB of dynamic shared memory is a per-device attribute of the kernel.
-template <bool kExt>
+template <bool kExt, int kShare>
 static cudaError_t configure() {
     static std::mutex mu;
     static bool done[64] = {};
@@ -846,7 +872,7 @@ static cudaError_t configure() {
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> guard(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-    e = cudaFuncSetAttribute(paired_fp8_kernel<kExt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    e = cudaFuncSetAttribute(paired_fp8_kernel<kExt, kShare>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev] = true;
     return cudaSuccess;
@@ -867,34 +893,36 @@ static void fill_launch(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int 
     cfg->numAttrs = 2;
 }
 
-template <bool kExt>
+template <bool kExt, int kShare>
 static cudaError_t launch(int num_lists, const AttnParams& p, cudaStream_t stream) {
-    cudaError_t e = configure<kExt>();
+    cudaError_t e = configure<kExt, kShare>();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     fill_launch(&cfg, attr, num_lists, stream);
-    return cudaLaunchKernelEx(&cfg, paired_fp8_kernel<kExt>, p);
+    return cudaLaunchKernelEx(&cfg, paired_fp8_kernel<kExt, kShare>, p);
 }
 
 }  // namespace paired_fp8
 
 int max_resident_pairs_fp8(int* out) {
-    cudaError_t e = paired_fp8::configure<false>();
+    cudaError_t e = paired_fp8::configure<false, paired_fp8::kRows>();
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     int n = 0;
     paired_fp8::fill_launch(&cfg, attr, 1, nullptr);
-    e = cudaOccupancyMaxActiveClusters(&n, paired_fp8::paired_fp8_kernel<false>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, paired_fp8::paired_fp8_kernel<false, paired_fp8::kRows>, &cfg);
     if (e != cudaSuccess) return (int)e;
     *out = n;
     return 0;
 }
 
-// ext: a sink or peers are given, or rows of out are aligned to 16 bytes only
-cudaError_t launch_paired_fp8(bool ext, int num_lists, const AttnParams& p, cudaStream_t stream) {
-    return ext ? paired_fp8::launch<true>(num_lists, p, stream) : paired_fp8::launch<false>(num_lists, p, stream);
+// ext: a sink or peers are given, rows are stacked, or rows of out are aligned to 16 bytes only; tile_rows: the most rows an item of the plan has
+cudaError_t launch_paired_fp8(bool ext, int tile_rows, int num_lists, const AttnParams& p, cudaStream_t stream) {
+    using namespace paired_fp8;
+    if (tile_rows > kRows) return ext ? launch<true, kRows>(num_lists, p, stream) : launch<false, kRows>(num_lists, p, stream);
+    return ext ? launch<true, kRows / 2>(num_lists, p, stream) : launch<false, kRows / 2>(num_lists, p, stream);
 }
 
 }  // namespace dsa
