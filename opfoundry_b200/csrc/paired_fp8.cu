@@ -153,21 +153,16 @@ __device__ __forceinline__ int tiles_of(const dsa_v32_work_info& w) { return (w.
 __device__ __forceinline__ void split_e4m3(const uint4& x, float mul, uint2& hi, uint2& lo) {
     const uint32_t in[4] = {x.x, x.y, x.z, x.w};
     uint32_t h[4], l[4];
-    const uint64_t m2 = pack2(mul, mul), neg1 = pack2(-1.0f, -1.0f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const uint64_t u = mul2(pack2u(in[i] << 16, in[i] & 0xFFFF0000u), m2);
         float u0, u1;
-        unpack2(u, u0, u1);
-        h[i] = pack_e4m3x2(u0, u1);
-        float h0, h1;
-        unpack_f16x2(e4m3x2_to_f16x2(h[i]), h0, h1);
-        float d0, d1;
-        unpack2(fma2(pack2(h0, h1), neg1, u), d0, d1);
-        l[i] = pack_e4m3x2(d0, d1);
+        unpack2(mul2(pack2u(in[i] << 16, in[i] & 0xFFFF0000u), pack2(mul, mul)), u0, u1);
+        const uint32_t u = pack_f16x2(u0, u1);   // exact where e4m3 resolves anything
+        h[i] = f16x2_to_e4m3x2(u);
+        l[i] = f16x2_to_e4m3x2(sub_f16x2(u, e4m3x2_to_f16x2(h[i])));
     }
-    hi = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-    lo = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+    hi = make_uint2(__byte_perm(h[0], h[1], 0x5410), __byte_perm(h[2], h[3], 0x5410));
+    lo = make_uint2(__byte_perm(l[0], l[1], 0x5410), __byte_perm(l[2], l[3], 0x5410));
 }
 
 // kShare: tile rows that a CTA owns, 64, or 32 for plans without items of more than 64: softmax warps without a live row only take part in the

@@ -689,9 +689,14 @@ __device__ __forceinline__ uint32_t pack_bf16x2_from2(uint64_t v) {
     return r;
 }
 // e4m3 (saturating, to nearest even) and f16, two at a time: element 0 in the low half
-__device__ __forceinline__ uint32_t pack_e4m3x2(float lo, float hi) {
+__device__ __forceinline__ uint32_t f16x2_to_e4m3x2(uint32_t v) {   // in the low half
     uint32_t r;
-    asm("{\n\t.reg .b16 t;\n\tcvt.rn.satfinite.e4m3x2.f32 t, %1, %2;\n\tmov.b32 %0, {t, 0};\n\t}" : "=r"(r) : "f"(hi), "f"(lo));
+    asm("{\n\t.reg .b16 t;\n\tcvt.rn.satfinite.e4m3x2.f16x2 t, %1;\n\tmov.b32 %0, {t, 0};\n\t}" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t sub_f16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
 __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t v) {   // the two low bytes; exact
