@@ -320,7 +320,16 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                     // denominator, counted once per query row and head: in the piece that starts the list
                     const float sink2 = rm.live ? __ldg(p.attn_sink + rm.head) * 1.4426950408889634f : -INFINITY;
                     if (m_out == -INFINITY) m_out = sink2;                      // no valid score in this piece: the sink is the reference
-                    if (wi.k_begin == 0 && sink2 > -INFINITY) ls += ex2_approx(sink2 - m_out + kPShift);
+                    if (wi.k_begin == 0 && sink2 > -INFINITY) {
+                        const float d = sink2 - m_out;
+                        if (d > 0.0f) {   // a sink above the scores is the reference, so that nothing overflows
+                            const float f = ex2_approx(-d);
+                            ls *= f;
+                            v_unit *= f;
+                            m_out = sink2;
+                        }
+                        ls += ex2_approx(fminf(d, 0.0f) + kPShift);
+                    }
                 }
                 const float inv = ls > 0.0f ? v_unit / ls : 0.0f;
                 const float lse_nat = ls > 0.0f ? (m_out - kPShift + __log2f(ls)) * 0.69314718055994531f : INFINITY;

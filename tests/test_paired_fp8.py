@@ -95,3 +95,27 @@ def test_nan_codes_and_scales_reach_only_their_own_queries(built_lib):
         out, _, _ = run_gpu(dict(case, kv=bad), SCALE)
         assert np.isnan(_f32(out)[1]).any(axis=-1).all()
         np.testing.assert_array_equal(out[[0, 2]], clean[[0, 2]])
+
+
+@pytest.mark.parametrize("num_sms", [6, 148])
+def test_sinks_far_above_the_scores(built_lib, num_sms):
+    """A sink 10 nats above a row's lse leaves e^-10 of its output, one 85 or 300 above it next to nothing, and lse is theirs (whole and split items)."""
+    import torch
+    from gpu_util import to_dev
+    from opfoundry_b200 import api
+    H, topk = 48, 700
+    case = synth.make_decode_case(3, H, 1024, topk, fp8=True, paged=True, seed=9)
+    d = to_dev(case)
+    plan = api.mla_decode_plan_create(3, H, topk, num_sms=num_sms)
+    assert (plan.info.num_partials > 0) == (num_sms == 148)
+    kw = dict(block_table=d["block_table"], page_block_size=case["page_block_size"], kv_batch_stride_rows=case["kv_batch_stride_rows"])
+    run = lambda sink: [x.float() for x in api.mla_v4_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, attn_sink=sink, **kw)]
+    out0, lse0 = run(torch.full((H,), -float("inf"), device="cuda"))
+    above = torch.tensor([10.0, 85.0, 300.0] * (H // 3), device="cuda")
+    sink = lse0[0] + above      # of query row 0
+    out, lse = run(sink)
+    assert torch.isfinite(out).all() and torch.isfinite(lse).all()
+    torch.testing.assert_close(lse[0], torch.logaddexp(lse0[0], sink), rtol=1e-5, atol=1e-3)
+    weight = torch.sigmoid(lse0[0] - sink)[:, None]
+    scale = out0[0].abs().amax(dim=1, keepdim=True) * weight
+    assert ((out[0] - out0[0] * weight).abs() <= 1e-2 * scale + 1e-37).all()
