@@ -252,12 +252,12 @@ inline int build_plan_split(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
 }
 
 // Largest cost (tile steps + per-piece overhead) any list of the plan carries.
-inline int64_t plan_makespan(const HostPlan& P) {
+inline int64_t plan_makespan(const HostPlan& P, int overhead) {
     int64_t worst = 0;
     for (size_t l = 0; l + 1 < P.list_indptr.size(); ++l) {
         int64_t c = 0;
         for (int w = P.list_indptr[l]; w < P.list_indptr[l + 1]; ++w)
-            c += (P.works[w].k_end - P.works[w].k_begin + kTileRows - 1) / kTileRows + kPieceOverheadTiles;
+            c += (P.works[w].k_end - P.works[w].k_begin + kTileRows - 1) / kTileRows + overhead;
         worst = std::max(worst, c);
     }
     return worst;
@@ -318,7 +318,16 @@ inline int build_plan_whole(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
 // The plan a shape gets: the balanced one, unless the plan without splits is nearly as even.  A split
 // costs what the makespan does not show: fp32 partial results written and read back (4x the bytes of
 // the bf16 output) and the merge after the attention kernel, together worth about kMergeCostTiles steps.
+// On the 128-row kernels (more than kSmallHeads heads) a piece costs more than the cuts assume - Q, the refilled pipeline and 128 fp32
+// rows to store, about 10 000 cycles where a step takes 600 - so there the two plans are compared with dearer pieces, too, where
+// every second list gets a unit at least (and none has stacked rows, which were not measured).  By how much longer the whole plan's
+// longest list then is (in steps): rows x slots, split -> whole, 128 heads, us
+//   -7: 134 x 2048 fp8 114.1 -> 106.0, bf16 88.3 -> 79.3      -6: 47 x 1000 39.0 -> 33.0, 31.3 -> 26.2      -4: 56 x 2048 60.2 -> 55.5, 49.1 -> 40.6
+//   -1: 128 x 2048 114.5 -> 105.8, 87.4 -> 79.6       2: 50 x 2048 56.3 -> 55.2, 45.5 -> 40.2; 30 x 1000 31.1 -> 31.8, 25.4 -> 23.4
+//    4: 26 x 1000 28.3 -> 31.8, 24.0 -> 22.9; 40 x 1500 42.6 -> 43.4, 33.8 -> 32.3       6: 105 x 1300 73.5 -> 76.3, 56.0 -> 53.7
+//   10: 10 x 512 18.2 -> 20.8, 15.6 -> 15.8      13: 112 x 2048 100.0 -> 105.4, 78.2 -> 75.4      25: 100 x 2048 92.2 -> 105.5, 73.2 -> 73.4
 constexpr int kMergeCostTiles = 6;
+constexpr int kWidePieceOverheadTiles = 20, kWideMergeCostTiles = 2;
 inline int build_plan(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
     int rc = build_plan_split(sh, num_sms, P);
     if (rc) return rc;
@@ -326,7 +335,9 @@ inline int build_plan(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
     HostPlan W;
     rc = build_plan_whole(sh, num_sms, W);
     if (rc) return rc;
-    if (plan_makespan(W) <= plan_makespan(P) + kMergeCostTiles) P = W;
+    const auto whole_within = [&](int overhead, int steps) { return plan_makespan(W, overhead) <= plan_makespan(P, overhead) + steps; };
+    const bool wide = sh.H > kSmallHeads && !P.hdr.has_stacked && 2 * int(W.works.size()) >= P.hdr.num_lists;
+    if (whole_within(kPieceOverheadTiles, kMergeCostTiles) || (wide && whole_within(kWidePieceOverheadTiles, kWideMergeCostTiles))) P = W;
     return DSA_V32_OK;
 }
 
