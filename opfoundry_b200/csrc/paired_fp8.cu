@@ -34,17 +34,17 @@
 //   warps 20-23  row loaders: 16-byte cp.async copies into the swizzled tile, eight rows of every tile each
 //   warps 24-31  converters: e4m3 -> f16, eight of a tile's rows each; four of them fetch the own output columns of the other CTA's rows
 //
-// What bounds it (cycle stamps of an instrumented copy, 64 sequences x 128 heads x 2048 slots): a tile of 64 slots every 2 780 cycles.  Its MMAs
+// What bounds it (cycle stamps of an instrumented copy, 64 sequences x 128 heads x 2048 slots): a tile of 64 slots every 2 300 cycles.  Its MMAs
 // take 1 430 (measured alone; the scores' 25 an instruction are the rate of shared memory, 3 KB of operands each), all its traffic in shared
-// memory 2 100; what is in flight - three raw tiles, one and a half converted ones - over the 10 500 cycles from a load to the end of P V gives the rest:
+// memory 2 000; what is in flight - four raw tiles, one and a half converted ones - over the 10 000 cycles from a load to the end of P V gives the rest:
 // landing 1 900, scores 1 500, softmax 3 100, a converter's turn 2 200.  Every role pays for the number of its instructions, 6 700 a tile and SM:
-// seven or eight warps of a scheduler on five loops miss the instruction cache (4.7 of 19.6 cycles an instruction in a form of 85 KB; a warp number known
+// eight warps of a scheduler on five loops miss the instruction cache (4.7 of 19.6 cycles an instruction in a form of 85 KB; a warp number known
 // to be uniform, short waits and rolled loops brought 81 us to 61).  Tried: four teams of four warps with 32 slots a thread (fewer instructions, but
-// a tile takes 5 000 cycles from scores to P: 2 880 a tile), two teams of four (2 750, and 1.5 us more for one sequence), a converter on
-// both units of a tile (3 240).
+// a tile takes 5 000 cycles from scores to P: 2 880 a tile where two teams of eight took 2 780), two teams of four (2 750, and 1.5 us more for one
+// sequence), a converter on both units of a tile (3 240).  The other CTA's rows in the raw tiles, three of 28 KB: 60.6 us instead of 56.5.
 // Against the kernel before it (the 576 columns split over the pair, partial scores summed through distributed shared memory in 16 bits, four tile
-// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots: one sequence 19.6 -> 16.8 us, 8192 positions each: 16 33.8 -> 29.0, 37 58.7 -> 43.8,
-// 64 84.4 -> 59.7, 128 161 -> 117; 32768 positions each: 16 35.5 -> 31.0, 64 82.8 -> 65.9.
+// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots: one sequence 19.5 -> 16.4 us, 16 35.6 -> 30.3, 64 84.2 -> 62.1 (32768 positions each,
+// other inputs every pass); 37 58.7 -> 43.7, 128 161 -> 106 (8192 positions).
 // Against 64 bits, six shapes of 40 to 128 heads: out 1.68e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to 2.30e-3),
 // lse at most 1.9e-6 (7e-5).
 //
