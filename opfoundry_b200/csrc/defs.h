@@ -10,9 +10,9 @@ namespace dsa {
 constexpr int kDQK = DSA_V32_D_QK;      // 576
 constexpr int kDV = DSA_V32_D_V;        // 512
 constexpr int kDRope = DSA_V32_D_ROPE;  // 64
-constexpr int kHeadsPerBlock = 128;     // MMA M: one head per TMEM lane
+constexpr int kHeadsPerBlock = 128;     // tile rows: M of the pair MMAs
 constexpr int kDvHalf = 256;            // output columns accumulated by one CTA of a pair
-constexpr int kTileRows = 32;           // top-k slots per pipeline step
+constexpr int kTileRows = 32;           // top-k slots per step of the planner
 constexpr int kSmallHeads = 32;         // most tile rows an item may have for the few-heads kernel
 constexpr int kFp8RowBytes = DSA_V32_FP8_ROW_BYTES;
 

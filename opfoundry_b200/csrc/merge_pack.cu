@@ -22,21 +22,23 @@ __global__ void debug_rows_kernel(AttnParams p, int total_q, int32_t* rows_out) 
 // empty -> 0, +inf.
 // The partials were written by the kernel before and come from L2 (16 splits x 128 heads: 4 MB), so the time is a
 // chain of load latencies, not bytes: the plan's tables are read before the wait for the attention kernel, lane i then
-// fetches the lse of split i while the first partial rows (eight float4 per lane) are already on their way.
+// fetches the lse of split i while the first partial rows (eight or sixteen float4 per lane) are already on their way.
 // kV = float4 per lane and split: a warp covers 128 kV columns of one tile row, a block four warps.  kV = 1 (a block per
 // row) while all blocks are resident at once, else kV = 4 (a warp per row), which needs a quarter of the blocks.
 // Measured: decode of one sequence (16 splits) 25.3 -> 19.8 us, batch 16 37.1 -> 35.4 us, two sequences of 16 heads on a bf16
 // cache 21.5 -> 15.9 us, against one warp per row that walked the splits one by one (slot, then lse, then four float4).
 // With kV = 1 throughout, a prefill chunk of 64 split rows x 64 heads took 8.9 us for its merge instead of 5.2.
-constexpr int kMergeFlight = 8;                       // float4 in flight per lane
-constexpr int kMergeBlocks = 8;                       // blocks per SM of the form with kV = 1 (64 registers per thread)
-template <int kV>
-__global__ void __launch_bounds__(128, kV == 1 ? kMergeBlocks : kMergeBlocks - 1) combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
+// kFlight = float4 in flight per lane: 16, so that the 16 splits of a row come in one round, where four blocks an SM are enough (one sequence 16.55 -> 16.15 us,
+// two sequences of 16 heads on a bf16 cache 12.42 -> 12.00; with 16 throughout, 16 sequences 30.35 -> 30.45, 100 92.2 -> 94.5), else 8.
+constexpr int kMergeBlocks = 8;                       // blocks per SM of the form with kV = 1, kFlight = 8 (64 registers per thread)
+constexpr int kMergeBlocksDeep = 4;                   // and with kFlight = 16
+template <int kV, int kFlight>
+__global__ void __launch_bounds__(128, kFlight == 16 ? kMergeBlocksDeep : kV == 1 ? kMergeBlocks : kMergeBlocks - 1) combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
                                                       const int32_t* __restrict__ reduce_indptr,
                                                       const int32_t* __restrict__ reduce_slots,
                                                       const ReduceDst* __restrict__ reduce_dst, const OutTargets tgt,
                                                       int64_t stride_o_row, int64_t stride_o_head, int H) {
-    constexpr int kF = kMergeFlight / kV;    // splits in flight
+    constexpr int kF = kFlight / kV;    // splits in flight
     const int rr = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hrow = kV == 1 ? blockIdx.y : blockIdx.y * 4 + warp;   // row of the 128-row tile
@@ -225,7 +227,8 @@ cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const i
     int sms = 0;
     cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
-    const bool wide = (int64_t)num_reduce_rows * tile_rows > int64_t(sms) * kMergeBlocks;
+    const int64_t rows = (int64_t)num_reduce_rows * tile_rows;
+    const bool wide = rows > int64_t(sms) * kMergeBlocks, deep = rows <= int64_t(sms) * kMergeBlocksDeep;
     dim3 grid(num_reduce_rows, wide ? (tile_rows + 3) / 4 : tile_rows);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -236,7 +239,7 @@ cudaError_t launch_combine(const float* o_accum, const float* lse_accum, const i
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, wide ? combine_kernel<4> : combine_kernel<1>, o_accum, lse_accum, reduce_indptr, reduce_slots, reduce_dst, tgt, stride_o_row,
+    return cudaLaunchKernelEx(&cfg, wide ? combine_kernel<4, 8> : deep ? combine_kernel<1, 16> : combine_kernel<1, 8>, o_accum, lse_accum, reduce_indptr, reduce_slots, reduce_dst, tgt, stride_o_row,
                               stride_o_head, H);
 }
 

@@ -43,7 +43,7 @@
 // a tile takes 5 000 cycles from scores to P: 2 880 a tile where two teams of eight took 2 780), two teams of four (2 750, and 1.5 us more for one
 // sequence), a converter on both units of a tile (3 240).  The other CTA's rows in the raw tiles, three of 28 KB: 60.6 us instead of 56.5.
 // Against the kernel before it (the 576 columns split over the pair, partial scores summed through distributed shared memory in 16 bits, four tile
-// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots: one sequence 19.5 -> 16.4 us, 16 35.6 -> 30.3, 64 84.2 -> 62.1 (32768 positions each,
+// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots: one sequence 19.5 -> 16.0 us with its merge, 16 35.6 -> 30.2, 64 84.2 -> 62.1 (32768 positions each,
 // other inputs every pass); 37 58.7 -> 43.7, 128 161 -> 106 (8192 positions).
 // Against 64 bits, six shapes of 40 to 128 heads: out 1.68e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to 2.30e-3),
 // lse at most 1.9e-6 (7e-5).

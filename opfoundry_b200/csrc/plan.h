@@ -7,8 +7,8 @@
 // kTileRows top-k slots plus a fixed per-piece overhead (query load + epilogue), mirroring the
 // reference's "kv blocks + fixed_overhead" cost (get_mla_metadata.hpp:27-37).  A work list
 // belongs to one CTA pair, so there are num_sms / 2 lists instead of the reference's 256 compute units.
-// The two CTAs of a pair split an item by columns (fp8 cache) or heads (bf16 cache) in the 128-row kernels and by slots in the few-heads kernel; the
-// plan is the same for all, its unit and its overhead being those of the 128-row kernel of the fp8 cache.  (Of the few-heads kernel's own: an
+// The two CTAs of a pair split an item by heads in the 128-row kernels and by slots in the few-heads kernel; the plan is the same for all, in steps of 32 slots
+// with the overhead that suited the 128-row kernel of an fp8 cache when its tiles had 32.  (Of the few-heads kernel's own: an
 // overhead of 12 steps was neutral, a merge cost of 60 made 128 sequences of 2 x 16 heads 195 us instead of 186, least pieces of
 // two or three steps 19.1-20.3 us for one sequence against 19.6.)
 //
