@@ -15,10 +15,12 @@
 // Numbers.  Scores: an element of Q has 8 significant bits, so after a power-of-two factor per row (largest magnitude into
 // [128, 256)) it is hi + lo with both in e4m3, exact down to 2^-10 of the row's largest magnitude and to 2^-18 of that magnitude below;
 // products and sums are those of the bytes themselves, and the scales (fp32) multiply the finished group sums.
-// P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15; V = byte x scale 2^-e
-// with one e for the tile's 64 rows, so that the largest |V| stays below 2^16.  e starts at the exponent of the largest scale of an
-// item's first tile and moves up when a scale exceeds it by 2^7; O is then brought to the new e like it is to a new reference maximum.
-// What falls below f16's smallest step is 2^-33 of the largest V.
+// P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15; V = byte x scale 2^-e, rounded once,
+// with one e per scale group for the tile's 64 rows, so that the largest |V| stays below 2^16.  e starts at the exponent of the group's largest
+// scale in an item's first tile and moves up when a scale exceeds it by 2^7; the group's columns of O are then brought to the new e like they are to a
+// new reference maximum.  A row whose scales all lie more than 2^8 below their e lends V the difference, x = 20 octaves at most, and P takes it
+// back (V 2^x, P 2^-x): f16 alone would lose the rows' bits beside a large row from 2^-14 on.  What is left below f16's normal range then is
+// 2^-41 of the largest V at full weight (a group of a row that is small only beside another group of the same row: 2^-21).
 //
 // S in TMEM: lanes 0-63 = the CTA's 64 rows x slots of CTA 0, lanes 64-127 = the same rows x slots of CTA 1.
 // O in TMEM: lanes 0-63 = the rows x columns of CTA 0, lanes 64-127 = the rows x columns of CTA 1.
@@ -85,7 +87,7 @@ constexpr int kOffRaw = 9 * kQBlock;
 constexpr int kOffV = kOffRaw + kStages * kRawBytes;
 constexpr int kOffP = kOffV + kVUnits * kVUnit;
 constexpr int kOffCtl = kOffP + 2 * kPBytes;
-constexpr int kCtlBytes = 9216;
+constexpr int kCtlBytes = 10240;
 constexpr int kSmemBytes = kOffCtl + kCtlBytes;
 static_assert(kSmemBytes <= 232448, "227 KB per CTA");
 // TMEM columns: O 256 | S: groups 0-2 of even tiles, of odd tiles, group 3, rope, 32 columns each
@@ -98,8 +100,11 @@ struct Ctl {
     uint8_t q_exp[kRows];                    // biased exponent of 2^a, Q = 2^a (hi + lo); 255: a row with an infinity or a NaN
     int32_t late_row[kStages][kOwn];         // rows of the tile that the other CTA gathers
     uint32_t tile_mask[kStages][2];          // which slots of CTA 0 / CTA 1 hold a row
-    float v_mul[kStages], v_unit[kStages], v_fix[kStages];   // 2^-e of the tile, 2^e, and 2^(e of the tile before - e)
-    float v_fin;                             // 2^e of the item's last tile
+    alignas(8) float2 v_move[kStages][kGroups];          // 2^(e of the tile before - e), 2^e
+    alignas(8) float2 v_mul[kStages][kGroups];           // 2^-e, and 1 where some group of a row needs more than that, else 0
+    float v_lent[kStages][kSlots];           // then: 2^x of the rows
+    alignas(16) uint16_t p_back[kStages][kSlots];        // and 2^-x in f16
+    float v_fin[kGroups];                    // 2^e of the item's last tile
     uint64_t late_known[kStages];                      // late_row is written
     uint64_t kv_full[kStages], raw_empty[kStages];     // rows landed | scores complete, rows converted, scales read
     uint64_t prep[kStages];                            // ... and e known
@@ -302,7 +307,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         int item_n = 0;
         Ring<kStages> ring;   // of this team's tiles: every other one
         if (team) ring.next();
-        float ls = 0.0f, m_out = 0.0f, v_unit = 1.0f;   // of the last item: its row sum, last reference and 2^e
+        float ls = 0.0f, m_out = 0.0f, v_unit = 1.0f;   // of the last item: its row sum, last reference and 2^e of the columns that this thread reads out
 #pragma unroll 1
         for (int w = w_begin; w <= w_end; ++w, ++item_n) {
             // ---- Q of this item, so that its scores can start; then the output of the one before
@@ -434,6 +439,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 uint64_t sv[8];
                 uint32_t mask;
                 float v_fix;
+                bool lent;
                 {
                     const uint32_t ca = lane_base + kColS + 96 * team + 16 * cs;
                     const float* sc = &ctl->scale[ring.s][0][kOwn * h + 16 * cs];
@@ -441,8 +447,10 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                     tmem_ld16(lane_base + kColS3 + 16 * cs, x[1]);
                     tmem_ld16(lane_base + kColRope + 16 * cs, sr);
                     mask = ctl->tile_mask[ring.s][h] >> (16 * cs);
-                    v_fix = ctl->v_fix[ring.s];
-                    v_unit = ctl->v_unit[ring.s];
+                    const float2 move = ctl->v_move[ring.s][2 * h + cs];
+                    v_fix = move.x;
+                    v_unit = move.y;
+                    lent = __any_sync(0xffffffffu, ctl->v_mul[ring.s][0].y != 0.0f);
                     tmem_wait_ld();
                     tmem_loaded(x[1]);
                     tmem_loaded(sr);
@@ -467,7 +475,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             warp_arrive_lead(&ctl->s_empty[team], lane);
                         }
                     }
-                    warp_arrive(&ctl->raw_empty[ring.s], lane);
+                    if (!lent) warp_arrive(&ctl->raw_empty[ring.s], lane);
                 }
                 if ((mask & 0xFFFFu) != 0xFFFFu) {
 #pragma unroll
@@ -530,6 +538,14 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 }
                 if (l != 0.0f && m_was != m_ref) l *= ex2_approx(m_was - m_ref);
                 l += lsum;
+                if (lent) {   // what V was lent
+                    const uint4* back = reinterpret_cast<const uint4*>(&ctl->p_back[ring.s][kOwn * h + 16 * cs]);
+                    const uint4 b0 = back[0], b1 = back[1];
+                    const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) pk[j] = mul_f16x2(pk[j], b[j]);
+                    warp_arrive(&ctl->raw_empty[ring.s], lane);
+                }
                 // ---- into the P buffer, once the product that read it last is complete
                 if (it >= 2)
                     if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) goto done;
@@ -562,14 +578,14 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             const float m_fin = ctl->m_ref[last_team][r];
             if (l != 0.0f && m_ref != m_fin) l *= ex2_approx(m_ref - m_fin);
             ctl->post[team][2 * h + cs][r] = l;
-            if (team == static_cast<int>(last_team) && (warp & (kTeamWarps - 1)) == 0 && lane == 0) ctl->v_fin = v_unit;
+            if (team == static_cast<int>(last_team) && rq == 0 && lane == 0) ctl->v_fin[2 * h + cs] = v_unit;
             warp_arrive(&ctl->e_bar, lane);
             if (!wait_on(&ctl->e_bar, item_n & 1, abort_flag)) goto done;
             m_out = m_fin;
             ls = 0.0f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) ls += ctl->post[i >> 2][i & 3][r];
-            v_unit = ctl->v_fin;
+            v_unit = ctl->v_fin[2 * h + team];   // the read-out's 64 columns lie in this group
         }
     } else if (warp < kLoadWarp0) {
         setmaxnreg_dec<kRegsIssuers>();
@@ -654,30 +670,74 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             // ======================================================== this CTA's rows' arrival, passed on to the issuers; e
             uint32_t it = 0;
             Ring<kStages> ring;
+            int e = 0;   // lane: that of group lane % 4
             for (int w = w_begin; w < w_end; ++w) {
                 const int n_tiles = tiles_of(p.works[w]);
-                int e = 0;
                 for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
                     if (!wait_on(&ctl->kv_full[ring.s], ring.ph, abort_flag)) goto done;
                     fence_proxy_async_smem();   // written by cp.async (generic proxy)
                     warp_arrive_lead(&ctl->tile_ready[it & 1u][ring.s], lane);
-                    // largest finite scale of the tile's rows (of both CTAs' slots and all groups, so both CTAs follow the same e)
-                    uint32_t m = 0u;
+                    // exponents of the scales of slots 2 lane (low half) and 2 lane + 1 (biased; 0: none that counts)
+                    uint32_t a[kGroups];
 #pragma unroll
                     for (int g = 0; g < kGroups; ++g) {
                         const float2 s = *reinterpret_cast<const float2*>(&ctl->scale[ring.s][g][2 * lane]);
-                        const uint32_t a = __float_as_uint(s.x) & 0x7FFFFFFFu, b = __float_as_uint(s.y) & 0x7FFFFFFFu;
-                        m = max(m, max(a < 0x7F800000u ? a : 0u, b < 0x7F800000u ? b : 0u));
+                        const uint32_t x = (__float_as_uint(s.x) >> 23) & 0xFFu, y = (__float_as_uint(s.y) >> 23) & 0xFFu;
+                        a[g] = (x < 255u ? x : 0u) | (y < 255u ? y : 0u) << 16;
                     }
-                    m = __reduce_max_sync(0xffffffffu, m);
-                    const int em = max(static_cast<int>(m >> 23) - 127, -120);
+                    uint32_t most = max_u16x2(max_u16x2(a[0], a[1]), max_u16x2(a[2], a[3]));
+                    const uint32_t spread = most - min_u16x2(min_u16x2(a[0], a[1]), min_u16x2(a[2], a[3]));
+                    if (__any_sync(0xffffffffu, max(spread & 0xFFFFu, spread >> 16) > 12u)) {
+                        // a group may be zeros under any scale (the cache writer gives it 1): then the scale does not count and becomes 0
+                        const uint32_t odd = __ballot_sync(0xffffffffu, (spread & 0xFFFFu) > 12u), odd1 = __ballot_sync(0xffffffffu, (spread >> 16) > 12u);
+#pragma unroll 1
+                        for (int slot = 0; slot < kSlots; ++slot) {
+                            if (!(((slot & 1 ? odd1 : odd) >> (slot >> 1)) & 1u)) continue;
+                            const bool own = slot / kOwn == rank;
+                            const int late = ctl->late_row[ring.s][slot % kOwn];
+#pragma unroll
+                            for (int g = 0; g < kGroups; ++g) {
+                                uint32_t v = 0u;
+                                if (own) v = *reinterpret_cast<const uint32_t*>(sRaw + ring.s * kRawBytes + g * kBlock + (slot % kOwn) * 128 + 4 * lane);
+                                else if (late >= 0) v = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(p.kv) + (size_t)late * kFp8RowBytes + 128 * g) + lane);
+                                const uint32_t half = slot & 1 ? 0xFFFF0000u : 0xFFFFu;
+                                if (!__any_sync(0xffffffffu, (v & 0x7F7F7F7Fu) != 0u) && lane == slot >> 1 && (a[g] & half) != 0u) {
+                                    a[g] &= ~half;
+                                    ctl->scale[ring.s][g][slot] = 0.0f;   // (f16 may not hold what is left of it below)
+                                }
+                            }
+                        }
+                    }
+                    // the largest of the tile's rows (of both CTAs' slots, so both CTAs follow the same e)
+                    uint32_t top = 0u;
+#pragma unroll
+                    for (int g = 0; g < kGroups; ++g) {
+                        const uint32_t m = __reduce_max_sync(0xffffffffu, max(a[g] & 0xFFFFu, a[g] >> 16));
+                        if ((lane & 3) == g) top = m;
+                    }
+                    const int em = max(static_cast<int>(top) - 127, -120);
                     const int e_old = e;
                     if (t == 0 || em >= e + 7) e = min(em, 126);
-                    if (lane == 0) {
-                        ctl->v_mul[ring.s] = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
-                        ctl->v_unit[ring.s] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+                    // how far a row's groups lie below their e, 512 added: the least and the most of them
+                    uint32_t low = 0xFFFFFFFFu, deep = 0u;
+                    most = 0u;
+#pragma unroll
+                    for (int g = 0; g < kGroups; ++g) {
+                        const uint32_t d = __shfl_sync(0xffffffffu, (e + 127 + 512) * 0x10001, g) - a[g];
+                        low = min_u16x2(low, d);
+                        deep = max_u16x2(deep, d);
+                        most |= a[g];
+                    }
+                    const int x0 = most & 0xFFFFu ? min(max(static_cast<int>(low & 0xFFFFu) - 520, 0), 20) : 0, x1 = most >> 16 ? min(max(static_cast<int>(low >> 16) - 520, 0), 20) : 0;
+                    const bool lent = __any_sync(0xffffffffu, (most & 0xFFFFu && static_cast<int>(deep & 0xFFFFu) > 520) || (most >> 16 && static_cast<int>(deep >> 16) > 520));
+                    if (lent) {
+                        *reinterpret_cast<float2*>(&ctl->v_lent[ring.s][2 * lane]) = make_float2(__uint_as_float((127 + x0) << 23), __uint_as_float((127 + x1) << 23));
+                        reinterpret_cast<uint32_t*>(ctl->p_back[ring.s])[lane] = pow2_f16(-x0) | pow2_f16(-x1) << 16;
+                    }
+                    if (lane < kGroups) {
                         const int d = t == 0 ? 0 : e_old - e;
-                        ctl->v_fix[ring.s] = d < -126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 + d) << 23);
+                        ctl->v_move[ring.s][lane] = make_float2(d < -126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 + d) << 23), __uint_as_float(static_cast<uint32_t>(127 + e) << 23));
+                        ctl->v_mul[ring.s][lane] = make_float2(__uint_as_float(static_cast<uint32_t>(127 - e) << 23), lent ? 1.0f : 0.0f);
                     }
                     warp_arrive(&ctl->prep[ring.s], lane);
                 }
@@ -758,9 +818,25 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         const int r = 8 * (cw & 3) + r4;   // of the first two steps; the others take the row four further
         const uint32_t v0 = smem_u32(sV) + half * kBlock + r * 128 + (((2 * k) ^ (r & 7)) << 4);
         // lane i < 16 (and i + 16): the scale of block i / 8, row i % 8
-        const float* const scale0 = &ctl->scale[0][2 * rank + ((lane >> 3) & 1)][kOwn * u + 8 * (cw & 3) + (lane & 7)];
+        const int sg = 2 * rank + ((lane >> 3) & 1), ss = kOwn * u + 8 * (cw & 3) + (lane & 7);
+        // ... times 2^-e as a sum of two f16 with 22 significant bits, and, where that takes more than f16's range, the power of two that the bytes are
+        // multiplied with before (exact)
+        uint32_t scales = 0u, pre = 0u;
+        bool lent = false;
+        auto load_scale = [&](uint32_t st) {
+            const float2 m = ctl->v_mul[st][sg];
+            float f = ctl->scale[st][sg][ss] * m.x;
+            lent = __any_sync(0xffffffffu, m.y != 0.0f);   // (a vote, so that it is known to be the same in all lanes)
+            if (lent) {
+                f *= ctl->v_lent[st][ss];
+                const int k = min(max(123 - static_cast<int>((__float_as_uint(f) >> 23) & 0xFFu), 0), 15);
+                f *= __uint_as_float((127 + k) << 23);
+                pre = pow2_f16(-k) * 0x10001u;
+            }
+            scales = split_f16(f);
+        };
         // one chunk of either block of a row, scaled, to V
-        auto convert = [&](const uint4 (&x)[2], uint32_t scales, int i, uint32_t dst) {
+        auto convert = [&](const uint4 (&x)[2], int i, uint32_t dst) {
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint32_t s = __shfl_sync(0xffffffffu, scales, 8 * b + 4 * i + r4);
@@ -768,10 +844,14 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 const uint32_t v[4] = {x[b].x, x[b].y, x[b].z, x[b].w};
                 uint32_t y[8];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    y[2 * j] = scale_f16x2(e4m3x2_to_f16x2(v[j]), hi, lo);
-                    y[2 * j + 1] = scale_f16x2(e4m3x2_to_f16x2(v[j] >> 16), hi, lo);
+                for (int j = 0; j < 8; ++j) y[j] = e4m3x2_to_f16x2(v[j >> 1] >> (16 * (j & 1)));
+                if (lent) {
+                    const uint32_t m = __shfl_sync(0xffffffffu, pre, 8 * b + 4 * i + r4);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) y[j] = mul_f16x2(y[j], m);
                 }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] = scale_f16x2(y[j], hi, lo);
                 sts_16(dst + 2 * b * kBlock, y[0], y[1], y[2], y[3]);
                 sts_16((dst ^ 16u) + 2 * b * kBlock, y[4], y[5], y[6], y[7]);
             }
@@ -788,7 +868,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
 #pragma unroll 1
                 for (int t = 0; t < n_tiles; ++t, ring.next(), unit.next(), unit.next()) {
                     if (!wait_on2(&ctl->prep[ring.s], ring.ph, &ctl->v_empty[unit.s], unit.ph, abort_flag)) goto done;
-                    const uint32_t scales = split_f16(scale0[ring.s * (kGroups * kSlots)] * ctl->v_mul[ring.s]);   // as a sum of two f16
+                    load_scale(ring.s);
                     uint32_t src = raw0 + ring.s * kRawBytes, dst = v0 + unit.s * kVUnit;
                     uint4 x[2] = {lds_16(src), lds_16(src + kBlock)};
 #pragma unroll 1
@@ -801,7 +881,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                         } else {
                             warp_arrive(&ctl->raw_empty[ring.s], lane);
                         }
-                        convert(cur, scales, i, dst);
+                        convert(cur, i, dst);
                         dst = (dst ^ 64u) + 512u;
                     }
                     fence_proxy_async_smem();
@@ -837,12 +917,12 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                         known.next();
                     }
                     if (!wait_on2(&ctl->prep[ring.s], ring.ph, &ctl->v_empty[unit.s], unit.ph, abort_flag)) goto done;
-                    const uint32_t scales = split_f16(scale0[ring.s * (kGroups * kSlots)] * ctl->v_mul[ring.s]);
+                    load_scale(ring.s);
                     const uint32_t dst = v0 + unit.s * kVUnit;
-                    convert(x[0], scales, 0, dst);
+                    convert(x[0], 0, dst);
                     load(x[0], next0);
                     warp_arrive(&ctl->raw_empty[ring.s], lane);
-                    convert(x[1], scales, 1, (dst ^ 64u) + 512u);
+                    convert(x[1], 1, (dst ^ 64u) + 512u);
                     load(x[1], next1);
                     fence_proxy_async_smem();
                     warp_arrive_lead(&ctl->v_full[unit.s], lane);

@@ -712,7 +712,14 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
 __device__ __forceinline__ void unpack_f16x2(uint32_t v, float& lo, float& hi) {
     asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.f32.f16 %0, a;\n\tcvt.f32.f16 %1, b;\n\t}" : "=f"(lo), "=f"(hi) : "r"(v));
 }
-// s = hi + lo in f16, hi in the low half: 22 significant bits
+__device__ __forceinline__ uint32_t mul_f16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// 2^n in f16, n from -24 to 15
+__device__ __forceinline__ uint32_t pow2_f16(int n) { return n >= -14 ? static_cast<uint32_t>(n + 15) << 10 : 1u << (n + 24); }
+// s = hi + lo in f16, hi in the low half: 22 significant bits from 2^-3 on, 2^-25 off below
 __device__ __forceinline__ uint32_t split_f16(float s) {
     const uint32_t hi = pack_f16x2(s, s);
     float a, b;
@@ -727,6 +734,11 @@ __device__ __forceinline__ uint32_t scale_f16x2(uint32_t v, uint32_t hi, uint32_
 }
 // two bf16 times a power of two
 __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float mul) { return pack_bf16x2(__uint_as_float(v << 16) * mul, __uint_as_float(v & 0xFFFF0000u) * mul); }
+__device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
 __device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));

@@ -1,5 +1,5 @@
-"""The 128-row kernel of an fp8 cache: Q as a sum of two e4m3 numbers per row factor, V scaled to f16 with one exponent for a tile that
-moves with the largest scale.  Tile edges, split and stacked items are in test_paired_heads."""
+"""The 128-row kernel of an fp8 cache: Q as a sum of two e4m3 numbers per row factor, V scaled to f16 with one exponent per scale group
+for a tile, which moves with the largest scale.  Tile edges, split and stacked items are in test_paired_heads."""
 import math
 
 import numpy as np
@@ -119,3 +119,58 @@ def test_sinks_far_above_the_scores(built_lib, num_sms):
     weight = torch.sigmoid(lse0[0] - sink)[:, None]
     scale = out0[0].abs().amax(dim=1, keepdim=True) * weight
     assert ((out[0] - out0[0] * weight).abs() <= 1e-2 * scale + 1e-37).all()
+
+
+def _in_list_order(case):
+    """Cache rows that a query's list names, slot by slot."""
+    idx, page = case["indices"], case["page_block_size"]
+    return [case["block_table"][b][idx[b] // page] * page + idx[b] % page for b in range(idx.shape[0])]
+
+
+def _check_groups(oracle, case, rel=4e-3):
+    """As _check, but each group of 128 columns against its own largest output, so that a small group counts as much as a large one."""
+    from gpu_util import run_gpu, run_oracle
+    g_out, g_lse, _ = run_gpu(case, SCALE, num_sms=4)
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    g, r = [_f32(x).reshape(x.shape[0], x.shape[1], 4, 128) for x in (g_out, r_out)]
+    assert np.isfinite(g).all()
+    assert (np.abs(g - r) <= rel * np.abs(r).max(axis=-1, keepdims=True) + 2.0 ** -8 * np.abs(r)).all()
+    check_lse(g_lse, r_lse)
+
+
+@pytest.mark.parametrize("amax", [1e-2, 1e-3, 1e-4, 1e-5, 1e-7])
+def test_rows_of_zeros_from_the_cache_writer_beside_small_ones(built_lib, oracle, amax):
+    """The cache writer gives a group of zeros the scale 1: it must not take precision from the other rows, whose scales are far smaller."""
+    case = _case(10)
+    latent = synth.stream(10, "kv").standard_normal(size=(case["kv"].shape[0], 512), dtype=np.float32) * np.float32(amax)
+    for rows in _in_list_order(case):
+        latent[rows[0]] = 0.0
+        latent[rows[5], 128:256] = 0.0      # a row with one such group
+    kv = synth.pack_fp8_rows(latent, np.ascontiguousarray(case["kv"][:, 528:]).view(np.uint16))
+    _check_groups(oracle, dict(case, kv=kv))
+
+
+@pytest.mark.parametrize("power", [-12, -24, -36])
+def test_one_group_far_smaller_than_the_others(built_lib, oracle, power):
+    case = _case(11)
+    kv = case["kv"].copy()
+    kv[:, 512:528].view(np.float32)[:, 2] *= np.float32(2.0 ** power)
+    _check_groups(oracle, dict(case, kv=kv))
+
+
+@pytest.mark.parametrize("power", [-14, -22, -30, -38])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_small_rows_that_carry_the_weight(built_lib, oracle, power, mixed):
+    """The rows with next to no weight (2^-60 and less) have the large scales, those that make the result the small ones: at the start of the list, or in every tile."""
+    case = _case(12, topk=512, B=2)
+    kv, q = case["kv"].copy(), _f32(case["q"]).copy()
+    rope = _f32(np.ascontiguousarray(kv[:, 528:]).view(np.uint16)).copy()
+    q[..., 512] = 24.0
+    rope[:, 0] = 0.0
+    for rows in _in_list_order(case):
+        few = rows[::7] if mixed else rows[:64]
+        rope[few, 0] = -32.0        # 24 x -32 / sqrt(192) = -55 nats
+        rest = np.setdiff1d(rows, few)
+        kv[rest, 512:528] = (kv[rest, 512:528].copy().view(np.float32) * np.float32(2.0 ** power)).view(np.uint8)
+    kv[:, 528:] = _bf16(rope).view(np.uint8).reshape(kv.shape[0], 128)
+    _check_groups(oracle, dict(case, kv=kv, q=_bf16(q)))

@@ -52,7 +52,8 @@ class PairFp8(Pair):
         self.prob, self.acc = [[[None] * TEAM, [None] * TEAM] for _ in range(2)], [None, None]
         self.post = [[[[None] * 4 for _ in range(2)] for _ in range(2)] for _ in range(2)]   # [cta][team][rows][quarter]
         self.ref = [[[None] * 2 for _ in range(2)] for _ in range(2)]                        # [cta][tile mod 2][rows]
-        self.v_fin = [None, None]
+        self.v_fin = [[None] * 4 for _ in range(2)]                              # [cta][scale group]
+        self.lent = [rng.random() < 0.3 for _ in range(7)]
         self.procs, self.queues = {}, []
         for c in range(2):
             for w in range(WARPS):
@@ -122,7 +123,9 @@ class PairFp8(Pair):
                 self.s_empty[team].arrive()
                 yield None
                 assert self.raw[c][ring.s] == [it] * LOADERS, "scales of another tile"
-                self.raw_empty[c][ring.s].arrive()
+                lent = self.lent[it % len(self.lent)]       # rows took more than 2^-e: P is multiplied with what stands beside e
+                if not lent:
+                    self.raw_empty[c][ring.s].arrive()
                 self.post[c][team][rq][2 * h + cs] = ("max", it)
                 self.posted[c][team][rq].arrive()
                 yield self.posted[c][team][rq], ph2
@@ -133,6 +136,10 @@ class PairFp8(Pair):
                 if h == 0 and cs == 0:
                     self.ref[c][team][rq] = it
                 self.moved[c][team][rq].arrive()
+                if lent:
+                    yield None
+                    assert self.e[c][ring.s] == it, "powers of two of another tile"
+                    self.raw_empty[c][ring.s].arrive()
                 if it >= 2:
                     yield self.pv_done[c][team], ph2 ^ 1
                 self.prob[c][team][w & 7] = it
@@ -148,12 +155,12 @@ class PairFp8(Pair):
             yield self.moved[c][last & 1][rq], (last >> 1) & 1
             assert self.idle(c, rq, n) or self.ref[c][last & 1][rq] == last, "references of another tile"   # (those of rows that are not live serve nobody)
             self.post[c][team][rq][2 * h + cs] = ("sum", n)
-            if team == last & 1 and w & 7 == 0:
-                self.v_fin[c] = n
+            if team == last & 1 and rq == 0:
+                self.v_fin[c][2 * h + cs] = n
             self.e_bar[c].arrive()
             yield self.e_bar[c], n & 1
             for _ in range(2):
-                assert all(x == ("sum", n) for t in range(2) for x in self.post[c][t][rq]) and self.v_fin[c] == n, "sums of another item"
+                assert all(x == ("sum", n) for t in range(2) for x in self.post[c][t][rq]) and self.v_fin[c][2 * h + team] == n, "sums of another item"
                 yield None
 
     def issuer(self, par, mma):
@@ -226,7 +233,7 @@ class PairFp8(Pair):
                 yield self.kv_full[c][ring.s], ring.ph
                 self.tile_ready[it & 1][ring.s].arrive()
                 yield None
-                assert self.raw[c][ring.s] == [it] * LOADERS, "scales of another tile"
+                assert self.raw[c][ring.s] == self.late[c][ring.s] == [it] * LOADERS, "scales of another tile"
                 self.e[c][ring.s] = it
                 self.prep[c][ring.s].arrive()
                 it += 1
