@@ -254,6 +254,7 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     if (peers) {
         p.n_peers = peers->num_peers;
         p.lse_stride_row = peers->lse_stride_row;
+        p.out = peers->out[peers->my_rank];   // (paired_fp8.cu uses this GPU's rows while their items run)
         for (int i = 0; i < peers->num_peers; ++i) {
             p.out_peers[i] = peers->out[i];
             p.lse_peers[i] = peers->lse[i];

@@ -7,14 +7,18 @@
 //
 // CTA c of the pair owns tile rows (heads) [64 c, 64 c + 64), or [32 c, 32 c + 32) where no item has more than 64, and, of every tile of 64 slots, gathers slots [32 c, 32 c + 32).
 //       S_g [128 x 64]  = Q_g K_g^T  cta_group::2, M = 128, N = 64, kind::f8f6f4, one accumulator per 128-column scale group g: B = the
-//                                    gathered e4m3 bytes, A = Q as the sum of two e4m3 numbers (below); the rope with bf16 operands
+//                                    gathered e4m3 bytes, A = Q as the sum of an e5m2 and an e4m3 number (below); the rope with bf16 operands
 //       O [128 x 512] += P V         cta_group::2, M = 128, N = 256, twice, kind::f16 on f16: A = each CTA's 64 rows of P, B = each
 //                                    CTA's 256 columns of all 64 gathered rows, scale x byte rounded once to f16
 // so a CTA holds the whole softmax of its heads: scores, maxima, P and output rows never cross to the other SM.
 //
 // Numbers.  Scores: an element of Q has 8 significant bits, so after a power-of-two factor per row (largest magnitude into
-// [128, 256)) it is hi + lo with both in e4m3, exact down to 2^-10 of the row's largest magnitude and to 2^-18 of that magnitude below;
-// products and sums are those of the bytes themselves, and the scales (fp32) multiply the finished group sums.
+// [2^11, 2^12)) it is hi + lo with hi in e5m2 (3 bits and the sign of what is left) and lo in e4m3 (4), exact down to 2^-13 of the row's largest magnitude
+// and to 2^-22 of that magnitude below; products and sums are those of the bytes themselves, and the scales (fp32) multiply the finished group
+// sums.  A row with more than kWideElements, zeros aside, below that line has a few far above the others, which the cache may answer with
+// zeros: there the softmax warps add what hi + lo leave out (residual_group), so the row is as exact as with bf16 operands.  (With an element X times the rest in a
+// column where the cache holds zeros, the error of lse is 2e-6 to 1.4e-5, the most at X = 2^8; the kernel before this one had 2.5e-5 to 6e-5 for any X.  A row of
+// normal numbers needs one of 2^9 for that; if all rows have one, 64 sequences of 128 heads take 392 us instead of 57, one 40 instead of 16.5.)
 // P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15; V = byte x scale 2^-e, rounded once,
 // with one e per scale group for the tile's 64 rows, so that the largest |V| stays below 2^16.  e starts at the exponent of the group's largest
 // scale in an item's first tile and moves up when a scale exceeds it by 2^7; the group's columns of O are then brought to the new e like they are to a
@@ -57,6 +61,7 @@
 #include <cfloat>
 #include <cstddef>
 #include <mutex>
+#include <type_traits>
 #include "defs.h"
 #include "ptx.cuh"
 #include "rows.cuh"
@@ -97,7 +102,7 @@ struct Ctl {
     float scale[kStages][kGroups][kSlots];   // row scales of a tile (0 where the slot holds no row)
     float post[2][4][kRows];                 // by team and quarter of a tile's slots: the rows' maxima (log2 domain); at the end of an item its row sums
     float m_ref[2][kRows];                   // by tile number mod 2: the rows' reference maxima after the tile
-    uint8_t q_exp[kRows];                    // biased exponent of 2^a, Q = 2^a (hi + lo); 255: a row with an infinity or a NaN
+    uint16_t q_exp[kRows];                   // biased exponent of 2^a, Q = 2^a (hi + lo), 255: a row with an infinity or a NaN; 256 more: hi + lo leave out too much
     int32_t late_row[kStages][kOwn];         // rows of the tile that the other CTA gathers
     uint32_t tile_mask[kStages][2];          // which slots of CTA 0 / CTA 1 hold a row
     alignas(8) float2 v_move[kStages][kGroups];          // 2^(e of the tile before - e), 2^e
@@ -114,6 +119,7 @@ struct Ctl {
     uint64_t posted[2][2], moved[2][2];      // by team and half of the rows: a tile's maxima are posted | its reference maxima are written and those before it read
     uint64_t q_here;                         // this CTA's Q and q_exp are written; what the item before left in post, m_ref and v_fin has been read
     uint64_t q_full, q_empty, o_full, o_free, e_bar;
+    uint64_t residual_here[2];               // by half of the rows: the residuals of an item that has some are written
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -153,21 +159,74 @@ __device__ __forceinline__ void warp_arrive_lead(uint64_t* bar, int lane) {
 __device__ __forceinline__ int rows_of(const dsa_v32_work_info& w, int H) { return w.stacked_rows > 1 ? w.stacked_rows * H : H - w.head_block * kHeadsPerBlock; }
 __device__ __forceinline__ int tiles_of(const dsa_v32_work_info& w) { return (w.k_end - w.k_begin + kSlots - 1) / kSlots; }
 
-// ------------------------------------------------------------------ Q as a sum of two e4m3 numbers
-// Eight bf16 elements times the power of two `mul` -> eight bytes each of hi = e4m3(x) and lo = e4m3(x - hi)
-__device__ __forceinline__ void split_e4m3(const uint4& x, float mul, uint2& hi, uint2& lo) {
+// ------------------------------------------------------------------ Q as a sum of an e5m2 and an e4m3 number
+constexpr int kWideElements = 16;   // elements of a row that may lie below what hi + lo hold exactly
+// Two elements of Q in f16 (after the row's factor) -> hi = e5m2(x) and lo = e4m3(x - hi), in the low halves
+__device__ __forceinline__ void split_q(uint32_t u, uint32_t& hi, uint32_t& lo) {
+    hi = f16x2_to_e5m2x2(u);
+    lo = f16x2_to_e4m3x2(sub_f16x2(u, __byte_perm(hi, 0, 0x1404)));   // (e5m2 is the upper byte of f16)
+}
+// Eight bf16 elements times the power of two `mul` -> eight bytes each of hi and lo
+__device__ __forceinline__ void split_q8(const uint4& x, float mul, uint2& hi, uint2& lo) {
     const uint32_t in[4] = {x.x, x.y, x.z, x.w};
     uint32_t h[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         float u0, u1;
         unpack2(mul2(pack2u(in[i] << 16, in[i] & 0xFFFF0000u), pack2(mul, mul)), u0, u1);
-        const uint32_t u = pack_f16x2(u0, u1);   // exact where e4m3 resolves anything
-        h[i] = f16x2_to_e4m3x2(u);
-        l[i] = f16x2_to_e4m3x2(sub_f16x2(u, e4m3x2_to_f16x2(h[i])));
+        split_q(pack_f16x2(u0, u1), h[i], l[i]);   // exact where hi or lo resolve anything
     }
     hi = make_uint2(__byte_perm(h[0], h[1], 0x5410), __byte_perm(h[2], h[3], 0x5410));
     lo = make_uint2(__byte_perm(l[0], l[1], 0x5410), __byte_perm(l[2], l[3], 0x5410));
+}
+
+// What hi + lo leave out of eight elements, in the same units: exact in bf16
+__device__ __forceinline__ uint4 residual8(const uint4& x, float mul) {
+    const uint32_t in[4] = {x.x, x.y, x.z, x.w};
+    uint32_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float u0 = __uint_as_float(in[i] << 16) * mul, u1 = __uint_as_float(in[i] & 0xFFFF0000u) * mul;
+        uint32_t hi, lo;
+        split_q(pack_f16x2(u0, u1), hi, lo);
+        float h0, h1, l0, l1;
+        unpack_f16x2(__byte_perm(hi, 0, 0x1404), h0, h1);
+        unpack_f16x2(e4m3x2_to_f16x2(lo), l0, l1);
+        r[i] = pack_bf16x2((u0 - h0) - l0, (u1 - h1) - l1);
+    }
+    return make_uint4(r[0], r[1], r[2], r[3]);
+}
+// Where a row's residual waits while its item runs: the row of the output that the item's end overwrites
+__device__ __forceinline__ __nv_bfloat16* residual_row(const AttnParams& p, const dsa_v32_work_info& wi, int row, const RowMap& rm) {
+    if (wi.partial_slot >= 0) return reinterpret_cast<__nv_bfloat16*>(p.o_accum + ((size_t)wi.partial_slot * kHeadsPerBlock + row) * kDV);
+    return reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)rm.q_row * p.stride_o_row + (size_t)rm.head * p.stride_o_head;
+}
+// Residuals of sixteen rows (q: rows lane / 4 and that + 8; null: zeros) times 16 rows of the cache (k: the same), 128 columns: bf16 operands, sums in fp32.
+// By mma.sync, operands from L2: rows that need it are rare.
+__device__ __forceinline__ void residual_group(const __nv_bfloat16* q0, const __nv_bfloat16* q1, const uint8_t* k0, const uint8_t* k1, int lane, float (&acc)[2][4]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j >> 2][j & 3] = 0.0f;
+#pragma unroll 2
+    for (int c = 8 * (lane & 3); c < 128; c += 32) {   // eight columns a lane; which one the MMA takes for which is the same in Q and the cache
+        uint4 x[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+        uint2 y[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
+        if (q0) x[0] = *reinterpret_cast<const uint4*>(q0 + c);
+        if (q1) x[1] = *reinterpret_cast<const uint4*>(q1 + c);
+        if (k0) y[0] = __ldg(reinterpret_cast<const uint2*>(k0 + c));
+        if (k1) y[1] = __ldg(reinterpret_cast<const uint2*>(k1 + c));
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            uint32_t b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float lo, hi;
+                unpack_f16x2(e4m3x2_to_f16x2((j < 2 ? y[n].x : y[n].y) >> (16 * (j & 1))), lo, hi);
+                b[j] = pack_bf16x2(lo, hi);
+            }
+            mma_bf16_16816(acc[n], x[0].x, x[1].x, x[0].y, x[1].y, b[0], b[1]);
+            mma_bf16_16816(acc[n], x[0].z, x[1].z, x[0].w, x[1].w, b[2], b[3]);
+        }
+    }
 }
 
 // kShare: tile rows that a CTA owns, 64, or 32 for plans without items of more than 64: softmax warps without a live row only take part in the
@@ -222,6 +281,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         mbar_init(smem_u32(&ctl->o_full), 1);
         mbar_init(smem_u32(&ctl->o_free), 2 * kSoftmaxWarps);
         mbar_init(smem_u32(&ctl->e_bar), kSoftmaxWarps);
+        mbar_init(smem_u32(&ctl->residual_here[0]), kSoftmaxWarps / 2);
+        mbar_init(smem_u32(&ctl->residual_here[1]), kSoftmaxWarps / 2);
         ctl->abort_flag = 0;
         fence_mbar_init();
     }
@@ -271,6 +332,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 if (live) xr = __ldg(reinterpret_cast<const uint4*>(src));
             }
             float rope_mul = 1.0f;
+            uint32_t row_e[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int row = row0 + i;
@@ -280,15 +342,15 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                     m = max_u16x2(max_u16x2(max_u16x2(x[i][k].x & 0x7FFF7FFFu, x[i][k].y & 0x7FFF7FFFu),
                                             max_u16x2(x[i][k].z & 0x7FFF7FFFu, x[i][k].w & 0x7FFF7FFFu)), m);
                 m = __reduce_max_sync(0xffffffffu, max(m >> 16, m & 0xFFFFu));
-                // the largest magnitude into [128, 256)
+                // the largest magnitude into [2^11, 2^12)
                 const uint32_t e = max(m >> 7, 64u);
-                const float mul = __uint_as_float((261u - min(e, 254u)) << 23);
+                const float mul = __uint_as_float((265u - min(e, 254u)) << 23);
                 if ((lane >> 3) == i) rope_mul = mul;
-                if (lane == 0) ctl->q_exp[row] = static_cast<uint8_t>(e == 255u ? 255u : e - 7u);
+                row_e[i] = e;
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     uint2 hi, lo;
-                    split_e4m3(x[i][k], mul, hi, lo);
+                    split_q8(x[i][k], mul, hi, lo);
                     uint8_t* dst = sQ + (2 * k + (lane >> 4)) * kQBlock + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + 8 * (lane & 1);
                     *reinterpret_cast<uint2*>(dst) = hi;
                     *reinterpret_cast<uint2*>(dst + kGroups * kQBlock) = lo;
@@ -301,6 +363,23 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             }
             fence_proxy_async_smem();
             warp_arrive_lead(&ctl->q_full, lane);
+            // The scores may start; meanwhile, elements that are not 0 and lie below 2^-2 with the row's factor: their magnitudes' bits less 1 (a 0 becomes
+            // the largest), cut off to [line - 2, line - 1], in sums of eight modulo 2^16
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t line = ((row_e[i] - 13u) << 7) * 0x10001u;
+                uint32_t n = 0u;
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t w = (j == 0 ? x[i][k].x : j == 1 ? x[i][k].y : j == 2 ? x[i][k].z : x[i][k].w) & 0x7FFF7FFFu;
+                        n = add_u16x2(n, max_u16x2(min_u16x2(add_u16x2(w, 0xFFFFFFFFu), line - 0x10001u), line - 0x20002u));
+                    }
+                n = sub_u16x2(n, (((row_e[i] - 13u) * 1024u - 16u) & 0xFFFFu) * 0x10001u);
+                const uint32_t below = 512u - __reduce_add_sync(0xffffffffu, (n & 0xFFFFu) + (n >> 16));
+                if (lane == 0) ctl->q_exp[row0 + i] = static_cast<uint16_t>(row_e[i] == 255u ? 255u : row_e[i] - 11u + (below > kWideElements ? 256u : 0u));
+            }
             warp_arrive(&ctl->q_here, lane);
         };
         uint32_t it_base = 0;
@@ -308,285 +387,378 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         Ring<kStages> ring;   // of this team's tiles: every other one
         if (team) ring.next();
         float ls = 0.0f, m_out = 0.0f, v_unit = 1.0f;   // of the last item: its row sum, last reference and 2^e of the columns that this thread reads out
+        // The list's items.  Two forms, one after the other: the first leaves with `true` at the first item with rows for residual_group, and the second goes
+        // on from there, so that the registers of the first are given out as if the second were not there (both in one loop: 128 sequences of 2 x 16 heads
+        // 140 -> 149 us; the residual as a function that is called: 156).
+        int w = w_begin;
+        auto items = [&](auto residual, bool resume) -> bool {
+            constexpr bool kResidual = decltype(residual)::value;
+            int n_wide = 0;
 #pragma unroll 1
-        for (int w = w_begin; w <= w_end; ++w, ++item_n) {
-            // ---- Q of this item, so that its scores can start; then the output of the one before
-            if (w < w_end) {
-                if (item_n > 0)
-                    if (!wait_on(&ctl->q_empty, (item_n - 1) & 1, abort_flag)) goto done;
-                store_q(p.works[w]);
-            }
-            if (item_n > 0) {
-                const dsa_v32_work_info wi = p.works[w - 1];
-                const int row = kShare * rank + r;   // of the item's tile
-                const RowMap rm = map_row(wi, row, p.H);
-                if (kExt && p.attn_sink != nullptr) {
-                    // attention sink (opus_attn/dsa_v4/common/mla_v4_host.cc:469-472): one more term exp(sink - m) in the
-                    // denominator, counted once per query row and head: in the piece that starts the list
-                    const float sink2 = rm.live ? __ldg(p.attn_sink + rm.head) * 1.4426950408889634f : -INFINITY;
-                    if (m_out == -INFINITY) m_out = sink2;                      // no valid score in this piece: the sink is the reference
-                    if (wi.k_begin == 0 && sink2 > -INFINITY) {
-                        const float d = sink2 - m_out;
-                        if (d > 0.0f) {   // a sink above the scores is the reference, so that nothing overflows
-                            const float f = ex2_approx(-d);
-                            ls *= f;
-                            v_unit *= f;
-                            m_out = sink2;
-                        }
-                        ls += ex2_approx(fminf(d, 0.0f) + kPShift);
+            for (; w <= w_end; ++w, ++item_n, resume = false) {
+                if (!resume) {
+                    // ---- Q of this item, so that its scores can start; then the output of the one before
+                    if (w < w_end) {
+                        if (item_n > 0)
+                            if (!wait_on(&ctl->q_empty, (item_n - 1) & 1, abort_flag)) return false;
+                        store_q(p.works[w]);
                     }
-                }
-                const float inv = ls > 0.0f ? v_unit / ls : 0.0f;
-                const float lse_nat = ls > 0.0f ? (m_out - kPShift + __log2f(ls)) * 0.69314718055994531f : INFINITY;
-                if (!wait_on(&ctl->o_full, (item_n - 1) & 1, abort_flag)) goto done;
-                tc_fence_after();
-                // this thread's 64 columns of the row
-                const int col0 = 64 * (warp >> 2);   // of the 256 in its lane
-                if (32 * rq >= kShare) {   // none of the warp's rows is live
-                    tc_fence_before();
-                    warp_arrive_lead(&ctl->o_free, lane);
-                } else if (wi.partial_slot < 0) {
-                    const size_t off = (size_t)rm.q_row * p.stride_o_row + (size_t)rm.head * p.stride_o_head + 256 * h;
-                    const int n_dst = kExt && p.n_peers > 0 ? p.n_peers : 1;
-#pragma unroll 1
-                    for (int oc = col0; oc < col0 + 64; oc += 32) {
-                        uint32_t o[32];
-                        tmem_ld32(lane_base + kColO + oc, o);
-                        tmem_wait_ld();
-                        if (oc != col0) {   // the next item's products may overwrite O
-                            tc_fence_before();
-                            warp_arrive_lead(&ctl->o_free, lane);
-                        }
-                        if (rm.live) {
-                            // thread = row, so a store touches 32 lines whatever its width: 32-byte stores
-                            uint32_t u[16];
-#pragma unroll
-                            for (int v = 0; v < 16; ++v) u[v] = pack_bf16x2(__uint_as_float(o[2 * v]) * inv, __uint_as_float(o[2 * v + 1]) * inv);
-#pragma unroll 1
-                            for (int d = 0; d < n_dst; ++d) {
-                                __nv_bfloat16* o_dst = reinterpret_cast<__nv_bfloat16*>(kExt && p.n_peers > 0 ? p.out_peers[d] : p.out) + off + oc;
-                                stg_32<kExt>(o_dst, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], p.wide);
-                                stg_32<kExt>(o_dst + 16, u[8], u[9], u[10], u[11], u[12], u[13], u[14], u[15], p.wide);
+                    if (item_n > 0) {
+                        const dsa_v32_work_info wi = p.works[w - 1];
+                        const int row = kShare * rank + r;   // of the item's tile
+                        const RowMap rm = map_row(wi, row, p.H);
+                        if (kExt && p.attn_sink != nullptr) {
+                            // attention sink (opus_attn/dsa_v4/common/mla_v4_host.cc:469-472): one more term exp(sink - m) in the
+                            // denominator, counted once per query row and head: in the piece that starts the list
+                            const float sink2 = rm.live ? __ldg(p.attn_sink + rm.head) * 1.4426950408889634f : -INFINITY;
+                            if (m_out == -INFINITY) m_out = sink2;                      // no valid score in this piece: the sink is the reference
+                            if (wi.k_begin == 0 && sink2 > -INFINITY) {
+                                const float d = sink2 - m_out;
+                                if (d > 0.0f) {   // a sink above the scores is the reference, so that nothing overflows
+                                    const float f = ex2_approx(-d);
+                                    ls *= f;
+                                    v_unit *= f;
+                                    m_out = sink2;
+                                }
+                                ls += ex2_approx(fminf(d, 0.0f) + kPShift);
                             }
                         }
-                    }
-                    if (rm.live && warp < 2) {   // the rows' first quarter of the left half
-                        const size_t l_off = (size_t)rm.q_row * p.lse_stride_row + rm.head;
-                        if (kExt && p.n_peers > 0) {
-                            for (int d = 0; d < p.n_peers; ++d)
-                                if (p.lse_peers[d] != nullptr) p.lse_peers[d][l_off] = lse_nat;
-                        } else if (p.lse != nullptr) {
-                            p.lse[l_off] = lse_nat;
-                        }
-                    }
-                } else {
-                    float* o_dst = p.o_accum + ((size_t)wi.partial_slot * kHeadsPerBlock + row) * kDV + 256 * h;
-#pragma unroll 1
-                    for (int oc = col0; oc < col0 + 64; oc += 32) {
-                        uint32_t o[32];
-                        tmem_ld32(lane_base + kColO + oc, o);
-                        tmem_wait_ld();
-                        if (oc != col0) {
+                        const float inv = ls > 0.0f ? v_unit / ls : 0.0f;
+                        const float lse_nat = ls > 0.0f ? (m_out - kPShift + __log2f(ls)) * 0.69314718055994531f : INFINITY;
+                        if (!wait_on(&ctl->o_full, (item_n - 1) & 1, abort_flag)) return false;
+                        tc_fence_after();
+                        // this thread's 64 columns of the row
+                        const int col0 = 64 * (warp >> 2);   // of the 256 in its lane
+                        if (32 * rq >= kShare) {   // none of the warp's rows is live
                             tc_fence_before();
                             warp_arrive_lead(&ctl->o_free, lane);
-                        }
-                        if (rm.live) {
+                        } else if (wi.partial_slot < 0) {
+                            const size_t off = (size_t)rm.q_row * p.stride_o_row + (size_t)rm.head * p.stride_o_head + 256 * h;
+                            const int n_dst = kExt && p.n_peers > 0 ? p.n_peers : 1;
+#pragma unroll 1
+                            for (int oc = col0; oc < col0 + 64; oc += 32) {
+                                uint32_t o[32];
+                                tmem_ld32(lane_base + kColO + oc, o);
+                                tmem_wait_ld();
+                                if (oc != col0) {   // the next item's products may overwrite O
+                                    tc_fence_before();
+                                    warp_arrive_lead(&ctl->o_free, lane);
+                                }
+                                if (rm.live) {
+                                    // thread = row, so a store touches 32 lines whatever its width: 32-byte stores
+                                    uint32_t u[16];
 #pragma unroll
-                            for (int v = 0; v < 4; ++v)
-                                stg_256(o_dst + oc + 8 * v, __float_as_uint(__uint_as_float(o[8 * v + 0]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 1]) * inv),
-                                        __float_as_uint(__uint_as_float(o[8 * v + 2]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 3]) * inv),
-                                        __float_as_uint(__uint_as_float(o[8 * v + 4]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 5]) * inv),
-                                        __float_as_uint(__uint_as_float(o[8 * v + 6]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 7]) * inv));
+                                    for (int v = 0; v < 16; ++v) u[v] = pack_bf16x2(__uint_as_float(o[2 * v]) * inv, __uint_as_float(o[2 * v + 1]) * inv);
+#pragma unroll 1
+                                    for (int d = 0; d < n_dst; ++d) {
+                                        __nv_bfloat16* o_dst = reinterpret_cast<__nv_bfloat16*>(kExt && p.n_peers > 0 ? p.out_peers[d] : p.out) + off + oc;
+                                        stg_32<kExt>(o_dst, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], p.wide);
+                                        stg_32<kExt>(o_dst + 16, u[8], u[9], u[10], u[11], u[12], u[13], u[14], u[15], p.wide);
+                                    }
+                                }
+                            }
+                            if (rm.live && warp < 2) {   // the rows' first quarter of the left half
+                                const size_t l_off = (size_t)rm.q_row * p.lse_stride_row + rm.head;
+                                if (kExt && p.n_peers > 0) {
+                                    for (int d = 0; d < p.n_peers; ++d)
+                                        if (p.lse_peers[d] != nullptr) p.lse_peers[d][l_off] = lse_nat;
+                                } else if (p.lse != nullptr) {
+                                    p.lse[l_off] = lse_nat;
+                                }
+                            }
+                        } else {
+                            float* o_dst = p.o_accum + ((size_t)wi.partial_slot * kHeadsPerBlock + row) * kDV + 256 * h;
+#pragma unroll 1
+                            for (int oc = col0; oc < col0 + 64; oc += 32) {
+                                uint32_t o[32];
+                                tmem_ld32(lane_base + kColO + oc, o);
+                                tmem_wait_ld();
+                                if (oc != col0) {
+                                    tc_fence_before();
+                                    warp_arrive_lead(&ctl->o_free, lane);
+                                }
+                                if (rm.live) {
+#pragma unroll
+                                    for (int v = 0; v < 4; ++v)
+                                        stg_256(o_dst + oc + 8 * v, __float_as_uint(__uint_as_float(o[8 * v + 0]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 1]) * inv),
+                                                __float_as_uint(__uint_as_float(o[8 * v + 2]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 3]) * inv),
+                                                __float_as_uint(__uint_as_float(o[8 * v + 4]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 5]) * inv),
+                                                __float_as_uint(__uint_as_float(o[8 * v + 6]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 7]) * inv));
+                                }
+                            }
+                            if (rm.live && warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + row] = ls > 0.0f ? lse_nat : -FLT_MAX;
                         }
                     }
-                    if (rm.live && warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + row] = ls > 0.0f ? lse_nat : -FLT_MAX;
                 }
-            }
-            if (w == w_end) break;
-            const uint32_t it_end = it_base + tiles_of(p.works[w]);
-            float m_ref = -INFINITY;   // reference maximum after this team's last tile
-            float l = 0.0f;            // this thread's share of the row sum, against m_ref
-            const bool idle = 32 * rq >= kShare || kShare * rank + 32 * rq >= rows_of(p.works[w], p.H);   // none of the warp's rows is live
-            if (!wait_on(&ctl->q_here, item_n & 1, abort_flag)) goto done;
-            const uint32_t q_exp = ctl->q_exp[r];
-            const float c_log2 = p.scale_log2 * __uint_as_float(q_exp == 255u ? 0x7FC00000u : q_exp << 23);   // of scores in units of 2^a
-            uint32_t it = it_base + ((it_base ^ team) & 1u);
-            if (idle) {   // the warp's part in the barriers; what P holds for such rows is used for such rows of O only
+                if (w == w_end) break;
+                const uint32_t it_end = it_base + tiles_of(p.works[w]);
+                float m_ref = -INFINITY;   // reference maximum after this team's last tile
+                float l = 0.0f;            // this thread's share of the row sum, against m_ref
+                const bool idle = 32 * rq >= kShare || kShare * rank + 32 * rq >= rows_of(p.works[w], p.H);   // none of the warp's rows is live
+                if (!resume)
+                    if (!wait_on(&ctl->q_here, item_n & 1, abort_flag)) return false;
+                const uint32_t q_exp = ctl->q_exp[r] & 255u;
+                const bool wide = ctl->q_exp[r] >= 256u, any_wide = __any_sync(0xffffffffu, wide);
+                if (!kResidual && any_wide) return true;
+                if (kResidual && any_wide) {
+                    // four of the 32 rows for each of the warps that share them
+                    const dsa_v32_work_info& wi = p.works[w];
+#pragma unroll 1
+                    for (int row = 32 * rq + 4 * (4 * team + 2 * cs + h), end = row + 4; row < end; ++row) {
+                        const uint32_t e = ctl->q_exp[row];
+                        if (e < 256u) continue;
+                        const RowMap rm = map_row(wi, kShare * rank + row, p.H);   // (a live row)
+                        const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)rm.q_row * p.stride_q_row + (size_t)rm.head * p.stride_q_head);
+                        uint4* dst = reinterpret_cast<uint4*>(residual_row(p, wi, kShare * rank + row, rm));
+                        const float mul = __uint_as_float((254u - (e & 255u)) << 23);
+#pragma unroll 1
+                        for (int k = lane; k < kDV / 8; k += 32) dst[k] = residual8(__ldg(src + k), mul);
+                    }
+                    warp_arrive(&ctl->residual_here[rq], lane);
+                    if (!wait_on(&ctl->residual_here[rq], n_wide & 1, abort_flag)) return false;
+                    ++n_wide;
+                }
+                const float c_log2 = p.scale_log2 * __uint_as_float(q_exp == 255u ? 0x7FC00000u : q_exp << 23);   // of scores in units of 2^a
+                uint32_t it = it_base + ((it_base ^ team) & 1u);
+                if (idle) {   // the warp's part in the barriers; what P holds for such rows is used for such rows of O only
+#pragma unroll 1
+                    for (; it < it_end; it += 2, ring.next(), ring.next()) {
+                        const uint32_t ph2 = (it >> 1) & 1u;
+                        if (!wait_on(&ctl->s_full[team], ph2, abort_flag)) return false;
+                        warp_arrive_lead(&ctl->s3_empty, lane);
+                        warp_arrive_lead(&ctl->s_empty[team], lane);
+                        warp_arrive(&ctl->raw_empty[ring.s], lane);
+                        if (it >= 2)   // every warp of the team has come to the end of its last tile
+                            if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) return false;
+                        warp_arrive(&ctl->posted[team][rq], lane);
+                        warp_arrive(&ctl->moved[team][rq], lane);
+                        warp_arrive_lead(&ctl->p_full[team], lane);
+                    }
+                }
 #pragma unroll 1
                 for (; it < it_end; it += 2, ring.next(), ring.next()) {
-                    const uint32_t ph2 = (it >> 1) & 1u;
-                    if (!wait_on(&ctl->s_full[team], ph2, abort_flag)) goto done;
-                    warp_arrive_lead(&ctl->s3_empty, lane);
-                    warp_arrive_lead(&ctl->s_empty[team], lane);
-                    warp_arrive(&ctl->raw_empty[ring.s], lane);
-                    if (it >= 2)   // every warp of the team has come to the end of its last tile
-                        if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) goto done;
-                    warp_arrive(&ctl->posted[team][rq], lane);
-                    warp_arrive(&ctl->moved[team][rq], lane);
-                    warp_arrive_lead(&ctl->p_full[team], lane);
-                }
-            }
-#pragma unroll 1
-            for (; it < it_end; it += 2, ring.next(), ring.next()) {
-                const uint32_t ph2 = (it >> 1) & 1u;            // phase of the per-team barriers
-                const bool first = it == it_base;
-                // the tile's mask, scales and e, and its scores (the stage's phase before is complete: its tile was three earlier, and this team has
-                // seen the references move past that tile); the team has read its last tile's maxima
-                if (!wait_on3(&ctl->prep[ring.s], ring.ph, &ctl->s_full[team], ph2, &ctl->moved[team][rq], ph2 ^ 1u, abort_flag)) goto done;
-                tc_fence_after();
-                // ---- scores in units of 2^a: sum_g scale_g S_g + S_rope, in pairs of slots.  Group 3 and the rope, which have one
-                // accumulator for all tiles, first
-                uint64_t sv[8];
-                uint32_t mask;
-                float v_fix;
-                bool lent;
-                {
-                    const uint32_t ca = lane_base + kColS + 96 * team + 16 * cs;
-                    const float* sc = &ctl->scale[ring.s][0][kOwn * h + 16 * cs];
-                    uint32_t x[2][16], sr[16];
-                    tmem_ld16(lane_base + kColS3 + 16 * cs, x[1]);
-                    tmem_ld16(lane_base + kColRope + 16 * cs, sr);
-                    mask = ctl->tile_mask[ring.s][h] >> (16 * cs);
-                    const float2 move = ctl->v_move[ring.s][2 * h + cs];
-                    v_fix = move.x;
-                    v_unit = move.y;
-                    lent = __any_sync(0xffffffffu, ctl->v_mul[ring.s][0].y != 0.0f);
-                    tmem_wait_ld();
-                    tmem_loaded(x[1]);
-                    tmem_loaded(sr);
-                    tc_fence_before();
-                    warp_arrive_lead(&ctl->s3_empty, lane);
-#pragma unroll
-                    for (int g = kGroups - 1; g >= 0; --g) {   // the next group's scores are on their way while this one's are scaled
-                        if (g > 0) tmem_ld16(ca + 32 * (g - 1), x[(g - 1) & 1]);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const float4 f = *reinterpret_cast<const float4*>(sc + g * kSlots + 4 * c);
-                            const uint32_t* y = x[g & 1] + 4 * c;
-                            sv[2 * c] = fma2(pack2(f.x, f.y), pack2u(y[0], y[1]), g == kGroups - 1 ? pack2u(sr[4 * c], sr[4 * c + 1]) : sv[2 * c]);
-                            sv[2 * c + 1] = fma2(pack2(f.z, f.w), pack2u(y[2], y[3]), g == kGroups - 1 ? pack2u(sr[4 * c + 2], sr[4 * c + 3]) : sv[2 * c + 1]);
-                        }
-                        if (g > 0) {
-                            tmem_wait_ld();
-                            tmem_loaded(x[(g - 1) & 1]);
-                        }
-                        if (g == 1) {
-                            tc_fence_before();
-                            warp_arrive_lead(&ctl->s_empty[team], lane);
-                        }
-                    }
-                    if (!lent) warp_arrive(&ctl->raw_empty[ring.s], lane);
-                }
-                if ((mask & 0xFFFFu) != 0xFFFFu) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float s0, s1;
-                        unpack2(sv[j], s0, s1);
-                        sv[j] = pack2(((mask >> (2 * j)) & 1u) ? s0 : -INFINITY, ((mask >> (2 * j + 1)) & 1u) ? s1 : -INFINITY);
-                    }
-                }
-                // ---- maximum of this quarter, posted
-                {
-                    float t[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float s0, s1;
-                        unpack2(sv[j], s0, s1);
-                        t[j] = fmaxf(s0, s1);
-                    }
-                    ctl->post[team][2 * h + cs][r] = fmaxf(max3(max3(t[0], t[1], t[2]), t[3], t[4]), max3(t[5], t[6], t[7])) * c_log2;
-                    warp_arrive(&ctl->posted[team][rq], lane);
-                }
-                // ---- P = 2^(score - reference + 7): at most 2^15; a masked slot gives 0.  Taken against the last reference known while
-                // the other maxima are on their way, and again in the rare case that it has moved
-                const float m_was = m_ref;
-                float m_old = -INFINITY;
-                uint32_t pk[8];
-                float lsum = 0.0f;
-                bool settled = false;
-#pragma unroll 1
-                while (true) {
-                    if (settled || !first) {
-                        const float n = kPShift - (m_ref == -INFINITY ? 0.0f : m_ref);
-                        const uint64_t c2 = pack2(c_log2, c_log2), nm2 = pack2(n, n);
-                        uint64_t ls2 = pack2(0.0f, 0.0f);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            float e0, e1;
-                            unpack2(fma2(sv[j], c2, nm2), e0, e1);
-                            e0 = ex2_approx(e0);
-                            e1 = ex2_approx(e1);
-                            ls2 = add2(ls2, pack2(e0, e1));
-                            pk[j] = pack_f16x2(e0, e1);
-                        }
-                        float l0, l1;
-                        unpack2(ls2, l0, l1);
-                        lsum = l0 + l1;
-                    }
-                    if (settled) break;
-                    // the row's reference after the tile before this one, and after this one: it moves when the tile's maximum exceeds it by
-                    // more than the lazy margin
-                    // (before tile 0 the second barrier's phase -1 passes)
-                    if (!wait_on2(&ctl->posted[team][rq], ph2, &ctl->moved[team ^ 1][rq], ((it - 1) >> 1) & 1u, abort_flag)) goto done;
-                    const float mt = fmaxf(fmaxf(ctl->post[team][0][r], ctl->post[team][1][r]), fmaxf(ctl->post[team][2][r], ctl->post[team][3][r]));
-                    if (!first) m_old = ctl->m_ref[team ^ 1][r];
-                    m_ref = mt > m_old + 8.0f ? mt : m_old;
-                    if (h == 0 && cs == 0) ctl->m_ref[team][r] = m_ref;
-                    warp_arrive(&ctl->moved[team][rq], lane);
-                    if (!first && !__any_sync(0xffffffffu, m_ref != m_was)) break;
-                    settled = true;
-                }
-                if (l != 0.0f && m_was != m_ref) l *= ex2_approx(m_was - m_ref);
-                l += lsum;
-                if (lent) {   // what V was lent
-                    const uint4* back = reinterpret_cast<const uint4*>(&ctl->p_back[ring.s][kOwn * h + 16 * cs]);
-                    const uint4 b0 = back[0], b1 = back[1];
-                    const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) pk[j] = mul_f16x2(pk[j], b[j]);
-                    warp_arrive(&ctl->raw_empty[ring.s], lane);
-                }
-                // ---- into the P buffer, once the product that read it last is complete
-                if (it >= 2)
-                    if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) goto done;
-                sts_16(p_lo, pk[0], pk[1], pk[2], pk[3]);
-                sts_16(p_lo ^ 16u, pk[4], pk[5], pk[6], pk[7]);
-                fence_proxy_async_smem();
-                if (!first && __any_sync(0xffffffffu, m_ref != m_old || v_fix != 1.0f)) {
-                    // the reference or e moved: O so far (complete once the previous tile's product is) is brought to the new ones
-                    const float f = (m_old == m_ref ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2_approx(m_old - m_ref))) * v_fix;
-                    if (!wait_on(&ctl->pv_done[team ^ 1], ((it - 1) >> 1) & 1u, abort_flag)) goto done;
+                    const uint32_t ph2 = (it >> 1) & 1u;            // phase of the per-team barriers
+                    const bool first = it == it_base;
+                    // the tile's mask, scales and e, and its scores (the stage's phase before is complete: its tile was three earlier, and this team has
+                    // seen the references move past that tile); the team has read its last tile's maxima
+                    if (!wait_on3(&ctl->prep[ring.s], ring.ph, &ctl->s_full[team], ph2, &ctl->moved[team][rq], ph2 ^ 1u, abort_flag)) return false;
                     tc_fence_after();
+                    // ---- scores in units of 2^a: sum_g scale_g S_g + S_rope, in pairs of slots.  Group 3 and the rope, which have one
+                    // accumulator for all tiles, first
+                    uint64_t sv[8];
+                    uint32_t mask;
+                    float v_fix;
+                    bool lent;
+                    {
+                        const uint32_t ca = lane_base + kColS + 96 * team + 16 * cs;
+                        const float* sc = &ctl->scale[ring.s][0][kOwn * h + 16 * cs];
+                        uint32_t x[2][16], sr[16];
+                        tmem_ld16(lane_base + kColS3 + 16 * cs, x[1]);
+                        tmem_ld16(lane_base + kColRope + 16 * cs, sr);
+                        mask = ctl->tile_mask[ring.s][h] >> (16 * cs);
+                        const float2 move = ctl->v_move[ring.s][2 * h + cs];
+                        v_fix = move.x;
+                        v_unit = move.y;
+                        lent = __any_sync(0xffffffffu, ctl->v_mul[ring.s][0].y != 0.0f);
+                        tmem_wait_ld();
+                        tmem_loaded(x[1]);
+                        tmem_loaded(sr);
+                        tc_fence_before();
+                        warp_arrive_lead(&ctl->s3_empty, lane);
+#pragma unroll
+                        for (int g = kGroups - 1; g >= 0; --g) {   // the next group's scores are on their way while this one's are scaled
+                            if (g > 0) tmem_ld16(ca + 32 * (g - 1), x[(g - 1) & 1]);
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                const float4 f = *reinterpret_cast<const float4*>(sc + g * kSlots + 4 * c);
+                                const uint32_t* y = x[g & 1] + 4 * c;
+                                sv[2 * c] = fma2(pack2(f.x, f.y), pack2u(y[0], y[1]), g == kGroups - 1 ? pack2u(sr[4 * c], sr[4 * c + 1]) : sv[2 * c]);
+                                sv[2 * c + 1] = fma2(pack2(f.z, f.w), pack2u(y[2], y[3]), g == kGroups - 1 ? pack2u(sr[4 * c + 2], sr[4 * c + 3]) : sv[2 * c + 1]);
+                            }
+                            if (g > 0) {
+                                tmem_wait_ld();
+                                tmem_loaded(x[(g - 1) & 1]);
+                            }
+                            if (!kResidual && g == 1) {
+                                tc_fence_before();
+                                warp_arrive_lead(&ctl->s_empty[team], lane);
+                            }
+                        }
+                        if (!kResidual && !lent) warp_arrive(&ctl->raw_empty[ring.s], lane);
+                    }
+                    if (kResidual && any_wide) {   // what hi + lo leave out of some row of the warp's; meanwhile the scores wait in tensor memory
+                        const uint32_t own = lane_base + kColS + 96 * team + 16 * cs;
+                        {
+                            uint32_t y[16];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                y[2 * j] = static_cast<uint32_t>(sv[j]);
+                                y[2 * j + 1] = static_cast<uint32_t>(sv[j] >> 32);
+                            }
+                            tmem_st16(own, y);
+                            tmem_wait_st();
+                        }
+                        const dsa_v32_work_info& wi = p.works[w];
+                        const uint8_t* rows[2];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const int k = wi.k_begin + static_cast<int>(it - it_base) * kSlots + kOwn * h + 16 * cs + (lane >> 2) + 8 * i;
+                            const int row = k < wi.k_end ? translate_row(__ldg(p.indices + (size_t)wi.q_row * p.topk + k), wi.q_row / p.s_q, p) : -1;
+                            rows[i] = row < 0 ? nullptr : reinterpret_cast<const uint8_t*>(p.kv) + (size_t)row * kFp8RowBytes;
+                        }
 #pragma unroll 1
-                    for (int oc = 128 * cs; oc < 128 * cs + 128; oc += 16) {
-                        uint32_t o[16];
-                        tmem_ld16(lane_base + kColO + oc, o);
+                        for (int m = 0; m < 2; ++m) {   // sixteen rows of Q
+                            const __nv_bfloat16* q[2];
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const int row = 32 * rq + 16 * m + 8 * i + (lane >> 2);
+                                q[i] = ctl->q_exp[row] < 256u ? nullptr : residual_row(p, wi, kShare * rank + row, map_row(wi, kShare * rank + row, p.H));
+                            }
+                            float sum[2][4] = {};
+#pragma unroll 1
+                            for (int g = 0; g < kGroups; ++g) {
+                                float acc[2][4];
+                                residual_group(q[0] ? q[0] + 128 * g : nullptr, q[1] ? q[1] + 128 * g : nullptr, rows[0] ? rows[0] + 128 * g : nullptr, rows[1] ? rows[1] + 128 * g : nullptr, lane, acc);
+                                const float* sc = &ctl->scale[ring.s][g][kOwn * h + 16 * cs + 2 * (lane & 3)];
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) sum[j >> 2][j & 3] += acc[j >> 2][j & 3] * sc[8 * (j >> 2) + (j & 1)];
+                            }
+                            // a lane holds rows lane / 4 and that + 8, columns 2 (lane % 4) and the next of either half: a row's go to its own lane
+                            uint32_t y[16];
+                            tmem_ld16(own, y);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int n = 0; n < 16; ++n) {
+                                const int src = (lane & 7) * 4 + ((n & 7) >> 1);
+                                const float lo = __shfl_sync(0xffffffffu, sum[n >> 3][n & 1], src), hi = __shfl_sync(0xffffffffu, sum[n >> 3][2 + (n & 1)], src);
+                                if (wide && (lane >> 4) == m) y[n] = __float_as_uint(__uint_as_float(y[n]) + (lane & 8 ? hi : lo));
+                            }
+                            tmem_st16(own, y);
+                            tmem_wait_st();
+                        }
+                        uint32_t y[16];
+                        tmem_ld16(own, y);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-                        tmem_st16(lane_base + kColO + oc, o);
+                        for (int j = 0; j < 8; ++j) sv[j] = pack2u(y[2 * j], y[2 * j + 1]);
                     }
-                    tmem_wait_st();
-                }
-                tc_fence_before();
-                warp_arrive_lead(&ctl->p_full[team], lane);
-            }
-            // ---- the item's sums, last reference and last e
-            const uint32_t last = it_end - 1, last_team = last & 1u;
-            it_base = it_end;
-            if (!wait_on(&ctl->moved[last_team][rq], (last >> 1) & 1u, abort_flag)) goto done;   // the posted maxima have been read, too
-            const float m_fin = ctl->m_ref[last_team][r];
-            if (l != 0.0f && m_ref != m_fin) l *= ex2_approx(m_ref - m_fin);
-            ctl->post[team][2 * h + cs][r] = l;
-            if (team == static_cast<int>(last_team) && rq == 0 && lane == 0) ctl->v_fin[2 * h + cs] = v_unit;
-            warp_arrive(&ctl->e_bar, lane);
-            if (!wait_on(&ctl->e_bar, item_n & 1, abort_flag)) goto done;
-            m_out = m_fin;
-            ls = 0.0f;
+                    if (kResidual) {
+                        tc_fence_before();
+                        warp_arrive_lead(&ctl->s_empty[team], lane);
+                    }
+                    if ((mask & 0xFFFFu) != 0xFFFFu) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ls += ctl->post[i >> 2][i & 3][r];
-            v_unit = ctl->v_fin[2 * h + team];   // the read-out's 64 columns lie in this group
-        }
+                        for (int j = 0; j < 8; ++j) {
+                            float s0, s1;
+                            unpack2(sv[j], s0, s1);
+                            sv[j] = pack2(((mask >> (2 * j)) & 1u) ? s0 : -INFINITY, ((mask >> (2 * j + 1)) & 1u) ? s1 : -INFINITY);
+                        }
+                    }
+                    // ---- maximum of this quarter, posted
+                    {
+                        float t[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            float s0, s1;
+                            unpack2(sv[j], s0, s1);
+                            t[j] = fmaxf(s0, s1);
+                        }
+                        ctl->post[team][2 * h + cs][r] = fmaxf(max3(max3(t[0], t[1], t[2]), t[3], t[4]), max3(t[5], t[6], t[7])) * c_log2;
+                        warp_arrive(&ctl->posted[team][rq], lane);
+                    }
+                    // ---- P = 2^(score - reference + 7): at most 2^15; a masked slot gives 0.  Taken against the last reference known while
+                    // the other maxima are on their way, and again in the rare case that it has moved
+                    const float m_was = m_ref;
+                    float m_old = -INFINITY;
+                    uint32_t pk[8];
+                    float lsum = 0.0f;
+                    bool settled = false;
+#pragma unroll 1
+                    while (true) {
+                        if (settled || !first) {
+                            const float n = kPShift - (m_ref == -INFINITY ? 0.0f : m_ref);
+                            const uint64_t c2 = pack2(c_log2, c_log2), nm2 = pack2(n, n);
+                            uint64_t ls2 = pack2(0.0f, 0.0f);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                float e0, e1;
+                                unpack2(fma2(sv[j], c2, nm2), e0, e1);
+                                e0 = ex2_approx(e0);
+                                e1 = ex2_approx(e1);
+                                ls2 = add2(ls2, pack2(e0, e1));
+                                pk[j] = pack_f16x2(e0, e1);
+                            }
+                            float l0, l1;
+                            unpack2(ls2, l0, l1);
+                            lsum = l0 + l1;
+                        }
+                        if (settled) break;
+                        // the row's reference after the tile before this one, and after this one: it moves when the tile's maximum exceeds it by
+                        // more than the lazy margin
+                        // (before tile 0 the second barrier's phase -1 passes)
+                        if (!wait_on2(&ctl->posted[team][rq], ph2, &ctl->moved[team ^ 1][rq], ((it - 1) >> 1) & 1u, abort_flag)) return false;
+                        const float mt = fmaxf(fmaxf(ctl->post[team][0][r], ctl->post[team][1][r]), fmaxf(ctl->post[team][2][r], ctl->post[team][3][r]));
+                        if (!first) m_old = ctl->m_ref[team ^ 1][r];
+                        m_ref = mt > m_old + 8.0f ? mt : m_old;
+                        if (h == 0 && cs == 0) ctl->m_ref[team][r] = m_ref;
+                        warp_arrive(&ctl->moved[team][rq], lane);
+                        if (!first && !__any_sync(0xffffffffu, m_ref != m_was)) break;
+                        settled = true;
+                    }
+                    if (l != 0.0f && m_was != m_ref) l *= ex2_approx(m_was - m_ref);
+                    l += lsum;
+                    if (lent) {   // what V was lent
+                        const uint4* back = reinterpret_cast<const uint4*>(&ctl->p_back[ring.s][kOwn * h + 16 * cs]);
+                        const uint4 b0 = back[0], b1 = back[1];
+                        const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) pk[j] = mul_f16x2(pk[j], b[j]);
+                    }
+                    if (kResidual || lent) warp_arrive(&ctl->raw_empty[ring.s], lane);
+                    // ---- into the P buffer, once the product that read it last is complete
+                    if (it >= 2)
+                        if (!wait_on(&ctl->pv_done[team], ph2 ^ 1u, abort_flag)) return false;
+                    sts_16(p_lo, pk[0], pk[1], pk[2], pk[3]);
+                    sts_16(p_lo ^ 16u, pk[4], pk[5], pk[6], pk[7]);
+                    fence_proxy_async_smem();
+                    if (!first && __any_sync(0xffffffffu, m_ref != m_old || v_fix != 1.0f)) {
+                        // the reference or e moved: O so far (complete once the previous tile's product is) is brought to the new ones
+                        const float f = (m_old == m_ref ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2_approx(m_old - m_ref))) * v_fix;
+                        if (!wait_on(&ctl->pv_done[team ^ 1], ((it - 1) >> 1) & 1u, abort_flag)) return false;
+                        tc_fence_after();
+#pragma unroll 1
+                        for (int oc = 128 * cs; oc < 128 * cs + 128; oc += 16) {
+                            uint32_t o[16];
+                            tmem_ld16(lane_base + kColO + oc, o);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                            tmem_st16(lane_base + kColO + oc, o);
+                        }
+                        tmem_wait_st();
+                    }
+                    tc_fence_before();
+                    warp_arrive_lead(&ctl->p_full[team], lane);
+                }
+                // ---- the item's sums, last reference and last e
+                const uint32_t last = it_end - 1, last_team = last & 1u;
+                it_base = it_end;
+                if (!wait_on(&ctl->moved[last_team][rq], (last >> 1) & 1u, abort_flag)) return false;   // the posted maxima have been read, too
+                const float m_fin = ctl->m_ref[last_team][r];
+                if (l != 0.0f && m_ref != m_fin) l *= ex2_approx(m_ref - m_fin);
+                ctl->post[team][2 * h + cs][r] = l;
+                if (team == static_cast<int>(last_team) && rq == 0 && lane == 0) ctl->v_fin[2 * h + cs] = v_unit;
+                warp_arrive(&ctl->e_bar, lane);
+                if (!wait_on(&ctl->e_bar, item_n & 1, abort_flag)) return false;
+                m_out = m_fin;
+                ls = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) ls += ctl->post[i >> 2][i & 3][r];
+                v_unit = ctl->v_fin[2 * h + team];   // the read-out's 64 columns lie in this group
+            }
+            return false;
+        };
+        if (items(std::false_type(), false)) items(std::true_type(), true);
     } else if (warp < kLoadWarp0) {
         setmaxnreg_dec<kRegsIssuers>();
         if (warp < kPvWarp && rank == 0) {
@@ -624,7 +796,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                         const uint32_t d = g < kGroups - 1 ? d0 + 32 * g : tmem + kColS3;
 #pragma unroll
                         for (int v = 0; v < 2; ++v)
-                            umma_pair_f8_ss_x4_el(d, q_lo + (((v * kGroups + g) * kQBlock) >> 4), q_hi, k_lo + ((g * kBlock) >> 4), k_hi, idesc8, v, el);
+                            umma_pair_f8_ss_x4_el(d, q_lo + (((v * kGroups + g) * kQBlock) >> 4), q_hi, k_lo + ((g * kBlock) >> 4), k_hi, v ? idesc8 : idesc8 | kIdescAE5m2, v, el);
                     }
                     umma_pair_ss_x4_el(tmem + kColRope, q_lo + ((2 * kGroups * kQBlock) >> 4), q_hi, k_lo + ((kGroups * kBlock) >> 4), k_hi, idesc, 0u, el);
                     tc_commit_pair_el(smem_u32(&ctl->s_full[par]), el);

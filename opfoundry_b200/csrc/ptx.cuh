@@ -494,6 +494,7 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool b_mn_m
 // The same for f16 A and B, and for kind::f8f6f4 with e4m3 A and B (both K-major).
 __host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, bool b_mn_major) { return make_idesc_bf16(M, N, b_mn_major) & ~((1u << 7) | (1u << 10)); }
 __host__ __device__ constexpr uint32_t make_idesc_e4m3(int M, int N) { return make_idesc_f16(M, N, false); }
+constexpr uint32_t kIdescAE5m2 = 1u << 7;          // of kind::f8f6f4: A is e5m2
 constexpr uint32_t kIdescATransposed = 1u << 15;   // A is MN-major
 
 // D[tmem] (+)= A * B, A in shared memory (ss) or TMEM (ts), B in shared memory; accumulate == 0 overwrites D.
@@ -688,10 +689,21 @@ __device__ __forceinline__ uint32_t pack_bf16x2_from2(uint64_t v) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// e4m3 (saturating, to nearest even) and f16, two at a time: element 0 in the low half
+// D += A B of one warp, bf16 operands: A 16 x 16, B 16 x 8
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// e4m3 and e5m2 (saturating, to nearest even) and f16, two at a time: element 0 in the low half
 __device__ __forceinline__ uint32_t f16x2_to_e4m3x2(uint32_t v) {   // in the low half
     uint32_t r;
     asm("{\n\t.reg .b16 t;\n\tcvt.rn.satfinite.e4m3x2.f16x2 t, %1;\n\tmov.b32 %0, {t, 0};\n\t}" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t f16x2_to_e5m2x2(uint32_t v) {
+    uint32_t r;
+    asm("{\n\t.reg .b16 t;\n\tcvt.rn.satfinite.e5m2x2.f16x2 t, %1;\n\tmov.b32 %0, {t, 0};\n\t}" : "=r"(r) : "r"(v));
     return r;
 }
 __device__ __forceinline__ uint32_t sub_f16x2(uint32_t a, uint32_t b) {
@@ -734,6 +746,12 @@ __device__ __forceinline__ uint32_t scale_f16x2(uint32_t v, uint32_t hi, uint32_
 }
 // two bf16 times a power of two
 __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float mul) { return pack_bf16x2(__uint_as_float(v << 16) * mul, __uint_as_float(v & 0xFFFF0000u) * mul); }
+__device__ __forceinline__ uint32_t add_u16x2(uint32_t a, uint32_t b) {   // modulo 2^16, as the next
+    uint32_t r;
+    asm("add.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t sub_u16x2(uint32_t a, uint32_t b) { return add_u16x2(add_u16x2(a, ~b), 0x10001u); }
 __device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));

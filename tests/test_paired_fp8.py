@@ -1,4 +1,4 @@
-"""The 128-row kernel of an fp8 cache: Q as a sum of two e4m3 numbers per row factor, V scaled to f16 with one exponent per scale group
+"""The 128-row kernel of an fp8 cache: Q as a sum of an e5m2 and an e4m3 number per row factor, V scaled to f16 with one exponent per scale group
 for a tile, which moves with the largest scale.  Tile edges, split and stacked items are in test_paired_heads."""
 import math
 
@@ -174,3 +174,42 @@ def test_small_rows_that_carry_the_weight(built_lib, oracle, power, mixed):
         kv[rest, 512:528] = (kv[rest, 512:528].copy().view(np.float32) * np.float32(2.0 ** power)).view(np.uint8)
     kv[:, 528:] = _bf16(rope).view(np.uint8).reshape(kv.shape[0], 128)
     _check_groups(oracle, dict(case, kv=kv, q=_bf16(q)))
+
+
+@pytest.mark.parametrize("power", [8, 9, 11, 14, 20, 30])
+@pytest.mark.parametrize("H,columns,num_sms", [(72, 1, 4), (72, 200, 148), (128, 3, 148), (40, 1, 148), (48, 200, 4)])
+def test_elements_of_q_far_above_the_others(built_lib, oracle, power, H, columns, num_sms):
+    """Columns of Q that are 2^power times the others and that the cache holds zeros in: what is left of the row decides, and has all its bits.  In some
+    heads only, whole and split; lse to 2e-5: at most 16 elements lie below what the two parts hold, each rounded to 2^-22 of 2^9.5 (2^-12.5), which is
+    2^-12.5 / sqrt(3) x 4 / sqrt(192) = 3e-5 of a score, and lse averages over more than four of them."""
+    from gpu_util import run_gpu, run_oracle
+    case = _case(13, H=H, topk=500 if num_sms == 148 else 321)
+    q, kv = _f32(case["q"]).copy(), case["kv"].copy()
+    heads = [0, 3, 31, 32, H - 1] + ([63, 64] if H > 64 else [])
+    q[:, heads, 7:7 + columns] *= np.float32(2.0 ** power)
+    kv[:, 7:7 + columns] = 0
+    case = dict(case, kv=kv, q=_bf16(q))
+    g_out, g_lse, plan = run_gpu(case, SCALE, num_sms=num_sms)
+    assert (plan.info.num_partials > 0) == (num_sms == 148)
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    check_out(g_out, r_out, **TOL_FP8)
+    assert np.abs(g_lse - r_lse).max() < 2e-5
+    again = run_gpu(case, SCALE, num_sms=num_sms)
+    assert np.array_equal(again[0], g_out) and np.array_equal(again[1], g_lse)
+
+
+def test_stacked_rows_with_elements_far_above_the_others(built_lib, oracle):
+    """Both forms of the softmax warps in one list, stacked and single rows."""
+    from gpu_util import run_gpu, run_oracle
+    case = synth.make_decode_case(9, 24, 1024, 300, s_q=2, fp8=True, paged=True, seed=15)
+    shared = [b % 2 == 0 for b in range(9)]
+    q, kv, idx = _f32(case["q"]).copy(), case["kv"].copy(), case["indices"]
+    for b in range(0, 9, 2):
+        idx[2 * b + 1] = idx[2 * b]
+    q[6:, ::5, 300] *= np.float32(2.0 ** 15)
+    kv[:, 300] = 0
+    case = dict(case, kv=kv, q=_bf16(q))
+    g_out, g_lse, _ = run_gpu(case, SCALE, num_sms=4, mtp_shared=shared)
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    check_out(g_out, r_out, **TOL_FP8)
+    assert np.abs(g_lse - r_lse).max() < 2e-5

@@ -29,7 +29,7 @@ class Ring:
 
 
 class PairFp8(Pair):
-    def __init__(self, items, rng, wait_read=True, idle=lambda c, rq, n: False):
+    def __init__(self, items, rng, wait_read=True, idle=lambda c, rq, n: False, wide=0.0):
         self.items, self.rng, self.wait_read, self.idle = items, rng, wait_read, idle
         bars = lambda n, count: [[Bar(count) for _ in range(n)] for _ in range(2)]
         one = lambda count: [Bar(count) for _ in range(2)]
@@ -41,6 +41,9 @@ class PairFp8(Pair):
         self.s_full, self.s_empty, self.p_full, self.pv_done = bars(2, 1), [Bar(2 * TEAM) for _ in range(2)], [Bar(2 * TEAM) for _ in range(2)], bars(2, 1)
         self.s3_empty, self.q_full, self.o_free = Bar(2 * TEAM), Bar(2 * WARPS), Bar(2 * WARPS)
         self.posted, self.moved = [[[[Bar(TEAM // 2) for _ in range(2)] for _ in range(2)] for _ in range(2)] for _ in range(2)]
+        self.residual_here = [[Bar(WARPS // 2) for _ in range(2)] for _ in range(2)]
+        self.left = [[[None] * (WARPS // 2) for _ in range(2)] for _ in range(2)]   # residuals of an item that has some, [cta][rows]
+        self.wide = [[[rng.random() < wide for _ in items] for _ in range(2)] for _ in range(2)]
         self.q_here, self.q_empty, self.o_full, self.e_bar = one(WARPS), one(2), one(1), one(WARPS)
         # what the buffers hold
         self.raw = [[[None] * LOADERS for _ in range(STAGES)] for _ in range(2)]   # rows and scales, by loader warp
@@ -70,6 +73,7 @@ class PairFp8(Pair):
         team, cs, quad = w >> 3, (w >> 2) & 1, w & 3
         h, rq = quad >> 1, quad & 1
         ring, base, end = Ring(STAGES), 0, 0
+        second, n_wide = False, 0       # the form for items with residuals
         if team:
             ring.next()
         for n in range(len(self.items) + 1):
@@ -91,6 +95,14 @@ class PairFp8(Pair):
             base, end = end, end + self.items[n]
             yield self.q_here[c], n & 1
             assert self.q[c] == [n] * WARPS, "row factors of another item"
+            wide = self.wide[c][rq][n] and not self.idle(c, rq, n)
+            if wide:
+                second = True
+                self.left[c][rq][4 * team + 2 * cs + h] = n
+                yield None
+                self.residual_here[c][rq].arrive()
+                yield self.residual_here[c][rq], n_wide & 1
+                n_wide += 1
             for it in range(base + ((base ^ team) & 1), end, 2):
                 ph2, first = (it >> 1) & 1, it == base
                 if self.idle(c, rq, n):
@@ -120,8 +132,12 @@ class PairFp8(Pair):
                 self.s3_empty.arrive()
                 yield None
                 assert self.score[c][team] == it, "scores of another tile"
-                self.s_empty[team].arrive()
+                if not second:
+                    self.s_empty[team].arrive()
                 yield None
+                if second:
+                    assert self.score[c][team] == it and (not wide or self.left[c][rq] == [n] * (WARPS // 2)), "residuals of another item"
+                    self.s_empty[team].arrive()
                 assert self.raw[c][ring.s] == [it] * LOADERS, "scales of another tile"
                 lent = self.lent[it % len(self.lent)]       # rows took more than 2^-e: P is multiplied with what stands beside e
                 if not lent:
@@ -308,6 +324,12 @@ def test_warps_without_live_rows(idle):
     for items in ([1] * 9, [3, 1, 2, 5, 1, 1, 4]):
         for i, role in enumerate([None, "softmax0.0", "softmax1.3", "softmax0.5", "softmax1.14", "softmax0.2", "pv", "issuer1", "~pvmma", "conv1.3"]):
             PairFp8(items, random.Random(i), idle=idle).run(slow=role)
+
+
+def test_items_with_residuals():
+    for items in ([1] * 9, [3, 1, 2, 5, 1, 1, 4]):
+        for i, role in enumerate([None, "softmax0.0", "softmax1.3", "softmax0.5", "softmax1.14", "softmax0.2", "pv", "issuer1", "~score0"]):
+            PairFp8(items, random.Random(i), wide=0.5, idle=(lambda c, rq, n: rq == 1) if i % 3 == 2 else lambda c, rq, n: False).run(slow=role)
 
 
 def test_the_model_sees_a_missing_wait():
