@@ -326,10 +326,10 @@ void* dsa_v32_static_scratch_address(void);
 int dsa_v32_device_status(const dsa_v32_attn_args* args, void* stream);
 
 /*
- * Self-test of the bounded device-side wait: launches one warp that waits, for `budget_us` microseconds
- * (1 .. 1000000), on an initialised barrier nothing arrives at.  The wait must run out, the kernel must
- * record DSA_V32_ERR_DEVICE_WAIT in the status word of `workspace` (any planned workspace) and exit
- * normally; result_dev[0] = 1 when the wait gave up, result_dev[1] = the abort flag it raised.  Afterwards
+ * Self-test of the bounded device-side waits: launches four warps that wait, in the forms that the kernels have, on an
+ * initialised barrier nothing arrives at, one of them for `budget_us` microseconds (1 .. 1000000), the others until that one raises the abort
+ * flag.  All waits must end, the kernel must record DSA_V32_ERR_DEVICE_WAIT in the status word of `workspace` (any planned workspace) and exit
+ * normally; result_dev[0] = 1 when all waits gave up, result_dev[1] = the abort flag that was raised.  Afterwards
  * dsa_v32_device_status reports and clears the code.  Nothing traps and nothing is left waiting, so the
  * context stays usable.  No counterpart in the reference, whose kernels wait without a bound.
  */

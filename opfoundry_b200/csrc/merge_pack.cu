@@ -195,26 +195,33 @@ __global__ void __launch_bounds__(256) pack_fp8_rows_kernel(const float* __restr
     reinterpret_cast<uint32_t*>(row + kDV + 16)[lane] = rp;
 }
 
-// ------------------------------------------------------------------ self-test of the bounded wait
-// One warp waits, with a short budget, on an initialised barrier that nothing ever arrives at: the wait
-// must give up, raise the CTA's abort flag and record DSA_V32_ERR_DEVICE_WAIT in the status word - the
-// path every wait of the attention kernel takes when its peer never answers - and the kernel must exit
-// normally.  result[0] = 1 when the wait returned false, result[1] = the abort flag it left.
-__global__ void __launch_bounds__(32) wait_expiry_selftest_kernel(int32_t* status, int32_t* result, unsigned long long budget_ns) {
+// ------------------------------------------------------------------ self-test of the bounded waits
+// Four warps wait on an initialised barrier that nothing ever arrives at: one by time, with a short budget, three in the short forms (with a
+// complete phase beside the one that is not).  The first must give up and raise the CTA's abort flag, which must end the others; the kernel records
+// DSA_V32_ERR_DEVICE_WAIT in the status word - the path every wait of the attention kernels takes when its peer never answers - and must exit
+// normally.  result[0] = 1 when all waits returned false, result[1] = the abort flag they left.
+__global__ void __launch_bounds__(128) wait_expiry_selftest_kernel(int32_t* status, int32_t* result, unsigned long long budget_ns) {
     __shared__ uint64_t bar;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, gave_up;
+    const uint32_t b = smem_u32(&bar);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&bar), 1);
-        abort_flag = 0;
+        mbar_init(b, 1);
+        abort_flag = gave_up = 0;
         fence_mbar_init();
     }
-    __syncwarp();
-    const bool ok = __all_sync(0xffffffffu, mbar_wait_budget(smem_u32(&bar), 0, &abort_flag, budget_ns));
-    __syncwarp();
+    __syncthreads();
+    // phase 0 is not complete, the one before it (parity 1) is
+    const bool ok = warp == 0   ? __all_sync(0xffffffffu, mbar_wait_budget(b, 0, &abort_flag, budget_ns))
+                    : warp == 1 ? warp_wait_short(b, 0, &abort_flag)
+                    : warp == 2 ? warp_wait_short2(b, 1, b, 0, &abort_flag)
+                                : warp_wait_short3(b, 1, b, 0, b, 1, &abort_flag);
+    if (!ok && (threadIdx.x & 31) == 0) atomicAdd(&gave_up, 1);
+    __syncthreads();
     if (abort_flag) settle_in_flight();
     if (threadIdx.x == 0) {
         if (abort_flag) atomicExch(status, DSA_V32_ERR_DEVICE_WAIT);
-        result[0] = ok ? 0 : 1;
+        result[0] = gave_up == 4 ? 1 : 0;
         result[1] = abort_flag;
     }
 }
@@ -276,7 +283,7 @@ cudaError_t launch_peer_sync(const PeerSync& s, cudaStream_t stream) {
 }
 
 cudaError_t launch_wait_selftest(int32_t* status, int32_t* result, unsigned long long budget_ns, cudaStream_t stream) {
-    wait_expiry_selftest_kernel<<<1, 32, 0, stream>>>(status, result, budget_ns);
+    wait_expiry_selftest_kernel<<<1, 128, 0, stream>>>(status, result, budget_ns);
     return cudaGetLastError();
 }
 

@@ -36,7 +36,7 @@
 //                of an item all sixteen fetch the next one's Q (global -> hi and lo -> shared memory) and read out O
 //   warps 16, 17 CTA 0: score issuers on alternate tiles
 //   warp 18      CTA 0: P V issuer
-//   warp 19      tells the issuers that the CTA's rows of a tile have landed, and follows e
+//   warp 19      tells the issuers that the CTA's rows of a tile have landed, and follows e; watches that the CTA moves on
 //   warps 20-23  row loaders: 16-byte cp.async copies into the swizzled tile, eight rows of every tile each
 //   warps 24-31  converters: e4m3 -> f16, eight of a tile's rows each; four of them fetch the own output columns of the other CTA's rows
 //
@@ -54,7 +54,8 @@
 // Against 64 bits, six shapes of 40 to 128 heads: out 1.68e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to 2.30e-3),
 // lse at most 1.9e-6 (7e-5).
 //
-// Every mbarrier wait is bounded; on expiry the CTA raises its own and its peer's abort flag, records DSA_V32_ERR_DEVICE_WAIT in
+// Every mbarrier wait is bounded: warp 19 of either CTA, which sees every tile and stays until the other warps have finished, waits by time, the
+// others end by the abort flag that it raises.  On expiry the CTA raises its own and its peer's abort flag, records DSA_V32_ERR_DEVICE_WAIT in
 // the workspace status word and both drain to the normal exit.  A parity wait is only issued on a barrier whose previous phase
 // the waiting warp knows to be complete, and that cannot complete its next one before that warp has looked.
 #include <cuda_bf16.h>
@@ -119,6 +120,7 @@ struct Ctl {
     uint64_t posted[2][2], moved[2][2];      // by team and half of the rows: a tile's maxima are posted | its reference maxima are written and those before it read
     uint64_t q_here;                         // this CTA's Q and q_exp are written; what the item before left in post, m_ref and v_fin has been read
     uint64_t q_full, q_empty, o_full, o_free, e_bar;
+    uint64_t finished;                       // the other warps have come to their end
     uint64_t residual_here[2];               // by half of the rows: the residuals of an item that has some are written
     uint32_t tmem_base;
     int abort_flag;
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
         mbar_init(smem_u32(&ctl->o_full), 1);
         mbar_init(smem_u32(&ctl->o_free), 2 * kSoftmaxWarps);
         mbar_init(smem_u32(&ctl->e_bar), kSoftmaxWarps);
+        mbar_init(smem_u32(&ctl->finished), kWarps - 1);
         mbar_init(smem_u32(&ctl->residual_here[0]), kSoftmaxWarps / 2);
         mbar_init(smem_u32(&ctl->residual_here[1]), kSoftmaxWarps / 2);
         ctl->abort_flag = 0;
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 if (!resume)
                     if (!wait_on(&ctl->q_here, item_n & 1, abort_flag)) return false;
                 const uint32_t q_exp = ctl->q_exp[r] & 255u;
-                const bool wide = ctl->q_exp[r] >= 256u, any_wide = __any_sync(0xffffffffu, wide);
+                const bool any_wide = __any_sync(0xffffffffu, ctl->q_exp[r] >= 256u);
                 if (!kResidual && any_wide) return true;
                 if (kResidual && any_wide) {
                     // four of the 32 rows for each of the warps that share them
@@ -631,7 +634,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             for (int n = 0; n < 16; ++n) {
                                 const int src = (lane & 7) * 4 + ((n & 7) >> 1);
                                 const float lo = __shfl_sync(0xffffffffu, sum[n >> 3][n & 1], src), hi = __shfl_sync(0xffffffffu, sum[n >> 3][2 + (n & 1)], src);
-                                if (wide && (lane >> 4) == m) y[n] = __float_as_uint(__uint_as_float(y[n]) + (lane & 8 ? hi : lo));
+                                if (ctl->q_exp[r] >= 256u && (lane >> 4) == m) y[n] = __float_as_uint(__uint_as_float(y[n]) + (lane & 8 ? hi : lo));
                             }
                             tmem_st16(own, y);
                             tmem_wait_st();
@@ -846,7 +849,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             for (int w = w_begin; w < w_end; ++w) {
                 const int n_tiles = tiles_of(p.works[w]);
                 for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
-                    if (!wait_on(&ctl->kv_full[ring.s], ring.ph, abort_flag)) goto done;
+                    if (!warp_wait(smem_u32(&ctl->kv_full[ring.s]), ring.ph, abort_flag)) goto done;
                     fence_proxy_async_smem();   // written by cp.async (generic proxy)
                     warp_arrive_lead(&ctl->tile_ready[it & 1u][ring.s], lane);
                     // exponents of the scales of slots 2 lane (low half) and 2 lane + 1 (biased; 0: none that counts)
@@ -914,6 +917,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                     warp_arrive(&ctl->prep[ring.s], lane);
                 }
             }
+            if (!warp_wait(smem_u32(&ctl->finished), 0, abort_flag)) goto done;
         }
     } else if (warp < kConvWarp0) {
         // ============================================================ row loaders: eight rows of every tile per warp, four lanes per row
@@ -1102,6 +1106,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             }
         }
     }
+    if (warp != kReadyWarp) warp_arrive(&ctl->finished, lane);
 
 done:
     if (ctl->abort_flag) st_cluster_u32(peer_abort, 1u);   // let the peer stop waiting for us

@@ -84,8 +84,8 @@ __device__ __forceinline__ uint64_t global_ns() {
 #ifndef DSA_WAIT_HINT_NS
 #define DSA_WAIT_HINT_NS 20000u        // one parked try_wait
 #endif
-#ifndef DSA_WAIT_PARKS
-#define DSA_WAIT_PARKS 500000u         // the bound of warp_wait_short: a parked try_wait gives up after 4 us (measured, whatever the hint), so two seconds
+#ifndef DSA_WAIT_TRIES
+#define DSA_WAIT_TRIES (1u << 28)      // the last bound of warp_wait_short: more than two seconds even if a try came back at once
 #endif
 #ifndef DSA_WAIT_BUDGET_NS
 #define DSA_WAIT_BUDGET_NS 2000000000ull
@@ -125,7 +125,8 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // The same in few instructions, for code whose size counts (seven warps of a scheduler on five different loops miss the instruction
-// cache): the bound is a number of parked waits instead of a time.
+// cache): these end by the abort flag, which a warp of the CTA that waits by time for what the others bring (warp_wait) raises after two seconds,
+// and by themselves after DSA_WAIT_TRIES.  (A time in each of them: 128 sequences of 2 x 16 heads 142 -> 149 us.)
 __device__ __forceinline__ bool mbar_try_wait_all(uint32_t bar, uint32_t parity) {   // parked as above; what the whole warp has seen
     uint32_t ok;
     asm volatile(
@@ -142,7 +143,7 @@ __device__ __forceinline__ bool warp_wait_short(uint32_t bar, uint32_t parity, v
 #pragma unroll 1
     for (uint32_t n = 0; !mbar_try_wait_all(bar, parity); ++n) {
         if (*abort_flag) return false;
-        if (n > DSA_WAIT_PARKS) {
+        if (n > DSA_WAIT_TRIES) {
             *abort_flag = 1;
             return false;
         }
@@ -170,7 +171,7 @@ __device__ __forceinline__ bool warp_wait_short3(uint32_t bar_a, uint32_t parity
             : "memory");
         if (ok) return true;
         if (*abort_flag) return false;
-        if (n > DSA_WAIT_PARKS) {
+        if (n > DSA_WAIT_TRIES) {
             *abort_flag = 1;
             return false;
         }
@@ -194,7 +195,7 @@ __device__ __forceinline__ bool warp_wait_short2(uint32_t bar_a, uint32_t parity
             : "memory");
         if (ok) return true;
         if (*abort_flag) return false;
-        if (n > DSA_WAIT_PARKS) {
+        if (n > DSA_WAIT_TRIES) {
             *abort_flag = 1;
             return false;
         }

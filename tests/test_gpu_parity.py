@@ -292,6 +292,22 @@ def test_bounded_wait_expires_and_reports(built_lib):
     assert np.all(np.isfinite(lse))
 
 
+def test_waits_of_every_form_end_after_the_time_given(built_lib):
+    """5 ms and 50 ms, whatever a try takes to come back and however many there are."""
+    import ctypes as C
+    plan = api.mla_decode_plan_create(2, 16, 64, 1)
+    result = torch.zeros(2, dtype=torch.int32, device="cuda")
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    a, e0, e1 = api.AttnArgs(), torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.workspace = plan.workspace.data_ptr()
+    for us in (5000, 50000):
+        e0.record()
+        assert built_lib.dsa_v32_selftest_wait_expiry(plan.workspace.data_ptr(), result.data_ptr(), us, st) == 0
+        e1.record()
+        assert built_lib.dsa_v32_device_status(C.byref(a), st) == 1001 and result.cpu().tolist() == [1, 1]
+        assert us / 1000.0 <= e0.elapsed_time(e1) < us / 1000.0 + 4.0
+
+
 def test_copies_in_flight_land_after_a_wait_gave_up(built_lib):
     """The CTA keeps its memory for 200 us after a wait has given up (here one of 100 us): what it issued before may still land."""
     import ctypes as C
