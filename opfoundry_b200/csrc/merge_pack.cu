@@ -84,7 +84,8 @@ __global__ void __launch_bounds__(128, kFlight == 16 ? kMergeBlocksDeep : kV == 
             slot = c0 + lane < ns ? __ldg(reduce_slots + s0 + c0 + lane) : 0;
             lse_i = c0 + lane < ns ? lse_accum[(size_t)slot * kHeadsPerBlock + hrow] : -FLT_MAX;
         }
-        const float wgt = (lse_i > -FLT_MAX) ? exp2f((lse_i - m) * 1.4426950408889634f) : 0.0f;
+        // an empty piece has no weight, one of infinite lse (an infinite sink) all of it
+        const float wgt = !(lse_i > -FLT_MAX) ? 0.0f : lse_i == m ? 1.0f : exp2f((lse_i - m) * 1.4426950408889634f);
         const int n = min(32, ns - c0);
         for (int j = 0; j < n; j += kF) {
             if (c0 + j) load(j, n);

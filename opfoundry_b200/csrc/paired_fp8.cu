@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             // denominator, counted once per query row and head: in the piece that starts the list
                             const float sink2 = rm.live ? __ldg(p.attn_sink + rm.head) * 1.4426950408889634f : -INFINITY;
                             if (m_out == -INFINITY) m_out = sink2;                      // no valid score in this piece: the sink is the reference
-                            if (wi.k_begin == 0 && sink2 > -INFINITY) {
-                                const float d = sink2 - m_out;
+                            const float d = sink2 - m_out;
+                            if (wi.k_begin == 0 && sink2 > -INFINITY && d == d) {   // (a NaN is no term, nor an infinite sink where there is no score)
                                 if (d > 0.0f) {   // a sink above the scores is the reference, so that nothing overflows
                                     const float f = ex2_approx(-d);
                                     ls *= f;

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from helpers import TOL_FP8, check_lse, check_out
-from opfoundry_b200 import synth
+from opfoundry_b200 import api, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -102,7 +102,6 @@ def test_sinks_far_above_the_scores(built_lib, num_sms):
     """A sink 10 nats above a row's lse leaves e^-10 of its output, one 85 or 300 above it next to nothing, and lse is theirs (whole and split items)."""
     import torch
     from gpu_util import to_dev
-    from opfoundry_b200 import api
     H, topk = 48, 700
     case = synth.make_decode_case(3, H, 1024, topk, fp8=True, paged=True, seed=9)
     d = to_dev(case)
@@ -213,3 +212,34 @@ def test_stacked_rows_with_elements_far_above_the_others(built_lib, oracle):
     r_out, r_lse = run_oracle(oracle, case, SCALE)
     check_out(g_out, r_out, **TOL_FP8)
     assert np.abs(g_lse - r_lse).max() < 2e-5
+
+
+@pytest.mark.parametrize("B,H", [(2, 72), (2, 24), (74, 128)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_row_without_positions_under_an_infinite_or_nan_sink(built_lib, B, H, value):
+    """Zeros and +inf, whole or merged (the other kernels are in test_few_heads)."""
+    import torch
+    from gpu_util import to_dev
+    case = synth.make_decode_case(B, H, 1024, 1000, fp8=True, paged=True, seed=B)
+    case["indices"][0] = -1
+    d = to_dev(case)
+    plan = api.mla_decode_plan_create(B, H, 1000)
+    assert (plan.info.num_partials > 0) == (B == 2)
+    out, lse = api.mla_v4_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, attn_sink=torch.full((H,), value, device="cuda"), block_table=d["block_table"],
+                                          page_block_size=case["page_block_size"], kv_batch_stride_rows=case["kv_batch_stride_rows"])
+    assert torch.all(out[0] == 0) and torch.all(lse[0] == float("inf"))
+
+
+@pytest.mark.parametrize("B,H,num_sms", [(3, 72, 148), (3, 24, 148), (3, 16, 148), (3, 16, 2), (3, 72, 2)])
+def test_infinite_sinks_on_a_bf16_cache(built_lib, B, H, num_sms):
+    """An infinite sink takes all of a row's weight, whole or merged."""
+    import torch
+    from gpu_util import run_gpu, to_dev
+    case = synth.make_decode_case(B, H, 1024, 900, seed=16)
+    clean_out, clean_lse, plan = run_gpu(case, SCALE, num_sms=num_sms)
+    assert (plan.info.num_partials > 0) == (num_sms == 148)
+    d = to_dev(case)
+    sink = torch.tensor([float("inf") if h % 2 else -float("inf") for h in range(H)], device="cuda")
+    out, lse = api.mla_v4_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, attn_sink=sink, kv_batch_stride_rows=1024)
+    assert torch.all(out[:, 1::2] == 0) and torch.all(lse[:, 1::2] == float("inf"))
+    np.testing.assert_array_equal(out[:, ::2].cpu().view(torch.int16).numpy().view(np.uint16), clean_out[:, ::2])
