@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(128, kFlight == 16 ? kMergeBlocksDeep : kV == 
             slot = c0 + lane < ns ? __ldg(reduce_slots + s0 + c0 + lane) : 0;
             lse_i = c0 + lane < ns ? lse_accum[(size_t)slot * kHeadsPerBlock + hrow] : -FLT_MAX;
         }
-        // an empty piece has no weight, one of infinite lse (an infinite sink) all of it
-        const float wgt = !(lse_i > -FLT_MAX) ? 0.0f : lse_i == m ? 1.0f : exp2f((lse_i - m) * 1.4426950408889634f);
+        // an empty piece has no weight, one of infinite lse (an infinite sink) all of it; a NaN stays one
+        const float wgt = lse_i == -FLT_MAX ? 0.0f : lse_i == m ? 1.0f : exp2f((lse_i - m) * 1.4426950408889634f);
         const int n = min(32, ns - c0);
         for (int j = 0; j < n; j += kF) {
             if (c0 + j) load(j, n);
@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(128, kFlight == 16 ? kMergeBlocksDeep : kV == 
             }
         }
     }
-    const float inv = denom > 0.0f ? 1.0f / denom : 0.0f;
-    const float lse_val = denom > 0.0f ? m + log2f(denom) * 0.69314718055994531f : INFINITY;
+    const float inv = denom == 0.0f ? 0.0f : 1.0f / denom;
+    const float lse_val = denom == 0.0f ? INFINITY : m + log2f(denom) * 0.69314718055994531f;
     for (int d = 0; d < tgt.n_peers; ++d) {   // one destination, or every peer's gathered buffer
         __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(tgt.out[d]) + (size_t)q_row * stride_o_row + (size_t)head * stride_o_head + col;
 #pragma unroll

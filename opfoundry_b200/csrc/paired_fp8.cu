@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                                 ls += ex2_approx(fminf(d, 0.0f) + kPShift);
                             }
                         }
-                        const float inv = ls > 0.0f ? v_unit / ls : 0.0f;
-                        const float lse_nat = ls > 0.0f ? (m_out - kPShift + __log2f(ls)) * 0.69314718055994531f : INFINITY;
+                        const float inv = ls == 0.0f ? 0.0f : v_unit / ls;   // (a NaN stays one, in lse too)
+                        const float lse_nat = ls == 0.0f ? INFINITY : (m_out - kPShift + __log2f(ls)) * 0.69314718055994531f;
                         if (!wait_on(&ctl->o_full, (item_n - 1) & 1, abort_flag)) return false;
                         tc_fence_after();
                         // this thread's 64 columns of the row
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                                                 __float_as_uint(__uint_as_float(o[8 * v + 6]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 7]) * inv));
                                 }
                             }
-                            if (rm.live && warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + row] = ls > 0.0f ? lse_nat : -FLT_MAX;
+                            if (rm.live && warp < 2) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + row] = ls == 0.0f ? -FLT_MAX : lse_nat;
                         }
                     }
                 }

@@ -408,10 +408,11 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
                     // denominator, counted once per query row and head: in the piece that starts the list
                     const float sink2 = rm.live ? __ldg(p.attn_sink + rm.head) * 1.4426950408889634f : -INFINITY;
                     if (m_ref == -INFINITY) m_ref = sink2;                      // no valid score in this piece: the sink is the reference
-                    if (wi.k_begin == 0 && sink2 > -INFINITY) ls += ex2_approx(sink2 - m_ref);
+                    const float d = sink2 - m_ref;   // (a NaN is no term, nor an infinite sink where there is no score)
+                    if (wi.k_begin == 0 && sink2 > -INFINITY && d == d) ls += ex2_approx(d);
                 }
-                const float inv = ls > 0.0f ? 1.0f / ls : 0.0f;
-                const float lse_nat = ls > 0.0f ? (m_ref + __log2f(ls)) * 0.69314718055994531f : INFINITY;
+                const float inv = ls == 0.0f ? 0.0f : 1.0f / ls;   // (a NaN stays one, in lse too)
+                const float lse_nat = ls == 0.0f ? INFINITY : (m_ref + __log2f(ls)) * 0.69314718055994531f;
                 if (!wait_on(&ctl->o_full, (n - 1) & 1, abort_flag)) goto done;
                 tc_fence_after();
                 // this thread's 256 columns of the row
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_heads_kernel(const __gr
                                         __float_as_uint(__uint_as_float(o[8 * v + 6]) * inv), __float_as_uint(__uint_as_float(o[8 * v + 7]) * inv));
                         }
                     }
-                    if (h == 0) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + kRows * rank + r] = ls > 0.0f ? lse_nat : -FLT_MAX;
+                    if (h == 0) p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + kRows * rank + r] = ls == 0.0f ? -FLT_MAX : lse_nat;
                 }
             }
         }

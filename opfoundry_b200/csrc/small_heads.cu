@@ -428,10 +428,11 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     if (p.attn_sink != nullptr && wi.k_begin == 0 && half == 0) {
                         // attention sink: one more term exp(sink - m) in the denominator, in the piece that starts the list
                         const float sink2 = live ? __ldg(p.attn_sink + head) * 1.4426950408889634f : -INFINITY;
-                        // (a NaN is no term)
+                        // (a NaN is no term, nor an infinite sink where there is no score)
                         if (sink2 > -INFINITY) {
                             if (m == -INFINITY) m = sink2;
-                            ls += ex2_approx(sink2 - m);
+                            const float d = sink2 - m;
+                            if (d == d) ls += ex2_approx(d);
                         }
                     }
                     // this CTA's P buffer is free (every product of the item is complete; all four warps have met since they
@@ -473,12 +474,12 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     const float f_peer = pm == -INFINITY ? 0.0f : (pm == mm ? 1.0f : ex2_approx(pm - mm));
                     ls = ls * f_own + pl * f_peer;
                     m = mm;
-                    const float inv = ls > 0.0f ? 1.0f / ls : 0.0f;
-                    const float lse_nat = ls > 0.0f ? (m + __log2f(ls)) * 0.69314718055994531f : INFINITY;
+                    const float inv = ls == 0.0f ? 0.0f : 1.0f / ls;   // (a NaN stays one, in lse too)
+                    const float lse_nat = ls == 0.0f ? INFINITY : (m + __log2f(ls)) * 0.69314718055994531f;
                     const float k_own = f_own * inv, k_peer = f_peer * inv;
                     if (warp == 0 && lane < 16 && live && half == 0) {
                         if (wi.partial_slot >= 0) {
-                            p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + r] = ls > 0.0f ? lse_nat : -FLT_MAX;
+                            p.lse_accum[(size_t)wi.partial_slot * kHeadsPerBlock + r] = ls == 0.0f ? -FLT_MAX : lse_nat;
                         } else {
                             const size_t off = (size_t)(wi.q_row + sub) * p.lse_stride_row + head;
                             if (p.n_peers > 0) {

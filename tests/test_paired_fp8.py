@@ -243,3 +243,41 @@ def test_infinite_sinks_on_a_bf16_cache(built_lib, B, H, num_sms):
     out, lse = api.mla_v4_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, attn_sink=sink, kv_batch_stride_rows=1024)
     assert torch.all(out[:, 1::2] == 0) and torch.all(lse[:, 1::2] == float("inf"))
     np.testing.assert_array_equal(out[:, ::2].cpu().view(torch.int16).numpy().view(np.uint16), clean_out[:, ::2])
+
+
+@pytest.mark.parametrize("B,H,num_sms", [(3, 72, 148), (3, 24, 148), (3, 16, 148), (3, 16, 2), (3, 72, 2)])
+def test_nan_in_a_row_of_a_bf16_cache(built_lib, B, H, num_sms):
+    """A NaN in a row of the cache reaches out and lse of its queries, whole or merged."""
+    from gpu_util import run_gpu
+    case = synth.make_decode_case(B, H, 1024, 900, seed=16)
+    clean_out, clean_lse, plan = run_gpu(case, SCALE, num_sms=num_sms)
+    assert (plan.info.num_partials > 0) == (num_sms == 148)
+    kv = case["kv"].copy()
+    kv[1024 + case["indices"][1, 800], 300] = 0x7FC0
+    out, lse, _ = run_gpu(dict(case, kv=kv), SCALE, num_sms=num_sms)
+    assert np.isnan(_f32(out)[1]).any(axis=-1).all() and np.isnan(lse[1]).all()
+    np.testing.assert_array_equal(out[[0, 2]], clean_out[[0, 2]])
+    np.testing.assert_array_equal(lse[[0, 2]], clean_lse[[0, 2]])
+
+
+@pytest.mark.parametrize("H,topk,num_sms", [(72, 100, 2), (72, 700, 148), (24, 700, 148), (24, 100, 2)])
+@pytest.mark.parametrize("poison", ["code", "scale", "rope"])
+def test_nan_in_a_row_reaches_out_and_lse(built_lib, H, topk, num_sms, poison):
+    """The e4m3 NaN code, a NaN scale or a NaN in the rope of a row makes out and lse of the queries that select it NaN, whole or split."""
+    from gpu_util import run_gpu
+    case = synth.make_decode_case(3, H, 1024, topk, fp8=True, paged=True, seed=14)
+    kv, idx = case["kv"].copy(), case["indices"]
+    clean_out, clean_lse, plan = run_gpu(case, SCALE, num_sms=num_sms)
+    assert (plan.info.num_partials > 0) == (num_sms == 148)
+    pos, page = int(idx[1, 70]), case["page_block_size"]
+    row = int(case["block_table"][1][pos // page]) * page + pos % page
+    if poison == "code":
+        kv[row, 130] = 0xFF if H == 72 else 0x7F
+    elif poison == "scale":
+        kv[row, 516:520].view(np.float32)[0] = np.nan
+    else:
+        kv[row, 540:542].view(np.uint16)[0] = 0x7FC0
+    out, lse, _ = run_gpu(dict(case, kv=kv), SCALE, num_sms=num_sms)
+    assert np.isnan(_f32(out)[1]).any(axis=-1).all() and np.isnan(lse[1]).all()
+    np.testing.assert_array_equal(out[[0, 2]], clean_out[[0, 2]])
+    np.testing.assert_array_equal(lse[[0, 2]], clean_lse[[0, 2]])
