@@ -59,8 +59,9 @@ __device__ __forceinline__ int translate_row(int idx, int seq, const AttnParams&
 // Input: the two e4m3 bytes in the high byte of each 16-bit half.  Moving the 7 magnitude bits down
 // by 4 puts the 4 exponent bits and 3 mantissa bits where bf16 keeps them; read as bf16 that number
 // is the e4m3 value times 2^-120 (normal and subnormal codes alike), so one exact multiply by 2^120
-// finishes the conversion without going through the conversion unit.  (0x7F, the e4m3 NaN, becomes
-// 480 instead of NaN; a cache row that is never selected is never converted.)
+// finishes the conversion without going through the conversion unit.  (The e4m3 NaN, 0x7F or 0xFF, becomes +-480: the caller
+// looks for it with nan_codes.)
+__device__ __forceinline__ uint32_t nan_codes(uint32_t bytes) { return (bytes & 0x7F7F7F7Fu) + 0x01010101u; }   // bit 7 of each byte that is one
 __device__ __forceinline__ uint32_t e4m3x2_to_bf16x2(uint32_t hi_bytes) {
     const uint32_t y = (hi_bytes & 0x80008000u) | ((hi_bytes >> 4) & 0x07F007F0u);
     uint32_t z;

@@ -711,16 +711,17 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                     };
                     Row next = load_row(row0);
                     for (int t = 0; t < pt.n_tiles; ++t, ring.next()) {
-                        const Row cur = next;
+                        Row cur = next;
                         advance(t);
                         next = load_row(row0);   // a whole tile ahead
                         // e4m3 -> bf16 before the wait for a stage: a stage is the scarce resource
-                        uint32_t o[32];
+                        uint32_t o[32], codes = 0u;
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             const uint32_t wv[4] = {cur.raw[k].x, cur.raw[k].y, cur.raw[k].z, cur.raw[k].w};
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
+                                codes |= nan_codes(wv[q]);
                                 o[8 * k + 2 * q + 0] = e4m3x2_to_bf16x2(__byte_perm(wv[q], 0u, 0x1404u));
                                 o[8 * k + 2 * q + 1] = e4m3x2_to_bf16x2(__byte_perm(wv[q], 0u, 0x3424u));
                             }
@@ -741,6 +742,9 @@ small_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const AttnParams p)
                             *reinterpret_cast<uint4*>(dst_row + (((2 * c + h0) ^ (r & 7)) * 16)) = h0 ? hi : lo;
                             *reinterpret_cast<uint4*>(dst_row + (((2 * c + (h0 ^ 1)) ^ (r & 7)) * 16)) = h0 ? lo : hi;
                         }
+                        // (an e4m3 NaN makes the row's scores NaN by the rope, and with them out and lse of its queries, as in paired_fp8.cu; the conversion
+                        // gives 480.  64 rows of 16 heads x 2048 slots 49.5 -> 50.7 us; a vote and a second conversion of such rows: 52.6)
+                        if (codes & 0x80808080u) cur.rope.x |= 0x7FFF7FFFu;
                         *reinterpret_cast<uint4*>(tile + 8 * kKvBlock + ((oc ^ (r & 7)) * 16)) = cur.rope;
                         fence_proxy_async_smem();
                         warp_arrive(&ctl->kv_full[ring.s], lane);

@@ -260,10 +260,10 @@ def test_nan_in_a_row_of_a_bf16_cache(built_lib, B, H, num_sms):
     np.testing.assert_array_equal(lse[[0, 2]], clean_lse[[0, 2]])
 
 
-@pytest.mark.parametrize("H,topk,num_sms", [(72, 100, 2), (72, 700, 148), (24, 700, 148), (24, 100, 2)])
+@pytest.mark.parametrize("H,topk,num_sms", [(72, 100, 2), (72, 700, 148), (24, 700, 148), (24, 100, 2), (16, 700, 148), (16, 700, 2), (16, 100, 2)])
 @pytest.mark.parametrize("poison", ["code", "scale", "rope"])
-def test_nan_in_a_row_reaches_out_and_lse(built_lib, H, topk, num_sms, poison):
-    """The e4m3 NaN code, a NaN scale or a NaN in the rope of a row makes out and lse of the queries that select it NaN, whole or split."""
+def test_nan_in_a_row_reaches_out_and_lse_on_every_route(built_lib, H, topk, num_sms, poison):
+    """The e4m3 NaN code, a NaN scale or a NaN in the rope of a row makes out and lse of the queries that select it NaN, whole or split, whatever the number of heads."""
     from gpu_util import run_gpu
     case = synth.make_decode_case(3, H, 1024, topk, fp8=True, paged=True, seed=14)
     kv, idx = case["kv"].copy(), case["indices"]
