@@ -273,9 +273,8 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
     CUtensorMap tq;
     std::memset(&tq, 0, sizeof(tq));
     const bool fp8 = want_dtype == DSA_V32_KV_FP8;
-    // Few heads: the kernel that puts the slots on the tensor-core tile's rows, where the plan says so (few_heads_form); with an fp8 cache
-    // items of 17 to 32 rows are faster on the 128-row kernel (the figures are beside the rule)
-    const int few_heads = !fp8 ? h.few_heads_bf16 : h.few_heads <= 16 ? h.few_heads : 0;
+    // Few heads: the kernel that puts the slots on the tensor-core tile's rows, where the plan says so (few_heads_form)
+    const int few_heads = fp8 ? h.few_heads : h.few_heads_bf16;
     if (few_heads) {
         const uint64_t qdims[3] = {uint64_t(kDQK), uint64_t(a->H), uint64_t(a->total_q)};
         const uint64_t qstr[2] = {uint64_t(a->stride_q_head) * 2, uint64_t(a->stride_q_row) * 2};

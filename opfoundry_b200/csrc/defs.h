@@ -44,8 +44,8 @@ struct WorkspaceHeader {
     int32_t has_stacked;  // 1 when some work item stacks several query rows
     int64_t off_list_indptr, off_works, off_reduce_indptr, off_reduce_slots, off_reduce_dst;
     int64_t off_o_accum, off_lse_accum, total_bytes;
-    int32_t few_heads;    // fp8 cache: tile rows (16 or 32) of the few-heads kernel when the plan's items suit it, else 0; launches follow a 16 only
-    int32_t few_heads_bf16;   // the same for a bf16 cache
+    int32_t few_heads;    // fp8 cache: 16, the tile rows of the few-heads kernel, when the plan's items run on it, else 0
+    int32_t few_heads_bf16;   // bf16 cache: the same, 16 or 32
 };
 static_assert(sizeof(WorkspaceHeader) <= 256, "header must fit its slot");
 

@@ -60,25 +60,24 @@ inline void enumerate_units(const dsa_v32_shape& sh, std::vector<PlanUnit>& unit
     }
 }
 
-// The kernel a plan's items run on: 16 or 32 = the few-heads kernel's form for that many tile rows, 0 = the 128-row kernel.
+// The kernel a plan's items run on: 16 or 32 = the few-heads kernel's form for that many tile rows (fp8 cache: 16 only), 0 = the 128-row kernel.
 // Beyond 32 rows Q, the P copies and three tile stages of the few-heads kernel do not fit shared memory.
 // Up to 32 rows it takes less time per slot but more per change of item (its softmax group is also its epilogue), so the line is
 // drawn by the slots that an item has on average.  Measured time over that of the 128-row kernel, fp8, 1 to 3 items per list:
 //   16 rows, whole items of  64: 1.06   128: 1.04-1.07   256: 0.96-0.97   512: 0.87-0.92   1024: 0.81-0.88   2048: 0.84-0.88   pieces: 0.89-0.99
 //   32 rows, whole items of  64: 1.53   128: 1.51-1.58   512: 1.23-1.29   2048: 1.19-1.23   pieces: 1.13-1.21
-// so a launch with an fp8 cache takes the few-heads kernel for at most 16 rows only; the plan's word still says 32 for such items, and so do plans
-// that were saved before.
+// so with an fp8 cache the few-heads kernel takes at most 16 rows.
 // bf16, over its own 128-row kernel (paired_heads.cu), both from one build, 1 to 16 items per list, short runs | after 0.8 s of the same
 // launches, when the 128-row kernel, not the few-heads one, has run into the power cap (1965 -> 1300-1900 MHz):
 //   16 rows, whole items of 128: 1.16-1.26 | 1.20-1.27   320: 1.07-1.23 | 1.00-1.12   400: 1.02-1.09 | 0.95-1.02   512: 0.97-1.07 | 0.82-1.02
 //                           640: 0.99-1.03 | 0.87-0.99   1024: 0.91-0.98 | 0.78-0.94   pieces: 0.93-0.98 | 0.93-0.98
 //   32 rows, whole items of 300: 1.38-1.69 | 1.39-1.52   640: 1.30 | 1.10-1.31   1024: 1.15-1.27 | 0.98-1.20   1500: 0.99-1.14 | 0.90-0.99
 //                          2048: 0.99-1.12 | 0.91-0.93   pieces: 1.17-1.24 | 1.18-1.21
-// The line for 17 to 32 rows is that of the fp8 cache; by these figures a bf16 cache wants its own, later one, and none for pieces.
+// The lines for 17 to 32 rows were drawn by a former kernel of an fp8 cache; by these figures a bf16 cache wants a later one, and none for pieces.
 constexpr int kFewRows16Slots = 160;       // least slots of a whole item of at most 16 rows, on average
 constexpr int kFewRows16SlotsBf16 = 512;   // the same for a bf16 cache
-constexpr int kFewRows32Slots = 768;       // the same for 17 to 32 rows, either cache
-constexpr int kFewRows32PieceSlots = 128;  // the same for a piece of a split item of 17 to 32 rows
+constexpr int kFewRows32Slots = 768;       // the same for 17 to 32 rows (bf16)
+constexpr int kFewRows32PieceSlots = 128;  // the same for a piece of a split item of 17 to 32 rows (bf16)
 inline int few_heads_form(const dsa_v32_shape& sh, const std::vector<dsa_v32_work_info>& works, bool fp8) {
     int rows = 0;
     int64_t slots = 0, wanted = 0;
@@ -89,7 +88,7 @@ inline int few_heads_form(const dsa_v32_shape& sh, const std::vector<dsa_v32_wor
         if (w.partial_slot < 0) wanted += r > 16 ? kFewRows32Slots : (fp8 ? kFewRows16Slots : kFewRows16SlotsBf16);
         else if (r > 16) wanted += kFewRows32PieceSlots;
     }
-    if (rows > kSmallHeads || slots < wanted) return 0;
+    if (rows > (fp8 ? 16 : kSmallHeads) || slots < wanted) return 0;
     return rows <= 16 ? 16 : 32;
 }
 

@@ -5,7 +5,7 @@ import math
 import numpy as np
 import pytest
 
-from helpers import TOL_FP8, check_lse, check_out
+from helpers import TOL_FP8, check_lse, check_out, few_heads_form
 from opfoundry_b200 import api, synth
 
 pytestmark = pytest.mark.gpu
@@ -281,3 +281,24 @@ def test_nan_in_a_row_reaches_out_and_lse_on_every_route(built_lib, H, topk, num
     assert np.isnan(_f32(out)[1]).any(axis=-1).all() and np.isnan(lse[1]).all()
     np.testing.assert_array_equal(out[[0, 2]], clean_out[[0, 2]])
     np.testing.assert_array_equal(lse[[0, 2]], clean_lse[[0, 2]])
+
+
+@pytest.mark.parametrize("H,s_q,num_sms", [(17, 1, 2), (24, 1, 148), (32, 1, 6), (16, 2, 4), (8, 3, 148)])
+def test_17_to_32_rows(built_lib, oracle, H, s_q, num_sms):
+    """Heads or stacked rows that the few-heads kernel would take from a bf16 cache, at the edges of this kernel's tiles of 64 slots."""
+    from gpu_util import run_gpu, run_oracle
+    edges = [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 191, 193, 257, 321, 1100]
+    lens = np.repeat(np.array(edges + edges[::-1], np.int32), s_q)
+    T = len(lens)
+    case = synth.make_decode_case(T // s_q, H, 1216, 1100, s_q=s_q, fp8=True, paged=True, seed=H)
+    for r, n in enumerate(lens):
+        if r % s_q:
+            case["indices"][r] = case["indices"][r - r % s_q]
+        case["indices"][r, n:] = -1
+    kw = dict(num_sms=num_sms, valid_len_hint=lens, mtp_shared=[True] * (T // s_q) if s_q > 1 else None)
+    assert few_heads_form(api.plan_host(T, H, 1100, s_q, **kw)) == 0
+    g_out, g_lse, plan = run_gpu(case, SCALE, **kw)
+    assert s_q == 1 or any(w.stacked_rows == s_q for w in plan.read_works()[0])
+    r_out, r_lse = run_oracle(oracle, case, SCALE)
+    check_out(g_out, r_out, **TOL_FP8)
+    check_lse(g_lse, r_lse)

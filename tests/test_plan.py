@@ -176,10 +176,10 @@ def test_mtp_rows_that_share_a_list_are_planned_as_one_stacked_item():
 
 @pytest.mark.parametrize("form,total_q,H,topk,kw", [
     (0, 200, 16, 128, {}), (16, 200, 16, 160, {}), (16, 200, 1, 2048, {}),       # whole items of at most 16 rows: 160 slots and more
-    (0, 200, 17, 640, {}), (0, 200, 32, 767, {}), (32, 200, 32, 768, {}), (32, 64, 17, 2048, {}),    # 17 to 32 rows: 768
-    (16, 1, 16, 2048, {}), (32, 1, 32, 2048, {}),                                # pieces of 128 slots of a split item
+    (0, 200, 17, 640, {}), (0, 200, 32, 768, {}), (0, 64, 17, 2048, {}),         # not 17 to 32 rows with an fp8 cache
+    (16, 1, 16, 2048, {}), (0, 1, 32, 2048, {}),                                 # pieces of a split item
     (0, 2, 33, 2048, {}), (0, 2, 128, 2048, {}),                                 # more rows than it takes
-    (32, 64, 16, 2048, dict(s_q=2, mtp_shared=[True] + [False] * 31)), (0, 400, 16, 300, dict(s_q=2, mtp_shared=[True] * 200)),
+    (0, 64, 16, 2048, dict(s_q=2, mtp_shared=[True] + [False] * 31)), (0, 400, 16, 300, dict(s_q=2, mtp_shared=[True] * 200)),
     (16, 400, 16, 300, dict(s_q=2, mtp_shared=[False] * 200)), (0, 64, 32, 2048, dict(s_q=2, mtp_shared=[True] * 32)),
     (0, 300, 16, 2048, dict(valid_len_hint=[100] * 300)), (16, 300, 16, 2048, dict(valid_len_hint=[100, 300] * 150)),   # by the mean length
 ])
