@@ -317,16 +317,19 @@ inline int build_plan_whole(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
 // The plan a shape gets: the balanced one, unless the plan without splits is nearly as even.  A split
 // costs what the makespan does not show: fp32 partial results written and read back (4x the bytes of
 // the bf16 output) and the merge after the attention kernel, together worth about kMergeCostTiles steps.
-// On the 128-row kernels (more than kSmallHeads heads) a piece costs more than the cuts assume - Q, the refilled pipeline and 128 fp32
-// rows to store, about 10 000 cycles where a step takes 600 - so there the two plans are compared with dearer pieces, too, where
-// every second list gets a unit at least (and none has stacked rows, which were not measured).  By how much longer the whole plan's
-// longest list then is (in steps): rows x slots, split -> whole, 128 heads, us
-//   -7: 134 x 2048 fp8 114.1 -> 106.0, bf16 88.3 -> 79.3      -6: 47 x 1000 39.0 -> 33.0, 31.3 -> 26.2      -4: 56 x 2048 60.2 -> 55.5, 49.1 -> 40.6
-//   -1: 128 x 2048 114.5 -> 105.8, 87.4 -> 79.6       2: 50 x 2048 56.3 -> 55.2, 45.5 -> 40.2; 30 x 1000 31.1 -> 31.8, 25.4 -> 23.4
-//    4: 26 x 1000 28.3 -> 31.8, 24.0 -> 22.9; 40 x 1500 42.6 -> 43.4, 33.8 -> 32.3       6: 105 x 1300 73.5 -> 76.3, 56.0 -> 53.7
-//   10: 10 x 512 18.2 -> 20.8, 15.6 -> 15.8      13: 112 x 2048 100.0 -> 105.4, 78.2 -> 75.4      25: 100 x 2048 92.2 -> 105.5, 73.2 -> 73.4
+// On the 128-row kernels a piece costs more than the cuts assume: Q, the refilled pipeline and 128 fp32 rows to store, about 10 000 cycles where a step
+// takes 1 150 (fp8 cache) or 700 (bf16).  So there the two plans are compared with dearer pieces, too, where every second list gets a unit at least (and
+// none has stacked rows, which were not measured).  By how much longer the whole plan's longest list then is (in steps, at 20 a piece): rows x slots, time of
+// the whole plan over that of the split one.
+//   more than 64 heads (96 and 128), fp8 | bf16
+//     -7: 49 x 1000 0.79-0.82 | 0.82   134 x 2048 0.90-0.93 | 0.89-0.92    -3: 38 x 1000 0.80-0.93 | 0.80-0.84   113 x 1000 0.94-0.96 | 0.88-0.91
+//      1: 38 x 1300 0.94-0.97 | 0.91-0.97   112 x 1300 1.00-1.01 | 0.94-0.96    2: 50 x 2048 0.91-0.94 | 0.84   104 x 1000 1.00-1.01 | 0.90-0.96
+//      4: 26 x 1000 1.12 | 0.95    6: 105 x 1300 1.04 | 0.96   10: 10 x 512 1.14 | 1.01   25: 100 x 2048 1.14 | 1.00   (128 heads)
+//   33 to 64 heads (40 and 64), where the pieces are cheaper
+//     -7: 49 x 1000 0.93-0.94 | 0.88-0.90   60 x 2048 0.94 | 0.87-0.91   134 x 2048 0.89-1.01 | 0.91-0.96   128 x 1300 1.00-1.01 | 0.92-0.98
+//     -5: 44 x 1000 0.97-1.08 | 0.91-1.00   -3: 38 x 1000 0.99-1.11 | 0.95-1.01   2: 50 x 2048 1.07-1.12 | 0.95-1.00   104 x 1000 1.07-1.10 | 1.00
 constexpr int kMergeCostTiles = 6;
-constexpr int kWidePieceOverheadTiles = 20, kWideMergeCostTiles = 2;
+constexpr int kWidePieceOverheadTiles = 20, kWideMergeCostTiles = 2, kHalfWideMergeCostTiles = -7;
 inline int build_plan(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
     int rc = build_plan_split(sh, num_sms, P);
     if (rc) return rc;
@@ -336,7 +339,7 @@ inline int build_plan(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
     if (rc) return rc;
     const auto whole_within = [&](int overhead, int steps) { return plan_makespan(W, overhead) <= plan_makespan(P, overhead) + steps; };
     const bool wide = sh.H > kSmallHeads && !P.hdr.has_stacked && 2 * int(W.works.size()) >= P.hdr.num_lists;
-    if (whole_within(kPieceOverheadTiles, kMergeCostTiles) || (wide && whole_within(kWidePieceOverheadTiles, kWideMergeCostTiles))) P = W;
+    if (whole_within(kPieceOverheadTiles, kMergeCostTiles) || (wide && whole_within(kWidePieceOverheadTiles, sh.H > kHeadsPerBlock / 2 ? kWideMergeCostTiles : kHalfWideMergeCostTiles))) P = W;
     return DSA_V32_OK;
 }
 
