@@ -300,6 +300,8 @@ int launch_attention(const dsa_v32_attn_args* a, int want_dtype, cudaStream_t st
         cudaError_t e = launch_paired_heads(use_ext, h.num_lists, tq, p, stream);
         return e == cudaSuccess ? DSA_V32_OK : (int)e;
     }
+    // (no tensor map here, but one on the route for at most 16 rows: what a call may be does not depend on the number of heads)
+    if (a->stride_q_head >= (int64_t(1) << 39) || a->stride_q_row >= (int64_t(1) << 39)) return DSA_V32_ERR_DRIVER;
     cudaError_t e = launch_paired_fp8(use_ext, live_tile_rows(h), h.num_lists, p, stream);
     return e == cudaSuccess ? DSA_V32_OK : (int)e;
 }

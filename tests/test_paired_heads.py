@@ -71,6 +71,17 @@ def test_any_stride_of_a_single_row_or_head(built_lib, T, H, topk, strides):
     assert torch.equal(out.view(torch.int16), want.view(torch.int16)) and torch.equal(lse, want_lse)
 
 
+@pytest.mark.parametrize("T,H,strides", [(1, 128, (1 << 40, 576, 1)), (1, 8, (1 << 40, 576, 1)), (3, 1, (576, 1 << 41, 1)), (1, 40, (1 << 39, 576, 1))])
+def test_strides_beyond_a_tensor_map_stay_refused_with_an_fp8_cache(built_lib, T, H, strides):
+    """Whichever kernel the number of heads would lead to."""
+    from gpu_util import to_dev
+    case = synth.make_decode_case(T, H, 1024, 100, fp8=True, paged=True, seed=H)
+    d = to_dev(case)
+    plan = api.mla_decode_plan_create(T, H, 100)
+    with pytest.raises(api.DsaError):
+        api.mla_decode_launch_pipeline(d["q"].as_strided((T, H, 576), strides), d["kv"], d["indices"], plan, SCALE, block_table=d["block_table"], page_block_size=64)
+
+
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("B,H", [(3, 128), (80, 72)])
 def test_repeated_launches_give_the_same_bits(built_lib, B, H, fp8):
