@@ -331,6 +331,109 @@ def test_items_with_residuals():
         for i, role in enumerate([None, "softmax0.0", "softmax1.3", "softmax0.5", "softmax1.14", "softmax0.2", "pv", "issuer1", "~score0"]):
             PairFp8(items, random.Random(i), wide=0.5, idle=(lambda c, rq, n: rq == 1) if i % 3 == 2 else lambda c, rq, n: False).run(slow=role)
 
+def sync_points(src):
+    """Every wait, arrival and commit of the kernel, in the order of the source, with its barrier and parity."""
+    src, out = re.sub(r"//[^\n]*", "", src), []
+    for m in re.finditer(r"\b(wait_on[23]?|warp_wait|warp_arrive(?:_lead)?|tc_commit_pair_el|cp_async_mbar_arrive_noinc)\(", src):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(src[i], 0)
+            i += 1
+        args = re.sub(r"\s+", " ", re.sub(r"smem_u32\(&ctl->([^()]*)\)", r"&ctl->\1", src[m.end():i - 1]))
+        if "ctl->" in args:     # (else a wrapper's own)
+            for part in ("&ctl->", ", abort_flag", ", lane", ", el"):
+                args = args.replace(part, "")
+            out.append(m.group(1) + " " + args)
+    return out
+
+
+# What the roles above restate, role by role.  A line that differs from the source means that the model has to be looked at again.
+SYNC_POINTS = """
+warp_arrive_lead q_full
+warp_arrive q_here
+wait_on q_empty, (item_n - 1) & 1
+wait_on o_full, (item_n - 1) & 1
+warp_arrive_lead o_free
+warp_arrive_lead o_free
+warp_arrive_lead o_free
+wait_on q_here, item_n & 1
+warp_arrive residual_here[rq]
+wait_on residual_here[rq], n_wide & 1
+wait_on s_full[team], ph2
+warp_arrive_lead s3_empty
+warp_arrive_lead s_empty[team]
+warp_arrive raw_empty[ring.s]
+wait_on pv_done[team], ph2 ^ 1u
+warp_arrive posted[team][rq]
+warp_arrive moved[team][rq]
+warp_arrive_lead p_full[team]
+wait_on3 prep[ring.s], ring.ph, s_full[team], ph2, moved[team][rq], ph2 ^ 1u
+warp_arrive_lead s3_empty
+warp_arrive_lead s_empty[team]
+warp_arrive raw_empty[ring.s]
+warp_arrive_lead s_empty[team]
+warp_arrive posted[team][rq]
+wait_on2 posted[team][rq], ph2, moved[team ^ 1][rq], ((it - 1) >> 1) & 1u
+warp_arrive moved[team][rq]
+warp_arrive raw_empty[ring.s]
+wait_on pv_done[team], ph2 ^ 1u
+wait_on pv_done[team ^ 1], ((it - 1) >> 1) & 1u
+warp_arrive_lead p_full[team]
+wait_on moved[last_team][rq], (last >> 1) & 1u
+warp_arrive e_bar
+wait_on e_bar, item_n & 1
+wait_on q_full, item_n & 1
+wait_on tile_ready[par][ring.s], (ready_bits >> ring.s) & 1u
+wait_on s_empty[par], ((it >> 1) & 1u) ^ 1u
+wait_on s3_empty, (it - 1) & 1u
+tc_commit_pair_el s_full[par]
+tc_commit_pair_el raw_empty[ring.s]
+tc_commit_pair_el q_empty
+wait_on o_free, (item_n - 1) & 1
+wait_on p_full[sb], (it >> 1) & 1u
+wait_on v_full[unit.s], unit.ph
+tc_commit_pair_el v_empty[unit.s]
+tc_commit_pair_el pv_done[sb]
+tc_commit_pair_el o_full
+warp_wait kv_full[ring.s], ring.ph
+warp_arrive_lead tile_ready[it & 1u][ring.s]
+warp_arrive prep[ring.s]
+warp_wait finished, 0
+wait_on raw_empty[ring.s], ring.ph
+warp_arrive late_known[ring.s]
+cp_async_mbar_arrive_noinc kv_full[ring.s]
+warp_arrive kv_full[ring.s]
+wait_on2 prep[ring.s], ring.ph, v_empty[unit.s], unit.ph
+warp_arrive raw_empty[ring.s]
+warp_arrive_lead v_full[unit.s]
+wait_on late_known[known.s], known.ph
+wait_on late_known[known.s], known.ph
+wait_on2 prep[ring.s], ring.ph, v_empty[unit.s], unit.ph
+warp_arrive raw_empty[ring.s]
+warp_arrive_lead v_full[unit.s]
+warp_arrive finished
+"""
+
+
+def test_the_model_restates_the_kernels_waits_and_arrivals():
+    assert sync_points(SRC) == SYNC_POINTS.strip().split("\n")
+
+
+def test_the_model_counts_arrivals_as_the_kernel_does():
+    names = ("kLoadWarps", "kConvWarps", "kTeamWarps", "kSoftmaxWarps", "kWarps")
+    values = {n: _const(n) for n in names}
+    model = PairFp8([1], random.Random(0))
+    found = re.findall(r"mbar_init\(smem_u32\(&ctl->(\w+)[^)]*\), ([^;]+)\);", SRC)
+    assert len({n for n, _ in found}) == 22
+    for name, count in found:
+        if name == "finished":      # at the end of every other warp; the model ends by itself
+            continue
+        bar = getattr(model, name)
+        while isinstance(bar, list):
+            bar = bar[0]
+        assert bar.count == eval(count.replace("/", "//"), {}, values), name
+
+
 
 def test_the_model_sees_a_missing_wait():
     """A warp that posts a tile's maxima before its team has read those of the team's last tile."""
