@@ -367,7 +367,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             fence_proxy_async_smem();
             warp_arrive_lead(&ctl->q_full, lane);
             // The scores may start; meanwhile, elements that are not 0 and lie below 2^-2 with the row's factor: their magnitudes' bits less 1 (a 0 becomes
-            // the largest), cut off to [line - 2, line - 1], in sums of eight modulo 2^16
+            // the largest), cut off to line - 2 or line - 1, two halves in 32-bit sums, from which line - 2 is taken at the end (a 0 in the lower half lends
+            // its neighbour's last bit, which an element on the line may cost its place)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const uint32_t line = ((row_e[i] - 13u) << 7) * 0x10001u;
@@ -377,9 +378,9 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const uint32_t w = (j == 0 ? x[i][k].x : j == 1 ? x[i][k].y : j == 2 ? x[i][k].z : x[i][k].w) & 0x7FFF7FFFu;
-                        n = add_u16x2(n, max_u16x2(min_u16x2(add_u16x2(w, 0xFFFFFFFFu), line - 0x10001u), line - 0x20002u));
+                        n += max_u16x2(min_u16x2(w - 0x10001u, line - 0x10001u), line - 0x20002u);
                     }
-                n = sub_u16x2(n, (((row_e[i] - 13u) * 1024u - 16u) & 0xFFFFu) * 0x10001u);
+                n -= 8u * (line - 0x20002u);
                 const uint32_t below = 512u - __reduce_add_sync(0xffffffffu, (n & 0xFFFFu) + (n >> 16));
                 if (lane == 0) ctl->q_exp[row0 + i] = static_cast<uint16_t>(row_e[i] == 255u ? 255u : row_e[i] - 11u + (below > kWideElements ? 256u : 0u));
             }

@@ -747,12 +747,6 @@ __device__ __forceinline__ uint32_t scale_f16x2(uint32_t v, uint32_t hi, uint32_
 }
 // two bf16 times a power of two
 __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float mul) { return pack_bf16x2(__uint_as_float(v << 16) * mul, __uint_as_float(v & 0xFFFF0000u) * mul); }
-__device__ __forceinline__ uint32_t add_u16x2(uint32_t a, uint32_t b) {   // modulo 2^16, as the next
-    uint32_t r;
-    asm("add.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ uint32_t sub_u16x2(uint32_t a, uint32_t b) { return add_u16x2(add_u16x2(a, ~b), 0x10001u); }
 __device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
