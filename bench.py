@@ -61,7 +61,7 @@ def measured_traffic(batch):
     """DRAM bytes (read + write) of one attention launch of the headline workload, from the ncu capture
     recorded beside its summary (taken at a smaller batch; traffic is proportional to the batch because
     every sequence has its own cache pages).  None when no capture of the current kernel is recorded."""
-    path = os.path.join(ROOT, "profiles", "sparse_mla_fp8_decode_traffic.json")
+    path = os.path.join(ROOT, "profiles", "paired_fp8_decode_traffic.json")
     if not os.path.exists(path):
         return None
     with open(path) as f:

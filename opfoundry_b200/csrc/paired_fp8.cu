@@ -18,13 +18,14 @@
 // sums.  A row with more than kWideElements, zeros aside, below that line has a few far above the others, which the cache may answer with
 // zeros: there the softmax warps add what hi + lo leave out (residual_group), so the row is as exact as with bf16 operands.  (With an element X times the rest in a
 // column where the cache holds zeros, the error of lse is 2e-6 to 1.4e-5, the most at X = 2^8; the kernel before this one had 2.5e-5 to 6e-5 for any X.  A row of
-// normal numbers needs one of 2^9 for that; if all rows have one, 64 sequences of 128 heads take 392 us instead of 57, one 40 instead of 16.5.)
+// normal numbers needs one of 2^9 for that; if all rows have one, 64 sequences of 128 heads take 392 us instead of 57, one 40 instead of 17.)
 // P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15; V = byte x scale 2^-e, rounded once,
 // with one e per scale group for the tile's 64 rows, so that the largest |V| stays below 2^16.  e starts at the exponent of the group's largest
 // scale in an item's first tile and moves up when a scale exceeds it by 2^7; the group's columns of O are then brought to the new e like they are to a
 // new reference maximum.  A row whose scales all lie more than 2^8 below their e lends V the difference, x = 20 octaves at most, and P takes it
-// back (V 2^x, P 2^-x): f16 alone would lose the rows' bits beside a large row from 2^-14 on.  What is left below f16's normal range then is
-// 2^-41 of the largest V at full weight (a group of a row that is small only beside another group of the same row: 2^-21).
+// back (V 2^x, P 2^-x): f16 alone would lose bits of a row at 2^-21 of a large row's scale and less.  What is lost then lies at
+// 2^-41 of the largest V at full weight (a group of a row that is small only beside another group of the same row: 2^-21).  The scale of a group of zeros
+// does not count where it differs from the row's other scales by more than 2^12 (the cache writer gives such a group 1).
 //
 // S in TMEM: lanes 0-63 = the CTA's 64 rows x slots of CTA 0, lanes 64-127 = the same rows x slots of CTA 1.
 // O in TMEM: lanes 0-63 = the rows x columns of CTA 0, lanes 64-127 = the rows x columns of CTA 1.
@@ -43,16 +44,17 @@
 // What bounds it (cycle stamps of an instrumented copy, 64 sequences x 128 heads x 2048 slots): a tile of 64 slots every 2 300 cycles.  Its MMAs
 // take 1 430 (measured alone; the scores' 25 an instruction are the rate of shared memory, 3 KB of operands each), all its traffic in shared
 // memory 2 000; what is in flight - four raw tiles, one and a half converted ones - over the 10 000 cycles from a load to the end of P V gives the rest:
-// landing 1 900, scores 1 500, softmax 3 100, a converter's turn 2 200.  Every role pays for the number of its instructions, 6 700 a tile and SM:
+// landing 1 900, scores 1 500, softmax 3 100, a converter's turn 2 200.  Every role pays for the number of its instructions, about 6 900 a tile and SM:
 // eight warps of a scheduler on five loops miss the instruction cache (4.7 of 19.6 cycles an instruction in a form of 85 KB; a warp number known
 // to be uniform, short waits and rolled loops brought 81 us to 61).  Tried: four teams of four warps with 32 slots a thread (fewer instructions, but
 // a tile takes 5 000 cycles from scores to P: 2 880 a tile where two teams of eight took 2 780), two teams of four (2 750, and 1.5 us more for one
 // sequence), a converter on both units of a tile (3 240).  The other CTA's rows in the raw tiles, three of 28 KB: 60.6 us instead of 56.5.
 // Against the kernel before it (the 576 columns split over the pair, partial scores summed through distributed shared memory in 16 bits, four tile
-// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots: one sequence 19.5 -> 16.0 us with its merge, 16 35.6 -> 30.2, 64 84.2 -> 62.1 (32768 positions each,
-// other inputs every pass); 37 58.7 -> 43.7, 128 161 -> 106 (8192 positions).
-// Against 64 bits, six shapes of 40 to 128 heads: out 1.68e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to 2.30e-3),
-// lse at most 1.9e-6 (7e-5).
+// stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots, 32768 positions each, other inputs every pass: one sequence 19.4 -> 16.65 us with its merge,
+// 16 35.6 -> 31.2, 64 84.0 -> 63.2.  (Of these 0.5, 0.9 and 1.3 us are what keeps Q and V exact beside elements, rows and groups that are far larger: the count of
+// Q's small elements at the start of an item takes 0.3 of the first two, the rest lies in instructions here and there.)
+// Against 64 bits, nine shapes of 24 to 128 heads: out 1.67e-3 to 1.69e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to
+// 2.30e-3), lse at most 1.7e-6 (7e-5; the few-heads kernel that took 17 to 32 rows before 1.4e-6).
 //
 // Every mbarrier wait is bounded: warp 19 of either CTA, which sees every tile and stays until the other warps have finished, waits by time, the
 // others end by the abort flag that it raises.  On expiry the CTA raises its own and its peer's abort flag, records DSA_V32_ERR_DEVICE_WAIT in
@@ -234,7 +236,7 @@ __device__ __forceinline__ void residual_group(const __nv_bfloat16* q0, const __
 // kShare: tile rows that a CTA owns, 64, or 32 for plans without items of more than 64: softmax warps without a live row only take part in the
 // barriers (128 sequences of 2 x 16 heads 144 -> 134 us), and with 32 that is half of either CTA's (64 sequences of 64 heads 55.5 -> 52.5 us; decided
 // at run time it costs 0.4 us a launch).
-// kExt: a sink, peers, stacked rows, or rows of out on 16-byte boundaries
+// kExt: a sink, peers, or rows of out on 16-byte boundaries (stacked rows need nothing of it, but come with it, as they do on the bf16 kernel)
 template <bool kExt, int kShare>
 __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnParams p) {
     extern __shared__ __align__(1024) uint8_t smem_paired_fp8[];   // the same offset in both CTAs of a pair

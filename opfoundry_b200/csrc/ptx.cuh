@@ -581,7 +581,7 @@ __device__ __forceinline__ void umma_pair_ss_el(uint32_t d_tmem, uint64_t a_desc
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
-// four K = 16 steps of one 64-column block, as umma_ts_x4_el and umma_ss_x4_el
+// four K = 16 steps of one 64-column block, as umma_ss_x4_el
 __device__ __forceinline__ void umma_pair_ts_x4_el(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                                    uint32_t first_accumulates, uint32_t elected) {
     asm volatile(

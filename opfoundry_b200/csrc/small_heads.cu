@@ -30,10 +30,10 @@
 // rows 700, scores 2 000, softmax 2 100, P V 750 and the hand-offs between them), three stages: 2 850-3 300 cycles per
 // 48 slots; its MMAs take 2 000 of them to issue (36 for the scores of M = 64, N = 16 at 33 cycles, 12 for P V at 62), though
 // the counter has the tensor pipe active for 8 %.
-// Measured against paired_fp8.cu: 74 rows of 16 heads x 2048 slots 57.8 -> 50.9 us, 200 x 1024 90.3 -> 73.1.  (For 17 to 32 rows of an fp8 cache it
+// Measured against paired_fp8.cu: 74 rows of 16 heads x 2048 slots 57.8 -> 50.9 us, 200 x 1024 90.3 -> 73.1 (52 and 75 since its loaders look for NaN codes).  (For 17 to 32 rows of an fp8 cache it
 // had a form, too: 71 us for 74 x 2048 where paired_fp8.cu takes 60.)  Against paired_heads.cu: bf16, 296 rows of 16 heads x 1024 slots 86.6 -> 78.9,
 // eight sequences of 16 heads x 2048 in pieces 15.1 -> 14.2 with the merge; more shapes beside the rule (few_heads_form in plan.h).
-// out against 64 bits: 2.08e-3 (1.68e-3 in paired_fp8.cu), lse 2e-7 (2e-6).
+// out against 64 bits: 2.08e-3 (1.68e-3 in paired_fp8.cu), lse at most 1.4e-6 (1.7e-6).
 //
 // Every mbarrier wait is bounded, as in the 128-row kernels, and the warps of the softmax group meet on mbarriers only, so a
 // warp that gave up never leaves the others in a hardware barrier.
