@@ -25,7 +25,7 @@
 // new reference maximum.  A row whose scales all lie more than 2^8 below their e lends V the difference, x = 20 octaves at most, and P takes it
 // back (V 2^x, P 2^-x): f16 alone would lose bits of a row at 2^-21 of a large row's scale and less.  What is lost then lies at
 // 2^-41 of the largest V at full weight (a group of a row that is small only beside another group of the same row: 2^-21).  The scale of a group of zeros
-// does not count where it differs from the row's other scales by more than 2^12 (the cache writer gives such a group 1).
+// does not count where it would make its row lose bits (the cache writer gives such a group 1).
 //
 // S in TMEM: lanes 0-63 = the CTA's 64 rows x slots of CTA 0, lanes 64-127 = the same rows x slots of CTA 1.
 // O in TMEM: lanes 0-63 = the rows x columns of CTA 0, lanes 64-127 = the rows x columns of CTA 1.
@@ -863,51 +863,55 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                         const uint32_t x = (__float_as_uint(s.x) >> 23) & 0xFFu, y = (__float_as_uint(s.y) >> 23) & 0xFFu;
                         a[g] = (x < 255u ? x : 0u) | (y < 255u ? y : 0u) << 16;
                     }
-                    uint32_t most = max_u16x2(max_u16x2(a[0], a[1]), max_u16x2(a[2], a[3]));
-                    const uint32_t spread = most - min_u16x2(min_u16x2(a[0], a[1]), min_u16x2(a[2], a[3]));
-                    if (__any_sync(0xffffffffu, max(spread & 0xFFFFu, spread >> 16) > 12u)) {
-                        // a group may be zeros under any scale (the cache writer gives it 1): then the scale does not count and becomes 0
-                        const uint32_t odd = __ballot_sync(0xffffffffu, (spread & 0xFFFFu) > 12u), odd1 = __ballot_sync(0xffffffffu, (spread >> 16) > 12u);
+                    const int e_old = e;
+                    int x0, x1;   // octaves that the two rows take more than 2^-e
+                    bool lent;
 #pragma unroll 1
-                        for (int slot = 0; slot < kSlots; ++slot) {
-                            if (!(((slot & 1 ? odd1 : odd) >> (slot >> 1)) & 1u)) continue;
-                            const bool own = slot / kOwn == rank;
-                            const int late = ctl->late_row[ring.s][slot % kOwn];
+                    for (bool looked = false;; looked = true) {
+                        // the largest of the tile's rows (of both CTAs' slots, so both CTAs follow the same e)
+                        uint32_t top = 0u;
 #pragma unroll
-                            for (int g = 0; g < kGroups; ++g) {
-                                uint32_t v = 0u;
-                                if (own) v = *reinterpret_cast<const uint32_t*>(sRaw + ring.s * kRawBytes + g * kBlock + (slot % kOwn) * 128 + 4 * lane);
-                                else if (late >= 0) v = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(p.kv) + (size_t)late * kFp8RowBytes + 128 * g) + lane);
-                                const uint32_t half = slot & 1 ? 0xFFFF0000u : 0xFFFFu;
-                                if (!__any_sync(0xffffffffu, (v & 0x7F7F7F7Fu) != 0u) && lane == slot >> 1 && (a[g] & half) != 0u) {
+                        for (int g = 0; g < kGroups; ++g) {
+                            const uint32_t m = __reduce_max_sync(0xffffffffu, max(a[g] & 0xFFFFu, a[g] >> 16));
+                            if ((lane & 3) == g) top = m;
+                        }
+                        const int em = max(static_cast<int>(top) - 127, -120);
+                        e = t == 0 || em >= e_old + 7 ? min(em, 126) : e_old;
+                        // how far a row's groups lie below their e, 512 added: the least and the most of them
+                        uint32_t low = 0xFFFFFFFFu, deep = 0u;
+#pragma unroll
+                        for (int g = 0; g < kGroups; ++g) {
+                            const uint32_t d = __shfl_sync(0xffffffffu, (e + 127 + 512) * 0x10001, g) - a[g];
+                            const uint32_t counts = (((a[g] + 0x00FF00FFu) >> 8) & 0x00010001u) * 0xFFFFu;   // (a is not 0)
+                            low = min_u16x2(low, d | ~counts);
+                            deep = max_u16x2(deep, d & counts);
+                        }
+                        x0 = (low & 0xFFFFu) == 0xFFFFu ? 0 : min(max(static_cast<int>(low & 0xFFFFu) - 520, 0), 20);
+                        x1 = (low >> 16) == 0xFFFFu ? 0 : min(max(static_cast<int>(low >> 16) - 520, 0), 20);
+                        lent = __any_sync(0xffffffffu, max(deep & 0xFFFFu, deep >> 16) > 520u);
+                        if (!lent || looked) break;
+                        const int y0 = static_cast<int>(deep & 0xFFFFu) - x0, y1 = static_cast<int>(deep >> 16) - x1;
+                        uint32_t rows0 = __ballot_sync(0xffffffffu, y0 > 512 + 18), rows1 = __ballot_sync(0xffffffffu, y1 > 512 + 18);
+                        if ((rows0 | rows1) == 0u) break;
+                        // A group of some row would lose bits.  The reason may be another group of that row, of zeros under any scale (the cache
+                        // writer gives it 1): its scale does not count and becomes 0 (f16 may not hold what is left of it).
+#pragma unroll 4
+                        for (int slot = 0; slot < kSlots; ++slot) {
+                            if (!(((slot & 1 ? rows1 : rows0) >> (slot >> 1)) & 1u)) continue;
+                            // sixteen bytes a lane, eight lanes a group
+                            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                            const int late = ctl->late_row[ring.s][slot % kOwn];
+                            if (slot / kOwn == rank) v = *reinterpret_cast<const uint4*>(sRaw + ring.s * kRawBytes + (lane >> 3) * kBlock + (slot % kOwn) * 128 + 16 * (lane & 7));
+                            else if (late >= 0) v = ldg_stream_16(reinterpret_cast<const uint8_t*>(p.kv) + (size_t)late * kFp8RowBytes + 16 * lane);
+                            const uint32_t full = __ballot_sync(0xffffffffu, ((v.x | v.y | v.z | v.w) & 0x7F7F7F7Fu) != 0u), half = slot & 1 ? 0xFFFF0000u : 0xFFFFu;
+#pragma unroll
+                            for (int g = 0; g < kGroups; ++g)
+                                if (((full >> (8 * g)) & 0xFFu) == 0u && lane == slot >> 1 && (a[g] & half) != 0u) {
                                     a[g] &= ~half;
-                                    ctl->scale[ring.s][g][slot] = 0.0f;   // (f16 may not hold what is left of it below)
+                                    ctl->scale[ring.s][g][slot] = 0.0f;
                                 }
-                            }
                         }
                     }
-                    // the largest of the tile's rows (of both CTAs' slots, so both CTAs follow the same e)
-                    uint32_t top = 0u;
-#pragma unroll
-                    for (int g = 0; g < kGroups; ++g) {
-                        const uint32_t m = __reduce_max_sync(0xffffffffu, max(a[g] & 0xFFFFu, a[g] >> 16));
-                        if ((lane & 3) == g) top = m;
-                    }
-                    const int em = max(static_cast<int>(top) - 127, -120);
-                    const int e_old = e;
-                    if (t == 0 || em >= e + 7) e = min(em, 126);
-                    // how far a row's groups lie below their e, 512 added: the least and the most of them
-                    uint32_t low = 0xFFFFFFFFu, deep = 0u;
-                    most = 0u;
-#pragma unroll
-                    for (int g = 0; g < kGroups; ++g) {
-                        const uint32_t d = __shfl_sync(0xffffffffu, (e + 127 + 512) * 0x10001, g) - a[g];
-                        low = min_u16x2(low, d);
-                        deep = max_u16x2(deep, d);
-                        most |= a[g];
-                    }
-                    const int x0 = most & 0xFFFFu ? min(max(static_cast<int>(low & 0xFFFFu) - 520, 0), 20) : 0, x1 = most >> 16 ? min(max(static_cast<int>(low >> 16) - 520, 0), 20) : 0;
-                    const bool lent = __any_sync(0xffffffffu, (most & 0xFFFFu && static_cast<int>(deep & 0xFFFFu) > 520) || (most >> 16 && static_cast<int>(deep >> 16) > 520));
                     if (lent) {
                         *reinterpret_cast<float2*>(&ctl->v_lent[ring.s][2 * lane]) = make_float2(__uint_as_float((127 + x0) << 23), __uint_as_float((127 + x1) << 23));
                         reinterpret_cast<uint32_t*>(ctl->p_back[ring.s])[lane] = pow2_f16(-x0) | pow2_f16(-x1) << 16;

@@ -157,6 +157,18 @@ def test_one_group_far_smaller_than_the_others(built_lib, oracle, power):
     _check_groups(oracle, dict(case, kv=kv))
 
 
+@pytest.mark.parametrize("power", [-12, -20, -30, None])
+def test_groups_small_by_turns(built_lib, oracle, power):
+    """Some rows have one group far smaller (None: of scale 0) than their others, other rows another: neither takes bits from the large ones.
+    (Against 64 bits the kernel is up to 2.0e-3 of a group's largest output off here, the oracle, which rounds P to 8 bits, 4.0e-3: together 6e-3.)"""
+    case = _case(17)
+    kv = case["kv"].copy()
+    scales, factor = kv[:, 512:528].view(np.float32), np.float32(0.0 if power is None else 2.0 ** power)
+    scales[::3, 0] *= factor
+    scales[1::3, 1] *= factor
+    _check_groups(oracle, dict(case, kv=kv), rel=6e-3)
+
+
 @pytest.mark.parametrize("power", [-14, -22, -30, -38])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_small_rows_that_carry_the_weight(built_lib, oracle, power, mixed):
