@@ -325,11 +325,12 @@ inline int build_plan_whole(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
 //     -7: 49 x 1000 0.79-0.82 | 0.82   134 x 2048 0.90-0.93 | 0.89-0.92    -3: 38 x 1000 0.80-0.93 | 0.80-0.84   113 x 1000 0.94-0.96 | 0.88-0.91
 //      1: 38 x 1300 0.94-0.97 | 0.91-0.97   112 x 1300 1.00-1.01 | 0.94-0.96    2: 50 x 2048 0.91-0.94 | 0.84   104 x 1000 1.00-1.01 | 0.90-0.96
 //      4: 26 x 1000 1.12 | 0.95    6: 105 x 1300 1.04 | 0.96   10: 10 x 512 1.14 | 1.01   25: 100 x 2048 1.14 | 1.00   (128 heads)
-//   33 to 64 heads (40 and 64), where the pieces are cheaper
-//     -7: 49 x 1000 0.93-0.94 | 0.88-0.90   60 x 2048 0.94 | 0.87-0.91   134 x 2048 0.89-1.01 | 0.91-0.96   128 x 1300 1.00-1.01 | 0.92-0.98
-//     -5: 44 x 1000 0.97-1.08 | 0.91-1.00   -3: 38 x 1000 0.99-1.11 | 0.95-1.01   2: 50 x 2048 1.07-1.12 | 0.95-1.00   104 x 1000 1.07-1.10 | 1.00
+//   33 to 64 heads (40 and 64; medians of four runs), where the pieces are cheaper
+//     -5: 44 x 1000 0.92-0.94 | 0.89-0.90   -3: 38 x 1000 0.96-0.99 | 0.94-0.95   113 x 1000 1.00-1.01 | 0.94-0.96   120 x 1300 1.01 | 0.95-0.98
+//     -2: 55 x 2048 0.97-0.98 | 0.91-0.93   129 x 2048 0.93-1.00 | 0.95-0.98       1: 38 x 1300 1.01-1.04 | 0.96-1.01   112 x 1300 1.05 | 1.00-1.02
+//      2: 50 x 2048 0.97-0.99 | 0.91-0.97   104 x 1000 1.08 | 0.98-1.02   124 x 2048 1.01 | 0.96-0.98
 constexpr int kMergeCostTiles = 6;
-constexpr int kWidePieceOverheadTiles = 20, kWideMergeCostTiles = 2, kHalfWideMergeCostTiles = -7;
+constexpr int kWidePieceOverheadTiles = 20, kWideMergeCostTiles = 2, kHalfWideMergeCostTiles = -2;
 inline int build_plan(const dsa_v32_shape& sh, int num_sms, HostPlan& P) {
     int rc = build_plan_split(sh, num_sms, P);
     if (rc) return rc;
