@@ -103,8 +103,8 @@ constexpr uint32_t kColO = 0, kColS = 256, kColS3 = kColS + 6 * 32, kColRope = k
 
 struct Ctl {
     float scale[kStages][kGroups][kSlots];   // row scales of a tile (0 where the slot holds no row)
-    float post[2][4][kRows];                 // by team and quarter of a tile's slots: the rows' maxima (log2 domain); at the end of an item its row sums
-    float m_ref[2][kRows];                   // by tile number mod 2: the rows' reference maxima after the tile
+    float post[2][4][kRows];                 // by team and quarter of a tile's slots: the rows' maxima (in the scores' units); at the end of an item its row sums
+    float m_ref[2][kRows];                   // by tile number mod 2: the rows' reference maxima after the tile (scores' units)
     uint16_t q_exp[kRows];                   // biased exponent of 2^a, Q = 2^a (hi + lo), 255: a row with an infinity or a NaN; 256 more: hi + lo leave out too much
     int32_t late_row[kStages][kOwn];         // rows of the tile that the other CTA gathers
     uint32_t tile_mask[kStages][2];          // which slots of CTA 0 / CTA 1 hold a row
@@ -669,10 +669,11 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             unpack2(sv[j], s0, s1);
                             t[j] = fmaxf(s0, s1);
                         }
-                        ctl->post[team][2 * h + cs][r] = fmaxf(max3(max3(t[0], t[1], t[2]), t[3], t[4]), max3(t[5], t[6], t[7])) * c_log2;
+                        ctl->post[team][2 * h + cs][r] = fmaxf(max3(max3(t[0], t[1], t[2]), t[3], t[4]), max3(t[5], t[6], t[7]));
                         warp_arrive(&ctl->posted[team][rq], lane);
                     }
-                    // ---- P = 2^(score - reference + 7): at most 2^15; a masked slot gives 0.  Taken against the last reference known while
+                    // ---- P = 2^(score - reference + 7), the difference taken before it is scaled (rounded products would lie octaves apart from scores of 2^24
+                    // on, and P in f16 would overflow; 64 sequences 57.75 -> 58.0 us): at most 2^15; a masked slot gives 0.  Taken against the last reference known while
                     // the other maxima are on their way, and again in the rare case that it has moved
                     const float m_was = m_ref;
                     float m_old = -INFINITY;
@@ -682,13 +683,13 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
 #pragma unroll 1
                     while (true) {
                         if (settled || !first) {
-                            const float n = kPShift - (m_ref == -INFINITY ? 0.0f : m_ref);
-                            const uint64_t c2 = pack2(c_log2, c_log2), nm2 = pack2(n, n);
+                            const float n = m_ref == -INFINITY ? 0.0f : -m_ref;
+                            const uint64_t c2 = pack2(c_log2, c_log2), n2 = pack2(n, n), s2 = pack2(kPShift, kPShift);
                             uint64_t ls2 = pack2(0.0f, 0.0f);
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
                                 float e0, e1;
-                                unpack2(fma2(sv[j], c2, nm2), e0, e1);
+                                unpack2(fma2(add2(sv[j], n2), c2, s2), e0, e1);
                                 e0 = ex2_approx(e0);
                                 e1 = ex2_approx(e1);
                                 ls2 = add2(ls2, pack2(e0, e1));
@@ -705,13 +706,13 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                         if (!wait_on2(&ctl->posted[team][rq], ph2, &ctl->moved[team ^ 1][rq], ((it - 1) >> 1) & 1u, abort_flag)) return false;
                         const float mt = fmaxf(fmaxf(ctl->post[team][0][r], ctl->post[team][1][r]), fmaxf(ctl->post[team][2][r], ctl->post[team][3][r]));
                         if (!first) m_old = ctl->m_ref[team ^ 1][r];
-                        m_ref = mt > m_old + 8.0f ? mt : m_old;
+                        m_ref = (mt - m_old) * c_log2 > 8.0f ? mt : m_old;
                         if (h == 0 && cs == 0) ctl->m_ref[team][r] = m_ref;
                         warp_arrive(&ctl->moved[team][rq], lane);
                         if (!first && !__any_sync(0xffffffffu, m_ref != m_was)) break;
                         settled = true;
                     }
-                    if (l != 0.0f && m_was != m_ref) l *= ex2_approx(m_was - m_ref);
+                    if (l != 0.0f && m_was != m_ref) l *= ex2_approx((m_was - m_ref) * c_log2);
                     l += lsum;
                     if (lent) {   // what V was lent
                         const uint4* back = reinterpret_cast<const uint4*>(&ctl->p_back[ring.s][kOwn * h + 16 * cs]);
@@ -729,7 +730,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                     fence_proxy_async_smem();
                     if (!first && __any_sync(0xffffffffu, m_ref != m_old || v_fix != 1.0f)) {
                         // the reference or e moved: O so far (complete once the previous tile's product is) is brought to the new ones
-                        const float f = (m_old == m_ref ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2_approx(m_old - m_ref))) * v_fix;
+                        const float f = (m_old == m_ref ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2_approx((m_old - m_ref) * c_log2))) * v_fix;
                         if (!wait_on(&ctl->pv_done[team ^ 1], ((it - 1) >> 1) & 1u, abort_flag)) return false;
                         tc_fence_after();
 #pragma unroll 1
@@ -751,12 +752,12 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 it_base = it_end;
                 if (!wait_on(&ctl->moved[last_team][rq], (last >> 1) & 1u, abort_flag)) return false;   // the posted maxima have been read, too
                 const float m_fin = ctl->m_ref[last_team][r];
-                if (l != 0.0f && m_ref != m_fin) l *= ex2_approx(m_ref - m_fin);
+                if (l != 0.0f && m_ref != m_fin) l *= ex2_approx((m_ref - m_fin) * c_log2);
                 ctl->post[team][2 * h + cs][r] = l;
                 if (team == static_cast<int>(last_team) && rq == 0 && lane == 0) ctl->v_fin[2 * h + cs] = v_unit;
                 warp_arrive(&ctl->e_bar, lane);
                 if (!wait_on(&ctl->e_bar, item_n & 1, abort_flag)) return false;
-                m_out = m_fin;
+                m_out = m_fin * c_log2;
                 ls = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) ls += ctl->post[i >> 2][i & 3][r];

@@ -314,3 +314,28 @@ def test_17_to_32_rows(built_lib, oracle, H, s_q, num_sms):
     r_out, r_lse = run_oracle(oracle, case, SCALE)
     check_out(g_out, r_out, **TOL_FP8)
     check_lse(g_lse, r_lse)
+
+
+@pytest.mark.parametrize("H,num_sms", [(72, 4), (24, 148)])
+@pytest.mark.parametrize("power", [20, 27, 40])
+def test_scores_beyond_the_resolution_of_their_reference(built_lib, H, num_sms, power):
+    """Scores of 2^power and more: the largest one's row is the output (or a mean of rows whose scores fp32 does not tell apart), and out and lse are finite."""
+    from gpu_util import run_gpu
+    case = _case(18, H=H, topk=500)
+    q = (_f32(case["q"]) * np.float32(2.0 ** power)).astype(np.float32)
+    out, lse, _ = run_gpu(dict(case, q=_bf16(q)), SCALE, num_sms=num_sms)
+    g, qd = _f32(out), _f32(_bf16(q)).astype(np.float64)
+    assert np.isfinite(g).all() and np.isfinite(lse).all()
+    from opfoundry_b200.synth import bf16_bits_to_f32
+    import torch
+    for b, rows in enumerate(_in_list_order(case)):
+        kv = torch.from_numpy(case["kv"][rows])
+        v = (kv[:, :512].view(torch.float8_e4m3fn).double() * kv[:, 512:528].contiguous().view(torch.float32).double().repeat_interleave(128, 1)).numpy()
+        rope = bf16_bits_to_f32(np.ascontiguousarray(case["kv"][rows][:, 528:]).view(np.uint16))
+        s = qd[b] @ np.concatenate([v, rope], axis=1).T * SCALE
+        order = np.sort(s, axis=1)
+        clear = order[:, -1] - order[:, -2] > 1e-6 * np.abs(qd[b]).max() * 576      # to the rounding of the sums
+        assert clear.sum() > H // 2
+        want = v[s.argmax(axis=1)]
+        assert (np.abs(g[b] - want) <= 1e-2 * np.abs(want) + 1e-3)[clear].all()
+        assert (np.abs(lse[b] - s.max(axis=1)) <= 1e-6 * np.abs(qd[b]).max() * 576)[clear].all()
