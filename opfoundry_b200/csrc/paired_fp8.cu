@@ -19,13 +19,14 @@
 // zeros: there the softmax warps add what hi + lo leave out (residual_group), so the row is as exact as with bf16 operands.  (With an element X times the rest in a
 // column where the cache holds zeros, the error of lse is 2e-6 to 1.4e-5, the most at X = 2^8; the kernel before this one had 2.5e-5 to 6e-5 for any X.  A row of
 // normal numbers needs one of 2^9 for that; if all rows have one, 64 sequences of 128 heads take 392 us instead of 57, one 40 instead of 17.)
-// P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15; V = byte x scale 2^-e, rounded once,
+// P and V in f16 (11 significant bits, where P in bf16 has 8): P = 2^(s - reference + 7), at most 2^15 (a weight of less than 2^-32 of the reference's is
+// lost, which shows only where all larger weights meet zeros); V = byte x scale 2^-e, rounded once,
 // with one e per scale group for the tile's 64 rows, so that the largest |V| stays below 2^16.  e starts at the exponent of the group's largest
-// scale in an item's first tile and moves up when a scale exceeds it by 2^7; the group's columns of O are then brought to the new e like they are to a
-// new reference maximum.  A row whose scales all lie more than 2^8 below their e lends V the difference, x = 20 octaves at most, and P takes it
-// back (V 2^x, P 2^-x): f16 alone would lose bits of a row at 2^-21 of a large row's scale and less.  What is lost then lies at
-// 2^-41 of the largest V at full weight (a group of a row that is small only beside another group of the same row: 2^-21).  The scale of a group of zeros
-// does not count where it would make its row lose bits (the cache writer gives such a group 1).
+// scale in an item's first tile and moves up when a scale exceeds it by 2^7, down when a tile's scales all lie 2^24 below; the group's columns of O are then
+// brought to the new e like they are to a new reference maximum.  A row whose scales all lie more than 2^16 below their e lends V the difference, x = 20
+// octaves at most, and P takes it back (V 2^x, P 2^-x): f16 alone would lose bits of a row at 2^-21 of a large row's scale and less.  What is lost then lies at
+// 2^-41 of the tile's largest V at full weight (a group of a row that is small only beside another group of the same row: 2^-21).  The scale of a group of zeros
+// does not count where a row would lose bits by it (the cache writer gives such a group 1).
 //
 // S in TMEM: lanes 0-63 = the CTA's 64 rows x slots of CTA 0, lanes 64-127 = the same rows x slots of CTA 1.
 // O in TMEM: lanes 0-63 = the rows x columns of CTA 0, lanes 64-127 = the rows x columns of CTA 1.
@@ -849,7 +850,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             // ======================================================== this CTA's rows' arrival, passed on to the issuers; e
             uint32_t it = 0;
             Ring<kStages> ring;
-            int e = 0;   // lane: that of group lane % 4
+            int e = 0, e_most = 0;   // lane: those of group lane % 4; the largest of the item
             for (int w = w_begin; w < w_end; ++w) {
                 const int n_tiles = tiles_of(p.works[w]);
                 for (int t = 0; t < n_tiles; ++t, ++it, ring.next()) {
@@ -877,7 +878,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             if ((lane & 3) == g) top = m;
                         }
                         const int em = max(static_cast<int>(top) - 127, -120);
-                        e = t == 0 || em >= e_old + 7 ? min(em, 126) : e_old;
+                        // (down only from far, and not so far that O, brought to the new e, could overflow)
+                        e = t == 0 || em >= e_old + 7 ? min(em, 126) : top != 0u && em + 24 <= e_old ? min(max(em, e_most - 60), e_old) : e_old;
                         // how far a row's groups lie below their e, 512 added: the least and the most of them
                         uint32_t low = 0xFFFFFFFFu, deep = 0u;
 #pragma unroll
@@ -887,18 +889,16 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                             low = min_u16x2(low, d | ~counts);
                             deep = max_u16x2(deep, d & counts);
                         }
-                        x0 = (low & 0xFFFFu) == 0xFFFFu ? 0 : min(max(static_cast<int>(low & 0xFFFFu) - 520, 0), 20);
-                        x1 = (low >> 16) == 0xFFFFu ? 0 : min(max(static_cast<int>(low >> 16) - 520, 0), 20);
+                        x0 = (low & 0xFFFFu) == 0xFFFFu ? 0 : min(max(static_cast<int>(low & 0xFFFFu) - (512 + 16), 0), 20);
+                        x1 = (low >> 16) == 0xFFFFu ? 0 : min(max(static_cast<int>(low >> 16) - (512 + 16), 0), 20);
                         lent = __any_sync(0xffffffffu, max(deep & 0xFFFFu, deep >> 16) > 520u);
                         if (!lent || looked) break;
                         const int y0 = static_cast<int>(deep & 0xFFFFu) - x0, y1 = static_cast<int>(deep >> 16) - x1;
-                        uint32_t rows0 = __ballot_sync(0xffffffffu, y0 > 512 + 18), rows1 = __ballot_sync(0xffffffffu, y1 > 512 + 18);
-                        if ((rows0 | rows1) == 0u) break;
-                        // A group of some row would lose bits.  The reason may be another group of that row, of zeros under any scale (the cache
+                        if (!__any_sync(0xffffffffu, max(y0, y1) > 512 + 18)) break;
+                        // A group of some row would lose bits.  The reason may be a group of zeros under any scale, in that row or in another (the cache
                         // writer gives it 1): its scale does not count and becomes 0 (f16 may not hold what is left of it).
-#pragma unroll 4
+#pragma unroll 1   // (four at a time: 128 sequences of 2 x 16 heads 142.3 -> 151.3 us, by their code alone)
                         for (int slot = 0; slot < kSlots; ++slot) {
-                            if (!(((slot & 1 ? rows1 : rows0) >> (slot >> 1)) & 1u)) continue;
                             // sixteen bytes a lane, eight lanes a group
                             uint4 v = make_uint4(0u, 0u, 0u, 0u);
                             const int late = ctl->late_row[ring.s][slot % kOwn];
@@ -913,6 +913,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                                 }
                         }
                     }
+                    e_most = t == 0 ? e : max(e_most, e);
                     if (lent) {
                         *reinterpret_cast<float2*>(&ctl->v_lent[ring.s][2 * lane]) = make_float2(__uint_as_float((127 + x0) << 23), __uint_as_float((127 + x1) << 23));
                         reinterpret_cast<uint32_t*>(ctl->p_back[ring.s])[lane] = pow2_f16(-x0) | pow2_f16(-x1) << 16;

@@ -149,6 +149,23 @@ def test_rows_of_zeros_from_the_cache_writer_beside_small_ones(built_lib, oracle
     _check_groups(oracle, dict(case, kv=kv))
 
 
+@pytest.mark.parametrize("power", [-30, -60])
+@pytest.mark.parametrize("where", ["first tile", "here and there", "with other groups of scale 0"])
+def test_rows_of_zeros_whose_scale_is_far_above_all_others(built_lib, oracle, power, where):
+    """Scales of 2^power, and rows of zeros of scale 1, which set no exponent that the others could not leave."""
+    case = _case(19, topk=500, B=2)
+    kv = case["kv"].copy()
+    scales, q = kv[:, 512:528].copy().view(np.float32) * np.float32(2.0 ** power), _f32(case["q"]).copy()
+    q[..., :512] *= np.float32(2.0 ** -power)
+    for rows in _in_list_order(case):
+        zeros = rows[:64] if where == "first tile" else rows[::9]
+        kv[zeros, :512], scales[zeros] = 0, 1.0
+        if where == "with other groups of scale 0":
+            scales[zeros, 1:] = 0.0
+    kv[:, 512:528] = scales.view(np.uint8).reshape(-1, 16)
+    _check_groups(oracle, dict(case, kv=kv, q=_bf16(q)))
+
+
 @pytest.mark.parametrize("power", [-12, -24, -36])
 def test_one_group_far_smaller_than_the_others(built_lib, oracle, power):
     case = _case(11)
