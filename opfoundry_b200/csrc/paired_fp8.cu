@@ -45,7 +45,7 @@
 // What bounds it (cycle stamps of an instrumented copy, 64 sequences x 128 heads x 2048 slots): a tile of 64 slots every 2 300 cycles.  Its MMAs
 // take 1 430 (measured alone; the scores' 25 an instruction are the rate of shared memory, 3 KB of operands each), all its traffic in shared
 // memory 2 000; what is in flight - four raw tiles, one and a half converted ones - over the 10 000 cycles from a load to the end of P V gives the rest:
-// landing 1 900, scores 1 500, softmax 3 100, a converter's turn 2 200.  Every role pays for the number of its instructions, about 6 900 a tile and SM:
+// landing 1 900, scores 1 500, softmax 3 100, a converter's turn 2 200.  Every role pays for the number of its instructions, 6 700 a tile and SM (before V had an exponent per group):
 // eight warps of a scheduler on five loops miss the instruction cache (4.7 of 19.6 cycles an instruction in a form of 85 KB; a warp number known
 // to be uniform, short waits and rolled loops brought 81 us to 61).  Tried: four teams of four warps with 32 slots a thread (fewer instructions, but
 // a tile takes 5 000 cycles from scores to P: 2 880 a tile where two teams of eight took 2 780), two teams of four (2 750, and 1.5 us more for one

@@ -356,3 +356,43 @@ def test_scores_beyond_the_resolution_of_their_reference(built_lib, H, num_sms, 
         want = v[s.argmax(axis=1)]
         assert (np.abs(g[b] - want) <= 1e-2 * np.abs(want) + 1e-3)[clear].all()
         assert (np.abs(lse[b] - s.max(axis=1)) <= 1e-6 * np.abs(qd[b]).max() * 576)[clear].all()
+
+
+@pytest.mark.parametrize("B,H,s_q", [(3, 24, 1), (80, 40, 1), (3, 72, 1), (74, 128, 1), (40, 32, 2)])
+def test_residuals_with_peers_and_a_sink(built_lib, B, H, s_q):
+    """Rows of Q with residuals, which wait in this GPU's rows of the gathered buffer: both peers' buffers hold the bits of the call without peers, nothing else is
+    written; and the sink's weight is that of the call without one."""
+    import ctypes as C
+    import torch
+    from gpu_util import to_dev
+    topk, T = 700, B * s_q
+    case = synth.make_decode_case(B, H, 1024, topk, s_q=s_q, fp8=True, paged=True, share_mtp="coin" if s_q > 1 else None, seed=B)
+    q = _f32(case["q"]).copy()
+    q[:, ::3, 9] *= np.float32(2.0 ** 16)
+    kv = case["kv"].copy()
+    kv[:, 9] = 0
+    plan = api.mla_decode_plan_create(T, H, topk, s_q, mtp_shared=case["mtp_shared"] if s_q > 1 else None)
+    d = to_dev(dict(case, q=_bf16(q), kv=kv))
+    kw = dict(block_table=d["block_table"], page_block_size=64)
+    want_out, want_lse = api.mla_decode_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, **kw)
+    outs = [torch.full((T, 3 * H, 512), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    lses = [torch.full((T, 3 * H), 7.0, device="cuda") for _ in range(2)]
+    flags = torch.zeros(2, api.MAX_PEERS, dtype=torch.int32, device="cuda")
+    flags[0, 1] = 1
+    a = api.make_args(d["q"], d["kv"], d["indices"], plan, SCALE, out=outs[0][:, H:2 * H], lse=None, **kw)
+    po = api.PeerOutputs()
+    po.num_peers, po.my_rank, po.lse_stride_row, po.step = 2, 0, 3 * H, 1
+    for r in range(2):
+        po.out[r], po.lse[r], po.flags[r] = outs[r].data_ptr() + H * 1024, lses[r].data_ptr() + H * 4, flags[r].data_ptr()
+    torch.cuda.synchronize()
+    api._check(api.lib().dsa_v32_decode_pipeline_allgather(C.byref(a), C.byref(po), api._stream()), "dsa_v32_decode_pipeline_allgather")
+    api._check(api.lib().dsa_v32_device_status(C.byref(a), api._stream()), "dsa_v32_device_status")
+    for o, l in zip(outs, lses):
+        assert torch.equal(o[:, H:2 * H].view(torch.int16), want_out.view(torch.int16)) and torch.equal(l[:, H:2 * H], want_lse)
+        assert torch.all(o[:, :H] == 7) and torch.all(o[:, 2 * H:] == 7) and torch.all(l[:, :H] == 7) and torch.all(l[:, 2 * H:] == 7)
+    sink = want_lse.mean(dim=0).contiguous()
+    out, lse = api.mla_v4_launch_pipeline(d["q"], d["kv"], d["indices"], plan, SCALE, attn_sink=sink, **kw)
+    torch.testing.assert_close(lse, torch.logaddexp(want_lse, sink[None]), rtol=1e-5, atol=1e-4)
+    weight = torch.sigmoid(want_lse - sink[None])[..., None]
+    ref = want_out.float() * weight
+    assert ((out.float() - ref).abs() <= 2.0 ** -7 * ref.abs() + 1e-3 * ref.abs().amax(dim=-1, keepdim=True)).all()
