@@ -338,7 +338,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 if (live) xr = __ldg(reinterpret_cast<const uint4*>(src));
             }
             float rope_mul = 1.0f;
-            uint32_t row_e[4];
+            uint2 hi[4][2];
+            int maybe = 0;   // rows that may have elements below what hi and lo hold: those that are not all zeros, nor have an infinity or a NaN
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int row = row0 + i;
@@ -352,13 +353,14 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
                 const uint32_t e = max(m >> 7, 64u);
                 const float mul = __uint_as_float((265u - min(e, 254u)) << 23);
                 if ((lane >> 3) == i) rope_mul = mul;
-                row_e[i] = e;
+                if (m != 0u && e < 255u) maybe |= 1 << i;
+                if (lane == 0) ctl->q_exp[row] = static_cast<uint16_t>(e == 255u ? 255u : e - 11u);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    uint2 hi, lo;
-                    split_q8(x[i][k], mul, hi, lo);
+                    uint2 lo;
+                    split_q8(x[i][k], mul, hi[i][k], lo);
                     uint8_t* dst = sQ + (2 * k + (lane >> 4)) * kQBlock + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + 8 * (lane & 1);
-                    *reinterpret_cast<uint2*>(dst) = hi;
+                    *reinterpret_cast<uint2*>(dst) = hi[i][k];
                     *reinterpret_cast<uint2*>(dst + kGroups * kQBlock) = lo;
                 }
             }
@@ -369,23 +371,37 @@ __global__ void __launch_bounds__(32 * kWarps, 1) paired_fp8_kernel(const AttnPa
             }
             fence_proxy_async_smem();
             warp_arrive_lead(&ctl->q_full, lane);
-            // The scores may start; meanwhile, elements that are not 0 and lie below 2^-2 with the row's factor: their magnitudes' bits less 1 (a 0 becomes
-            // the largest), cut off to line - 2 or line - 1, two halves in 32-bit sums, from which line - 2 is taken at the end (a 0 in the lower half lends
-            // its neighbour's last bit, which an element on the line may cost its place)
+            // The scores may start; meanwhile, rows with more than kWideElements below 2^-2 (with the row's factor): two lanes hold such an element, or a 0, by their
+            // bytes of hi ...
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const uint32_t line = ((row_e[i] - 13u) << 7) * 0x10001u;
+                uint32_t large = 0xFFFFFFFFu;   // bit 7 of a byte: magnitudes of 2^-2 and more only
+#pragma unroll
+                for (int k = 0; k < 2; ++k) large &= ((hi[i][k].x & 0x7F7F7F7Fu) + 0x4C4C4C4Cu) & ((hi[i][k].y & 0x7F7F7F7Fu) + 0x4C4C4C4Cu);
+                const uint32_t lanes = __ballot_sync(0xffffffffu, (large & 0x80808080u) != 0x80808080u);
+                if ((lanes & (lanes - 1u)) == 0u) maybe &= ~(1 << i);
+            }
+            // ... and then they are counted: their magnitudes' bits less 1 (a 0 becomes the largest), cut off to line - 2 or line - 1, two halves in 32-bit sums,
+            // from which line - 2 is taken at the end (a 0 in the lower half lends its neighbour's last bit, which may cost an element its place on the line)
+            __syncwarp();
+#pragma unroll 1
+            for (; maybe != 0; maybe &= maybe - 1) {
+                const int row = row0 + __ffs(maybe) - 1;
+                bool live;
+                const uint4* src = reinterpret_cast<const uint4*>(row_ptr(row, live)) + lane;
+                const uint4 y[2] = {__ldg(src), __ldg(src + 32)};
+                const uint32_t e = ctl->q_exp[row], line = ((e - 2u) << 7) * 0x10001u;
                 uint32_t n = 0u;
 #pragma unroll
                 for (int k = 0; k < 2; ++k)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const uint32_t w = (j == 0 ? x[i][k].x : j == 1 ? x[i][k].y : j == 2 ? x[i][k].z : x[i][k].w) & 0x7FFF7FFFu;
+                        const uint32_t w = (j == 0 ? y[k].x : j == 1 ? y[k].y : j == 2 ? y[k].z : y[k].w) & 0x7FFF7FFFu;
                         n += max_u16x2(min_u16x2(w - 0x10001u, line - 0x10001u), line - 0x20002u);
                     }
                 n -= 8u * (line - 0x20002u);
                 const uint32_t below = 512u - __reduce_add_sync(0xffffffffu, (n & 0xFFFFu) + (n >> 16));
-                if (lane == 0) ctl->q_exp[row0 + i] = static_cast<uint16_t>(row_e[i] == 255u ? 255u : row_e[i] - 11u + (below > kWideElements ? 256u : 0u));
+                if (lane == 0 && below > kWideElements) ctl->q_exp[row] = static_cast<uint16_t>(e + 256u);
             }
             warp_arrive(&ctl->q_here, lane);
         };
