@@ -52,8 +52,9 @@
 // sequence), a converter on both units of a tile (3 240).  The other CTA's rows in the raw tiles, three of 28 KB: 60.6 us instead of 56.5.
 // Against the kernel before it (the 576 columns split over the pair, partial scores summed through distributed shared memory in 16 bits, four tile
 // stages of 32 slots, rows converted to bf16), 128 heads x 2048 slots, 32768 positions each, other inputs every pass: one sequence 19.4 -> 16.7 us with its merge,
-// 16 35.6 -> 31.2, 64 84.0 -> 63.9.  (Of these 0.5, 1.0 and 1.7 us are what keeps Q and V exact beside elements, rows and groups that are far larger: the count of
-// Q's small elements at the start of an item takes 0.3 of the first two, the rest lies in instructions here and there.)
+// 16 35.6 -> 31.2, 64 84.0 -> 63.9.  (Of these 0.5, 1.0 and 1.7 us are what keeps Q and V exact beside elements, rows and groups that are far larger, in
+// instructions here and there: an exponent per group looked at only where a tile asks for it, and one register more a group, gave nothing back.)  Items of
+// one tile are slower than they were: 1184 rows of 64 heads x 32 slots 104 -> 130.
 // Against 64 bits, nine shapes of 24 to 128 heads: out 1.67e-3 to 1.69e-3 (2-norm, of which the output's own rounding 1.66e-3; the kernel before 2.11e-3 to
 // 2.30e-3), lse at most 1.7e-6 (7e-5; the few-heads kernel that took 17 to 32 rows before 1.4e-6).
 //
